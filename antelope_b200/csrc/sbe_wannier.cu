@@ -32,150 +32,12 @@
 #include <type_traits>
 
 #include "sbe_problem.h"
+#include "sbe_wandev.cuh"
 #include "sbe_wannier.h"
 
 namespace sbe {
 
 namespace {
-
-template <class Real> struct Cx;
-template <> struct Cx<double> { using T = double2; };
-template <> struct Cx<float> { using T = float2; };
-
-template <class T> __device__ __forceinline__ T cx(double re, double im)
-{
-    T r;
-    r.x = (decltype(r.x))re;
-    r.y = (decltype(r.y))im;
-    return r;
-}
-template <class T> __device__ __forceinline__ T cmul(T a, T b)
-{
-    T r;
-    r.x = fma(a.x, b.x, -(a.y * b.y));
-    r.y = fma(a.x, b.y, a.y * b.x);
-    return r;
-}
-template <class T> __device__ __forceinline__ T cmulc(T a, T b)  // conj(a) * b
-{
-    T r;
-    r.x = fma(a.x, b.x, a.y * b.y);
-    r.y = fma(a.x, b.y, -(a.y * b.x));
-    return r;
-}
-template <class T> __device__ __forceinline__ void cfma(T &acc, T a, T b)  // acc += a b
-{
-    acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
-    acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
-}
-template <class T> __device__ __forceinline__ void cfmac(T &acc, T a, T b)  // acc += conj(a) b
-{
-    acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
-    acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-}
-template <class T> __device__ __forceinline__ T cconj(T a)
-{
-    a.y = -a.y;
-    return a;
-}
-
-// ---- laser on the device (laser.h:150-322), FP64
-__device__ double envelope(const PulseDev &q, double t, bool d)
-{
-    const double ef = q.envfactor;
-    double to;
-    switch (q.env) {
-        case 2:  // cos4
-            if (fabs(t) > q.twidth) return 0;
-            if (d) return -4. * ef * sin(t * ef) * pow(cos(t * ef), 3.);
-            return pow(cos(t * ef), 4.);
-        case 4:  // sin2 (extension)
-            if (fabs(t) > q.twidth) return 0;
-            if (d) return -2. * ef * sin(t * ef) * cos(t * ef);
-            return cos(t * ef) * cos(t * ef);
-        case 3:  // cos4_clipped
-            if (fabs(t) > q.twidth) return 0;
-            if (t > q.twidth_clipped) to = t - q.twidth_clipped;
-            else if (t > -q.twidth_clipped) return d ? 0. : 1.;
-            else to = t + q.twidth_clipped;
-            if (d) return -4. * ef * sin(to * ef) * pow(cos(to * ef), 3.);
-            return pow(cos(to * ef), 4.);
-        case 0:  // gauss
-            if (d) return 2 * t * ef * exp(ef * t * t);
-            return exp(ef * t * t);
-        default:  // gauss_clipped
-            if (t > q.twidth_clipped) to = t - q.twidth_clipped;
-            else if (t > -q.twidth_clipped) return d ? 0. : 1.;
-            else to = t + q.twidth_clipped;
-            if (d) return 2 * to * ef * exp(ef * to * to);
-            return exp(ef * to * to);
-    }
-}
-
-__device__ void laser_eval(const LaserDev &L, double t, double *A, double *E)
-{
-    double a[3] = {0, 0, 0}, e[3] = {0, 0, 0};
-    for (int i = 0; i < L.npulses; ++i) {
-        const PulseDev &q = L.p[i];
-        const double kt = t - q.t0;
-        double s, c;
-        sincos(kt * q.w0 - q.cep, &s, &c);
-        const double f = envelope(q, kt, false), fp = envelope(q, kt, true);
-        const double ax = -q.A0x * s * f, ay = q.A0y * c * f;
-        const double ex = q.E0x * c * f - q.A0x * s * fp;
-        const double ey = q.E0y * s * f + q.A0y * c * fp;
-        for (int dd = 0; dd < 3; ++dd) {
-            a[dd] += ax * q.xdir[dd] + ay * q.ydir[dd];
-            e[dd] += ex * q.xdir[dd] + ey * q.ydir[dd];
-        }
-    }
-    for (int dd = 0; dd < 3; ++dd) {
-        A[dd] = a[dd] - L.init_A[dd];
-        E[dd] = e[dd] - L.init_E[dd];
-    }
-}
-
-// ---- tableaux (SBEs.h:395-416; Cash-Karp 4(5) for the adaptive steps)
-struct WTab {
-    int S;
-    double c[6], a[6][6], b[6], e[6];  // e = b - b* (error weights)
-};
-__device__ void tableau(int rk, WTab &T)
-{
-    for (int i = 0; i < 6; ++i) {
-        T.c[i] = T.b[i] = T.e[i] = 0;
-        for (int j = 0; j < 6; ++j) T.a[i][j] = 0;
-    }
-    if (rk == 4) {
-        T.S = 4;
-        T.c[1] = 0.5; T.c[2] = 0.5; T.c[3] = 1.0;
-        T.a[1][0] = 0.5; T.a[2][1] = 0.5; T.a[3][2] = 1.0;
-        T.b[0] = 1.0 / 6.0; T.b[1] = 2.0 / 6.0; T.b[2] = 2.0 / 6.0; T.b[3] = 1.0 / 6.0;
-    } else if (rk == 5) {
-        T.S = 6;
-        T.c[1] = 0.25; T.c[2] = 3. / 8.; T.c[3] = 12. / 13.; T.c[4] = 1.0; T.c[5] = 0.5;
-        T.a[1][0] = 1.0 / 4.0;
-        T.a[2][0] = 3. / 32.; T.a[2][1] = 9. / 32.;
-        T.a[3][0] = 1932. / 2197.; T.a[3][1] = -7200. / 2197.; T.a[3][2] = 7296. / 2197.;
-        T.a[4][0] = 439. / 216.; T.a[4][1] = -8.; T.a[4][2] = 3680. / 513.; T.a[4][3] = -845. / 4104.;
-        T.a[5][0] = -8. / 27.; T.a[5][1] = 2.; T.a[5][2] = -3544. / 2565; T.a[5][3] = 1859. / 4104;
-        T.a[5][4] = -11. / 40.;
-        T.b[0] = 16. / 135.; T.b[2] = 6656. / 12825.; T.b[3] = 28561. / 56430.; T.b[4] = -9. / 50.;
-        T.b[5] = 2. / 55.;
-    } else {  // Cash-Karp (J. R. Cash, A. H. Karp, ACM TOMS 16 (1990) 201)
-        T.S = 6;
-        T.c[1] = 1. / 5.; T.c[2] = 3. / 10.; T.c[3] = 3. / 5.; T.c[4] = 1.; T.c[5] = 7. / 8.;
-        T.a[1][0] = 1. / 5.;
-        T.a[2][0] = 3. / 40.; T.a[2][1] = 9. / 40.;
-        T.a[3][0] = 3. / 10.; T.a[3][1] = -9. / 10.; T.a[3][2] = 6. / 5.;
-        T.a[4][0] = -11. / 54.; T.a[4][1] = 5. / 2.; T.a[4][2] = -70. / 27.; T.a[4][3] = 35. / 27.;
-        T.a[5][0] = 1631. / 55296.; T.a[5][1] = 175. / 512.; T.a[5][2] = 575. / 13824.;
-        T.a[5][3] = 44275. / 110592.; T.a[5][4] = 253. / 4096.;
-        T.b[0] = 37. / 378.; T.b[2] = 250. / 621.; T.b[3] = 125. / 594.; T.b[5] = 512. / 1771.;
-        const double bs[6] = {2825. / 27648., 0., 18575. / 48384., 13525. / 55296., 277. / 14336., 1. / 4.};
-        for (int i = 0; i < 6; ++i) T.e[i] = T.b[i] - bs[i];
-    }
-}
 
 // upper-triangle element u of an N x N matrix -> (m, n), m <= n
 __device__ __forceinline__ void upper_mn(int u, int N, int &m, int &n)
@@ -632,23 +494,6 @@ __device__ __forceinline__ double warp_max(double v)
 {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
-}
-
-// k-grid point (momaxis.h:147-186, 349-383) and its trapezoid weight
-__device__ void kpoint(const WanDev &P, int kl, double kv[3], double &wt)
-{
-    const int N0 = P.Ngrid[0], N1 = P.Ngrid[1], N2 = P.Ngrid[2];
-    const int k = P.k_offset + kl;  // local index -> flat grid index
-    const int ii[3] = {k / (N1 * N2), (k / N2) % N1, k % N2};
-    const int NNg[3] = {N0, N1, N2};
-    double f[3];
-    wt = 1.0;
-    for (int dd = 0; dd < 3; ++dd) {
-        f[dd] = (NNg[dd] == 1) ? 0.0 : double(ii[dd]) / (NNg[dd] - 1) - 0.5;
-        if (NNg[dd] != 1 && (ii[dd] == 0 || ii[dd] == NNg[dd] - 1)) wt /= 2;
-    }
-    for (int dd = 0; dd < 3; ++dd)
-        kv[dd] = P.origin[dd] + f[0] * P.axes[0 * 3 + dd] + f[1] * P.axes[1 * 3 + dd] + f[2] * P.axes[2 * 3 + dd];
 }
 
 template <class RF> __device__ void load_lattice(const WanDev &P, RF *Rc)

@@ -94,6 +94,13 @@ struct WanDev {
     int shot_every;
     double *snap_nc;
     double *snap_pi;
+    // many steps per launch (wan_steps): A at the distinct stage times of
+    // every step [Nt][wan_steps_fields][3], the output partials of a launch
+    // [WAN_STEPS][step_rows][WAN_NSLOT] and the finishing blocks' counter
+    double *step_fld;
+    double *step_part;
+    unsigned *step_ticket;
+    int step_rows;
 };
 
 // A tile of a batched launch: tile `tile` (WAN_WARPS k-points) of solve
@@ -147,6 +154,21 @@ cudaError_t launch_wan_snapshot(const WanDev &w, const WanDev *dw, int precision
 cudaError_t launch_wan_attempt_batch(int N, int nR_max, bool vg, const WanDev *const *descs, const WanTileRef *tiles,
                                      int ntiles, int precision, cudaStream_t st, int grouped_rk = 0);
 cudaError_t launch_wan_control_batch(const WanDev *const *descs, int nsolves, int precision, cudaStream_t st);
+// Fixed-step solves that advance many steps per launch (sbe_wanstep.cu):
+// wan_steps says which; a launch takes at most WAN_STEPS steps of each solve
+// and launch_wan_finish then sums the steps' outputs and moves the
+// controllers on.  A block covers wan_steps_unit() tiles (tile = the first
+// one); N, na (components of A.P: 3 for the continuum model) and rk pick the
+// instance, `descs` / `tiles` null for a single solve (`dw`).
+constexpr int WAN_STEPS = 64;
+int wan_steps(const WanDev &w);   // 0: no; otherwise the kernel form (mode)
+int wan_steps_rows(const WanDev &w);
+int wan_steps_fields(int rk);
+int wan_steps_unit(int mode, int N);
+cudaError_t launch_wan_steps(int mode, int N, int na, int rk, const WanDev *dw, const WanDev *const *descs,
+                             const WanTileRef *tiles, int nblocks, int S, cudaStream_t st);
+cudaError_t launch_wan_finish(const WanDev *dw, const WanDev *const *descs, int nsolves, int S, cudaStream_t st);
+cudaError_t launch_wan_step_fields(const WanDev &w, const WanDev *dw, cudaStream_t st);
 cudaError_t launch_wan_snapshot_batch(int N, int nR_max, const WanDev *const *descs, const WanTileRef *tiles,
                                       int ntiles, int precision, cudaStream_t st);
 

@@ -95,6 +95,18 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
         dalloc(&w_.snap_nc, sizeof(double) * nshots_ * nk, st, "alloc snapshots");
         dalloc(&w_.snap_pi, sizeof(double) * 2 * nshots_ * nk, st, "alloc snapshots");
     }
+    if (wan_steps(w_)) {
+        w_.step_rows = wan_steps_rows(w_);
+        dalloc(&w_.step_fld, sizeof(double) * (size_t)w_.Nt * wan_steps_fields(w_.rk) * 3, st, "alloc step fields");
+        dalloc(&w_.step_part, sizeof(double) * (size_t)std::min(WAN_STEPS, w_.Nt) * w_.step_rows * WAN_NSLOT, st,
+               "alloc step partials");
+        // slots that a model has no values for stay zero
+        cuda_check(cudaMemsetAsync(w_.step_part, 0,
+                                   sizeof(double) * (size_t)std::min(WAN_STEPS, w_.Nt) * w_.step_rows * WAN_NSLOT, st),
+                   "clear step partials");
+        dalloc(&w_.step_ticket, sizeof(unsigned), st, "alloc step counter");
+        cuda_check(cudaMemsetAsync(w_.step_ticket, 0, sizeof(unsigned), st), "clear step counter");
+    }
     dalloc(&d_w_, sizeof(WanDev), st, "alloc descriptor");
     w_.V = V;
     w_.h = h;
@@ -204,7 +216,8 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     ring.upload(w_.ctl, &c, sizeof(c), st);
     ring.upload(d_w_, &w_, sizeof(w_), st);
     cuda_check(launch_wan_init(w_, precision_, st), "Wannier init kernel");
-    cuda_check(launch_wan_prepare(d_w_, precision_, st), "Wannier stage preparation");
+    if (wan_steps(w_)) cuda_check(launch_wan_step_fields(w_, d_w_, st), "Wannier step fields");
+    else cuda_check(launch_wan_prepare(d_w_, precision_, st), "Wannier stage preparation");
     cuda_check(cudaMallocHost(&h_ctl_, sizeof(WanCtl)), "cudaMallocHost(control)");
 }
 
@@ -232,6 +245,9 @@ WannierSolve::~WannierSolve()
     cudaFreeAsync(w_.ctl, stream_);
     cudaFreeAsync(w_.stage_AE, stream_);
     cudaFreeAsync(w_.stage_cA, stream_);
+    if (w_.step_fld) cudaFreeAsync(w_.step_fld, stream_);
+    if (w_.step_part) cudaFreeAsync(w_.step_part, stream_);
+    if (w_.step_ticket) cudaFreeAsync(w_.step_ticket, stream_);
     cudaFreeAsync(d_w_, stream_);
     if (w_.snap_nc) cudaFreeAsync(w_.snap_nc, stream_);
     if (w_.snap_pi) cudaFreeAsync(w_.snap_pi, stream_);
@@ -242,6 +258,25 @@ WannierSolve::~WannierSolve()
 void WannierSolve::run(cudaStream_t st)
 {
     stream_ = st;
+    if (wan_steps(w_)) {   // a fixed number of launches, each of many steps
+        const int mode = wan_steps(w_), na = w_.cont ? 3 : 2, unit = wan_steps_unit(mode, w_.N), F = w_.shot_every;
+        launches_ = 0;
+        for (int n = 0; n < w_.Nt;) {
+            // the steps the kernels take from n (a launch ends at a snapshot)
+            int m = std::min(WAN_STEPS, w_.Nt - n);
+            if (F > 0) m = std::min(m, (n + F - 1) / F * F + 1 - n);
+            cuda_check(launch_wan_steps(mode, w_.N, na, w_.rk, d_w_, nullptr, nullptr, (w_.ntiles + unit - 1) / unit,
+                                        WAN_STEPS, st),
+                       "Wannier step kernel");
+            cuda_check(launch_wan_finish(d_w_, nullptr, 1, WAN_STEPS, st), "Wannier finish kernel");
+            cuda_check(launch_wan_snapshot(w_, d_w_, precision_, st), "Wannier snapshot kernel");
+            launches_ += F > 0 ? 3 : 2;
+            n += m;
+        }
+        cuda_check(cudaMemcpyAsync(h_ctl_, w_.ctl, sizeof(WanCtl), cudaMemcpyDeviceToHost, st), "copy control");
+        cuda_check(cudaStreamSynchronize(st), "sync");
+        return;
+    }
     // attempts are launched in chunks; the controller makes surplus launches
     // after the last step no-ops, and the host checks progress per chunk
     const int chunk = 64;
@@ -283,10 +318,11 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
     // lead the tile list, so their blocks are scheduled first
     for (int i = 0; i < (int)solves_.size(); ++i) {
         const WanDev &w = solves_[i]->dev();
-        const int grk = wan_grouped(w) ? w.rk : 0;
+        const int grk = wan_grouped(w) ? w.rk : 0, smode = wan_steps(w), srk = smode ? w.rk : 0, na = w.cont ? 3 : 2;
         Class *c = nullptr;
         for (Class &x : classes_)
-            if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == solves_[i]->precision() && x.grouped_rk == grk)
+            if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == solves_[i]->precision() && x.grouped_rk == grk &&
+                x.steps_rk == srk && x.steps_mode == smode && (!srk || x.na == na))
                 c = &x;
         if (!c) {
             classes_.emplace_back();
@@ -295,6 +331,9 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
             c->vg = w.vg != 0;
             c->precision = solves_[i]->precision();
             c->grouped_rk = grk;
+            c->steps_rk = srk;
+            c->steps_mode = smode;
+            c->na = na;
         }
         c->members.push_back(i);
         c->nR = std::max(c->nR, w.nR);
@@ -315,7 +354,7 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         // interleave the solves' tiles round-robin (longest first), so that
         // the blocks of one launch spread every solve over the whole GPU
         // (grouped classes: one entry per block of WAN_GROUP_TILES tiles)
-        const int unit = c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps_rk ? wan_steps_unit(c.steps_mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
         int maxt = 0;
         for (int m : c.members) maxt = std::max(maxt, solves_[m]->dev().ntiles);
         for (int t = 0; t < maxt; t += unit)
@@ -326,7 +365,14 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         dalloc(&c.d_tiles, sizeof(WanTileRef) * tiles.size(), st, "alloc batch tiles");
         ring.upload(c.d_descs, descs.data(), sizeof(WanDev *) * descs.size(), st);
         ring.upload(c.d_tiles, tiles.data(), sizeof(WanTileRef) * tiles.size(), st);
-        per_iter_ += c.shots ? 3 : 2;
+        if (c.shots) {   // the snapshot kernel's blocks cover one tile each
+            tiles.clear();
+            for (int j = 0; j < (int)c.members.size(); ++j)
+                for (int t = 0; t < solves_[c.members[j]]->dev().ntiles; ++t) tiles.push_back(WanTileRef{j, t});
+            c.nsnap_tiles = (int)tiles.size();
+            dalloc(&c.d_snap_tiles, sizeof(WanTileRef) * tiles.size(), st, "alloc snapshot tiles");
+            ring.upload(c.d_snap_tiles, tiles.data(), sizeof(WanTileRef) * tiles.size(), st);
+        }
     }
     cuda_check(cudaMallocHost(&h_ctls_, sizeof(WanCtl) * std::max<size_t>(1, solves_.size())),
                "cudaMallocHost(batch control)");
@@ -338,25 +384,44 @@ WannierBatch::~WannierBatch()
     for (Class &c : classes_) {
         if (c.d_descs) cudaFreeAsync(c.d_descs, stream_);
         if (c.d_tiles) cudaFreeAsync(c.d_tiles, stream_);
+        if (c.d_snap_tiles) cudaFreeAsync(c.d_snap_tiles, stream_);
     }
     cudaStreamSynchronize(stream_);
     solves_.clear();
     if (h_ctls_) cudaFreeHost(h_ctls_);
 }
 
-void WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
+int WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
 {
+    int launched = 0;
     for (int it = 0; it < iters; ++it)
         for (const Class &c : classes_) {
+            if (c.steps_rk) {   // WAN_STEPS iterations in one launch
+                if (it % WAN_STEPS) continue;
+                cuda_check(launch_wan_steps(c.steps_mode, c.N, c.na, c.steps_rk, nullptr, c.d_descs, c.d_tiles, c.ntiles,
+                                            std::min(WAN_STEPS, iters - it), st),
+                           "Wannier step kernel (batch)");
+                cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.members.size(), std::min(WAN_STEPS, iters - it), st),
+                           "Wannier finish kernel (batch)");
+                launched += 2;
+                if (c.shots) {
+                    cuda_check(launch_wan_snapshot_batch(c.N, c.nR, c.d_descs, c.d_snap_tiles, c.nsnap_tiles, c.precision, st),
+                               "Wannier snapshot kernel (batch)");
+                    ++launched;
+                }
+                continue;
+            }
+            launched += c.shots ? 3 : 2;
             cuda_check(launch_wan_attempt_batch(c.N, c.nR, c.vg, c.d_descs, c.d_tiles, c.ntiles, c.precision, st,
                                                 c.grouped_rk),
                        "Wannier attempt kernel (batch)");
             cuda_check(launch_wan_control_batch(c.d_descs, (int)c.members.size(), c.precision, st),
                        "Wannier control kernel (batch)");
             if (c.shots)
-                cuda_check(launch_wan_snapshot_batch(c.N, c.nR, c.d_descs, c.d_tiles, c.ntiles, c.precision, st),
+                cuda_check(launch_wan_snapshot_batch(c.N, c.nR, c.d_descs, c.d_snap_tiles, c.nsnap_tiles, c.precision, st),
                            "Wannier snapshot kernel (batch)");
         }
+    return launched;
 }
 
 void WannierBatch::run(cudaStream_t st, bool use_graph)
@@ -369,10 +434,12 @@ void WannierBatch::run(cudaStream_t st, bool use_graph)
     for (auto &s : solves_) max_nt = std::max<long long>(max_nt, s->dev().Nt);
     const long long max_iters = 64LL * max_nt + 1000;
     cudaGraphExec_t ge = nullptr;
+    int per_chunk = 0;
+    launches_ = 0;
     if (use_graph) {
         cudaGraph_t g;
         cuda_check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-        enqueue_chunk(st, chunk);
+        per_chunk = enqueue_chunk(st, chunk);
         cuda_check(cudaStreamEndCapture(st, &g), "end capture");
         cuda_check(cudaGraphInstantiate(&ge, g, 0), "graph instantiate");
         cudaGraphDestroy(g);
@@ -381,7 +448,8 @@ void WannierBatch::run(cudaStream_t st, bool use_graph)
     bool all_done = false;
     while (!all_done) {
         if (ge) cuda_check(cudaGraphLaunch(ge, st), "graph launch");
-        else enqueue_chunk(st, chunk);
+        else per_chunk = enqueue_chunk(st, chunk);
+        launches_ += per_chunk;
         iters += chunk;
         for (int i = 0; i < (int)solves_.size(); ++i)
             cuda_check(cudaMemcpyAsync(&h_ctls_[i], solves_[i]->dev().ctl, sizeof(WanCtl), cudaMemcpyDeviceToHost, st),
@@ -395,7 +463,6 @@ void WannierBatch::run(cudaStream_t st, bool use_graph)
         }
     }
     if (ge) cudaGraphExecDestroy(ge);
-    launches_ = (int)(per_iter_ * iters);
     for (int i = 0; i < (int)solves_.size(); ++i) solves_[i]->finish_batched(h_ctls_[i], launches_);
 }
 
@@ -427,6 +494,8 @@ size_t WannierPool::bytes_needed(const Problem &p, int precision)
     b += nR * NN * cplx * 5 + nR * 16 + nR * 216 * cplx;               // h, d, current, re-laid and stage tables, vectors
     b += ntiles * 8 * (1 + WAN_NSLOT) + (size_t)p.laser.Nt * WAN_NSLOT * 8;   // tile results, per-step sums
     if (p.gauge == GAUGE_VELOCITY) b += nk * N * 16 + nk * 3 * NN * 16;  // bands, momentum matrices
+    if (p.gauge == GAUGE_VELOCITY && p.rk != 45)   // step fields and partials
+        b += (size_t)p.laser.Nt * 6 * 24 + (size_t)WAN_STEPS * (nk / 4 + 1) * WAN_NSLOT * 8;
     return b + 4096;
 }
 
@@ -490,10 +559,12 @@ void WannierPool::rebuild()
         if (kv.second.done) continue;
         const WannierSolve &s = *kv.second.s;
         const WanDev &w = s.dev();
-        const int grk = wan_grouped(w) ? w.rk : 0;
+        const int grk = wan_grouped(w) ? w.rk : 0, smode = wan_steps(w), srk = smode ? w.rk : 0, na = w.cont ? 3 : 2;
         Class *c = nullptr;
         for (Class &x : classes_)
-            if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == s.precision() && x.grouped_rk == grk) c = &x;
+            if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == s.precision() && x.grouped_rk == grk &&
+                x.steps_rk == srk && x.steps_mode == smode && (!srk || x.na == na))
+                c = &x;
         if (!c) {
             classes_.emplace_back();
             c = &classes_.back();
@@ -501,6 +572,9 @@ void WannierPool::rebuild()
             c->vg = w.vg != 0;
             c->precision = s.precision();
             c->grouped_rk = grk;
+            c->steps_rk = srk;
+            c->steps_mode = smode;
+            c->na = na;
         }
         c->ids.push_back(kv.first);
         c->nR = std::max(c->nR, w.nR);
@@ -509,7 +583,7 @@ void WannierPool::rebuild()
     for (Class &c : classes_) {
         std::vector<const WanDev *> descs;
         std::vector<WanTileRef> tiles;
-        const int unit = c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps_rk ? wan_steps_unit(c.steps_mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
         int maxt = 0;
         for (int id : c.ids) {
             descs.push_back(solves_.at(id).s->dev_ptr());
@@ -535,6 +609,16 @@ void WannierPool::step(int iters)
     if (classes_.empty()) return;
     for (int it = 0; it < iters; ++it)
         for (const Class &c : classes_) {
+            if (c.steps_rk) {   // up to WAN_STEPS iterations in one launch
+                if (it % WAN_STEPS) continue;
+                const int S = std::min(WAN_STEPS, iters - it);
+                cuda_check(launch_wan_steps(c.steps_mode, c.N, c.na, c.steps_rk, nullptr, c.d_descs, c.d_tiles, c.ntiles, S, st_),
+                           "Wannier step kernel (server)");
+                cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.ids.size(), S, st_),
+                           "Wannier finish kernel (server)");
+                last_launches_ += 2;
+                continue;
+            }
             cuda_check(launch_wan_attempt_batch(c.N, c.nR, c.vg, c.d_descs, c.d_tiles, c.ntiles, c.precision, st_,
                                                 c.grouped_rk),
                        "Wannier attempt kernel (server)");

@@ -72,16 +72,17 @@ private:
     struct Class {
         int N = 0, nR = 0, precision = 0;
         int grouped_rk = 0;   // the grouped attempt kernel (and its RK order), or 0
+        int steps_rk = 0, steps_mode = 0, na = 2;   // the many-step kernels (RK order, form) or 0; components of A.P
         bool vg = false, shots = false;
         std::vector<int> members;
         const WanDev **d_descs = nullptr;
-        WanTileRef *d_tiles = nullptr;
-        int ntiles = 0;
+        WanTileRef *d_tiles = nullptr, *d_snap_tiles = nullptr;   // launch units; single tiles for snapshots
+        int ntiles = 0, nsnap_tiles = 0;
     };
-    void enqueue_chunk(cudaStream_t st, int iters);
+    int enqueue_chunk(cudaStream_t st, int iters);   // returns the launches queued
     std::vector<std::unique_ptr<WannierSolve>> solves_;
     std::vector<Class> classes_;
-    int device_ = 0, launches_ = 0, per_iter_ = 0;
+    int device_ = 0, launches_ = 0;
     cudaStream_t stream_ = nullptr;
     WanCtl *h_ctls_ = nullptr;
 };
@@ -128,7 +129,7 @@ private:
     cudaStream_t st_;
     bool dirty_ = true;
     struct Class {
-        int N = 0, nR = 0, precision = 0, grouped_rk = 0;
+        int N = 0, nR = 0, precision = 0, grouped_rk = 0, steps_rk = 0, steps_mode = 0, na = 2;
         bool vg = false;
         std::vector<int> ids;
         const WanDev **d_descs = nullptr;

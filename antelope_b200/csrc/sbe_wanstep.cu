@@ -1,0 +1,581 @@
+// Fixed-step N-band solves, many steps per launch (sm_100a).
+//
+// With a fixed step (RK4 / Fehlberg-5, SBEs.h:395-416, 596-624) the k-points
+// of a solve are independent until the k-sum of the outputs, so a launch
+// advances every k-point by up to S steps with its state on chip and writes
+// one partial row of the outputs per warp and step; `wan_finish` sums the
+// rows of each step and moves the solve's controller on.  One attempt launch
+// and one control launch per step (wan_vg_attempt / wan_control) cost 30 + 12
+// us on 14 520 k-points of the four-band KaneMele model, of which the
+// arithmetic is under 2.
+//
+// wan_vg_steps: velocity gauge (SBEs.h:284-373, 787-805, 862-871) at N <= 3,
+// one thread per k-point.  rho (the upper triangle) and H = diag(eps) + A.P
+// live in registers, P in shared memory (one column per thread, so a warp's
+// 16-byte loads are contiguous).
+// wan_vg_rows: the same at N = 4 ... 8, one row of the matrices per lane.
+// Both are FP64 in both methods, as wan_vg_attempt, which runs the adaptive
+// Cash-Karp steps.
+//
+// Measured (RK4, 367 steps, whole solve with its set-up): three bands 1.8 us a
+// step at 14 520 k-points and 5.5 at 90 300 (rows: 3.7, 14.9); four bands rows
+// 5.2 and 21 (one thread per k-point spills: 5.5, 21; with RK5 8.1 and 34
+// against 9.7 and 39).
+#include <cuda_runtime.h>
+
+#include "sbe_wandev.cuh"
+#include "sbe_wannier.h"
+
+namespace sbe {
+
+namespace {
+
+constexpr int WS_T = 64;   // threads (k-points) per block
+
+// Compile-time tableaux (SBEs.h:395-416).  ti(i): field-table column of
+// stage i (NT distinct stage times); c: the fractions of those columns.
+template <int RK> struct StepTab;
+template <> struct StepTab<4> {
+    static constexpr int S = 4, NT = 3;
+    __host__ __device__ static constexpr double c(int t) { return t == 0 ? 0.0 : t == 1 ? 0.5 : 1.0; }
+    __device__ static constexpr double a(int i, int j)
+    {
+        return (i == 1 && j == 0) ? 0.5 : (i == 2 && j == 1) ? 0.5 : (i == 3 && j == 2) ? 1.0 : 0.0;
+    }
+    __device__ static constexpr double b(int i) { return (i == 0 || i == 3) ? 1.0 / 6.0 : 2.0 / 6.0; }
+    __device__ static constexpr int ti(int i) { return i == 0 ? 0 : (i == 3 ? 2 : 1); }
+};
+template <> struct StepTab<5> {
+    static constexpr int S = 6, NT = 6;
+    __host__ __device__ static constexpr double c(int t)
+    {
+        return t == 0 ? 0.0 : t == 1 ? 0.25 : t == 2 ? 3. / 8. : t == 3 ? 12. / 13. : t == 4 ? 1.0 : 0.5;
+    }
+    __device__ static constexpr double a(int i, int j)
+    {
+        return i == 1 ? (j == 0 ? 1.0 / 4.0 : 0.0)
+             : i == 2 ? (j == 0 ? 3. / 32. : j == 1 ? 9. / 32. : 0.0)
+             : i == 3 ? (j == 0 ? 1932. / 2197. : j == 1 ? -7200. / 2197. : j == 2 ? 7296. / 2197. : 0.0)
+             : i == 4 ? (j == 0 ? 439. / 216. : j == 1 ? -8. : j == 2 ? 3680. / 513. : j == 3 ? -845. / 4104. : 0.0)
+             : i == 5 ? (j == 0 ? -8. / 27. : j == 1 ? 2. : j == 2 ? -3544. / 2565 : j == 3 ? 1859. / 4104
+                        : j == 4 ? -11. / 40. : 0.0)
+             : 0.0;
+    }
+    __device__ static constexpr double b(int i)
+    {
+        return i == 0 ? 16. / 135. : i == 1 ? 0.0 : i == 2 ? 6656. / 12825. : i == 3 ? 28561. / 56430.
+             : i == 4 ? -9. / 50. : 2. / 55.;
+    }
+    __device__ static constexpr int ti(int i) { return i; }
+};
+
+// Steps a launch of at most S takes from output step n: up to the end, and not
+// past a step whose density snapshot is due (it is taken between launches).
+__device__ __forceinline__ int launch_steps(const WanDev &P, int n, int S)
+{
+    int m = min(S, P.Nt - n);
+    if (P.shot_every > 0) m = min(m, ((n + P.shot_every - 1) / P.shot_every) * P.shot_every + 1 - n);
+    return m;
+}
+
+// Start of output step n and its length as the step controller forms them:
+// steps end exactly on t_{n+1}.
+__device__ __forceinline__ double step_start(const WanDev &P, int n)
+{
+    return n == 0 ? P.atmin : P.atmin + P.dt * n;
+}
+__device__ __forceinline__ double step_length(const WanDev &P, int n)
+{
+    return (P.atmin + P.dt * (n + 1)) - step_start(P, n);
+}
+
+// Sum of 16 values over a warp by halving exchanges: lanes 2i return value i
+// (fixed pattern; 16 shuffles instead of 80).
+__device__ __forceinline__ double warp_sum16(const double (&v)[16], int lane)
+{
+    double u[8], x[4], y[2];
+    const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4, h1 = lane & 2;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        u[i] = (h4 ? v[i + 8] : v[i]) + __shfl_xor_sync(0xffffffffu, h4 ? v[i] : v[i + 8], 16);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        x[i] = (h3 ? u[i + 4] : u[i]) + __shfl_xor_sync(0xffffffffu, h3 ? u[i] : u[i + 4], 8);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        y[i] = (h2 ? x[i + 2] : x[i]) + __shfl_xor_sync(0xffffffffu, h2 ? x[i] : x[i + 2], 4);
+    double z = (h1 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, h1 ? y[0] : y[1], 2);
+    return z + __shfl_xor_sync(0xffffffffu, z, 1);
+}
+
+// upper-triangle index of (m, n), m < n, among the off-diagonal elements
+__host__ __device__ constexpr int oidx(int m, int n, int N) { return m * N - m * (m + 1) / 2 + (n - m - 1); }
+
+}  // namespace
+
+// A at the distinct stage times of every step: step_fld[n][NT][3]
+__global__ void __launch_bounds__(128) wan_step_fields(const WanDev *__restrict__ Pp, int nt, int rk)
+{
+    const WanDev &P = *Pp;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.Nt * nt) return;
+    const int n = i / nt, j = i % nt;
+    const double tc = step_start(P, n), hs = step_length(P, n);
+    const double c = rk == 4 ? StepTab<4>::c(j) : StepTab<5>::c(j);
+    double A[3], E[3];
+    laser_eval(P.laser, j == 0 ? tc : tc + c * hs, A, E);
+    for (int d = 0; d < 3; ++d) P.step_fld[(size_t)i * 3 + d] = A[d];
+}
+
+// FP64-pipe bound where the grid fills the GPU, latency-bound (one warp per
+// scheduler) below: at N = 3 an RK4 step is ~0.7e3 FP64 instructions per
+// thread against 3 passes over P in shared memory (54 16-byte loads).
+template <int N, int RK, int NA>
+__global__ void __launch_bounds__(WS_T) wan_vg_steps(const WanDev *__restrict__ Pp,
+                                                     const WanDev *const *__restrict__ descs,
+                                                     const WanTileRef *__restrict__ tiles, int S)
+{
+    using TB = StepTab<RK>;
+    constexpr int NN = N * N, NO = N * (N - 1) / 2;
+    extern __shared__ __align__(16) double2 sP[];   // [NA][NN][WS_T] P, then [N][WS_T] (eps, f)
+    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
+    const int tile0 = tiles ? tiles[blockIdx.x].tile : (int)blockIdx.x * (WS_T / WAN_WARPS);
+    if (P.ctl->done) return;
+    const int n0 = P.ctl->n, steps = launch_steps(P, n0, S);
+    const int t = threadIdx.x, lane = t & 31;
+    const int k = tile0 * WAN_WARPS + t;
+    const bool live = k < P.nk;
+    const int kc = live ? k : P.nk - 1;   // a thread past the grid shadows the last k-point
+    double2 *const sE = sP + NA * NN * WS_T;
+    for (int e = 0; e < NA * NN; ++e) sP[e * WS_T + t] = P.vg_P[(size_t)kc * (NA * NN) + e];
+#pragma unroll
+    for (int m = 0; m < N; ++m)
+        sE[m * WS_T + t] = make_double2(P.vg_eps[(size_t)kc * N + m], P.vg_f[(size_t)kc * N + m]);
+    const double wk = live ? P.weight[kc] : 0.0;
+    const double g1 = P.g1, g2 = P.g2;
+    double2 *rho = P.rho[0] + (size_t)kc * NN;
+    double yd[N];
+    double2 yo[NO];
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+        yd[m] = rho[m * N + m].x;
+#pragma unroll
+        for (int n = m + 1; n < N; ++n) yo[oidx(m, n, N)] = rho[m * N + n];
+    }
+    const int ce = (P.nval * N + P.nval + 1) % NN;   // antelope.cpp:539-542
+    const int nw = (P.nk + 31) / 32;
+    double *part = P.step_part + (size_t)((tile0 * WAN_WARPS + t) >> 5) * WAN_NSLOT + (lane >> 1);
+    const bool put = (lane & 1) == 0 && tile0 * WAN_WARPS + (t & ~31) < P.nk;
+
+    for (int j = 0; j < steps; ++j) {
+        const double *fl = P.step_fld + (size_t)(n0 + j) * TB::NT * 3;
+        const double h = step_length(P, n0 + j);
+        double2 H[NN];
+        // one pass over P: H at the start of the step, and the currents there
+        // (SBEs.h:694-760): Re sum_ij rho_ij P_a,ji, the diagonal -> intraband
+        {
+            double A[NA], v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = 0.0;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+                A[a] = fl[a];
+                double ie = 0.0, ia = 0.0;
+#pragma unroll
+                for (int e = 0; e < NN; ++e) {
+                    const int m = e / N, n = e % N;
+                    const double2 p = sP[(a * NN + e) * WS_T + t];
+                    if (a == 0) H[e] = make_double2(m == n ? fma(A[a], p.x, sE[m * WS_T + t].x) : A[a] * p.x, A[a] * p.y);
+                    else H[e] = make_double2(fma(A[a], p.x, H[e].x), fma(A[a], p.y, H[e].y));
+                    // rho_nm P_mn
+                    if (m == n) ia = fma(yd[m], p.x, ia);
+                    else if (m < n) ie = fma(yo[oidx(m, n, N)].x, p.x, fma(yo[oidx(m, n, N)].y, p.y, ie));
+                    else ie = fma(yo[oidx(n, m, N)].x, p.x, fma(-yo[oidx(n, m, N)].y, p.y, ie));
+                }
+                v[a < 2 ? a : WAN_SLOT_INTER_Z] = wk * ie;
+                v[a < 2 ? 2 + a : WAN_SLOT_INTRA_Z] = wk * ia;
+            }
+#pragma unroll
+            for (int m = 0; m < N; ++m) v[4 + m] = wk * yd[m];
+#pragma unroll
+            for (int e = 0; e < NN; ++e)
+                if (e == ce) {
+                    const int m = e / N, n = e % N;
+                    v[4 + N] = wk * (m == n ? yd[m] : m < n ? yo[oidx(m, n, N)].x : yo[oidx(n, m, N)].x);
+                    v[5 + N] = m == n ? 0.0 : wk * (m < n ? yo[oidx(m, n, N)].y : -yo[oidx(n, m, N)].y);
+                }
+            const double s = warp_sum16(v, lane);
+            if (put) part[(size_t)j * nw * WAN_NSLOT] = s;
+        }
+        // the step
+        double kd[TB::S][N], id[N];
+        double2 ko[TB::S][NO], io[NO];
+#pragma unroll
+        for (int m = 0; m < N; ++m) id[m] = 0.0;
+#pragma unroll
+        for (int o = 0; o < NO; ++o) io[o] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int s = 0; s < TB::S; ++s) {
+            double xd[N];
+            double2 xo[NO];
+#pragma unroll
+            for (int m = 0; m < N; ++m) xd[m] = yd[m];
+#pragma unroll
+            for (int o = 0; o < NO; ++o) xo[o] = yo[o];
+#pragma unroll
+            for (int q = 0; q < s; ++q)
+                if (TB::a(s, q) != 0.0) {
+                    const double a = h * TB::a(s, q);
+#pragma unroll
+                    for (int m = 0; m < N; ++m) xd[m] = fma(a, kd[q][m], xd[m]);
+#pragma unroll
+                    for (int o = 0; o < NO; ++o)
+                        xo[o] = make_double2(fma(a, ko[q][o].x, xo[o].x), fma(a, ko[q][o].y, xo[o].y));
+                }
+            if (s > 0 && TB::ti(s) != TB::ti(s - 1)) {
+#pragma unroll
+                for (int a = 0; a < NA; ++a) {
+                    const double Aa = fl[TB::ti(s) * 3 + a];
+#pragma unroll
+                    for (int e = 0; e < NN; ++e) {
+                        const double2 p = sP[(a * NN + e) * WS_T + t];
+                        if (a == 0)
+                            H[e] = make_double2(e / N == e % N ? fma(Aa, p.x, sE[(e / N) * WS_T + t].x) : Aa * p.x, Aa * p.y);
+                        else H[e] = make_double2(fma(Aa, p.x, H[e].x), fma(Aa, p.y, H[e].y));
+                    }
+                }
+            }
+            // -i((HY) - (HY)^dag) - Gamma o (Y - rho0)   (SBEs.h:808-819, 862-871)
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                double im = H[m * N + m].y * xd[m];   // Im (HY)_mm
+#pragma unroll
+                for (int l = 0; l < N; ++l) {
+                    if (l == m) continue;
+                    const double2 y = l < m ? xo[oidx(l, m, N)] : cconj(xo[oidx(m, l, N)]);
+                    im = fma(H[m * N + l].x, y.y, fma(H[m * N + l].y, y.x, im));
+                }
+                kd[s][m] = 2.0 * im - g1 * (xd[m] - sE[m * WS_T + t].y);
+#pragma unroll
+                for (int n = m + 1; n < N; ++n) {
+                    // c = (HY)_mn - conj (HY)_nm
+                    const double2 w = xo[oidx(m, n, N)];
+                    double2 c = make_double2(H[m * N + n].x * xd[n] - H[n * N + m].x * xd[m],
+                                             H[m * N + n].y * xd[n] + H[n * N + m].y * xd[m]);
+                    cfma(c, H[m * N + m], w);
+                    // conj(H_nn conj(w)) = conj(H_nn) w
+                    cfma(c, make_double2(-H[n * N + n].x, H[n * N + n].y), w);
+#pragma unroll
+                    for (int l = 0; l < N; ++l) {
+                        if (l == m || l == n) continue;
+                        const double2 yn = l < n ? xo[oidx(l, n, N)] : cconj(xo[oidx(n, l, N)]);   // Y_ln
+                        const double2 ym = l < m ? xo[oidx(l, m, N)] : cconj(xo[oidx(m, l, N)]);   // Y_lm
+                        cfma(c, H[m * N + l], yn);
+                        // - conj(H_nl Y_lm)
+                        const double2 hn = H[n * N + l];
+                        c.x = fma(-hn.x, ym.x, fma(hn.y, ym.y, c.x));
+                        c.y = fma(hn.x, ym.y, fma(hn.y, ym.x, c.y));
+                    }
+                    ko[s][oidx(m, n, N)] = make_double2(fma(-g2, w.x, c.y), fma(-g2, w.y, -c.x));
+                }
+            }
+            if (TB::b(s) != 0.0) {
+                const double b = h * TB::b(s);
+#pragma unroll
+                for (int m = 0; m < N; ++m) id[m] = fma(b, kd[s][m], id[m]);
+#pragma unroll
+                for (int o = 0; o < NO; ++o) io[o] = make_double2(fma(b, ko[s][o].x, io[o].x), fma(b, ko[s][o].y, io[o].y));
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < N; ++m) yd[m] += id[m];
+#pragma unroll
+        for (int o = 0; o < NO; ++o) yo[o] = make_double2(yo[o].x + io[o].x, yo[o].y + io[o].y);
+    }
+    if (!live) return;
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+        rho[m * N + m] = make_double2(yd[m], 0.0);
+#pragma unroll
+        for (int n = m + 1; n < N; ++n) {
+            rho[m * N + n] = yo[oidx(m, n, N)];
+            rho[n * N + m] = cconj(yo[oidx(m, n, N)]);
+        }
+    }
+}
+
+// ---------------------------------------------------- one row per lane
+// Lanes per k-point and the shared-memory strides (in complex numbers) of a
+// k-point's regions: Y, the packed upper triangle, read element by element at
+// one address per group (odd stride: the groups of a warp hit distinct
+// banks), and T, rows of LDT for the transpose (stride GT: the 8 lanes of a
+// 16-byte phase hit distinct banks on row writes and on column reads).
+template <int N> struct RowDim {
+    static constexpr int G = N <= 4 ? 4 : 8, KW = 32 / G, NU = N * (N + 1) / 2;
+    static constexpr int GY = NU | 1, LDT = N | 1;
+    static constexpr int GT = G == 8 ? (N * LDT) | 1 : (N * LDT + 3) / 8 * 8 + 4;
+};
+constexpr int WR_T = 64;   // threads per block of the row kernel
+
+// Velocity gauge at N = 4 ... 8: lane m of a k-point's group holds row m of
+// rho, of P and of H in registers; H Y is formed one row per lane with Y read
+// by element, and its conjugate transpose read back from shared memory.  Bound
+// by shared memory (58 wavefronts per warp and stage at N = 4) and the FP64
+// pipe (112 instructions) about equally, at 12 warps per SM.
+template <int N, int RK>
+__global__ void __launch_bounds__(WR_T, N <= 4 ? 6 : 4) wan_vg_rows(const WanDev *__restrict__ Pp,
+                                                    const WanDev *const *__restrict__ descs,
+                                                    const WanTileRef *__restrict__ tiles, int S)
+{
+    using TB = StepTab<RK>;
+    using D = RowDim<N>;
+    constexpr int NN = N * N, G = D::G, KW = D::KW;
+    __shared__ double2 sY[WR_T / G * D::GY], sT[WR_T / G * D::GT];
+    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
+    const int k0 = (tiles ? tiles[blockIdx.x].tile * WAN_WARPS : (int)blockIdx.x * (WR_T / G));
+    if (P.ctl->done) return;
+    const int n0 = P.ctl->n, steps = launch_steps(P, n0, S);
+    const int lane = threadIdx.x & 31, grp = threadIdx.x / G, m = threadIdx.x % G;
+    const int warp_k = k0 + (threadIdx.x >> 5) * KW;   // the warp's first k-point
+    if (warp_k >= P.nk) return;                        // no block-wide barrier below
+    const int k = k0 + grp;
+    const bool live = k < P.nk;
+    const int kc = live ? k : P.nk - 1;   // a group past the grid shadows the last k-point
+    const int mr = m < N ? m : N - 1;     // idle lanes shadow the last row (and store nothing)
+    const bool own = m < N;
+    double2 *const Y = sY + grp * D::GY, *const T = sT + grp * D::GT;
+    double2 p[2][N], y0[N];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int n = 0; n < N; ++n) p[a][n] = P.vg_P[((size_t)kc * 2 + a) * NN + mr * N + n];
+    double2 *rho = P.rho[0] + (size_t)kc * NN;
+#pragma unroll
+    for (int n = 0; n < N; ++n) y0[n] = mr <= n ? rho[mr * N + n] : cconj(rho[n * N + mr]);
+    const double eps = P.vg_eps[(size_t)kc * N + mr], f = P.vg_f[(size_t)kc * N + mr];
+    const double wk = live && own ? P.weight[kc] : 0.0;
+    const double g1 = P.g1, g2 = P.g2;
+    const int ce = (P.nval * N + P.nval + 1) % NN, cr = ce / N, cc = ce % N;   // antelope.cpp:539-542
+    double *const part = P.step_part + (size_t)(warp_k / KW) * WAN_NSLOT;
+    const size_t pstride = (size_t)P.step_rows * WAN_NSLOT;
+
+    for (int j = 0; j < steps; ++j) {
+        const double *fl = P.step_fld + (size_t)(n0 + j) * TB::NT * 3;
+        const double h = step_length(P, n0 + j);
+        {   // currents at the start of the step (SBEs.h:694-760), occupations, coherence
+            double v[4] = {0.0, 0.0, 0.0, 0.0}, oc = 0.0, co = 0.0;
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const bool dg = n == m;
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    const double q = fma(y0[n].x, p[a][n].x, y0[n].y * p[a][n].y);   // Re rho_nm P_mn
+                    v[a] += dg ? 0.0 : q;
+                    v[2 + a] += dg ? q : 0.0;
+                }
+                if (dg) oc = y0[n].x;
+                // element ce: its real part from row cr, its imaginary part (of
+                // the conjugate) from row cc
+                if (m == cr && n == cc) co = y0[n].x;
+                else if (m == cc && n == cr) co = -y0[n].y;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] *= wk;
+            oc *= wk;
+            co *= wk;
+            const bool h4 = lane & 16, h3 = lane & 8;
+            double u0 = (h4 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h4 ? v[0] : v[2], 16);
+            double u1 = (h4 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h4 ? v[1] : v[3], 16);
+            double z = (h3 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, h3 ? u0 : u1, 8);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+#pragma unroll
+            for (int o = 16; o >= G; o >>= 1) {
+                oc += __shfl_xor_sync(0xffffffffu, oc, o);
+                co += __shfl_xor_sync(0xffffffffu, co, o);
+            }
+            double *row = part + (size_t)j * pstride;
+            if ((lane & 7) == 0) row[lane >> 3] = z;
+            if (lane < N) {
+                row[4 + lane] = oc;
+                if (lane == cr) row[4 + N] = co;
+                if (lane == cc && cr != cc) row[5 + N] = co;
+            }
+        }
+        double2 ks[TB::S][N], inc[N], H[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) inc[n] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int s = 0; s < TB::S; ++s) {
+            double2 y[N];
+#pragma unroll
+            for (int n = 0; n < N; ++n) y[n] = y0[n];
+#pragma unroll
+            for (int q = 0; q < s; ++q)
+                if (TB::a(s, q) != 0.0) {
+                    const double a = h * TB::a(s, q);
+#pragma unroll
+                    for (int n = 0; n < N; ++n)
+                        y[n] = make_double2(fma(a, ks[q][n].x, y[n].x), fma(a, ks[q][n].y, y[n].y));
+                }
+#pragma unroll
+            for (int n = 0; n < N; ++n)
+                if (own && n >= m) Y[m * N - m * (m - 1) / 2 + (n - m)] = y[n];
+            if (s == 0 || TB::ti(s) != TB::ti(s - 1)) {   // row m of diag(eps) + A.P (SBEs.h:787-805)
+                const double Ax = fl[TB::ti(s) * 3], Ay = fl[TB::ti(s) * 3 + 1];
+#pragma unroll
+                for (int n = 0; n < N; ++n)
+                    H[n] = make_double2(fma(Ax, p[0][n].x, fma(Ay, p[1][n].x, n == m ? eps : 0.0)),
+                                        fma(Ax, p[0][n].y, Ay * p[1][n].y));
+            }
+            __syncwarp();
+            double2 c[N];
+#pragma unroll
+            for (int n = 0; n < N; ++n) c[n] = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int l = 0; l < N; ++l)
+#pragma unroll
+                for (int n = l; n < N; ++n) {
+                    const double2 v = Y[l * N - l * (l - 1) / 2 + (n - l)];   // Y_ln
+                    cfma(c[n], H[l], v);
+                    if (n != l) cfma(c[l], H[n], cconj(v));
+                }
+#pragma unroll
+            for (int n = 0; n < N; ++n)
+                if (own) T[m * D::LDT + n] = c[n];
+            __syncwarp();
+            // -i((HY) - (HY)^dag) - Gamma o (Y - rho0)   (SBEs.h:808-819, 862-871)
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const double2 d = T[n * D::LDT + mr];
+                const double re = c[n].y + d.y, im = d.x - c[n].x;
+                ks[s][n] = n == m ? make_double2(fma(-g1, y[n].x - f, re), 0.0)
+                                  : make_double2(fma(-g2, y[n].x, re), fma(-g2, y[n].y, im));
+                if (TB::b(s) != 0.0) {
+                    const double b = h * TB::b(s);
+                    inc[n] = make_double2(fma(b, ks[s][n].x, inc[n].x), fma(b, ks[s][n].y, inc[n].y));
+                }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) y0[n] = make_double2(y0[n].x + inc[n].x, y0[n].y + inc[n].y);
+    }
+    if (live && own)
+#pragma unroll
+        for (int n = 0; n < N; ++n) rho[m * N + n] = y0[n];
+}
+
+// Block (j, solve): the sums of the launch's step j over the solve's partial
+// rows (fixed order).  The solve's last block to finish moves its controller
+// past the launch's steps; every block has read it by then.
+__global__ void __launch_bounds__(256) wan_finish(const WanDev *__restrict__ Pp, const WanDev *const *__restrict__ descs,
+                                                  int S)
+{
+    __shared__ double red[16][WAN_NSLOT];
+    const WanDev &P = descs ? *descs[blockIdx.y] : *Pp;
+    WanCtl *ctl = P.ctl;
+    const int j = blockIdx.x, t = threadIdx.x;
+    if (ctl->done) {
+        if (j == 0 && t == 0) ctl->shot = -1;   // a snapshot is taken once
+        return;
+    }
+    const int n0 = ctl->n, steps = launch_steps(P, n0, S);
+    if (j < steps) {
+        const int slot = t % WAN_NSLOT, g = t / WAN_NSLOT, nw = P.step_rows;
+        const double *p = P.step_part + (size_t)j * nw * WAN_NSLOT + slot;
+        double s0 = 0.0, s1 = 0.0;
+        int i = g;
+        for (; i + 16 < nw; i += 32) {
+            s0 += p[(size_t)i * WAN_NSLOT];
+            s1 += p[(size_t)(i + 16) * WAN_NSLOT];
+        }
+        if (i < nw) s0 += p[(size_t)i * WAN_NSLOT];
+        red[g][slot] = s0 + s1;
+        __syncthreads();
+        if (t < WAN_NSLOT) {
+            double s = 0.0;
+            for (int q = 0; q < 16; ++q) s += red[q][t];
+            P.jout[(size_t)(n0 + j) * WAN_NSLOT + t] = s;
+        }
+    }
+    __syncthreads();
+    if (t == 0) {
+        __threadfence();
+        if (atomicAdd(P.step_ticket, 1u) == gridDim.x - 1) {
+            *P.step_ticket = 0u;
+            ctl->shot = -1;
+            ctl->n = n0 + steps;
+            // a step whose end the sum t + dt misses by rounding counts one
+            // more (empty) step, as the step controller counts it
+            long long cnt = steps;
+            for (int n = n0; n < n0 + steps; ++n)
+                cnt += !(step_start(P, n) + P.dt >= P.atmin + P.dt * (n + 1) - 1e-12 * P.dt);
+            ctl->steps += cnt;
+            ctl->attempts += cnt;
+            ctl->tc = step_start(P, n0 + steps);
+            ctl->need_current = 1;
+            if (P.shot_every > 0 && (n0 + steps - 1) % P.shot_every == 0) ctl->shot = n0 + steps - 1;
+            if (n0 + steps >= P.Nt) ctl->done = 1;
+        }
+    }
+}
+
+// ============================================================= launchers
+// One thread per k-point (1) while a k-point's matrices fit a thread's
+// registers without spilling (N <= 3), else one row per lane (2); both sides
+// measured at the head of this file.
+int wan_steps(const WanDev &w)
+{
+    if (!w.vg || (w.rk != 4 && w.rk != 5) || w.N < 2 || w.N > WAN_MAXN) return 0;
+    return w.N <= 3 ? 1 : 2;
+}
+static int row_lanes(int N) { return N <= 4 ? 4 : 8; }
+int wan_steps_rows(const WanDev &w)
+{
+    const int kw = wan_steps(w) == 2 ? 32 / row_lanes(w.N) : 32;
+    return (w.nk + kw - 1) / kw;
+}
+int wan_steps_fields(int rk) { return rk == 4 ? StepTab<4>::NT : StepTab<5>::NT; }
+int wan_steps_unit(int mode, int N) { return (mode == 2 ? WR_T / row_lanes(N) : WS_T) / WAN_WARPS; }
+
+using StepKernel = void (*)(const WanDev *, const WanDev *const *, const WanTileRef *, int);
+template <int RK> static StepKernel vg_steps_n(int mode, int N, int na)
+{
+    if (mode == 1) {
+        if (N == 2) return na == 3 ? wan_vg_steps<2, RK, 3> : wan_vg_steps<2, RK, 2>;   // 3: the continuum model
+        return N == 3 ? wan_vg_steps<3, RK, 2> : nullptr;
+    }
+    switch (N) {
+    case 4: return wan_vg_rows<4, RK>;
+    case 5: return wan_vg_rows<5, RK>;
+    case 6: return wan_vg_rows<6, RK>;
+    case 7: return wan_vg_rows<7, RK>;
+    case 8: return wan_vg_rows<8, RK>;
+    default: return nullptr;
+    }
+}
+
+cudaError_t launch_wan_steps(int mode, int N, int na, int rk, const WanDev *dw, const WanDev *const *descs,
+                             const WanTileRef *tiles, int nblocks, int S, cudaStream_t st)
+{
+    const StepKernel f = rk == 4 ? vg_steps_n<4>(mode, N, na) : rk == 5 ? vg_steps_n<5>(mode, N, na) : nullptr;
+    if (!f) return cudaErrorInvalidValue;
+    const int sm = mode == 1 ? (na * N * N + N) * WS_T * 16 : 0;   // at most 21 KB
+    f<<<nblocks, mode == 1 ? WS_T : WR_T, sm, st>>>(dw, descs, tiles, S);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_wan_finish(const WanDev *dw, const WanDev *const *descs, int nsolves, int S, cudaStream_t st)
+{
+    wan_finish<<<dim3(S, nsolves), 256, 0, st>>>(dw, descs, S);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_wan_step_fields(const WanDev &w, const WanDev *dw, cudaStream_t st)
+{
+    const int nt = wan_steps_fields(w.rk);
+    wan_step_fields<<<(w.Nt * nt + 127) / 128, 128, 0, st>>>(dw, nt, w.rk);
+    return cudaGetLastError();
+}
+
+}  // namespace sbe
