@@ -543,6 +543,21 @@ __global__ void __launch_bounds__(32 * WAN_WARPS) wan_init(WanDev P)
     for (int e = lane; e < NN; e += 32) w.B[e] = w.H0[e];
     __syncwarp();
     jacobi_sweeps<RF>(w, bh, N, 16, 1e-30, lane);
+    if (P.band_gap) {   // smallest gap between bands and largest width of the spectrum over the grid
+        double gap = 1e300, wid = 0.0;
+        if (lane < N)
+            for (int j = 0; j < N; ++j) {
+                const double d = fabs(w.B[j * N + j].x - w.B[lane * N + lane].x);
+                if (j != lane) gap = fmin(gap, d);
+                wid = fmax(wid, d);
+            }
+        gap = -warp_max(-gap);
+        wid = warp_max(wid);
+        if (lane == 0) {   // non-negative doubles order as their bits
+            atomicMin(P.band_gap, (unsigned long long)__double_as_longlong(gap));
+            atomicMax(P.band_gap + 1, (unsigned long long)__double_as_longlong(wid));
+        }
+    }
     // occupations of the eigenstates: the Nval lowest filled, or Fermi-Dirac (SBEs.h:319-340)
     if (lane < N) {
         const double ev = w.B[lane * N + lane].x;

@@ -101,6 +101,16 @@ struct WanDev {
     double *step_part;
     unsigned *step_ticket;
     int step_rows;
+    // ... in the length gauge the launch's phase factors e^{iA(t)R}
+    // [WAN_STEPS][wan_steps_fields][npair] at the pairs' vectors gpair (gmate:
+    // the index of a pair's other vector, or -1)
+    double2 *step_cA;
+    const int *gmate;
+    int mixed;              // the mixed method (FP32 Fourier sums)
+    // length gauge: bits of the smallest gap between two bands and of the
+    // largest spread of the bands over the grid (wan_init), or null
+    unsigned long long *band_gap;
+    int degenerate;   // bands meet at a grid point: wan_steps does not apply
 };
 
 // A tile of a batched launch: tile `tile` (WAN_WARPS k-points) of solve
@@ -157,15 +167,23 @@ cudaError_t launch_wan_control_batch(const WanDev *const *descs, int nsolves, in
 // Fixed-step solves that advance many steps per launch (sbe_wanstep.cu):
 // wan_steps says which; a launch takes at most WAN_STEPS steps of each solve
 // and launch_wan_finish then sums the steps' outputs and moves the
-// controllers on.  A block covers wan_steps_unit() tiles (tile = the first
-// one); N, na (components of A.P: 3 for the continuum model) and rk pick the
-// instance, `descs` / `tiles` null for a single solve (`dw`).
+// controllers on.  Solves of one class (equal but for npair, of which the
+// launch gets the largest) share launches; a block covers wan_steps_unit() tiles
+// (tile = the first one).  `descs` / `tiles` null: a single solve (`dw`).
 constexpr int WAN_STEPS = 64;
 int wan_steps(const WanDev &w);   // 0: no; otherwise the kernel form (mode)
 int wan_steps_rows(const WanDev &w);
 int wan_steps_fields(int rk);
 int wan_steps_unit(int mode, int N);
-cudaError_t launch_wan_steps(int mode, int N, int na, int rk, const WanDev *dw, const WanDev *const *descs,
+struct WanStepClass {
+    int mode = 0, N = 0, na = 2, rk = 0, npair = 0;   // na: components of A.P (3: the continuum model)
+    bool same(const WanStepClass &o) const
+    {
+        return mode == o.mode && (!mode || (N == o.N && na == o.na && rk == o.rk));
+    }
+};
+WanStepClass wan_step_class(const WanDev &w);
+cudaError_t launch_wan_steps(const WanStepClass &c, const WanDev *dw, const WanDev *const *descs,
                              const WanTileRef *tiles, int nblocks, int S, cudaStream_t st);
 cudaError_t launch_wan_finish(const WanDev *dw, const WanDev *const *descs, int nsolves, int S, cudaStream_t st);
 cudaError_t launch_wan_step_fields(const WanDev &w, const WanDev *dw, cudaStream_t st);

@@ -95,6 +95,7 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
         dalloc(&w_.snap_nc, sizeof(double) * nshots_ * nk, st, "alloc snapshots");
         dalloc(&w_.snap_pi, sizeof(double) * 2 * nshots_ * nk, st, "alloc snapshots");
     }
+    w_.mixed = precision_ != 0;
     if (wan_steps(w_)) {
         w_.step_rows = wan_steps_rows(w_);
         dalloc(&w_.step_fld, sizeof(double) * (size_t)w_.Nt * wan_steps_fields(w_.rk) * 3, st, "alloc step fields");
@@ -121,7 +122,8 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     // past the triangle or without dipoles.
     std::vector<double> gt;
     std::vector<int> gpair, mate(w_.nR, -1);
-    if (wan_grouped_applies(w_)) {
+    const bool lw_steps = !w_.vg && wan_steps(w_) != 0;
+    if (wan_grouped_applies(w_) || lw_steps) {
         const int nR = w_.nR;
         std::vector<char> used(nR, 0);
         for (int r = 0; r < nR; ++r) {
@@ -138,9 +140,23 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
         // more vectors without their negatives than R = 0 (the SyntheticWannier
         // reader already refuses such a model): the grouped kernel's per-k
         // phase arrays are sized for pairs, so wan_attempt would run it
-        if ((int)gpair.size() > wan_npair_cap(nR)) gpair.clear();
+        if (!lw_steps && (int)gpair.size() > wan_npair_cap(nR)) gpair.clear();
     }
-    if (!gpair.empty()) {
+    std::vector<int> gmate;
+    if (lw_steps) {
+        for (int r : gpair) gmate.push_back(mate[r]);
+        int *gp = nullptr, *gm = nullptr;
+        dalloc(&gp, sizeof(int) * gpair.size(), st, "alloc vector pairs");
+        dalloc(&gm, sizeof(int) * gpair.size(), st, "alloc vector pairs");
+        w_.gpair = gp;
+        w_.gmate = gm;
+        w_.npair = (int)gpair.size();
+        dalloc(&w_.band_gap, 16, st, "alloc band gap");
+        cuda_check(cudaMemsetAsync(w_.band_gap, 0x7f, 8, st), "clear band gap");   // a large double
+        cuda_check(cudaMemsetAsync(w_.band_gap + 1, 0, 8, st), "clear band gap");
+        dalloc(&w_.step_cA, sizeof(double2) * WAN_STEPS * (size_t)wan_steps_fields(w_.rk) * w_.npair, st,
+               "alloc step phases");
+    } else if (!gpair.empty()) {
         const int NU = N * (N + 1) / 2, NO = (NU + 7) / 8, row = wan_gtab_row(N);
         const int np = (int)gpair.size();
         gt.assign((size_t)np * row * 2, 0.0);
@@ -197,6 +213,7 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     if (w_.has_jtab && !w_.cont) up_real(j, p.w_j);
     if (w_.gtab) up_real(const_cast<void *>(w_.gtab), gt);
     if (w_.gpair) ring.upload(const_cast<int *>(w_.gpair), gpair.data(), sizeof(int) * gpair.size(), st);
+    if (w_.gmate) ring.upload(const_cast<int *>(w_.gmate), gmate.data(), sizeof(int) * gmate.size(), st);
     cuda_check(cudaMemsetAsync(w_.jout, 0, sizeof(double) * (size_t)w_.Nt * WAN_NSLOT, st), "clear outputs");
     // initial controller state: t = t_min, h = dt, currents first
     WanCtl c{};
@@ -216,6 +233,12 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     ring.upload(w_.ctl, &c, sizeof(c), st);
     ring.upload(d_w_, &w_, sizeof(w_), st);
     cuda_check(launch_wan_init(w_, precision_, st), "Wannier init kernel");
+    if (w_.band_gap) {   // bands that meet on the grid rule the many-step kernels out
+        double gw[2];
+        cuda_check(cudaMemcpyAsync(gw, w_.band_gap, 16, cudaMemcpyDeviceToHost, st), "copy band gap");
+        cuda_check(cudaStreamSynchronize(st), "sync");
+        w_.degenerate = !(gw[0] > 1e-7 * gw[1]);
+    }
     if (wan_steps(w_)) cuda_check(launch_wan_step_fields(w_, d_w_, st), "Wannier step fields");
     else cuda_check(launch_wan_prepare(d_w_, precision_, st), "Wannier stage preparation");
     cuda_check(cudaMallocHost(&h_ctl_, sizeof(WanCtl)), "cudaMallocHost(control)");
@@ -248,6 +271,9 @@ WannierSolve::~WannierSolve()
     if (w_.step_fld) cudaFreeAsync(w_.step_fld, stream_);
     if (w_.step_part) cudaFreeAsync(w_.step_part, stream_);
     if (w_.step_ticket) cudaFreeAsync(w_.step_ticket, stream_);
+    if (w_.step_cA) cudaFreeAsync(w_.step_cA, stream_);
+    if (w_.gmate) cudaFreeAsync((void *)w_.gmate, stream_);
+    if (w_.band_gap) cudaFreeAsync(w_.band_gap, stream_);
     cudaFreeAsync(d_w_, stream_);
     if (w_.snap_nc) cudaFreeAsync(w_.snap_nc, stream_);
     if (w_.snap_pi) cudaFreeAsync(w_.snap_pi, stream_);
@@ -259,14 +285,14 @@ void WannierSolve::run(cudaStream_t st)
 {
     stream_ = st;
     if (wan_steps(w_)) {   // a fixed number of launches, each of many steps
-        const int mode = wan_steps(w_), na = w_.cont ? 3 : 2, unit = wan_steps_unit(mode, w_.N), F = w_.shot_every;
+        const WanStepClass sc = wan_step_class(w_);
+        const int unit = wan_steps_unit(sc.mode, w_.N), F = w_.shot_every;
         launches_ = 0;
         for (int n = 0; n < w_.Nt;) {
             // the steps the kernels take from n (a launch ends at a snapshot)
             int m = std::min(WAN_STEPS, w_.Nt - n);
             if (F > 0) m = std::min(m, (n + F - 1) / F * F + 1 - n);
-            cuda_check(launch_wan_steps(mode, w_.N, na, w_.rk, d_w_, nullptr, nullptr, (w_.ntiles + unit - 1) / unit,
-                                        WAN_STEPS, st),
+            cuda_check(launch_wan_steps(sc, d_w_, nullptr, nullptr, (w_.ntiles + unit - 1) / unit, WAN_STEPS, st),
                        "Wannier step kernel");
             cuda_check(launch_wan_finish(d_w_, nullptr, 1, WAN_STEPS, st), "Wannier finish kernel");
             cuda_check(launch_wan_snapshot(w_, d_w_, precision_, st), "Wannier snapshot kernel");
@@ -318,11 +344,12 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
     // lead the tile list, so their blocks are scheduled first
     for (int i = 0; i < (int)solves_.size(); ++i) {
         const WanDev &w = solves_[i]->dev();
-        const int grk = wan_grouped(w) ? w.rk : 0, smode = wan_steps(w), srk = smode ? w.rk : 0, na = w.cont ? 3 : 2;
+        const int grk = wan_grouped(w) ? w.rk : 0;
+        const WanStepClass sc = wan_step_class(w);
         Class *c = nullptr;
         for (Class &x : classes_)
             if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == solves_[i]->precision() && x.grouped_rk == grk &&
-                x.steps_rk == srk && x.steps_mode == smode && (!srk || x.na == na))
+                x.steps.same(sc))
                 c = &x;
         if (!c) {
             classes_.emplace_back();
@@ -331,12 +358,11 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
             c->vg = w.vg != 0;
             c->precision = solves_[i]->precision();
             c->grouped_rk = grk;
-            c->steps_rk = srk;
-            c->steps_mode = smode;
-            c->na = na;
+            c->steps = sc;
         }
         c->members.push_back(i);
         c->nR = std::max(c->nR, w.nR);
+        c->steps.npair = std::max(c->steps.npair, sc.npair);
         c->shots = c->shots || w.shot_every > 0;
     }
     UploadRing &ring = UploadRing::shared();
@@ -354,7 +380,7 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         // interleave the solves' tiles round-robin (longest first), so that
         // the blocks of one launch spread every solve over the whole GPU
         // (grouped classes: one entry per block of WAN_GROUP_TILES tiles)
-        const int unit = c.steps_rk ? wan_steps_unit(c.steps_mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
         int maxt = 0;
         for (int m : c.members) maxt = std::max(maxt, solves_[m]->dev().ntiles);
         for (int t = 0; t < maxt; t += unit)
@@ -396,9 +422,9 @@ int WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
     int launched = 0;
     for (int it = 0; it < iters; ++it)
         for (const Class &c : classes_) {
-            if (c.steps_rk) {   // WAN_STEPS iterations in one launch
+            if (c.steps.mode) {   // WAN_STEPS iterations in one launch
                 if (it % WAN_STEPS) continue;
-                cuda_check(launch_wan_steps(c.steps_mode, c.N, c.na, c.steps_rk, nullptr, c.d_descs, c.d_tiles, c.ntiles,
+                cuda_check(launch_wan_steps(c.steps, nullptr, c.d_descs, c.d_tiles, c.ntiles,
                                             std::min(WAN_STEPS, iters - it), st),
                            "Wannier step kernel (batch)");
                 cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.members.size(), std::min(WAN_STEPS, iters - it), st),
@@ -494,8 +520,8 @@ size_t WannierPool::bytes_needed(const Problem &p, int precision)
     b += nR * NN * cplx * 5 + nR * 16 + nR * 216 * cplx;               // h, d, current, re-laid and stage tables, vectors
     b += ntiles * 8 * (1 + WAN_NSLOT) + (size_t)p.laser.Nt * WAN_NSLOT * 8;   // tile results, per-step sums
     if (p.gauge == GAUGE_VELOCITY) b += nk * N * 16 + nk * 3 * NN * 16;  // bands, momentum matrices
-    if (p.gauge == GAUGE_VELOCITY && p.rk != 45)   // step fields and partials
-        b += (size_t)p.laser.Nt * 6 * 24 + (size_t)WAN_STEPS * (nk / 4 + 1) * WAN_NSLOT * 8;
+    if (p.rk != 45)   // step fields, phases and partials
+        b += (size_t)WAN_STEPS * 6 * nR * cplx + (size_t)p.laser.Nt * 6 * 24 + (size_t)WAN_STEPS * (nk / 4 + 1) * WAN_NSLOT * 8;
     return b + 4096;
 }
 
@@ -559,11 +585,12 @@ void WannierPool::rebuild()
         if (kv.second.done) continue;
         const WannierSolve &s = *kv.second.s;
         const WanDev &w = s.dev();
-        const int grk = wan_grouped(w) ? w.rk : 0, smode = wan_steps(w), srk = smode ? w.rk : 0, na = w.cont ? 3 : 2;
+        const int grk = wan_grouped(w) ? w.rk : 0;
+        const WanStepClass sc = wan_step_class(w);
         Class *c = nullptr;
         for (Class &x : classes_)
             if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == s.precision() && x.grouped_rk == grk &&
-                x.steps_rk == srk && x.steps_mode == smode && (!srk || x.na == na))
+                x.steps.same(sc))
                 c = &x;
         if (!c) {
             classes_.emplace_back();
@@ -572,18 +599,17 @@ void WannierPool::rebuild()
             c->vg = w.vg != 0;
             c->precision = s.precision();
             c->grouped_rk = grk;
-            c->steps_rk = srk;
-            c->steps_mode = smode;
-            c->na = na;
+            c->steps = sc;
         }
         c->ids.push_back(kv.first);
         c->nR = std::max(c->nR, w.nR);
+        c->steps.npair = std::max(c->steps.npair, sc.npair);
     }
     UploadRing &ring = UploadRing::shared();
     for (Class &c : classes_) {
         std::vector<const WanDev *> descs;
         std::vector<WanTileRef> tiles;
-        const int unit = c.steps_rk ? wan_steps_unit(c.steps_mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
         int maxt = 0;
         for (int id : c.ids) {
             descs.push_back(solves_.at(id).s->dev_ptr());
@@ -609,10 +635,10 @@ void WannierPool::step(int iters)
     if (classes_.empty()) return;
     for (int it = 0; it < iters; ++it)
         for (const Class &c : classes_) {
-            if (c.steps_rk) {   // up to WAN_STEPS iterations in one launch
+            if (c.steps.mode) {   // up to WAN_STEPS iterations in one launch
                 if (it % WAN_STEPS) continue;
                 const int S = std::min(WAN_STEPS, iters - it);
-                cuda_check(launch_wan_steps(c.steps_mode, c.N, c.na, c.steps_rk, nullptr, c.d_descs, c.d_tiles, c.ntiles, S, st_),
+                cuda_check(launch_wan_steps(c.steps, nullptr, c.d_descs, c.d_tiles, c.ntiles, S, st_),
                            "Wannier step kernel (server)");
                 cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.ids.size(), S, st_),
                            "Wannier finish kernel (server)");

@@ -72,7 +72,7 @@ private:
     struct Class {
         int N = 0, nR = 0, precision = 0;
         int grouped_rk = 0;   // the grouped attempt kernel (and its RK order), or 0
-        int steps_rk = 0, steps_mode = 0, na = 2;   // the many-step kernels (RK order, form) or 0; components of A.P
+        WanStepClass steps;   // the many-step kernels (mode 0: not)
         bool vg = false, shots = false;
         std::vector<int> members;
         const WanDev **d_descs = nullptr;
@@ -129,7 +129,8 @@ private:
     cudaStream_t st_;
     bool dirty_ = true;
     struct Class {
-        int N = 0, nR = 0, precision = 0, grouped_rk = 0, steps_rk = 0, steps_mode = 0, na = 2;
+        int N = 0, nR = 0, precision = 0, grouped_rk = 0;
+        WanStepClass steps;
         bool vg = false;
         std::vector<int> ids;
         const WanDev **d_descs = nullptr;

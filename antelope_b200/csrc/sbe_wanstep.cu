@@ -16,6 +16,7 @@
 // wan_vg_rows: the same at N = 4 ... 8, one row of the matrices per lane.
 // Both are FP64 in both methods, as wan_vg_attempt, which runs the adaptive
 // Cash-Karp steps.
+// wan_lw_steps: the length gauge of the analytic materials at N = 2, 3, 4.
 //
 // Measured (RK4, 367 steps, whole solve with its set-up): three bands 1.8 us a
 // step at 14 520 k-points and 5.5 at 90 300 (rows: 3.7, 14.9); four bands rows
@@ -465,6 +466,415 @@ __global__ void __launch_bounds__(WR_T, N <= 4 ? 6 : 4) wan_vg_rows(const WanDev
         for (int n = 0; n < N; ++n) rho[m * N + n] = y0[n];
 }
 
+// ============================================================= length gauge
+// Models with their own current-operator tables (has_jtab: the analytic
+// materials), plain FP64 method: rho in the Wannier basis, H0(k + A) from its
+// Fourier tables, dephasing in the eigenbasis of H0 (SBEs.h:762-786, 831-861).
+// A pair of lattice vectors (R, -R) is summed together: c sig + s tau with
+// e^{iKR} = c + i s.
+
+// Phase factors e^{iA(t)R} of a launch that starts at step n0: row j of
+// step_cA, at the distinct stage times of step n0 + j.
+__device__ void launch_phases(const WanDev &P, int n0, int j)
+{
+    const int n = n0 + j, nt = P.rk == 4 ? StepTab<4>::NT : StepTab<5>::NT;
+    if (!P.step_cA || n >= P.Nt) return;
+    double2 *out = P.step_cA + (size_t)j * nt * P.npair;
+    for (int i = threadIdx.x; i < nt * P.npair; i += blockDim.x) {
+        const int r = P.gpair[i % P.npair];
+        const double *A = P.step_fld + ((size_t)n * nt + i / P.npair) * 3;
+        double sn, cs;
+        sincos(A[0] * P.V[2 * r] + A[1] * P.V[2 * r + 1], &sn, &cs);
+        out[i] = make_double2(cs, sn);
+    }
+}
+
+__global__ void __launch_bounds__(256) wan_step_phases(const WanDev *__restrict__ Pp)
+{
+    launch_phases(*Pp, Pp->ctl->n, blockIdx.x);
+}
+
+// Upper-triangle pair tables [np][2][NU] (sig, tau) of H (a < 0), or of the
+// Hermitian part of J_a (Re Tr(rho J) sees no more), into shared memory
+__device__ __forceinline__ void load_pairs(const WanDev &P, int N, int a, double2 *sh)
+{
+    const int NN = N * N, NU = N * (N + 1) / 2;
+    const double2 *tb = static_cast<const double2 *>(a < 0 ? P.h : P.jt) + (a > 0 ? NN : 0);
+    const int stride = a < 0 ? NN : 2 * NN;
+    const double2 zero = make_double2(0.0, 0.0);
+    for (int i = threadIdx.x; i < P.npair * NU; i += blockDim.x) {
+        const int q = i / NU, r = P.gpair[q], r2 = P.gmate[q];
+        int u = i % NU, m = 0;
+        while (u >= N - m) { u -= N - m; ++m; }
+        const int n = m + u;
+        double2 x = tb[(size_t)r * stride + m * N + n], y = r2 < 0 ? zero : tb[(size_t)r2 * stride + m * N + n];
+        if (a >= 0) {   // (T + T^dag) / 2: the adjoint of the entry at R belongs to -R
+            const double2 xt = cconj(tb[(size_t)r * stride + n * N + m]);
+            const double2 yt = r2 < 0 ? zero : cconj(tb[(size_t)r2 * stride + n * N + m]);
+            x = make_double2(0.5 * (x.x + yt.x), 0.5 * (x.y + yt.y));
+            y = make_double2(0.5 * (y.x + xt.x), 0.5 * (y.y + xt.y));
+        }
+        double2 *o = sh + q * 2 * NU + i % NU;
+        o[0] = make_double2(x.x + y.x, x.y + y.y);
+        o[NU] = make_double2(y.y - x.y, x.x - y.x);   // i (x - y)
+    }
+}
+
+// Hermitian N x N matrix of one thread: real diagonal, upper off-diagonal
+template <int N> struct Herm {
+    static constexpr int NO = N * (N - 1) / 2;
+    double d[N];
+    double2 o[NO];
+};
+template <int N> __device__ __forceinline__ double2 el(const Herm<N> &A, int m, int n)   // m != n
+{
+    return m < n ? A.o[oidx(m, n, N)] : cconj(A.o[oidx(n, m, N)]);
+}
+template <int N> __device__ __forceinline__ double tr2(const Herm<N> &A, const Herm<N> &B)   // Tr(A B)
+{
+    double s = 0.0, t = 0.0, u = 0.0;   // separate chains: latency counts at one warp per scheduler
+#pragma unroll
+    for (int m = 0; m < N; ++m) s = fma(A.d[m], B.d[m], s);
+#pragma unroll
+    for (int i = 0; i < Herm<N>::NO; ++i) {
+        t = fma(A.o[i].x, B.o[i].x, t);
+        u = fma(A.o[i].y, B.o[i].y, u);
+    }
+    return fma(2.0, t + u, s);
+}
+template <int N> __device__ __forceinline__ void axpy(Herm<N> &A, double c, const Herm<N> &B)   // A += c B
+{
+#pragma unroll
+    for (int m = 0; m < N; ++m) A.d[m] = fma(c, B.d[m], A.d[m]);
+#pragma unroll
+    for (int i = 0; i < Herm<N>::NO; ++i) A.o[i] = make_double2(fma(c, B.o[i].x, A.o[i].x), fma(c, B.o[i].y, A.o[i].y));
+}
+template <int N> __device__ __forceinline__ void clear(Herm<N> &A)
+{
+#pragma unroll
+    for (int m = 0; m < N; ++m) A.d[m] = 0.0;
+#pragma unroll
+    for (int i = 0; i < Herm<N>::NO; ++i) A.o[i] = make_double2(0.0, 0.0);
+}
+template <int N> __device__ __forceinline__ void traceless(Herm<N> &A)
+{
+    double t = 0.0;
+#pragma unroll
+    for (int m = 0; m < N; ++m) t += A.d[m];
+#pragma unroll
+    for (int m = 0; m < N; ++m) A.d[m] = fma(t, -1.0 / N, A.d[m]);
+}
+// W = traceless part of A B for commuting A, B
+template <int N> __device__ __forceinline__ void mul_traceless(Herm<N> &W, const Herm<N> &A, const Herm<N> &B)
+{
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+        double d = A.d[m] * B.d[m];
+#pragma unroll
+        for (int l = 0; l < N; ++l)
+            if (l != m) {
+                const double2 x = el<N>(A, m, l), y = el<N>(B, m, l);
+                d = fma(x.x, y.x, fma(x.y, y.y, d));
+            }
+        W.d[m] = d;
+#pragma unroll
+        for (int n = m + 1; n < N; ++n) {
+            const double2 x = A.o[oidx(m, n, N)], y = B.o[oidx(m, n, N)];
+            double2 w = make_double2(fma(A.d[m], y.x, x.x * B.d[n]), fma(A.d[m], y.y, x.y * B.d[n]));
+#pragma unroll
+            for (int l = 0; l < N; ++l)
+                if (l != m && l != n) cfma(w, el<N>(A, m, l), el<N>(B, l, n));
+            W.o[oidx(m, n, N)] = w;
+        }
+    }
+    traceless<N>(W);
+}
+
+// D = the band-diagonal part of Y in the eigenbasis of A, U diag(U^dag Y U)
+// U^dag, without the eigenbasis: for distinct eigenvalues it is the orthogonal
+// projection (inner product Tr(XY)) of Y on the span of I, A, ..., A^{N-1},
+// the matrices that commute with A.  The Lanczos recurrence from I (left
+// multiplication by A is self-adjoint) gives an orthogonal basis of Hermitian
+// matrices in N - 2 products, where a tracked eigenbasis takes B = U^dag A U,
+// rotations until it is diagonal, and U diag U^dag.  Conditioned like the
+// eigenvectors (rounding over the smallest gap).  N = 2 is the closed form
+// (s.n) n of the Bloch vector.  A is made traceless.
+template <int N> __device__ __forceinline__ void band_diagonal(Herm<N> &D, Herm<N> &A, const Herm<N> &Y)
+{
+    double ty = 0.0;
+#pragma unroll
+    for (int m = 0; m < N; ++m) ty += Y.d[m];
+    traceless<N>(A);
+    const double a2 = tr2<N>(A, A), ia = a2 > 0.0 ? 1.0 / a2 : 0.0;
+    clear<N>(D);
+#pragma unroll
+    for (int m = 0; m < N; ++m) D.d[m] = ty * (1.0 / N);
+    axpy<N>(D, tr2<N>(A, Y) * ia, A);
+    if constexpr (N > 2) {
+        // a basis matrix that is rounding only (two bands meet) is left out
+        Herm<N> W;
+        mul_traceless<N>(W, A, A);
+        axpy<N>(W, -tr2<N>(W, A) * ia, A);
+        const double w2 = tr2<N>(W, W), iw = w2 > 1e-26 * a2 * a2 ? 1.0 / w2 : 0.0;
+        axpy<N>(D, tr2<N>(W, Y) * iw, W);
+        if constexpr (N > 3) {
+            Herm<N> V;
+            mul_traceless<N>(V, A, W);
+            const double va = tr2<N>(V, A) * ia, vw = tr2<N>(V, W) * iw;
+            axpy<N>(V, -va, A);
+            axpy<N>(V, -vw, W);
+            const double v2 = tr2<N>(V, V), iv = v2 > 1e-26 * a2 * w2 ? 1.0 / v2 : 0.0;
+            axpy<N>(D, tr2<N>(V, Y) * iv, V);
+        }
+    }
+}
+
+// H += a pair's term: table entry s [2][NU], phase e
+template <int N> __device__ __forceinline__ void add_pair(Herm<N> &H, const double2 *s, double2 e)
+{
+    constexpr int NU = N * (N + 1) / 2;
+#pragma unroll
+    for (int m = 0; m < N; ++m)
+#pragma unroll
+        for (int n = m; n < N; ++n) {
+            const int u = m * N - m * (m - 1) / 2 + n - m;
+            const double2 sg = s[u], ta = s[NU + u];
+            if (m == n) {
+                H.d[m] = fma(e.x, sg.x, fma(e.y, ta.x, H.d[m]));
+            } else {
+                double2 &x = H.o[oidx(m, n, N)];
+                x = make_double2(fma(e.x, sg.x, fma(e.y, ta.x, x.x)), fma(e.x, sg.y, fma(e.y, ta.y, x.y)));
+            }
+        }
+}
+
+// the tableaux of StepTab, for the run-time stage loop
+__constant__ double c_step_a[2][6][6] = {
+    {{0}, {0.5}, {0, 0.5}, {0, 0, 1.0}},
+    {{0},
+     {1.0 / 4.0},
+     {3. / 32., 9. / 32.},
+     {1932. / 2197., -7200. / 2197., 7296. / 2197.},
+     {439. / 216., -8., 3680. / 513., -845. / 4104.},
+     {-8. / 27., 2., -3544. / 2565, 1859. / 4104, -11. / 40.}}};
+__constant__ double c_step_b[2][6] = {{1.0 / 6.0, 2.0 / 6.0, 2.0 / 6.0, 1.0 / 6.0},
+                                      {16. / 135., 0.0, 6656. / 12825., 28561. / 56430., -9. / 50., 2. / 55.}};
+
+constexpr int WL_T = 32;   // threads (k-points) per block
+// shared memory: H and J tables, the step's phase factors, per thread e^{ikR},
+// rho, its increment and the stage slopes
+static int lw_bytes(int N, int rk, int npair)
+{
+    const int nt = rk == 4 ? StepTab<4>::NT : StepTab<5>::NT;
+    return (3 * N * (N + 1) * npair + nt * npair + npair * WL_T) * 16 + (2 + (rk == 4 ? 1 : 5)) * N * N * WL_T * 8;
+}
+
+// N = 2, 3, 4, one thread per k-point.  H0, Y, D and the Lanczos basis are
+// registers; rho, its increment and the stage slopes wait in shared memory, a
+// column per thread.  The stage loop is a run-time loop, so that its body stays
+// in the instruction cache.  One-warp blocks: small grids spread over every
+// SM.  Latency-bound (a step is a serial chain of stages) until the grid gives
+// every scheduler a few warps, FP64-pipe bound beyond.  Measured (whole solves
+// of 367 steps with their set-up, us a step, 168 to 14 640 k-points alike): N =
+// 2, 3, 4 RK4 2.5, 5.7, 9.4, RK5 4.1, 9.2, 15; one attempt and one control
+// launch a step take 78 (N = 3, RK5, 2 400 k-points).
+template <int N, int RK>
+__global__ void __launch_bounds__(WL_T) wan_lw_steps(const WanDev *__restrict__ Pp,
+                                                     const WanDev *const *__restrict__ descs,
+                                                     const WanTileRef *__restrict__ tiles, int S)
+{
+    using TB = StepTab<RK>;
+    using HN = Herm<N>;
+    constexpr int NN = N * N, NU = N * (N + 1) / 2, NO = HN::NO, NK = RK == 4 ? 1 : 5;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
+    const int k0 = tiles ? tiles[blockIdx.x].tile * WAN_WARPS : (int)blockIdx.x * WL_T;
+    if (P.ctl->done) return;
+    const int n0 = P.ctl->n, steps = launch_steps(P, n0, S), np = P.npair, ncA = TB::NT * np;
+    const int t = threadIdx.x, lane = t & 31;
+    const int k = k0 + t;
+    const bool live = k < P.nk;
+    const int kc = live ? k : P.nk - 1;   // a thread past the grid shadows the last k-point
+    double2 *const htab = reinterpret_cast<double2 *>(smem), *const jtab = htab + 2 * NU * np;   // load_pairs; J_x, J_y
+    double2 *const cA = jtab + 4 * NU * np, *const pk = cA + ncA;                                // pk: [np][WL_T]
+    double *const sy = reinterpret_cast<double *>(pk + np * WL_T);   // [2 + NK][NN][WL_T]: rho, increment, slopes
+    auto put = [&](int slot, const HN &A) {
+#pragma unroll
+        for (int m = 0; m < N; ++m) sy[(slot * NN + m) * WL_T + t] = A.d[m];
+#pragma unroll
+        for (int i = 0; i < NO; ++i) {
+            sy[(slot * NN + N + 2 * i) * WL_T + t] = A.o[i].x;
+            sy[(slot * NN + N + 2 * i + 1) * WL_T + t] = A.o[i].y;
+        }
+    };
+    auto get = [&](int slot, HN &A) {
+#pragma unroll
+        for (int m = 0; m < N; ++m) A.d[m] = sy[(slot * NN + m) * WL_T + t];
+#pragma unroll
+        for (int i = 0; i < NO; ++i)
+            A.o[i] = make_double2(sy[(slot * NN + N + 2 * i) * WL_T + t], sy[(slot * NN + N + 2 * i + 1) * WL_T + t]);
+    };
+    load_pairs(P, N, -1, htab);
+    load_pairs(P, N, 0, jtab);
+    load_pairs(P, N, 1, jtab + 2 * NU * np);
+    double kv[3], wk;
+    kpoint(P, kc, kv, wk);
+    if (!live) wk = 0.0;
+    for (int q = 0; q < np; ++q) {
+        const int r = P.gpair[q];
+        double sn, cs;
+        sincos(kv[0] * P.V[2 * r] + kv[1] * P.V[2 * r + 1], &sn, &cs);
+        pk[q * WL_T + t] = make_double2(cs, sn);
+    }
+    double2 *rho = P.rho[0] + (size_t)kc * NN;
+    {
+        HN Y;
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            Y.d[m] = rho[m * N + m].x;
+#pragma unroll
+            for (int n = m + 1; n < N; ++n) Y.o[oidx(m, n, N)] = rho[m * N + n];
+        }
+        put(0, Y);
+    }
+    const double g1 = P.g1, g2 = P.g2, gd = g1 - g2;
+    const int ce = (P.nval * N + P.nval + 1) % NN;   // antelope.cpp:539-542
+    const int nw = P.step_rows;
+    double *part = P.step_part + (size_t)((k0 + t) >> 5) * WAN_NSLOT + (lane >> 1);
+    const bool wr = (lane & 1) == 0;
+    // the step's phase factors go to shared memory; the next step's first 64
+    // are on their way in registers meanwhile
+    const double2 *cg = P.step_cA;
+    double2 pre[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) pre[x] = t + x * WL_T < ncA ? cg[t + x * WL_T] : make_double2(0.0, 0.0);
+
+    for (int j = 0; j < steps; ++j, cg += ncA) {
+        __syncwarp();
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (t + x * WL_T < ncA) cA[t + x * WL_T] = pre[x];
+        for (int i = t + 2 * WL_T; i < ncA; i += WL_T) cA[i] = cg[i];
+        __syncwarp();
+        if (j + 1 < steps)
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+                if (t + x * WL_T < ncA) pre[x] = cg[ncA + t + x * WL_T];
+        const double h = step_length(P, n0 + j);
+        HN H;
+#pragma unroll 1
+        for (int s = 0; s < TB::S; ++s) {
+            const int ti = RK == 4 ? (s + 1) / 2 : s;
+            double z[4];   // current sums of the step's start
+            HN Y, K;
+            get(0, Y);
+            for (int q = RK == 4 ? max(0, s - 1) : 0; q < s; ++q) {
+                const double a = h * c_step_a[RK - 4][s][q];
+                get(2 + (RK == 4 ? 0 : q), K);
+                axpy<N>(Y, a, K);
+            }
+            HN X[2];
+            if (s == 0) {   // with the currents' operators (Hermitian parts)
+                clear<N>(H);
+                clear<N>(X[0]);
+                clear<N>(X[1]);
+#pragma unroll 1
+                for (int q = 0; q < np; ++q) {
+                    const double2 e = cmul(pk[q * WL_T + t], cA[q]);
+                    add_pair<N>(H, htab + q * 2 * NU, e);
+                    add_pair<N>(X[0], jtab + q * 2 * NU, e);
+                    add_pair<N>(X[1], jtab + (np + q) * 2 * NU, e);
+                }
+            } else if (!(RK == 4 && s == 2)) {   // RK4's midpoint stages share H0
+                clear<N>(H);
+#pragma unroll 2
+                for (int q = 0; q < np; ++q) add_pair<N>(H, htab + q * 2 * NU, cmul(pk[q * WL_T + t], cA[ti * np + q]));
+            }
+            {
+                HN A = H;
+                band_diagonal<N>(K, A, Y);   // K = D(Y)
+            }
+            if (s == 0) {   // currents at k + A(t_n) (SBEs.h:694-760): intraband Re Tr(D J), the rest interband
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    z[2 + a] = tr2<N>(K, X[a]);
+                    z[a] = tr2<N>(Y, X[a]) - z[2 + a];
+                }
+                double v[16];
+#pragma unroll
+                for (int q = 0; q < 16; ++q) v[q] = q < 4 ? wk * z[q] : 0.0;
+#pragma unroll
+                for (int m = 0; m < N; ++m) v[4 + m] = wk * Y.d[m];
+#pragma unroll
+                for (int e = 0; e < NN; ++e)
+                    if (e == ce) {
+                        const int m = e / N, n = e % N;
+                        const double2 y = m == n ? make_double2(Y.d[m], 0.0) : el<N>(Y, m, n);
+                        v[4 + N] = wk * y.x;
+                        v[5 + N] = wk * y.y;
+                    }
+                const double sum = warp_sum16(v, lane);
+                if (wr) part[(size_t)j * nw * WAN_NSLOT] = sum;
+            }
+            // -i((HY) - (HY)^dag) - (g2 Y + (g1 - g2) D)   (SBEs.h:808-861)
+            const double b = h * c_step_b[RK - 4][s];
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                double im = 0.0;   // Im (HY)_mm
+#pragma unroll
+                for (int l = 0; l < N; ++l) {
+                    if (l == m) continue;
+                    const double2 x = el<N>(H, m, l), y = el<N>(Y, l, m);
+                    im = fma(x.x, y.y, fma(x.y, y.x, im));
+                }
+                K.d[m] = fma(-gd, K.d[m], fma(-g2, Y.d[m], 2.0 * im));
+            }
+#pragma unroll
+            for (int m = 0; m < N; ++m)
+#pragma unroll
+                for (int n = m + 1; n < N; ++n) {
+                    const int o = oidx(m, n, N);
+                    const double2 w = Y.o[o], x = H.o[o];
+                    // c = (HY)_mn - conj (HY)_nm
+                    const double hd = H.d[m] - H.d[n], yd = Y.d[n] - Y.d[m];
+                    double2 c = make_double2(fma(hd, w.x, x.x * yd), fma(hd, w.y, x.y * yd));
+#pragma unroll
+                    for (int l = 0; l < N; ++l) {
+                        if (l == m || l == n) continue;
+                        cfma(c, el<N>(H, m, l), el<N>(Y, l, n));
+                        const double2 p = el<N>(Y, m, l), q = el<N>(H, l, n);   // - Y_ml H_ln
+                        c.x = fma(-p.x, q.x, fma(p.y, q.y, c.x));
+                        c.y = fma(-p.x, q.y, fma(-p.y, q.x, c.y));
+                    }
+                    K.o[o] = make_double2(fma(-gd, K.o[o].x, fma(-g2, w.x, c.y)), fma(-gd, K.o[o].y, fma(-g2, w.y, -c.x)));
+                }
+            if (RK == 4 || s < NK) put(2 + (RK == 4 ? 0 : s), K);
+            if (s > 0) get(1, Y);
+            else clear<N>(Y);
+            axpy<N>(Y, b, K);   // the increment
+            if (s + 1 < TB::S) {
+                put(1, Y);
+            } else {
+                get(0, K);
+                axpy<N>(K, 1.0, Y);
+                put(0, K);
+            }
+        }
+    }
+    if (!live) return;
+    HN Y;
+    get(0, Y);
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+        rho[m * N + m] = make_double2(Y.d[m], 0.0);
+#pragma unroll
+        for (int n = m + 1; n < N; ++n) {
+            rho[m * N + n] = Y.o[oidx(m, n, N)];
+            rho[n * N + m] = cconj(Y.o[oidx(m, n, N)]);
+        }
+    }
+}
+
 // Block (j, solve): the sums of the launch's step j over the solve's partial
 // rows (fixed order).  The solve's last block to finish moves its controller
 // past the launch's steps; every block has read it by then.
@@ -498,6 +908,7 @@ __global__ void __launch_bounds__(256) wan_finish(const WanDev *__restrict__ Pp,
             P.jout[(size_t)(n0 + j) * WAN_NSLOT + t] = s;
         }
     }
+    launch_phases(P, n0 + steps, j);   // of the next launch
     __syncthreads();
     if (t == 0) {
         __threadfence();
@@ -521,30 +932,52 @@ __global__ void __launch_bounds__(256) wan_finish(const WanDev *__restrict__ Pp,
 }
 
 // ============================================================= launchers
-// One thread per k-point (1) while a k-point's matrices fit a thread's
-// registers without spilling (N <= 3), else one row per lane (2); both sides
-// measured at the head of this file.
+// Velocity gauge: one thread per k-point while a k-point's matrices fit a
+// thread's registers without spilling (N <= 3), else one row per lane; both
+// sides measured at the head of this file.  Length gauge: the plain method on
+// models with current-operator tables, N <= 4.  The mixed method keeps the
+// FP32 Fourier sums and the tolerances of wan_attempt; more bands and dipole
+// tables stay with it and with wan_attempt_g, and so do solves with bands that
+// meet at a grid point (to 1e-7 of their spread): what the dephasing does
+// inside such a pair depends on its basis, which only a tracked eigenbasis
+// carries along.
+enum StepMode : int { VG_THREAD = 1, VG_ROWS = 2, LW_THREAD = 3 };
+static int row_lanes(int N) { return N <= 4 ? 4 : 8; }
+// dynamic shared memory of a block
+static int steps_bytes(int mode, int N, int na, int rk, int npair)
+{
+    if (mode == VG_THREAD) return (na * N * N + N) * WS_T * 16;
+    return mode == LW_THREAD ? lw_bytes(N, rk, npair) : 0;
+}
+constexpr int STEPS_MAX_BYTES = 96 * 1024;   // at least two blocks per SM
 int wan_steps(const WanDev &w)
 {
-    if (!w.vg || (w.rk != 4 && w.rk != 5) || w.N < 2 || w.N > WAN_MAXN) return 0;
-    return w.N <= 3 ? 1 : 2;
+    if ((w.rk != 4 && w.rk != 5) || w.N < 2 || w.N > WAN_MAXN) return 0;
+    if (w.vg) return w.N <= 3 ? VG_THREAD : VG_ROWS;
+    if (w.mixed || !w.has_jtab || w.has_dip || w.cont || w.N > 4 || w.degenerate) return 0;
+    return steps_bytes(LW_THREAD, w.N, 2, w.rk, w.nR) <= STEPS_MAX_BYTES ? LW_THREAD : 0;
 }
-static int row_lanes(int N) { return N <= 4 ? 4 : 8; }
+static int block_threads(int mode) { return mode == VG_ROWS ? WR_T : mode == LW_THREAD ? WL_T : WS_T; }
 int wan_steps_rows(const WanDev &w)
 {
-    const int kw = wan_steps(w) == 2 ? 32 / row_lanes(w.N) : 32;
+    const int kw = wan_steps(w) == VG_ROWS ? 32 / row_lanes(w.N) : 32;
     return (w.nk + kw - 1) / kw;
 }
 int wan_steps_fields(int rk) { return rk == 4 ? StepTab<4>::NT : StepTab<5>::NT; }
-int wan_steps_unit(int mode, int N) { return (mode == 2 ? WR_T / row_lanes(N) : WS_T) / WAN_WARPS; }
+int wan_steps_unit(int mode, int N)
+{
+    return block_threads(mode) / (mode == VG_ROWS ? row_lanes(N) : 1) / WAN_WARPS;
+}
 
 using StepKernel = void (*)(const WanDev *, const WanDev *const *, const WanTileRef *, int);
-template <int RK> static StepKernel vg_steps_n(int mode, int N, int na)
+template <int RK> static StepKernel steps_kernel(int mode, int N, int na)
 {
-    if (mode == 1) {
+    if (mode == VG_THREAD) {
         if (N == 2) return na == 3 ? wan_vg_steps<2, RK, 3> : wan_vg_steps<2, RK, 2>;   // 3: the continuum model
         return N == 3 ? wan_vg_steps<3, RK, 2> : nullptr;
     }
+    if (mode == LW_THREAD)
+        return N == 2 ? wan_lw_steps<2, RK> : N == 3 ? wan_lw_steps<3, RK> : N == 4 ? wan_lw_steps<4, RK> : nullptr;
     switch (N) {
     case 4: return wan_vg_rows<4, RK>;
     case 5: return wan_vg_rows<5, RK>;
@@ -555,14 +988,29 @@ template <int RK> static StepKernel vg_steps_n(int mode, int N, int na)
     }
 }
 
-cudaError_t launch_wan_steps(int mode, int N, int na, int rk, const WanDev *dw, const WanDev *const *descs,
+cudaError_t launch_wan_steps(const WanStepClass &c, const WanDev *dw, const WanDev *const *descs,
                              const WanTileRef *tiles, int nblocks, int S, cudaStream_t st)
 {
-    const StepKernel f = rk == 4 ? vg_steps_n<4>(mode, N, na) : rk == 5 ? vg_steps_n<5>(mode, N, na) : nullptr;
+    const StepKernel f = c.rk == 4 ? steps_kernel<4>(c.mode, c.N, c.na)
+                                   : c.rk == 5 ? steps_kernel<5>(c.mode, c.N, c.na) : nullptr;
     if (!f) return cudaErrorInvalidValue;
-    const int sm = mode == 1 ? (na * N * N + N) * WS_T * 16 : 0;   // at most 21 KB
-    f<<<nblocks, mode == 1 ? WS_T : WR_T, sm, st>>>(dw, descs, tiles, S);
+    const int sm = steps_bytes(c.mode, c.N, c.na, c.rk, c.npair);
+    if (sm > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, STEPS_MAX_BYTES);
+        if (e != cudaSuccess) return e;
+    }
+    f<<<nblocks, block_threads(c.mode), sm, st>>>(dw, descs, tiles, S);
     return cudaGetLastError();
+}
+WanStepClass wan_step_class(const WanDev &w)
+{
+    WanStepClass c;
+    c.mode = wan_steps(w);
+    c.N = w.N;
+    c.na = w.cont ? 3 : 2;
+    c.rk = w.rk;
+    c.npair = c.mode == LW_THREAD ? w.npair : 0;
+    return c;
 }
 
 cudaError_t launch_wan_finish(const WanDev *dw, const WanDev *const *descs, int nsolves, int S, cudaStream_t st)
@@ -575,6 +1023,7 @@ cudaError_t launch_wan_step_fields(const WanDev &w, const WanDev *dw, cudaStream
 {
     const int nt = wan_steps_fields(w.rk);
     wan_step_fields<<<(w.Nt * nt + 127) / 128, 128, 0, st>>>(dw, nt, w.rk);
+    if (w.step_cA) wan_step_phases<<<WAN_STEPS, 256, 0, st>>>(dw);
     return cudaGetLastError();
 }
 
