@@ -164,5 +164,61 @@ __device__ void kpoint(const WanDev &P, int kl, double kv[3], double &wt)
         kv[dd] = P.origin[dd] + f[0] * P.axes[0 * 3 + dd] + f[1] * P.axes[1 * 3 + dd] + f[2] * P.axes[2 * 3 + dd];
 }
 
+// Accept or reject an attempt of error emax and set up the next one.  The
+// step-size rule is the oracle's (oracle/sbe_oracle.c, run_adaptive).
+__device__ void control_decide(const WanDev &P, WanCtl *ctl, double emax)
+{
+    ctl->attempts++;
+    ctl->need_current = 0;
+    ctl->shot = -1;
+    ctl->emax = emax;
+    const double dt = P.dt, tend = P.atmin + dt * (ctl->n + 1);
+    bool accept = true;
+    if (P.rk == 45) {
+        if (emax <= P.tol) {
+            double fac = emax > 0 ? 0.9 * pow(P.tol / emax, 0.2) : 5.0;
+            if (fac > 5.0) fac = 5.0;
+            if (!ctl->last || fac < 1.0) ctl->h = ctl->hs * (fac < 0.2 ? 0.2 : fac);
+            if (ctl->h > dt) ctl->h = dt;
+        } else {
+            accept = false;
+            double fac = 0.9 * pow(P.tol / emax, 0.25);
+            ctl->h = ctl->hs * (fac < 0.1 ? 0.1 : fac);
+            ctl->rejects++;
+            if (!(ctl->h > 1e-12 * dt)) {
+                ctl->error = 1;
+                ctl->done = 1;
+                return;
+            }
+        }
+    }
+    if (accept) {
+        ctl->buf ^= 1;
+        ctl->steps++;
+        if (ctl->last) {
+            ctl->tc = tend;
+            // the state is now past interval n: its snapshot (after step n,
+            // antelope.cpp:342) is due when n is a multiple of the interval
+            if (P.shot_every > 0 && ctl->n % P.shot_every == 0) ctl->shot = ctl->n;
+            ctl->n++;
+            if (ctl->n >= P.Nt) {
+                ctl->done = 1;
+                return;
+            }
+            ctl->need_current = 1;
+        } else {
+            ctl->tc = ctl->tc + ctl->hs;
+        }
+    }
+    // next attempt
+    const double tend2 = P.atmin + dt * (ctl->n + 1);
+    ctl->hs = ctl->h;
+    ctl->last = 0;
+    if (ctl->tc + ctl->hs >= tend2 - 1e-12 * dt) {
+        ctl->hs = tend2 - ctl->tc;
+        ctl->last = 1;
+    }
+}
+
 }  // namespace
 }  // namespace sbe

@@ -1184,63 +1184,8 @@ template <class RF> __global__ void __launch_bounds__(256) wan_prepare(const Wan
 
 // ============================================================= control
 // One block: reduce the attempt's tile results (fixed order), record the
-// currents, accept or reject, and prepare the next attempt (its step, stage
-// fields and phase factors).  The step-size rule is the oracle's
-// (oracle/sbe_oracle.c, run_adaptive).
-__device__ void control_decide(const WanDev &P, WanCtl *ctl, double emax)
-{
-    ctl->attempts++;
-    ctl->need_current = 0;
-    ctl->shot = -1;
-    ctl->emax = emax;
-    const double dt = P.dt, tend = P.atmin + dt * (ctl->n + 1);
-    bool accept = true;
-    if (P.rk == 45) {
-        if (emax <= P.tol) {
-            double fac = emax > 0 ? 0.9 * pow(P.tol / emax, 0.2) : 5.0;
-            if (fac > 5.0) fac = 5.0;
-            if (!ctl->last || fac < 1.0) ctl->h = ctl->hs * (fac < 0.2 ? 0.2 : fac);
-            if (ctl->h > dt) ctl->h = dt;
-        } else {
-            accept = false;
-            double fac = 0.9 * pow(P.tol / emax, 0.25);
-            ctl->h = ctl->hs * (fac < 0.1 ? 0.1 : fac);
-            ctl->rejects++;
-            if (!(ctl->h > 1e-12 * dt)) {
-                ctl->error = 1;
-                ctl->done = 1;
-                return;
-            }
-        }
-    }
-    if (accept) {
-        ctl->buf ^= 1;
-        ctl->steps++;
-        if (ctl->last) {
-            ctl->tc = tend;
-            // the state is now past interval n: its snapshot (after step n,
-            // antelope.cpp:342) is due when n is a multiple of the interval
-            if (P.shot_every > 0 && ctl->n % P.shot_every == 0) ctl->shot = ctl->n;
-            ctl->n++;
-            if (ctl->n >= P.Nt) {
-                ctl->done = 1;
-                return;
-            }
-            ctl->need_current = 1;
-        } else {
-            ctl->tc = ctl->tc + ctl->hs;
-        }
-    }
-    // next attempt
-    const double tend2 = P.atmin + dt * (ctl->n + 1);
-    ctl->hs = ctl->h;
-    ctl->last = 0;
-    if (ctl->tc + ctl->hs >= tend2 - 1e-12 * dt) {
-        ctl->hs = tend2 - ctl->tc;
-        ctl->last = 1;
-    }
-}
-
+// currents, accept or reject (control_decide), and prepare the next attempt
+// (its step, stage fields and phase factors).
 template <class RF>
 __global__ void __launch_bounds__(1024) wan_control(const WanDev *__restrict__ Pp, const WanDev *const *__restrict__ descs)
 {
@@ -1482,8 +1427,9 @@ cudaError_t launch_wan_init(const WanDev &w, int precision, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_wan_prepare(const WanDev *dw, int precision, cudaStream_t st)
+cudaError_t launch_wan_prepare(const WanDev &w, const WanDev *dw, int precision, cudaStream_t st)
 {
+    if (wan_proj(w)) return launch_wan_next(w.N, dw, nullptr, 1, w.gr_rows * (w.rk == 4 ? 4 : 6), true, st);
     if (precision == 0) wan_prepare<double><<<1, 256, 0, st>>>(dw);
     else wan_prepare<float><<<1, 256, 0, st>>>(dw);
     return cudaGetLastError();
@@ -1537,6 +1483,10 @@ static cudaError_t launch_grouped(int N, int nR, int rk, const WanDev *dw, const
 
 cudaError_t launch_wan_attempt(const WanDev &w, const WanDev *dw, int precision, cudaStream_t st)
 {
+    if (wan_proj(w)) {
+        const int unit = wan_proj_unit(w.N);
+        return launch_wan_attempt_p(w.N, w.gr_n, dw, nullptr, nullptr, (w.ntiles + unit - 1) / unit, st);
+    }
     if (wan_grouped(w))
         return launch_grouped(w.N, w.nR, w.rk, dw, nullptr, nullptr, (w.ntiles + WG_WARPS - 1) / WG_WARPS,
                               precision, st);
@@ -1590,8 +1540,9 @@ cudaError_t launch_wan_snapshot_batch(int N, int nR_max, const WanDev *const *de
     return cudaGetLastError();
 }
 
-cudaError_t launch_wan_control(const WanDev *dw, int precision, cudaStream_t st)
+cudaError_t launch_wan_control(const WanDev &w, const WanDev *dw, int precision, cudaStream_t st)
 {
+    if (wan_proj(w)) return launch_wan_next(w.N, dw, nullptr, 1, w.gr_rows * (w.rk == 4 ? 4 : 6), false, st);
     if (precision == 0) wan_control<double><<<1, 1024, 0, st>>>(dw, nullptr);
     else wan_control<float><<<1, 1024, 0, st>>>(dw, nullptr);
     return cudaGetLastError();

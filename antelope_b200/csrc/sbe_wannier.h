@@ -110,7 +110,17 @@ struct WanDev {
     // length gauge: bits of the smallest gap between two bands and of the
     // largest spread of the bands over the grid (wan_init), or null
     unsigned long long *band_gap;
-    int degenerate;   // bands meet at a grid point: wan_steps does not apply
+    int degenerate;   // bands meet at a grid point: neither wan_steps nor wan_proj applies
+    // projection attempt kernel (wan_proj): the grid's rows along its fast axis
+    // (axis gr_fast, gr_nf points; the solve's rows start at gr_row0), the
+    // groups of vectors R with equal b.R = +-gr_a (b the fast axis; gr_n of
+    // them, 0 first; lists gr_idx[gr_off[2g] ...] at +, [gr_off[2g + 1] ...] at
+    // -), the row tables of the next attempt and the attempt's largest error
+    int gr_fast, gr_nf, gr_row0, gr_rows, gr_n;
+    const double *gr_a;
+    const int *gr_off, *gr_idx;
+    double2 *gr_tab, *gr_cur;
+    unsigned long long *gr_err;   // bits
 };
 
 // A tile of a batched launch: tile `tile` (WAN_WARPS k-points) of solve
@@ -150,9 +160,9 @@ int wan_gtab_row(int N);
 // but for R = 0)
 int wan_npair_cap(int nR);
 cudaError_t launch_wan_init(const WanDev &w, int precision, cudaStream_t st);
-cudaError_t launch_wan_prepare(const WanDev *dw, int precision, cudaStream_t st);
+cudaError_t launch_wan_prepare(const WanDev &w, const WanDev *dw, int precision, cudaStream_t st);
 cudaError_t launch_wan_attempt(const WanDev &w, const WanDev *dw, int precision, cudaStream_t st);
-cudaError_t launch_wan_control(const WanDev *dw, int precision, cudaStream_t st);
+cudaError_t launch_wan_control(const WanDev &w, const WanDev *dw, int precision, cudaStream_t st);
 // the snapshot of the interval the last control step completed, if one is due
 cudaError_t launch_wan_snapshot(const WanDev &w, const WanDev *dw, int precision, cudaStream_t st);
 // Batched forms: `descs` [nsolves] device pointers to the solves' descriptors,
@@ -187,6 +197,19 @@ cudaError_t launch_wan_steps(const WanStepClass &c, const WanDev *dw, const WanD
                              const WanTileRef *tiles, int nblocks, int S, cudaStream_t st);
 cudaError_t launch_wan_finish(const WanDev *dw, const WanDev *const *descs, int nsolves, int S, cudaStream_t st);
 cudaError_t launch_wan_step_fields(const WanDev &w, const WanDev *dw, cudaStream_t st);
+// Projection attempts (sbe_wanproj.cu): the plain method of the length gauge on
+// explicit tables at N = 3 ... 6, on grids where no bands meet.  A block covers
+// wan_proj_unit() tiles; solves of a class (equal N) share launches, ngrp and
+// nitems (rows x stages) being the largest of them.
+constexpr int WAN_PROJ_MAXGRP = 64;
+bool wan_proj_applies(const WanDev &w);   // before its tables exist
+bool wan_proj(const WanDev &w);
+int wan_proj_unit(int N);
+int wan_proj_entries(int N, int ngrp, int nq);
+cudaError_t launch_wan_attempt_p(int N, int ngrp, const WanDev *dw, const WanDev *const *descs, const WanTileRef *tiles,
+                                 int nblocks, cudaStream_t st);
+cudaError_t launch_wan_next(int N, const WanDev *dw, const WanDev *const *descs, int nsolves, int nitems, bool first,
+                            cudaStream_t st);
 cudaError_t launch_wan_snapshot_batch(int N, int nR_max, const WanDev *const *descs, const WanTileRef *tiles,
                                       int ntiles, int precision, cudaStream_t st);
 

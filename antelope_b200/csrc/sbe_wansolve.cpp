@@ -95,7 +95,39 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
         dalloc(&w_.snap_nc, sizeof(double) * nshots_ * nk, st, "alloc snapshots");
         dalloc(&w_.snap_pi, sizeof(double) * 2 * nshots_ * nk, st, "alloc snapshots");
     }
+    dalloc(&d_w_, sizeof(WanDev), st, "alloc descriptor");
+    w_.V = V;
+    w_.h = h;
+    w_.d = d;
+    w_.jt = j;
     w_.mixed = precision_ != 0;
+    UploadRing &ring = UploadRing::shared();
+    if (!p.w_vec.empty()) ring.upload(V, p.w_vec.data(), sizeof(double) * p.w_vec.size(), st);
+    auto up_real = [&](void *dst, const std::vector<double> &src) {
+        if (precision_ == 0) {
+            ring.upload(dst, src.data(), src.size() * 8, st);
+        } else {
+            std::vector<float> f(src.begin(), src.end());
+            ring.upload(dst, f.data(), f.size() * 4, st);
+        }
+    };
+    if (!p.w_h.empty()) up_real(h, p.w_h);
+    if (w_.has_dip) up_real(d, p.w_d);
+    if (w_.has_jtab && !w_.cont) up_real(j, p.w_j);
+    // the projections of the length gauge need bands that do not meet on the grid
+    const bool lw_new = !w_.vg && (wan_steps(w_) != 0 || wan_proj_applies(w_));
+    if (lw_new) {
+        dalloc(&w_.band_gap, 16, st, "alloc band gap");
+        cuda_check(cudaMemsetAsync(w_.band_gap, 0x7f, 8, st), "clear band gap");   // a large double
+        cuda_check(cudaMemsetAsync(w_.band_gap + 1, 0, 8, st), "clear band gap");
+    }
+    cuda_check(launch_wan_init(w_, precision_, st), "Wannier init kernel");
+    if (lw_new) {
+        double gw[2];
+        cuda_check(cudaMemcpyAsync(gw, w_.band_gap, 16, cudaMemcpyDeviceToHost, st), "copy band gap");
+        cuda_check(cudaStreamSynchronize(st), "sync");
+        w_.degenerate = !(gw[0] > 1e-7 * gw[1]);
+    }
     if (wan_steps(w_)) {
         w_.step_rows = wan_steps_rows(w_);
         dalloc(&w_.step_fld, sizeof(double) * (size_t)w_.Nt * wan_steps_fields(w_.rk) * 3, st, "alloc step fields");
@@ -108,11 +140,7 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
         dalloc(&w_.step_ticket, sizeof(unsigned), st, "alloc step counter");
         cuda_check(cudaMemsetAsync(w_.step_ticket, 0, sizeof(unsigned), st), "clear step counter");
     }
-    dalloc(&d_w_, sizeof(WanDev), st, "alloc descriptor");
-    w_.V = V;
-    w_.h = h;
-    w_.d = d;
-    w_.jt = j;
+    if (wan_proj_applies(w_)) setup_rows(p, st);
     // the tables re-laid for the grouped attempt kernel.  The lattice vectors
     // are taken in pairs (R, -R) (a vector without its negative, R = 0
     // included, stands alone): h_R e^{iKR} + h_-R e^{-iKR} = c sig + s tau
@@ -123,7 +151,7 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     std::vector<double> gt;
     std::vector<int> gpair, mate(w_.nR, -1);
     const bool lw_steps = !w_.vg && wan_steps(w_) != 0;
-    if (wan_grouped_applies(w_) || lw_steps) {
+    if ((wan_grouped_applies(w_) && !wan_proj(w_)) || lw_steps) {
         const int nR = w_.nR;
         std::vector<char> used(nR, 0);
         for (int r = 0; r < nR; ++r) {
@@ -151,9 +179,6 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
         w_.gpair = gp;
         w_.gmate = gm;
         w_.npair = (int)gpair.size();
-        dalloc(&w_.band_gap, 16, st, "alloc band gap");
-        cuda_check(cudaMemsetAsync(w_.band_gap, 0x7f, 8, st), "clear band gap");   // a large double
-        cuda_check(cudaMemsetAsync(w_.band_gap + 1, 0, 8, st), "clear band gap");
         dalloc(&w_.step_cA, sizeof(double2) * WAN_STEPS * (size_t)wan_steps_fields(w_.rk) * w_.npair, st,
                "alloc step phases");
     } else if (!gpair.empty()) {
@@ -198,19 +223,6 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
             w_.stage_gt = sg;
         }
     }
-    UploadRing &ring = UploadRing::shared();
-    if (!p.w_vec.empty()) ring.upload(V, p.w_vec.data(), sizeof(double) * p.w_vec.size(), st);
-    auto up_real = [&](void *dst, const std::vector<double> &src) {
-        if (precision_ == 0) {
-            ring.upload(dst, src.data(), src.size() * 8, st);
-        } else {
-            std::vector<float> f(src.begin(), src.end());
-            ring.upload(dst, f.data(), f.size() * 4, st);
-        }
-    };
-    if (!p.w_h.empty()) up_real(h, p.w_h);
-    if (w_.has_dip) up_real(d, p.w_d);
-    if (w_.has_jtab && !w_.cont) up_real(j, p.w_j);
     if (w_.gtab) up_real(const_cast<void *>(w_.gtab), gt);
     if (w_.gpair) ring.upload(const_cast<int *>(w_.gpair), gpair.data(), sizeof(int) * gpair.size(), st);
     if (w_.gmate) ring.upload(const_cast<int *>(w_.gmate), gmate.data(), sizeof(int) * gmate.size(), st);
@@ -232,16 +244,68 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     }
     ring.upload(w_.ctl, &c, sizeof(c), st);
     ring.upload(d_w_, &w_, sizeof(w_), st);
-    cuda_check(launch_wan_init(w_, precision_, st), "Wannier init kernel");
-    if (w_.band_gap) {   // bands that meet on the grid rule the many-step kernels out
-        double gw[2];
-        cuda_check(cudaMemcpyAsync(gw, w_.band_gap, 16, cudaMemcpyDeviceToHost, st), "copy band gap");
-        cuda_check(cudaStreamSynchronize(st), "sync");
-        w_.degenerate = !(gw[0] > 1e-7 * gw[1]);
-    }
     if (wan_steps(w_)) cuda_check(launch_wan_step_fields(w_, d_w_, st), "Wannier step fields");
-    else cuda_check(launch_wan_prepare(d_w_, precision_, st), "Wannier stage preparation");
+    else cuda_check(launch_wan_prepare(w_, d_w_, precision_, st), "Wannier stage preparation");
     cuda_check(cudaMallocHost(&h_ctl_, sizeof(WanCtl)), "cudaMallocHost(control)");
+}
+
+// The groups of lattice vectors that share their phase along the grid's rows,
+// and the row tables of the projection attempt kernel.  Left undone (the
+// other attempt kernels run the solve) where the tables would pass 1 GiB: grids
+// of very many short rows.
+void WannierSolve::setup_rows(const Problem &p, cudaStream_t st)
+{
+    const int nR = w_.nR, N = w_.N, fast = w_.Ngrid[1] > 1 ? 1 : 0;
+    std::vector<double> b(nR);
+    double bmax = 0.0;
+    for (int r = 0; r < nR; ++r) {
+        b[r] = p.bzaxes[3 * fast] * p.w_vec[2 * r] + p.bzaxes[3 * fast + 1] * p.w_vec[2 * r + 1];
+        bmax = std::max(bmax, std::fabs(b[r]));
+    }
+    const double tol = 1e-10 * bmax;   // the rounding of b.R
+    std::vector<double> ga{0.0};
+    std::vector<std::vector<int>> lists(2);
+    for (int r = 0; r < nR; ++r) {
+        int g = 0;
+        while (g < (int)ga.size() && std::fabs(ga[g] - std::fabs(b[r])) > tol) ++g;
+        if (g == (int)ga.size()) {
+            ga.push_back(std::fabs(b[r]));
+            lists.resize(2 * ga.size());
+        }
+        lists[2 * g + (g > 0 && b[r] < 0.0 ? 1 : 0)].push_back(r);
+    }
+    const int ng = (int)ga.size(), nq = w_.has_dip ? 2 : 1;
+    w_.gr_fast = fast;
+    w_.gr_nf = w_.Ngrid[fast];
+    w_.gr_row0 = w_.k_offset / w_.gr_nf;
+    w_.gr_rows = (w_.k_offset + w_.nk - 1) / w_.gr_nf - w_.gr_row0 + 1;
+    w_.gr_n = ng;
+    const int S = w_.rk == 4 ? 4 : 6;
+    const size_t nt = (size_t)w_.gr_rows * S * wan_proj_entries(N, ng, nq), nc = (size_t)w_.gr_rows * wan_proj_entries(N, ng, 2 * nq);
+    if (ng > WAN_PROJ_MAXGRP || (nt + nc) * 16 > ((size_t)1 << 30)) return;
+    std::vector<int> off{0}, idx;
+    for (const auto &l : lists) {
+        idx.insert(idx.end(), l.begin(), l.end());
+        off.push_back((int)idx.size());
+    }
+    double *a = nullptr;
+    int *o = nullptr, *i = nullptr;
+    dalloc(&a, sizeof(double) * ng, st, "alloc vector groups");
+    dalloc(&o, sizeof(int) * off.size(), st, "alloc vector groups");
+    dalloc(&i, sizeof(int) * idx.size(), st, "alloc vector groups");
+    w_.gr_a = a;
+    w_.gr_off = o;
+    w_.gr_idx = i;
+    dalloc(&w_.gr_tab, 16 * nt, st, "alloc row tables");
+    dalloc(&w_.gr_cur, 16 * nc, st, "alloc row tables");
+    dalloc(&w_.gr_err, 8, st, "alloc attempt error");
+    dalloc(&w_.step_ticket, sizeof(unsigned), st, "alloc step counter");
+    cuda_check(cudaMemsetAsync(w_.gr_err, 0, 8, st), "clear attempt error");
+    cuda_check(cudaMemsetAsync(w_.step_ticket, 0, sizeof(unsigned), st), "clear step counter");
+    UploadRing &ring = UploadRing::shared();
+    ring.upload(a, ga.data(), sizeof(double) * ng, st);
+    ring.upload(o, off.data(), sizeof(int) * off.size(), st);
+    ring.upload(i, idx.data(), sizeof(int) * idx.size(), st);
 }
 
 WannierSolve::~WannierSolve()
@@ -274,6 +338,12 @@ WannierSolve::~WannierSolve()
     if (w_.step_cA) cudaFreeAsync(w_.step_cA, stream_);
     if (w_.gmate) cudaFreeAsync((void *)w_.gmate, stream_);
     if (w_.band_gap) cudaFreeAsync(w_.band_gap, stream_);
+    if (w_.gr_a) cudaFreeAsync((void *)w_.gr_a, stream_);
+    if (w_.gr_off) cudaFreeAsync((void *)w_.gr_off, stream_);
+    if (w_.gr_idx) cudaFreeAsync((void *)w_.gr_idx, stream_);
+    if (w_.gr_tab) cudaFreeAsync(w_.gr_tab, stream_);
+    if (w_.gr_cur) cudaFreeAsync(w_.gr_cur, stream_);
+    if (w_.gr_err) cudaFreeAsync(w_.gr_err, stream_);
     cudaFreeAsync(d_w_, stream_);
     if (w_.snap_nc) cudaFreeAsync(w_.snap_nc, stream_);
     if (w_.snap_pi) cudaFreeAsync(w_.snap_pi, stream_);
@@ -311,7 +381,7 @@ void WannierSolve::run(cudaStream_t st)
     for (;;) {
         for (int c = 0; c < chunk; ++c) {
             cuda_check(launch_wan_attempt(w_, d_w_, precision_, st), "Wannier attempt kernel");
-            cuda_check(launch_wan_control(d_w_, precision_, st), "Wannier control kernel");
+            cuda_check(launch_wan_control(w_, d_w_, precision_, st), "Wannier control kernel");
             cuda_check(launch_wan_snapshot(w_, d_w_, precision_, st), "Wannier snapshot kernel");
         }
         launched += chunk;
@@ -346,10 +416,11 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         const WanDev &w = solves_[i]->dev();
         const int grk = wan_grouped(w) ? w.rk : 0;
         const WanStepClass sc = wan_step_class(w);
+        const bool proj = wan_proj(w);
         Class *c = nullptr;
         for (Class &x : classes_)
             if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == solves_[i]->precision() && x.grouped_rk == grk &&
-                x.steps.same(sc))
+                x.steps.same(sc) && x.proj == proj)
                 c = &x;
         if (!c) {
             classes_.emplace_back();
@@ -359,10 +430,13 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
             c->precision = solves_[i]->precision();
             c->grouped_rk = grk;
             c->steps = sc;
+            c->proj = proj;
         }
         c->members.push_back(i);
         c->nR = std::max(c->nR, w.nR);
         c->steps.npair = std::max(c->steps.npair, sc.npair);
+        c->ngrp = std::max(c->ngrp, w.gr_n);
+        c->nitems = std::max(c->nitems, w.gr_rows * (w.rk == 4 ? 4 : 6));
         c->shots = c->shots || w.shot_every > 0;
     }
     UploadRing &ring = UploadRing::shared();
@@ -380,7 +454,7 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         // interleave the solves' tiles round-robin (longest first), so that
         // the blocks of one launch spread every solve over the whole GPU
         // (grouped classes: one entry per block of WAN_GROUP_TILES tiles)
-        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.proj ? wan_proj_unit(c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
         int maxt = 0;
         for (int m : c.members) maxt = std::max(maxt, solves_[m]->dev().ntiles);
         for (int t = 0; t < maxt; t += unit)
@@ -438,11 +512,18 @@ int WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
                 continue;
             }
             launched += c.shots ? 3 : 2;
-            cuda_check(launch_wan_attempt_batch(c.N, c.nR, c.vg, c.d_descs, c.d_tiles, c.ntiles, c.precision, st,
-                                                c.grouped_rk),
-                       "Wannier attempt kernel (batch)");
-            cuda_check(launch_wan_control_batch(c.d_descs, (int)c.members.size(), c.precision, st),
-                       "Wannier control kernel (batch)");
+            if (c.proj) {
+                cuda_check(launch_wan_attempt_p(c.N, c.ngrp, nullptr, c.d_descs, c.d_tiles, c.ntiles, st),
+                           "Wannier attempt kernel (batch)");
+                cuda_check(launch_wan_next(c.N, nullptr, c.d_descs, (int)c.members.size(), c.nitems, false, st),
+                           "Wannier control kernel (batch)");
+            } else {
+                cuda_check(launch_wan_attempt_batch(c.N, c.nR, c.vg, c.d_descs, c.d_tiles, c.ntiles, c.precision, st,
+                                                    c.grouped_rk),
+                           "Wannier attempt kernel (batch)");
+                cuda_check(launch_wan_control_batch(c.d_descs, (int)c.members.size(), c.precision, st),
+                           "Wannier control kernel (batch)");
+            }
             if (c.shots)
                 cuda_check(launch_wan_snapshot_batch(c.N, c.nR, c.d_descs, c.d_snap_tiles, c.nsnap_tiles, c.precision, st),
                            "Wannier snapshot kernel (batch)");
@@ -520,6 +601,9 @@ size_t WannierPool::bytes_needed(const Problem &p, int precision)
     b += nR * NN * cplx * 5 + nR * 16 + nR * 216 * cplx;               // h, d, current, re-laid and stage tables, vectors
     b += ntiles * 8 * (1 + WAN_NSLOT) + (size_t)p.laser.Nt * WAN_NSLOT * 8;   // tile results, per-step sums
     if (p.gauge == GAUGE_VELOCITY) b += nk * N * 16 + nk * 3 * NN * 16;  // bands, momentum matrices
+    // row tables of the projection attempts (at most a group per vector pair)
+    if (p.gauge != GAUGE_VELOCITY && precision == 0)
+        b += (size_t)p.Nk[0] * 10 * wan_proj_entries((int)std::max<size_t>(N, 2), (int)nR / 2 + 1, 2) * 16;
     if (p.rk != 45)   // step fields, phases and partials
         b += (size_t)WAN_STEPS * 6 * nR * cplx + (size_t)p.laser.Nt * 6 * 24 + (size_t)WAN_STEPS * (nk / 4 + 1) * WAN_NSLOT * 8;
     return b + 4096;
@@ -587,10 +671,11 @@ void WannierPool::rebuild()
         const WanDev &w = s.dev();
         const int grk = wan_grouped(w) ? w.rk : 0;
         const WanStepClass sc = wan_step_class(w);
+        const bool proj = wan_proj(w);
         Class *c = nullptr;
         for (Class &x : classes_)
             if (x.N == w.N && x.vg == (w.vg != 0) && x.precision == s.precision() && x.grouped_rk == grk &&
-                x.steps.same(sc))
+                x.steps.same(sc) && x.proj == proj)
                 c = &x;
         if (!c) {
             classes_.emplace_back();
@@ -600,16 +685,19 @@ void WannierPool::rebuild()
             c->precision = s.precision();
             c->grouped_rk = grk;
             c->steps = sc;
+            c->proj = proj;
         }
         c->ids.push_back(kv.first);
         c->nR = std::max(c->nR, w.nR);
         c->steps.npair = std::max(c->steps.npair, sc.npair);
+        c->ngrp = std::max(c->ngrp, w.gr_n);
+        c->nitems = std::max(c->nitems, w.gr_rows * (w.rk == 4 ? 4 : 6));
     }
     UploadRing &ring = UploadRing::shared();
     for (Class &c : classes_) {
         std::vector<const WanDev *> descs;
         std::vector<WanTileRef> tiles;
-        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.proj ? wan_proj_unit(c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
         int maxt = 0;
         for (int id : c.ids) {
             descs.push_back(solves_.at(id).s->dev_ptr());
@@ -645,11 +733,18 @@ void WannierPool::step(int iters)
                 last_launches_ += 2;
                 continue;
             }
-            cuda_check(launch_wan_attempt_batch(c.N, c.nR, c.vg, c.d_descs, c.d_tiles, c.ntiles, c.precision, st_,
-                                                c.grouped_rk),
-                       "Wannier attempt kernel (server)");
-            cuda_check(launch_wan_control_batch(c.d_descs, (int)c.ids.size(), c.precision, st_),
-                       "Wannier control kernel (server)");
+            if (c.proj) {
+                cuda_check(launch_wan_attempt_p(c.N, c.ngrp, nullptr, c.d_descs, c.d_tiles, c.ntiles, st_),
+                           "Wannier attempt kernel (server)");
+                cuda_check(launch_wan_next(c.N, nullptr, c.d_descs, (int)c.ids.size(), c.nitems, false, st_),
+                           "Wannier control kernel (server)");
+            } else {
+                cuda_check(launch_wan_attempt_batch(c.N, c.nR, c.vg, c.d_descs, c.d_tiles, c.ntiles, c.precision, st_,
+                                                    c.grouped_rk),
+                           "Wannier attempt kernel (server)");
+                cuda_check(launch_wan_control_batch(c.d_descs, (int)c.ids.size(), c.precision, st_),
+                           "Wannier control kernel (server)");
+            }
             last_launches_ += 2;
         }
     // controllers of the running solves, read by a later poll()

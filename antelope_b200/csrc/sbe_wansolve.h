@@ -40,6 +40,7 @@ public:
     void finish_batched(const WanCtl &c, int launches);
 
 private:
+    void setup_rows(const Problem &p, cudaStream_t st);
     Problem prob_;
     int precision_, device_, nshots_ = 0;
     cudaStream_t stream_;
@@ -73,6 +74,8 @@ private:
         int N = 0, nR = 0, precision = 0;
         int grouped_rk = 0;   // the grouped attempt kernel (and its RK order), or 0
         WanStepClass steps;   // the many-step kernels (mode 0: not)
+        bool proj = false;    // the projection attempts
+        int ngrp = 0, nitems = 0;
         bool vg = false, shots = false;
         std::vector<int> members;
         const WanDev **d_descs = nullptr;
@@ -131,6 +134,8 @@ private:
     struct Class {
         int N = 0, nR = 0, precision = 0, grouped_rk = 0;
         WanStepClass steps;
+        bool proj = false;
+        int ngrp = 0, nitems = 0;
         bool vg = false;
         std::vector<int> ids;
         const WanDev **d_descs = nullptr;
