@@ -254,7 +254,7 @@ sbe_status create_solver(const sbe_problem *p, const sbe_opts *opts, int kb, int
             const int prec = (opts && opts->precision >= 0) ? opts->precision : p->p.precision;
             s->wan = std::make_unique<WannierSolve>(p->p, prec, s->device, s->own, kb, ke);
         } else {
-            s->eng = std::make_unique<Engine>(s->device, s->own, default_steps(opts));
+            s->eng = std::make_unique<Engine>(s->device, s->own, default_steps(opts), 1);
             EngineOptions eo = to_engine_opts(opts);
             eo.k_begin = kb;
             eo.k_end = ke;
@@ -555,7 +555,7 @@ extern "C" sbe_status sbe_batch_create(const sbe_problem *const *problems, int n
         std::vector<int> order, wan_order;
         for (int i = 0; i < n; ++i) (problems[i]->p.model == MODEL_HALDANE ? order : wan_order).push_back(i);
         if (!order.empty()) {
-            b->eng = std::make_unique<Engine>(b->device, b->own, default_steps(opts));
+            b->eng = std::make_unique<Engine>(b->device, b->own, default_steps(opts), std::min((int)order.size(), 4096));
             // longest solves first: their tiles lead every launch's tile list
             std::stable_sort(order.begin(), order.end(), [&](int a, int c) {
                 return (double)problems[a]->p.laser.Nt * problems[a]->p.ntotal() >
@@ -595,6 +595,8 @@ extern "C" sbe_status sbe_batch_run(sbe_batch *b, void *stream)
             run_engine(*b->eng, b->use_graph, &b->launches);
             for (int id : b->ids)
                 if (id >= 0) b->eng->fetch_async(id);
+            // host work of sbe_batch_get done while the GPU propagates
+            if (!b->wan) b->eng->prepare_outputs();
         }
         if (b->wan) {
             b->wan->run(st, b->use_graph);

@@ -138,6 +138,7 @@ struct Engine::Solve {
     double *snap_nc = nullptr, *snap_pi = nullptr;  // density snapshots (or null)
     int nshots = 0, k_begin = 0;
     double *h_jout = nullptr, *h_const = nullptr;  // pinned
+    std::vector<double> laser;                     // output columns (prepare_outputs), or empty
     cudaEvent_t ev = nullptr;
     bool fetched = false;
     size_t bytes = 0;
@@ -178,16 +179,18 @@ cudaMemPool_t engine_pool(int device)
 }
 }  // namespace
 
-Engine::Engine(int device, cudaStream_t stream, int steps_per_launch)
-    : device_(device), stream_(stream), S_(steps_per_launch > 0 ? steps_per_launch : 512)
+Engine::Engine(int device, cudaStream_t stream, int steps_per_launch, int capacity)
+    : device_(device), stream_(stream), S_(steps_per_launch > 0 ? steps_per_launch : 512), capacity_(capacity)
 {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     cuda_check(cudaStreamCreateWithFlags(&up_, cudaStreamNonBlocking), "stream create");
     pool_ = engine_pool(device_);
-    capacity_ = 4096;
-    cuda_check(cudaMalloc(&d_solves_, sizeof(SolveDev) * capacity_), "cudaMalloc(solves)");
-    h_solves_ = new SolveDev[capacity_];
-    cuda_check(cudaMalloc(&d_ids_, sizeof(int) * capacity_), "cudaMalloc(ids)");
+    // descriptors sized for the solves to come, from the pool: cudaMalloc and
+    // cudaFree (which waits for the whole device) around every solve took longer
+    // than a small solve
+    cuda_check(cudaMallocFromPoolAsync((void **)&d_solves_, sizeof(SolveDev) * capacity_, pool_, stream_), "alloc solves");
+    h_solves_.resize(capacity_);
+    cuda_check(cudaMallocFromPoolAsync((void **)&d_ids_, sizeof(int) * capacity_, pool_, stream_), "alloc ids");
     h_ids_.assign(capacity_, 0);
     for (int i = capacity_ - 1; i >= 0; --i) free_slots_.push_back(i);
     cudaMemPool_t pool;
@@ -219,15 +222,14 @@ Engine::~Engine()
         pinned_.put(s.h_const, (size_t)s.ntiles * NSLOT * 8);
     }
     for (auto &kv : groups_) cudaFreeAsync(kv.second->d_tiles, stream_);
+    cudaFreeAsync(d_solves_, stream_);
+    cudaFreeAsync(d_ids_, stream_);
     for (auto &e : prop_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     for (auto &e : red_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     cudaStreamSynchronize(stream_);
     for (auto ev : pending_) cudaEventDestroy(ev);
     for (auto ev : spare_ev_) cudaEventDestroy(ev);
     cudaStreamDestroy(up_);
-    cudaFree(d_solves_);
-    delete[] h_solves_;
-    cudaFree(d_ids_);
 }
 
 void Engine::drain_pending()
@@ -670,8 +672,20 @@ SolveOutputs Engine::outputs(int id, const std::vector<double> *laser)
     double cp[NSLOT];
     raw_outputs(id, j, cp);
     SolveOutputs o;
-    assemble_outputs(get(id).prob, j, cp, o, laser);
+    const Solve &s = get(id);
+    assemble_outputs(s.prob, j, cp, o, laser ? laser : &s.laser);
     return o;
+}
+
+void Engine::prepare_outputs()
+{
+    size_t bytes = 0;
+    for (auto &kv : live_) {
+        Solve &s = *kv.second;
+        bytes += (size_t)s.Nt * 56;
+        if (bytes > ((size_t)128 << 20)) return;
+        if (s.laser.empty()) s.laser = laser_rows(s.prob);
+    }
 }
 
 void Engine::remove(int id)

@@ -90,7 +90,8 @@ struct SolveOutputs {
 
 class Engine {
 public:
-    Engine(int device, cudaStream_t stream, int steps_per_launch);
+    // capacity: solves that may be resident at once
+    Engine(int device, cudaStream_t stream, int steps_per_launch, int capacity = 4096);
     ~Engine();
     Engine(const Engine &) = delete;
     Engine &operator=(const Engine &) = delete;
@@ -118,6 +119,9 @@ public:
     bool ready(int id);
     // `laser` may hold the problem's laser_rows() already built by the caller
     SolveOutputs outputs(int id, const std::vector<double> *laser = nullptr);
+    // Evaluate the laser columns of the resident solves' outputs (host work
+    // that can run while the GPU propagates), up to 128 MB of them
+    void prepare_outputs();
     // The raw per-step sums [Nt][NSLOT] and the summed constant parts of a
     // fetched solve (waits for the copy); assemble_outputs() turns them into
     // the output arrays.
@@ -174,7 +178,7 @@ private:
     std::map<int, std::unique_ptr<Solve>> live_;
     std::vector<int> free_slots_;
     SolveDev *d_solves_ = nullptr;
-    SolveDev *h_solves_ = nullptr;   // host mirror of the descriptors
+    std::vector<SolveDev> h_solves_;   // host mirror of the descriptors
     int *d_ids_ = nullptr;
     std::vector<int> h_ids_;
     UploadRing &ring_ = UploadRing::shared();

@@ -128,7 +128,7 @@ Shape autotune_shape(int device, const Problem &p, int precision)
     for (const Shape &c : cand) {
         float ms = 1e30f;
         try {
-            Engine e(device, st, S);
+            Engine e(device, st, S, 1);
             EngineOptions eo;
             eo.precision = precision;
             eo.tile_k = c.tile_k;

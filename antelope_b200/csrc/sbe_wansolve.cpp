@@ -246,7 +246,7 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     ring.upload(d_w_, &w_, sizeof(w_), st);
     if (wan_steps(w_)) cuda_check(launch_wan_step_fields(w_, d_w_, st), "Wannier step fields");
     else cuda_check(launch_wan_prepare(w_, d_w_, precision_, st), "Wannier stage preparation");
-    cuda_check(cudaMallocHost(&h_ctl_, sizeof(WanCtl)), "cudaMallocHost(control)");
+    h_ctl_ = static_cast<WanCtl *>(PinnedPool::shared().get(sizeof(WanCtl)));
 }
 
 // The groups of lattice vectors that share their phase along the grid's rows,
@@ -348,7 +348,7 @@ WannierSolve::~WannierSolve()
     if (w_.snap_nc) cudaFreeAsync(w_.snap_nc, stream_);
     if (w_.snap_pi) cudaFreeAsync(w_.snap_pi, stream_);
     cudaStreamSynchronize(stream_);
-    if (h_ctl_) cudaFreeHost(h_ctl_);
+    PinnedPool::shared().put(h_ctl_, sizeof(WanCtl));
 }
 
 void WannierSolve::run(cudaStream_t st)
@@ -474,8 +474,7 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
             ring.upload(c.d_snap_tiles, tiles.data(), sizeof(WanTileRef) * tiles.size(), st);
         }
     }
-    cuda_check(cudaMallocHost(&h_ctls_, sizeof(WanCtl) * std::max<size_t>(1, solves_.size())),
-               "cudaMallocHost(batch control)");
+    h_ctls_ = static_cast<WanCtl *>(PinnedPool::shared().get(sizeof(WanCtl) * std::max<size_t>(1, solves_.size())));
 }
 
 WannierBatch::~WannierBatch()
@@ -487,8 +486,8 @@ WannierBatch::~WannierBatch()
         if (c.d_snap_tiles) cudaFreeAsync(c.d_snap_tiles, stream_);
     }
     cudaStreamSynchronize(stream_);
+    PinnedPool::shared().put(h_ctls_, sizeof(WanCtl) * std::max<size_t>(1, solves_.size()));
     solves_.clear();
-    if (h_ctls_) cudaFreeHost(h_ctls_);
 }
 
 int WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
