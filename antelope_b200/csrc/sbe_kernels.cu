@@ -271,10 +271,30 @@ __device__ __forceinline__ void vg_rhs(const VgField<Real> &h, Real hc0, const R
     k[D_ZI] = fma(-g2, y[D_ZI], -xr);
 }
 
+// Shared memory of a propagate_vg block: the tile reducer's stage, the warps'
+// staged sums [VSTEP][4][VROW] double2 each, and two blocks of SUB steps of the
+// field table (the columns past the first).
+constexpr int VSTEP = 4;   // steps per warp sum: 4 x 8 (row, slot) sums, one per lane
+constexpr int VROW = 33;   // entries per staged row (32 lanes + 1 pad)
+template <class Real, int RK> constexpr int vg_stage_bytes(int threads)
+{
+    return red_stage_bytes(threads) + (threads / 32) * VSTEP * 4 * VROW * 16 +
+           2 * SUB * (Tableau<RK>::NT - 1) * 2 * (int)sizeof(Real);
+}
+
 // RK4 fits in 128 registers without spilling (4 CTAs of 128 threads per SM
 // instead of 3 at the compiler's unbounded choice); Fehlberg-5 would spill.
 // RK4 CTAs may have up to 512 threads at the same 128 registers, so that the
 // autotuner can choose a tile count that fills the last wave of CTAs.
+//
+// What bounds it: the FP64 pipe where the grid fills the GPU (82 FP64
+// instructions per k-step and RK4), the chain of the stages (17 dependent
+// operations of 8.5 cycles) at one or two warps per scheduler.  So the currents
+// of a step go to the warp's stage in shared memory -- 4 16-byte stores -- and
+// every VSTEP steps lane l sums (row l / 8, slot l % 8) over the 32 lanes: a
+// butterfly per step (18 shuffles, 28 selects, 9 adds) held up the warp's
+// in-order issue; and the field table is read SUB steps ahead into shared
+// memory, where a read in the step waited for L2 every third step.
 template <class Real, int RK, int KPT, bool G1>
 __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const TileDev *__restrict__ tiles,
                                                     const SolveDev *__restrict__ solves, int tick, int S)
@@ -282,7 +302,8 @@ __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const Til
     using T2 = typename V2<Real>::T;
     using TB = Tableau<RK>;
     constexpr bool F64 = std::is_same<Real, double>::value;
-    extern __shared__ double red_dyn[];   // red_stage_bytes(blockDim.x)
+    constexpr int NA = TB::NT - 1;
+    extern __shared__ __align__(16) double vg_dyn[];   // vg_stage_bytes(blockDim.x)
     const TileDev tl = tiles[blockIdx.x];
     const SolveDev &sd = solves[tl.solve];
     const int s0 = (tick - sd.admit_tick) * S;
@@ -295,6 +316,10 @@ __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const Til
     const T2 *__restrict__ tab = static_cast<const T2 *>(sd.tab);
     const Real g1 = Real(sd.g1), g2 = Real(sd.g2);
     double *partial = sd.partial;
+    const int nwarp = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double2 *const vst = reinterpret_cast<double2 *>(vg_dyn + 2 * SUB * nwarp * NSLOT) + warp * (VSTEP * 4 * VROW);
+    T2 *const sA = reinterpret_cast<T2 *>(reinterpret_cast<double2 *>(vg_dyn + 2 * SUB * nwarp * NSLOT) +
+                                          nwarp * (VSTEP * 4 * VROW));   // [2][SUB][NA]
 
     // the state (rho - rho0) is kept in FP64 in both methods; the mixed
     // method rounds it to FP32 once per step for the stage arithmetic and
@@ -314,10 +339,14 @@ __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const Til
 #pragma unroll
         for (int q = VG_PXR; q <= VG_PYI; ++q) c[j][q] = c[j][q] + c[j][q];   // see vg_rhs
         c[j][VG_C0] = c[j][VG_C0] * Real(0.5);
+        if (F64) {   // intraband weights of da alone (db = -da)
+            c[j][VG_WPX0] = c[j][VG_WPX0] - c[j][VG_WPX1];
+            c[j][VG_WPY0] = c[j][VG_WPY0] - c[j][VG_WPY1];
+        }
 #pragma unroll
         for (int q = 0; q < D_N; ++q) y64[j][q] = ok[j] ? st[(size_t)slot[q] * nkp + kidx[j]] : 0.0;
     }
-    TileReducer red(red_dyn, blockDim.x >> 5);
+    TileReducer red(vg_dyn, nwarp);
     // field terms at the start of the launch's first step (see vg_start_row)
     VgField<Real> hstart[KPT];
     {
@@ -326,45 +355,67 @@ __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const Til
         for (int j = 0; j < KPT; ++j) hstart[j] = vg_field<Real>(c[j], A0);
     }
     int next_shot = first_shot(s0, sd.shot_every);
+    // the table columns 1 ... NA of step s0 + i / NA, one entry i per thread
+    auto table = [&](int s, int i) { return __ldg(tab + (size_t)(s + i / NA) * TB::NT + 1 + i % NA); };
+    for (int i = threadIdx.x; i < min(SUB, s1 - s0) * NA; i += blockDim.x) sA[i] = table(s0, i);
+    __syncthreads();
 
-    for (int s = s0; s < s1; ++s) {
+    // one time step s, its sums staged in row r of the warp's stage
+    auto step = [&](int s, int r, const T2 *A) {
         Real y0[KPT][D_N];
 #pragma unroll
         for (int j = 0; j < KPT; ++j)
 #pragma unroll
             for (int q = 0; q < D_N; ++q) y0[j][q] = Real(y64[j][q]);
         // currents and occupations at t_s, before rho advances (antelope.cpp:309-334)
-        double v[8];
+        double v[7];
+        if constexpr (F64) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = 0.0;
+            for (int j = 0; j < KPT; ++j) {
+                const double *cc = c[j];
+                const double *yy = y0[j];
+                auto add = [&](int q, double a, double b) { v[q] = j == 0 ? a * b : fma(a, b, v[q]); };
+                add(0, yy[D_ZI], cc[VG_WQXI]);
+                v[0] = fma(yy[D_ZR], cc[VG_WQXR], v[0]);
+                add(1, yy[D_ZI], cc[VG_WQYI]);
+                v[1] = fma(yy[D_ZR], cc[VG_WQYR], v[1]);
+                add(2, yy[D_DA], cc[VG_WPX0]);
+                add(3, yy[D_DA], cc[VG_WPY0]);
+                add(4, cc[VG_W], yy[D_DA]);
+                add(5, cc[VG_W], yy[D_ZR]);
+                add(6, cc[VG_W], yy[D_ZI]);
+            }
+        } else {
 #pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-            const Real *cc = c[j];
-            const Real *yy = y0[j];
-            const Real db = -yy[D_DA];
-            v[0] += double(fma(yy[D_ZR], cc[VG_WQXR], yy[D_ZI] * cc[VG_WQXI]));
-            v[1] += double(fma(yy[D_ZR], cc[VG_WQYR], yy[D_ZI] * cc[VG_WQYI]));
-            v[2] += double(fma(yy[D_DA], cc[VG_WPX0], db * cc[VG_WPX1]));
-            v[3] += double(fma(yy[D_DA], cc[VG_WPY0], db * cc[VG_WPY1]));
-            v[4] += double(cc[VG_W] * yy[D_DA]);
-            v[6] += double(cc[VG_W] * yy[D_ZR]);
-            v[7] += double(cc[VG_W] * yy[D_ZI]);
+            for (int q = 0; q < 7; ++q) v[q] = 0.0;
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) {
+                const Real *cc = c[j];
+                const Real *yy = y0[j];
+                const Real db = -yy[D_DA];
+                v[0] += double(fma(yy[D_ZR], cc[VG_WQXR], yy[D_ZI] * cc[VG_WQXI]));
+                v[1] += double(fma(yy[D_ZR], cc[VG_WQYR], yy[D_ZI] * cc[VG_WQYI]));
+                v[2] += double(fma(yy[D_DA], cc[VG_WPX0], db * cc[VG_WPX1]));
+                v[3] += double(fma(yy[D_DA], cc[VG_WPY0], db * cc[VG_WPY1]));
+                v[4] += double(cc[VG_W] * yy[D_DA]);
+                v[5] += double(cc[VG_W] * yy[D_ZR]);
+                v[6] += double(cc[VG_W] * yy[D_ZI]);
+            }
         }
-        v[5] = -v[4];
-        const int r = (s - s0) % SUB;
-        red.push(v, r);
+        double2 *const o = vst + r * 4 * VROW + lane;
+        o[0] = make_double2(v[0], v[1]);
+        o[VROW] = make_double2(v[2], v[3]);
+        o[2 * VROW] = make_double2(v[4], v[5]);
+        o[3 * VROW].x = v[6];
 
         // one RK step of the thread's k-points, stage by stage so that their
         // independent dependency chains interleave
-        T2 A[TB::NT];
-#pragma unroll
-        for (int i = 1; i < TB::NT; ++i) A[i] = __ldg(tab + (size_t)s * TB::NT + i);
         VgField<Real> h[KPT][TB::NT];
 #pragma unroll
         for (int j = 0; j < KPT; ++j) {
             h[j][0] = hstart[j];
 #pragma unroll
-            for (int i = 1; i < TB::NT; ++i) h[j][i] = vg_field<Real>(c[j], A[i]);
+            for (int i = 1; i < TB::NT; ++i) h[j][i] = vg_field<Real>(c[j], A[i - 1]);
             hstart[j] = h[j][TB::END];
         }
         // FP64: acc = rho + sum_i dt b_i k_i in the reference's order
@@ -406,9 +457,38 @@ __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const Til
                                 y64[j][D_ZR], y64[j][D_ZI]);
             next_shot += sd.shot_every;
         }
-        // the staged sums reach the partial buffer after the step's arithmetic,
-        // so the warp reduction above can overlap it
-        if (r == SUB - 1 || s == s1 - 1) red.flush(r + 1, s - r - s0, ntiles, tl.tile, partial);
+    };
+
+    // this lane's sum: staged row lane / 8, slot lane % 8 (slot 5 = -slot 4)
+    const int vrow = lane >> 3, vslot = lane & 7;
+    const int vcol = vslot < 5 ? vslot : vslot == 5 ? 4 : vslot - 1;
+    const double *const vsrc = reinterpret_cast<const double *>(vst + (vrow * 4 + (vcol >> 1)) * VROW) + (vcol & 1);
+    int buf = 0;
+    for (int b0 = s0; b0 < s1; b0 += SUB, buf ^= 1) {
+        const int nb = min(SUB, s1 - b0), nn = min(SUB, s1 - b0 - SUB) * NA;   // this and the next block of steps
+        T2 pre{};
+        if ((int)threadIdx.x < nn) pre = table(b0 + SUB, threadIdx.x);
+        for (int e = 0; e < nb; e += VSTEP) {
+            const int m = min(VSTEP, nb - e);
+            const T2 *A = sA + (buf * SUB + e) * NA;
+            if (m == VSTEP) {
+#pragma unroll
+                for (int j = 0; j < VSTEP; ++j) step(b0 + e + j, j, A + j * NA);
+            } else {
+#pragma unroll 1
+                for (int j = 0; j < m; ++j) step(b0 + e + j, j, A + j * NA);
+            }
+            __syncwarp();
+            double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int i = 0; i < 32; ++i) s4[i & 3] += vsrc[2 * i];
+            const double sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            __syncwarp();
+            if (vrow < m) red.at(red.half, e + vrow, warp, vslot) = vslot == 5 ? -sum : sum;
+        }
+        if ((int)threadIdx.x < nn) sA[(buf ^ 1) * SUB * NA + threadIdx.x] = pre;
+        for (int i = threadIdx.x + blockDim.x; i < nn; i += blockDim.x) sA[(buf ^ 1) * SUB * NA + i] = table(b0 + SUB, i);
+        red.flush(nb, b0 - s0, ntiles, tl.tile, partial);
     }
 #pragma unroll
     for (int j = 0; j < KPT; ++j)
@@ -1431,37 +1511,48 @@ __global__ void __launch_bounds__(256) fma_peak_x2(float *out, int iters, float 
 
 // ------------------------------------------------------------- launchers
 #define SBE_CHECK_LAUNCH() return cudaGetLastError()
+constexpr int kMaxDev = 64;
 
-template <class Real, int RK, int KPT>
-static cudaError_t launch_vg_t(const LaunchArgs &la, bool g1)
+// The velocity-gauge kernels' stages live in dynamic shared memory, above the
+// 48 KiB default for large CTAs: the limit is raised once per device and
+// kernel instance.
+template <class K> static cudaError_t raise_smem(K kernel, std::atomic<int> *raised, int max_bytes)
 {
-    if (g1)
-        propagate_vg<Real, RK, KPT, true><<<la.ntiles, la.threads, red_stage_bytes(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    else
-        propagate_vg<Real, RK, KPT, false><<<la.ntiles, la.threads, red_stage_bytes(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    SBE_CHECK_LAUNCH();
-}
-
-// The packed kernel's warp stages live in dynamic shared memory (64 KiB at
-// 256 threads, above the 48 KiB default): the limit is raised once per device
-// and kernel instance.
-template <int RK, bool G1>
-static cudaError_t launch_vg_x2_t(const LaunchArgs &la)
-{
-    constexpr int kMaxDev = 64;
-    static std::atomic<int> raised[kMaxDev];
-    const int bytes = xstage_bytes(la.threads);
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
     if (raised[dev].load(std::memory_order_acquire) == 0) {
-        e = cudaFuncSetAttribute(propagate_vg_x2<RK, G1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 xstage_bytes(256));
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_bytes);
         if (e != cudaSuccess) return e;
         raised[dev].store(1, std::memory_order_release);
     }
-    propagate_vg_x2<RK, G1><<<la.ntiles, la.threads, bytes, la.stream>>>(la.tiles, la.solves, la.tick, la.S);
+    return cudaSuccess;
+}
+
+template <class Real, int RK, int KPT, bool G1>
+static cudaError_t launch_vg_g(const LaunchArgs &la)
+{
+    static std::atomic<int> raised[kMaxDev];
+    cudaError_t e = raise_smem(propagate_vg<Real, RK, KPT, G1>, raised, vg_stage_bytes<Real, RK>(RK == 4 ? 512 : 256));
+    if (e != cudaSuccess) return e;
+    propagate_vg<Real, RK, KPT, G1>
+        <<<la.ntiles, la.threads, vg_stage_bytes<Real, RK>(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
+    SBE_CHECK_LAUNCH();
+}
+template <class Real, int RK, int KPT>
+static cudaError_t launch_vg_t(const LaunchArgs &la, bool g1)
+{
+    return g1 ? launch_vg_g<Real, RK, KPT, true>(la) : launch_vg_g<Real, RK, KPT, false>(la);
+}
+
+template <int RK, bool G1>
+static cudaError_t launch_vg_x2_t(const LaunchArgs &la)
+{
+    static std::atomic<int> raised[kMaxDev];
+    cudaError_t e = raise_smem(propagate_vg_x2<RK, G1>, raised, xstage_bytes(256));
+    if (e != cudaSuccess) return e;
+    propagate_vg_x2<RK, G1><<<la.ntiles, la.threads, xstage_bytes(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
     SBE_CHECK_LAUNCH();
 }
 
