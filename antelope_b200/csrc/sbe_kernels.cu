@@ -26,6 +26,7 @@
 // FP64 from the warp level up.  In the velocity gauge the state is the
 // deviation rho - rho0, and the time-independent rho0 parts of the currents
 // are summed once, in FP64.
+#include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -140,36 +141,6 @@ template <class Real> struct V2;
 template <> struct V2<double> { using T = double2; };
 template <> struct V2<float> { using T = float2; };
 
-// ---------------------------------------------------- warp reduce-scatter
-// Sums 8 doubles over the 32 lanes of a warp.  Three halving exchanges leave
-// each lane with one partially summed value (index lane>>2 for lanes that are
-// multiples of 4), two more exchanges finish it: 9 shuffles instead of 40.
-// The pattern is fixed, so the result is deterministic.
-template <class T>
-__device__ __forceinline__ T warp_sum8(const T (&v)[8], int lane)
-{
-    const bool h4 = lane & 16, h2 = lane & 8, h1 = lane & 4;
-    T u[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        T send = h4 ? v[i] : v[i + 4];
-        T keep = h4 ? v[i + 4] : v[i];
-        u[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-    T x[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        T send = h2 ? u[i] : u[i + 2];
-        T keep = h2 ? u[i + 2] : u[i];
-        x[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-    T send = h1 ? x[0] : x[1];
-    T y = (h1 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, send, 4);
-    y += __shfl_xor_sync(0xffffffffu, y, 2);
-    y += __shfl_xor_sync(0xffffffffu, y, 1);
-    return y;  // lanes 4*i hold the sum of v[i]
-}
-
 constexpr int MAX_WARPS = 8;
 
 // Per-step tile reduction staged through shared memory: each warp deposits
@@ -193,15 +164,6 @@ struct TileReducer {
     __device__ __forceinline__ double &at(int h, int r, int w, int slot)
     {
         return red[((h * SUB + r) * nw + w) * NSLOT + slot];
-    }
-    __device__ __forceinline__ void put(double y, int r)
-    {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        if ((lane & 3) == 0) at(half, r, warp, lane >> 2) = y;
-    }
-    __device__ __forceinline__ void push(const double (&v)[8], int r)
-    {
-        put(warp_sum8<double>(v, threadIdx.x & 31), r);
     }
     __device__ __forceinline__ void flush(int nrows, int row0, int ntiles, int tile, double *partial)
     {
@@ -783,10 +745,10 @@ __device__ __forceinline__ void lw_field(const Real (&c)[LW_NCONST], const Real 
 #pragma unroll
     for (int i = 0; i < LW_NPHASE / PER; ++i) {
         if constexpr (sizeof(Real) == 4) {
-            const float4 u = __ldg(reinterpret_cast<const float4 *>(ph) + i);
+            const float4 u = reinterpret_cast<const float4 *>(ph)[i];
             p[4 * i] = u.x; p[4 * i + 1] = u.y; p[4 * i + 2] = u.z; p[4 * i + 3] = u.w;
         } else {
-            const double2 u = __ldg(reinterpret_cast<const double2 *>(ph) + i);
+            const double2 u = reinterpret_cast<const double2 *>(ph)[i];
             p[2 * i] = u.x; p[2 * i + 1] = u.y;
         }
     }
@@ -861,11 +823,11 @@ template <class Real> struct LwCurrentConsts {
 // Currents and density-matrix sums at k + A(t) (SBEs.h:694-760) from that
 // time's trig factors T and field terms F and the state y at t, in the stage
 // arithmetic (the per-k terms of the mixed method in FP32, like the velocity
-// gauge's), summed over the warp: lanes 4i return slot i.  The tile and
-// k-sums above the warp are FP64 in both methods.
+// gauge's): v[slot].  The tile and k-sums above the warp are FP64 in both
+// methods.
 template <class Real>
-__device__ __forceinline__ double lw_current_sum(const LwCurrentConsts<Real> &K, const LwTrig<Real> &T,
-                                                 const LwField<Real> &F, const Real (&y)[4], Real w)
+__device__ __forceinline__ void lw_current(const LwCurrentConsts<Real> &K, const LwTrig<Real> &T,
+                                           const LwField<Real> &F, const Real (&y)[4], Real w, Real (&v)[8])
 {
     Real j0[2], j1[2], j2[2], j3[2];
 #pragma unroll
@@ -878,7 +840,6 @@ __device__ __forceinline__ double lw_current_sum(const LwCurrentConsts<Real> &K,
     const Real al = y[LW_AL], sx = y[LW_SX], sy = y[LW_SY], sz = y[LW_SZ];
     const Real sBi = fma(sx, F.B1, fma(sy, F.B2, sz * F.B3)) * F.ib;   // (s.B) / |B|^2
     const Real w2 = w + w;
-    Real v[8];
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
         const Real sj = fma(sx, j1[a], fma(sy, j2[a], sz * j3[a]));
@@ -890,7 +851,70 @@ __device__ __forceinline__ double lw_current_sum(const LwCurrentConsts<Real> &K,
     v[5] = w * (al - sz);
     v[6] = w * sx;
     v[7] = -w * sy;
-    return double(warp_sum8<Real>(v, threadIdx.x & 31));
+}
+
+// The length-gauge kernels' sums over the warp: each lane stores its 8 values
+// of a step, and every VSTEP steps lane l sums row l / 8, slot l % 8 over the 32
+// lanes -- in the tree of a butterfly (lanes 16 apart, then 8, 4, 2, 1), which
+// the FP32 sums of the mixed method keep to the bit -- into row r0 + l / 8 of
+// the block's stage.  Rows are padded so that reads and stores are free of bank
+// conflicts.
+template <class Real> struct LwStage {
+    static constexpr int PER = 16 / sizeof(Real), COLS = 8 / PER;   // values and columns of 16 bytes
+    static constexpr int BYTES = VSTEP * COLS * VROW * 16;          // per warp
+    Real *base;
+    __device__ __forceinline__ explicit LwStage(unsigned char *p) : base(reinterpret_cast<Real *>(p)) {}
+    __device__ __forceinline__ void put(int r, const Real (&v)[8])
+    {
+        using V = typename std::conditional<sizeof(Real) == 4, float4, double2>::type;
+        V *o = reinterpret_cast<V *>(base) + r * COLS * VROW + (threadIdx.x & 31);
+#pragma unroll
+        for (int q = 0; q < COLS; ++q) {
+            if constexpr (sizeof(Real) == 4) o[q * VROW] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            else o[q * VROW] = make_double2(v[2 * q], v[2 * q + 1]);
+        }
+    }
+    __device__ __forceinline__ void sum(TileReducer &red, int r0, int m)
+    {
+        __syncwarp();
+        const int lane = threadIdx.x & 31, row = lane >> 3, slot = lane & 7;
+        const Real *p = base + ((row * COLS + slot / PER) * VROW) * PER + slot % PER;
+        const Real x = tree<1>(p, 0);
+        if (row < m) red.at(red.half, r0 + row, threadIdx.x >> 5, slot) = double(x);
+        __syncwarp();
+    }
+    // sum over the lanes = i mod S, depth first (few partial sums alive)
+    template <int S> static __device__ __forceinline__ Real tree(const Real *p, int i)
+    {
+        if constexpr (S == 16) {
+            return p[i * PER] + p[(i + 16) * PER];
+        } else {
+            const Real a = tree<2 * S>(p, i);
+            return a + tree<2 * S>(p, i + S);
+        }
+    }
+};
+// Shared memory of a length-gauge block: the tile reducer's stage, the warps'
+// staged sums and two blocks of SUB steps of the phase table (the columns past
+// the first)
+template <class Real, int RK> constexpr int lw_stage_bytes(int threads)
+{
+    return red_stage_bytes(threads) + (threads / 32) * LwStage<Real>::BYTES +
+           2 * SUB * (Tableau<RK>::NT - 1) * LW_NPHASE * (int)sizeof(Real);
+}
+// Start copying the table rows of nb steps from s on (columns past the first)
+// to shared memory; __pipeline_wait_prior before the block's next barrier
+template <class Real, int RK>
+__device__ __forceinline__ void lw_fetch(Real *dst, const Real *tab, int s, int nb)
+{
+    using TB = Tableau<RK>;
+    constexpr int V = (TB::NT - 1) * LW_NPHASE * (int)sizeof(Real) / 16;   // 16-byte pieces a step
+    for (int i = threadIdx.x; i < nb * V; i += blockDim.x) {
+        const int r = i / V, q = i % V;
+        __pipeline_memcpy_async(reinterpret_cast<char *>(dst) + (size_t)i * 16,
+                                reinterpret_cast<const char *>(tab + ((size_t)(s + r) * TB::NT + 1) * LW_NPHASE) + q * 16, 16);
+    }
+    __pipeline_commit();
 }
 
 // B of H0(k + A(t)) in FP64 from the field-table entry ph of time t (the
@@ -909,14 +933,16 @@ __device__ __forceinline__ void lw_B64(const Real (&c)[LW_NCONST], const Real *p
 // One k-point per thread.  Field terms once per distinct stage time (RK4:
 // t, t + dt/2 for stages 2 and 3, t + dt), the t + dt terms carried into the
 // next step (a launch beginning at s loads the entry of step s-1 at its end,
-// see vg_start_row); the currents of step s+1 are formed at the end of step s
-// from that entry's trig factors and the new state.
+// see vg_start_row); the currents of step s+1 are formed from that entry's trig
+// factors and the new state.  FP64-pipe bound on large grids, a serial chain on
+// small ones: the table is copied SUB steps ahead to shared memory (a read in
+// the step waited for L2) and the currents' sums go through LwStage.
 template <class Real, int RK, bool G1>
 __global__ void __launch_bounds__(256, 2) propagate_lw(const TileDev *__restrict__ tiles,
                                                     const SolveDev *__restrict__ solves, int tick, int S)
 {
     using TB = Tableau<RK>;
-    extern __shared__ double red_dyn[];   // red_stage_bytes(blockDim.x)
+    extern __shared__ __align__(16) double red_dyn[];   // lw_stage_bytes(blockDim.x)
     const TileDev tl = tiles[blockIdx.x];
     const SolveDev &sd = solves[tl.solve];
     const int s0 = (tick - sd.admit_tick) * S;
@@ -954,17 +980,35 @@ __global__ void __launch_bounds__(256, 2) propagate_lw(const TileDev *__restrict
     }
     if (!ok) c[LW_CA0] = c[LW_CB0] = Real(1);  // padding lanes: a harmless k = 0 point, weight 0
     const Real w = c[LW_W];
-    TileReducer red(red_dyn, blockDim.x >> 5);
+    const int nwarp = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    TileReducer red(red_dyn, nwarp);
+    unsigned char *const dyn = reinterpret_cast<unsigned char *>(red_dyn) + red_stage_bytes(blockDim.x);
+    LwStage<Real> stage(dyn + warp * LwStage<Real>::BYTES);
+    constexpr int NA = (TB::NT - 1) * LW_NPHASE;
+    Real *const sA = reinterpret_cast<Real *>(dyn + nwarp * LwStage<Real>::BYTES);   // [2][SUB][NA]
     int next_shot = first_shot(s0, sd.shot_every);
+    lw_fetch<Real, RK>(sA, tab, s0, min(SUB, s1 - s0));
 
-    // field and currents at the launch's first step
-    LwTrig<Real> Te;   // trig factors at the end of the step (t + dt)
+    // field at the launch's first step
+    LwTrig<Real> Te;   // trig factors at the end of the step before (t + dt)
     lw_field<Real>(c, tab + vg_start_row<TB>(s0) * LW_NPHASE, Te.ca, Te.sa, Te.cb, Te.sb);
     LwField<Real> F0 = lw_field_terms<Real>(Te, t1dt, t2sdt, Mdt, gd);
-    red.put(lw_current_sum<Real>(K, Te, F0, yr, w), 0);
+    __pipeline_wait_prior(0);
+    __syncthreads();
 
-    for (int s = s0; s < s1; ++s) {
-        const Real *row = tab + (size_t)s * TB::NT * LW_NPHASE;
+    int buf = 0;
+    for (int b0 = s0; b0 < s1; b0 += SUB, buf ^= 1) {
+      const int nb = min(SUB, s1 - b0), nn = min(SUB, s1 - b0 - SUB);   // this and the next block of steps
+      if (nn > 0) lw_fetch<Real, RK>(sA + (buf ^ 1) * SUB * NA, tab, b0 + SUB, nn);
+#pragma unroll 1
+      for (int e = 0; e < nb; ++e) {
+        const int s = b0 + e;
+        const Real *row = sA + (buf * SUB + e) * NA - LW_NPHASE;   // column i at row + i * LW_NPHASE
+        {   // currents at k + A(t_s) with the state before the step (antelope.cpp:309-334)
+            Real v[8];
+            lw_current<Real>(K, Te, F0, yr, w, v);
+            stage.put(e % VSTEP, v);
+        }
         LwField<Real> Fc = F0;   // field at the current stage's time; a new time evaluates it once
         Real kk[TB::S][4], y[4], acc[4];
 #pragma unroll
@@ -996,9 +1040,6 @@ __global__ void __launch_bounds__(256, 2) propagate_lw(const TileDev *__restrict
             y64[q] = F64 ? double(acc[q]) : y64[q] + double(acc[q]);
             yr[q] = Real(y64[q]);
         }
-        // currents of step s+1 at k + A(t_{s+1}) with the state after step s,
-        // summed over the warp now and staged after this step's flush
-        const double jsum = s + 1 < s1 ? lw_current_sum<Real>(K, Te, F0, yr, w) : 0.0;
         if (s == next_shot) {
             // density snapshot: rho after the step in the eigenbasis of
             // H0(k + A(t_s)) (SBEs::WannierToHamiltonian at the step's start
@@ -1025,9 +1066,10 @@ __global__ void __launch_bounds__(256, 2) propagate_lw(const TileDev *__restrict
             }
             next_shot += sd.shot_every;
         }
-        const int r = (s - s0) % SUB;
-        if (r == SUB - 1 || s == s1 - 1) red.flush(r + 1, s - r - s0, ntiles, tl.tile, sd.partial);
-        if (s + 1 < s1) red.put(jsum, (s + 1 - s0) % SUB);
+        if (e % VSTEP == VSTEP - 1 || e == nb - 1) stage.sum(red, e - e % VSTEP, e % VSTEP + 1);
+      }
+      __pipeline_wait_prior(0);
+      red.flush(nb, b0 - s0, ntiles, tl.tile, sd.partial);
     }
     if (ok)
 #pragma unroll
@@ -1050,7 +1092,7 @@ __device__ __forceinline__ void lw_trig2(const float2 (&c)[LW_NCONST], const flo
     float p[LW_NPHASE];
 #pragma unroll
     for (int i = 0; i < LW_NPHASE / 4; ++i) {
-        const float4 u = __ldg(reinterpret_cast<const float4 *>(ph) + i);
+        const float4 u = reinterpret_cast<const float4 *>(ph)[i];
         p[4 * i] = u.x; p[4 * i + 1] = u.y; p[4 * i + 2] = u.z; p[4 * i + 3] = u.w;
     }
 #pragma unroll
@@ -1093,10 +1135,10 @@ __device__ __forceinline__ void lw_rhs2(const LwField2 &F, const float2 (&y)[4],
 // j1 = t1 va.sin(ka), j2 = -t1 va.cos(ka), j3 = t2s vb.cos(kb) per axis
 struct LwCurK2 { float j0[2][3], j1[2][3], j2[2][3], j3[2][3]; };
 
-// The currents and density sums of both k-points (as lw_current_sum), added
-// over the pair in FP32 and over the warp: lanes 4i return slot i.
-__device__ __forceinline__ double lw_current_sum2(const LwCurK2 &K, const LwTrig2 &T, const LwField2 &F,
-                                                  const float2 (&y)[4], float2 w)
+// The currents and density sums of both k-points (as lw_current), added over
+// the pair in FP32.
+__device__ __forceinline__ void lw_current2(const LwCurK2 &K, const LwTrig2 &T, const LwField2 &F,
+                                            const float2 (&y)[4], float2 w, float (&v)[8])
 {
     float2 j0[2], j1[2], j2[2], j3[2];
 #pragma unroll
@@ -1109,7 +1151,6 @@ __device__ __forceinline__ double lw_current_sum2(const LwCurK2 &K, const LwTrig
     const float2 al = y[LW_AL], sx = y[LW_SX], sy = y[LW_SY], sz = y[LW_SZ];
     const float2 sBi = mul2(fma2(sx, F.B1, fma2(sy, F.B2, mul2(sz, F.B3))), F.ib);   // (s.B) / |B|^2
     const float2 w2 = add2(w, w);
-    float v[8];
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
         const float2 sj = fma2(sx, j1[a], fma2(sy, j2[a], mul2(sz, j3[a])));
@@ -1124,7 +1165,6 @@ __device__ __forceinline__ double lw_current_sum2(const LwCurK2 &K, const LwTrig
     v[5] = o1.x + o1.y;
     v[6] = o2.x + o2.y;
     v[7] = -(o3.x + o3.y);
-    return double(warp_sum8<float>(v, threadIdx.x & 31));
 }
 
 template <int RK, bool G1>
@@ -1132,7 +1172,7 @@ __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restr
                                                        const SolveDev *__restrict__ solves, int tick, int S)
 {
     using TB = Tableau<RK>;
-    extern __shared__ double red_dyn[];   // red_stage_bytes(blockDim.x)
+    extern __shared__ __align__(16) double red_dyn[];   // lw_stage_bytes(blockDim.x)
     const TileDev tl = tiles[blockIdx.x];
     const SolveDev &sd = solves[tl.solve];
     const int s0 = (tick - sd.admit_tick) * S;
@@ -1184,16 +1224,34 @@ __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restr
                              ok1 ? float(st[(size_t)(LW_ACC + q) * nkp + k1]) : 0.f);
         yr[q] = add2(yhi[q], acc[q]);
     }
-    TileReducer red(red_dyn, blockDim.x >> 5);
+    const int nwarp = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    TileReducer red(red_dyn, nwarp);
+    unsigned char *const dyn = reinterpret_cast<unsigned char *>(red_dyn) + red_stage_bytes(blockDim.x);
+    LwStage<float> stage(dyn + warp * LwStage<float>::BYTES);
+    constexpr int NA = (TB::NT - 1) * LW_NPHASE;
+    float *const sA = reinterpret_cast<float *>(dyn + nwarp * LwStage<float>::BYTES);   // [2][SUB][NA]
     int next_shot = first_shot(s0, sd.shot_every);
+    lw_fetch<float, RK>(sA, tab, s0, min(SUB, s1 - s0));
 
-    LwTrig2 Te;   // trig factors at the end of the step (t + dt)
+    LwTrig2 Te;   // trig factors at the end of the step before (t + dt)
     lw_trig2(c, tab + vg_start_row<TB>(s0) * LW_NPHASE, Te.ca, Te.sa, Te.cb, Te.sb);
     LwField2 F0 = lw_field_terms2(Te, t1dt, nt2sdt, Mdt, gd);
-    red.put(lw_current_sum2(K, Te, F0, yr, w), 0);
+    __pipeline_wait_prior(0);
+    __syncthreads();
 
-    for (int s = s0; s < s1; ++s) {
-        const float *row = tab + (size_t)s * TB::NT * LW_NPHASE;
+    int buf = 0;
+    for (int b0 = s0; b0 < s1; b0 += SUB, buf ^= 1) {
+      const int nb = min(SUB, s1 - b0), nn = min(SUB, s1 - b0 - SUB);   // this and the next block of steps
+      if (nn > 0) lw_fetch<float, RK>(sA + (buf ^ 1) * SUB * NA, tab, b0 + SUB, nn);
+#pragma unroll 1
+      for (int e = 0; e < nb; ++e) {
+        const int s = b0 + e;
+        const float *row = sA + (buf * SUB + e) * NA - LW_NPHASE;   // column i at row + i * LW_NPHASE
+        {   // currents at k + A(t_s) with the state before the step
+            float v[8];
+            lw_current2(K, Te, F0, yr, w, v);
+            stage.put(e % VSTEP, v);
+        }
         LwField2 Fc = F0;
         float2 kk[TB::S][4], y[4];
 #pragma unroll
@@ -1231,7 +1289,6 @@ __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restr
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) yr[q] = add2(yhi[q], acc[q]);
-        const double jsum = s + 1 < s1 ? lw_current_sum2(K, Te, F0, yr, w) : 0.0;
         if (s == next_shot) {
             // density snapshot of each k-point (as propagate_lw)
 #pragma unroll
@@ -1265,9 +1322,10 @@ __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restr
             }
             next_shot += sd.shot_every;
         }
-        const int r = (s - s0) % SUB;
-        if (r == SUB - 1 || s == s1 - 1) red.flush(r + 1, s - r - s0, ntiles, tl.tile, sd.partial);
-        if (s + 1 < s1) red.put(jsum, (s + 1 - s0) % SUB);
+        if (e % VSTEP == VSTEP - 1 || e == nb - 1) stage.sum(red, e - e % VSTEP, e % VSTEP + 1);
+      }
+      __pipeline_wait_prior(0);
+      red.flush(nb, b0 - s0, ntiles, tl.tile, sd.partial);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -1562,21 +1620,30 @@ static cudaError_t launch_vg_x2(const LaunchArgs &la, bool g1)
     return g1 ? launch_vg_x2_t<RK, true>(la) : launch_vg_x2_t<RK, false>(la);
 }
 
+template <class Real, int RK, bool G1>
+static cudaError_t launch_lw_g(const LaunchArgs &la)
+{
+    static std::atomic<int> raised[kMaxDev];
+    cudaError_t e = raise_smem(propagate_lw<Real, RK, G1>, raised, lw_stage_bytes<Real, RK>(256));
+    if (e != cudaSuccess) return e;
+    propagate_lw<Real, RK, G1>
+        <<<la.ntiles, la.threads, lw_stage_bytes<Real, RK>(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
+    SBE_CHECK_LAUNCH();
+}
 template <class Real, int RK>
 static cudaError_t launch_lw_t(const LaunchArgs &la, bool g1)
 {
-    if (g1)
-        propagate_lw<Real, RK, true><<<la.ntiles, la.threads, red_stage_bytes(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    else
-        propagate_lw<Real, RK, false><<<la.ntiles, la.threads, red_stage_bytes(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    SBE_CHECK_LAUNCH();
+    return g1 ? launch_lw_g<Real, RK, true>(la) : launch_lw_g<Real, RK, false>(la);
 }
 
 template <int RK, bool G1>
 static cudaError_t launch_lw_x2_t(const LaunchArgs &la)
 {
-    propagate_lw_x2<RK, G1><<<la.ntiles, la.threads, red_stage_bytes(la.threads), la.stream>>>(la.tiles, la.solves,
-                                                                                              la.tick, la.S);
+    static std::atomic<int> raised[kMaxDev];
+    cudaError_t e = raise_smem(propagate_lw_x2<RK, G1>, raised, lw_stage_bytes<float, RK>(256));
+    if (e != cudaSuccess) return e;
+    propagate_lw_x2<RK, G1>
+        <<<la.ntiles, la.threads, lw_stage_bytes<float, RK>(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
     SBE_CHECK_LAUNCH();
 }
 
