@@ -82,6 +82,7 @@ struct SolveDev {
     double t1, t2c, t2s;          // t1, 2*t2*cos(phi0), 2*t2*sin(phi0)
     double va[3][2], vb[3][2];    // NN and NNN vectors (bohr)
     int *status;                  // device status word (0 = ok)
+    int *prog;                    // [ntiles] first step each tile has yet to take (queued launches)
     // density snapshots (antelope.cpp:340-422): after every step s with
     // s % shot_every == 0 the kernels store, per k, the conduction occupation
     // snap_nc[s / shot_every][k] and the coherence snap_pi[..][k] (re, im) of
@@ -97,6 +98,18 @@ struct TileDev {
     int k0;      // first flat k index of the tile
     int kcount;  // number of k-points in the tile
     int tile;    // tile index within its solve (partial-buffer row)
+};
+
+// Queue of a launch whose tiles outnumber the CTAs the GPU holds: its steps are
+// cut into chunks, and the resident CTAs take (chunk, tile) items in that order
+// from the counter until none are left, so that only the last chunk of the last
+// tiles leaves SMs idle.  An item waits until its tile's chunk before is done:
+// that one was taken earlier, by a CTA that is running.  ctr: [0] next item,
+// [1] CTAs that are done (the last one clears both), [2] error; null: one tile
+// per CTA, all of its steps.
+struct TileQueue {
+    int *ctr;
+    int ntiles, chunk, nitems;
 };
 
 }  // namespace sbe

@@ -141,14 +141,18 @@ struct Engine::Solve {
     std::vector<double> laser;                     // output columns (prepare_outputs), or empty
     cudaEvent_t ev = nullptr;
     bool fetched = false;
+    int nqueues = 0;   // queue states copied behind h_const
     size_t bytes = 0;
 };
+
+constexpr int kMaxGroups = 32;   // launch classes: gauge x precision x RK x KPT x CTA size x T1 in use
 
 struct Engine::Group {
     int variant, precision, rk, kpt, threads;
     bool g1;
     std::vector<TileDev> tiles;
     TileDev *d_tiles = nullptr;
+    int *d_queue = nullptr;   // TileQueue counters
     int cap = 0;
 };
 
@@ -219,9 +223,12 @@ Engine::~Engine()
             cudaEventDestroy(s.ev);
         }
         pinned_.put(s.h_jout, (size_t)s.Nt * NSLOT * 8);
-        pinned_.put(s.h_const, (size_t)s.ntiles * NSLOT * 8);
+        pinned_.put(s.h_const, ((size_t)s.ntiles * NSLOT + kMaxGroups) * 8);
     }
-    for (auto &kv : groups_) cudaFreeAsync(kv.second->d_tiles, stream_);
+    for (auto &kv : groups_) {
+        cudaFreeAsync(kv.second->d_tiles, stream_);
+        cudaFreeAsync(kv.second->d_queue, stream_);
+    }
     cudaFreeAsync(d_solves_, stream_);
     cudaFreeAsync(d_ids_, stream_);
     for (auto &e : prop_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
@@ -341,7 +348,10 @@ int Engine::add(const Problem &p, const EngineOptions &o)
         throw std::runtime_error("field table not 16-byte aligned");
     alloc((void **)&s->partial, part_b, "alloc partials");
     alloc((void **)&s->jout, jout_b, "alloc outputs");
-    alloc((void **)&s->constpart, cp_b, "alloc constant parts");
+    // the tiles' progress follows their constant parts
+    alloc((void **)&s->constpart, cp_b + (size_t)s->ntiles * sizeof(int), "alloc constant parts");
+    int *prog = reinterpret_cast<int *>(s->constpart + (size_t)s->ntiles * NSLOT);
+    cuda_check(cudaMemsetAsync(prog, 0, (size_t)s->ntiles * sizeof(int), up_), "clear progress");
     if (snap_n > 0) {
         alloc((void **)&s->snap_nc, snap_n * 8, "alloc snapshots");
         alloc((void **)&s->snap_pi, snap_n * 16, "alloc snapshots");
@@ -402,6 +412,7 @@ int Engine::add(const Problem &p, const EngineOptions &o)
     d.tab = s->tab;
     d.partial = s->partial;
     d.jout = s->jout;
+    d.prog = prog;
     d.shot_every = s->nshots > 0 ? p.shot_every() : 0;
     d.snap_nc = s->snap_nc;
     d.snap_pi = s->snap_pi;
@@ -469,6 +480,8 @@ void Engine::rebuild_lists()
             g->kpt = s.shape.kpt;
             g->threads = s.shape.threads;
             g->g1 = s.g1;
+            cuda_check(cudaMallocFromPoolAsync((void **)&g->d_queue, 3 * sizeof(int), pool_, stream_), "alloc queue");
+            cuda_check(cudaMemsetAsync(g->d_queue, 0, 3 * sizeof(int), stream_), "clear queue");
         }
         for (int t = 0; t < s.ntiles; ++t) {
             TileDev td;
@@ -521,6 +534,7 @@ void Engine::step_frozen()
         la.rk = g.rk;
         la.kpt = g.kpt;
         la.has_g1 = g.g1;
+        la.queue = g.d_queue;
         la.stream = stream_;
         std::pair<cudaEvent_t, cudaEvent_t> ev{};
         if (profile_) {
@@ -584,11 +598,19 @@ void Engine::fetch_async(int id)
     // pinned result buffers are taken when a solve finishes, not when it is
     // admitted (a burst of admissions would otherwise wait on page locking)
     if (!s.h_jout) s.h_jout = static_cast<double *>(pinned_.get((size_t)s.Nt * NSLOT * 8));
-    if (!s.h_const) s.h_const = static_cast<double *>(pinned_.get((size_t)s.ntiles * NSLOT * 8));
+    if (!s.h_const) s.h_const = static_cast<double *>(pinned_.get(((size_t)s.ntiles * NSLOT + kMaxGroups) * 8));
     cuda_check(cudaMemcpyAsync(s.h_jout, s.jout, (size_t)s.Nt * NSLOT * 8, cudaMemcpyDeviceToHost, stream_),
                "copy outputs");
     cuda_check(cudaMemcpyAsync(s.h_const, s.constpart, (size_t)s.ntiles * NSLOT * 8, cudaMemcpyDeviceToHost, stream_),
                "copy constant parts");
+    // a queued launch that gave up waiting on a tile says so here
+    int i = 0;
+    for (auto &kv : groups_)
+        if (kv.second->d_queue && i < kMaxGroups)
+            cuda_check(cudaMemcpyAsync(s.h_const + (size_t)s.ntiles * NSLOT + i++, kv.second->d_queue + 2, sizeof(int),
+                                       cudaMemcpyDeviceToHost, stream_),
+                       "copy queue state");
+    s.nqueues = i;
     cuda_check(cudaEventRecord(s.ev, stream_), "event record");
     s.fetched = true;
 }
@@ -608,6 +630,11 @@ void Engine::raw_outputs(int id, std::vector<double> &jout, double cp[NSLOT])
     Solve &s = get(id);
     if (!s.fetched) fetch_async(id);
     cuda_check(cudaEventSynchronize(s.ev), "event sync");
+    for (int i = 0; i < s.nqueues; ++i) {
+        int err;
+        std::memcpy(&err, s.h_const + (size_t)s.ntiles * NSLOT + i, sizeof(int));
+        if (err) throw CudaError("a launch gave up waiting for a tile's earlier steps");
+    }
     for (int q = 0; q < NSLOT; ++q) cp[q] = 0.0;
     for (int t = 0; t < s.ntiles; ++t)
         for (int q = 0; q < NSLOT; ++q) cp[q] += s.h_const[(size_t)t * NSLOT + q];
@@ -704,7 +731,7 @@ void Engine::remove(int id)
     if (s.snap_pi) cudaFreeAsync(s.snap_pi, stream_);
     if (s.fetched) cudaEventSynchronize(s.ev);
     pinned_.put(s.h_jout, (size_t)s.Nt * NSLOT * 8);
-    pinned_.put(s.h_const, (size_t)s.ntiles * NSLOT * 8);
+    pinned_.put(s.h_const, ((size_t)s.ntiles * NSLOT + kMaxGroups) * 8);
     cudaEventDestroy(s.ev);
     bytes_in_use_ -= s.bytes;
     free_slots_.push_back(s.slot);

@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 
@@ -179,6 +180,50 @@ struct TileReducer {
     }
 };
 
+// -------------------------------------------------------------- tile queue
+// The CTA's next item, or -1 (see TileQueue).  The propagate kernels have an
+// instance with the queue (QU) and one without: the loop around the tile costs
+// registers (14 % of a small length-gauge solve, which needs no queue).
+__device__ __forceinline__ int next_item(const TileQueue &q)
+{
+    __shared__ int item;
+    __syncthreads();   // the item before is finished with shared memory
+    if (threadIdx.x == 0) {
+        item = atomicAdd(q.ctr, 1);
+        if (item >= q.nitems && atomicAdd(q.ctr + 1, 1) == (int)gridDim.x - 1) {
+            q.ctr[1] = 0;   // every CTA has taken its last item
+            __threadfence();
+            q.ctr[0] = 0;
+        }
+    }
+    __syncthreads();
+    return item < q.nitems ? item : -1;
+}
+// Wait until the tile's state at step s0 is in memory (bounded; false: gave up)
+__device__ __forceinline__ bool tile_ready(const TileQueue &q, const int *prog, int s0, bool first)
+{
+    __shared__ int ok;
+    if (first) return true;
+    if (threadIdx.x == 0) {
+        int v = 0, n = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(prog) : "memory");
+        } while (v < s0 && ++n < (1 << 25) && *(volatile int *)(q.ctr + 2) == 0);
+        if (v < s0) q.ctr[2] = 1;
+        ok = v >= s0;
+    }
+    __syncthreads();
+    return ok;
+}
+__device__ __forceinline__ void tile_done(const TileQueue &q, int *prog, int s1)
+{
+    __syncthreads();   // the CTA's state stores
+    if (threadIdx.x == 0) {
+        __threadfence();
+        asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(prog), "r"(s1) : "memory");
+    }
+}
+
 // ------------------------------------------------------ velocity gauge
 // The state is rho - rho0 in the band basis: (da, db, z) = (drho_00,
 // drho_11, rho_01).  Starting from rho = rho0, d(db)/dt = -d(da)/dt term by
@@ -257,21 +302,24 @@ template <class Real, int RK> constexpr int vg_stage_bytes(int threads)
 // butterfly per step (18 shuffles, 28 selects, 9 adds) held up the warp's
 // in-order issue; and the field table is read SUB steps ahead into shared
 // memory, where a read in the step waited for L2 every third step.
-template <class Real, int RK, int KPT, bool G1>
+template <class Real, int RK, int KPT, bool G1, bool QU>
 __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const TileDev *__restrict__ tiles,
-                                                    const SolveDev *__restrict__ solves, int tick, int S)
+                                                    const SolveDev *__restrict__ solves, int tick, int S,
+                                                    TileQueue queue)
 {
     using T2 = typename V2<Real>::T;
     using TB = Tableau<RK>;
     constexpr bool F64 = std::is_same<Real, double>::value;
     constexpr int NA = TB::NT - 1;
     extern __shared__ __align__(16) double vg_dyn[];   // vg_stage_bytes(blockDim.x)
-    const TileDev tl = tiles[blockIdx.x];
+    for (int item = QU ? next_item(queue) : (int)blockIdx.x; item >= 0; item = QU ? next_item(queue) : -1) {
+    const TileDev tl = tiles[QU ? item % queue.ntiles : item];
     const SolveDev &sd = solves[tl.solve];
-    const int s0 = (tick - sd.admit_tick) * S;
-    const int Nt = sd.Nt;
-    if (s0 < 0 || s0 >= Nt) return;
-    const int s1 = min(s0 + S, Nt);
+    const int sl = (tick - sd.admit_tick) * S;   // the launch's first step of this solve
+    const int s0 = QU ? sl + item / queue.ntiles * queue.chunk : sl;
+    const int s1 = min(QU ? min(sl + S, s0 + queue.chunk) : sl + S, sd.Nt);
+    if (sl < 0 || s0 >= s1) continue;
+    if (QU && !tile_ready(queue, sd.prog + tl.tile, s0, s0 == sl)) continue;
     const int nkp = sd.nk_pad, ntiles = sd.ntiles;
     const Real *__restrict__ kc = static_cast<const Real *>(sd.kc);
     double *__restrict__ st = static_cast<double *>(sd.st);
@@ -450,7 +498,7 @@ __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const Til
         }
         if ((int)threadIdx.x < nn) sA[(buf ^ 1) * SUB * NA + threadIdx.x] = pre;
         for (int i = threadIdx.x + blockDim.x; i < nn; i += blockDim.x) sA[(buf ^ 1) * SUB * NA + i] = table(b0 + SUB, i);
-        red.flush(nb, b0 - s0, ntiles, tl.tile, partial);
+        red.flush(nb, b0 - sl, ntiles, tl.tile, partial);
     }
 #pragma unroll
     for (int j = 0; j < KPT; ++j)
@@ -459,6 +507,8 @@ __global__ void __launch_bounds__(RK == 4 ? 512 : 256, 1) propagate_vg(const Til
             for (int q = 0; q < D_N; ++q) st[(size_t)slot[q] * nkp + kidx[j]] = y64[j][q];
             st[(size_t)VG_DB * nkp + kidx[j]] = -y64[j][D_DA];
         }
+    if (QU) tile_done(queue, sd.prog + tl.tile, s1);
+    }
 }
 
 // Mixed method, velocity gauge, two k-points per thread packed into f32x2
@@ -507,7 +557,8 @@ __device__ __forceinline__ void vg_rhs2(const VgField2 &h, float2 hc0, const flo
 
 template <int RK, bool G1>
 __global__ void __launch_bounds__(256) propagate_vg_x2(const TileDev *__restrict__ tiles,
-                                                       const SolveDev *__restrict__ solves, int tick, int S)
+                                                       const SolveDev *__restrict__ solves, int tick, int S,
+                                                       TileQueue)
 {
     using TB = Tableau<RK>;
     __shared__ RedStage red_s;
@@ -515,9 +566,8 @@ __global__ void __launch_bounds__(256) propagate_vg_x2(const TileDev *__restrict
     const TileDev tl = tiles[blockIdx.x];
     const SolveDev &sd = solves[tl.solve];
     const int s0 = (tick - sd.admit_tick) * S;
-    const int Nt = sd.Nt;
-    if (s0 < 0 || s0 >= Nt) return;
-    const int s1 = min(s0 + S, Nt);
+    const int s1 = min(s0 + S, sd.Nt);
+    if (s0 < 0 || s0 >= s1) return;
     const int nkp = sd.nk_pad, ntiles = sd.ntiles;
     const float *__restrict__ kc = static_cast<const float *>(sd.kc);
     double *__restrict__ st = static_cast<double *>(sd.st);
@@ -937,18 +987,21 @@ __device__ __forceinline__ void lw_B64(const Real (&c)[LW_NCONST], const Real *p
 // factors and the new state.  FP64-pipe bound on large grids, a serial chain on
 // small ones: the table is copied SUB steps ahead to shared memory (a read in
 // the step waited for L2) and the currents' sums go through LwStage.
-template <class Real, int RK, bool G1>
+template <class Real, int RK, bool G1, bool QU>
 __global__ void __launch_bounds__(256, 2) propagate_lw(const TileDev *__restrict__ tiles,
-                                                    const SolveDev *__restrict__ solves, int tick, int S)
+                                                    const SolveDev *__restrict__ solves, int tick, int S,
+                                                    TileQueue queue)
 {
     using TB = Tableau<RK>;
     extern __shared__ __align__(16) double red_dyn[];   // lw_stage_bytes(blockDim.x)
-    const TileDev tl = tiles[blockIdx.x];
+    for (int item = QU ? next_item(queue) : (int)blockIdx.x; item >= 0; item = QU ? next_item(queue) : -1) {
+    const TileDev tl = tiles[QU ? item % queue.ntiles : item];
     const SolveDev &sd = solves[tl.solve];
-    const int s0 = (tick - sd.admit_tick) * S;
-    const int Nt = sd.Nt;
-    if (s0 < 0 || s0 >= Nt) return;
-    const int s1 = min(s0 + S, Nt);
+    const int sl = (tick - sd.admit_tick) * S;   // the launch's first step of this solve
+    const int s0 = QU ? sl + item / queue.ntiles * queue.chunk : sl;
+    const int s1 = min(QU ? min(sl + S, s0 + queue.chunk) : sl + S, sd.Nt);
+    if (sl < 0 || s0 >= s1) continue;
+    if (QU && !tile_ready(queue, sd.prog + tl.tile, s0, s0 == sl)) continue;
     const int nkp = sd.nk_pad, ntiles = sd.ntiles;
     constexpr bool F64 = std::is_same<Real, double>::value;
     const Real *__restrict__ kc = static_cast<const Real *>(sd.kc);
@@ -975,7 +1028,7 @@ __global__ void __launch_bounds__(256, 2) propagate_lw(const TileDev *__restrict
     for (int q = 0; q < LW_NCONST; ++q) c[q] = ok ? kc[(size_t)q * nkp + kidx] : Real(0);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        y64[q] = ok ? st[(size_t)q * nkp + kidx] : 0.0;
+        y64[q] = ok ? __ldcg(st + (size_t)q * nkp + kidx) : 0.0;
         yr[q] = Real(y64[q]);
     }
     if (!ok) c[LW_CA0] = c[LW_CB0] = Real(1);  // padding lanes: a harmless k = 0 point, weight 0
@@ -1069,11 +1122,13 @@ __global__ void __launch_bounds__(256, 2) propagate_lw(const TileDev *__restrict
         if (e % VSTEP == VSTEP - 1 || e == nb - 1) stage.sum(red, e - e % VSTEP, e % VSTEP + 1);
       }
       __pipeline_wait_prior(0);
-      red.flush(nb, b0 - s0, ntiles, tl.tile, sd.partial);
+      red.flush(nb, b0 - sl, ntiles, tl.tile, sd.partial);
     }
     if (ok)
 #pragma unroll
         for (int q = 0; q < 4; ++q) st[(size_t)q * nkp + kidx] = y64[q];
+    if (QU) tile_done(queue, sd.prog + tl.tile, s1);
+    }
 }
 
 // Mixed method, length gauge, two k-points per thread in f32x2 registers (as
@@ -1167,18 +1222,21 @@ __device__ __forceinline__ void lw_current2(const LwCurK2 &K, const LwTrig2 &T, 
     v[7] = -(o3.x + o3.y);
 }
 
-template <int RK, bool G1>
+template <int RK, bool G1, bool QU>
 __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restrict__ tiles,
-                                                       const SolveDev *__restrict__ solves, int tick, int S)
+                                                       const SolveDev *__restrict__ solves, int tick, int S,
+                                                    TileQueue queue)
 {
     using TB = Tableau<RK>;
     extern __shared__ __align__(16) double red_dyn[];   // lw_stage_bytes(blockDim.x)
-    const TileDev tl = tiles[blockIdx.x];
+    for (int item = QU ? next_item(queue) : (int)blockIdx.x; item >= 0; item = QU ? next_item(queue) : -1) {
+    const TileDev tl = tiles[QU ? item % queue.ntiles : item];
     const SolveDev &sd = solves[tl.solve];
-    const int s0 = (tick - sd.admit_tick) * S;
-    const int Nt = sd.Nt;
-    if (s0 < 0 || s0 >= Nt) return;
-    const int s1 = min(s0 + S, Nt);
+    const int sl = (tick - sd.admit_tick) * S;   // the launch's first step of this solve
+    const int s0 = QU ? sl + item / queue.ntiles * queue.chunk : sl;
+    const int s1 = min(QU ? min(sl + S, s0 + queue.chunk) : sl + S, sd.Nt);
+    if (sl < 0 || s0 >= s1) continue;
+    if (QU && !tile_ready(queue, sd.prog + tl.tile, s0, s0 == sl)) continue;
     const int nkp = sd.nk_pad, ntiles = sd.ntiles;
     const float *__restrict__ kc = static_cast<const float *>(sd.kc);
     double *__restrict__ st = static_cast<double *>(sd.st);
@@ -1217,11 +1275,11 @@ __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restr
     float2 yhi[4], acc[4], yr[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        y64[0][q] = ok0 ? st[(size_t)q * nkp + k0] : 0.0;
-        y64[1][q] = ok1 ? st[(size_t)q * nkp + k1] : 0.0;
+        y64[0][q] = ok0 ? __ldcg(st + (size_t)q * nkp + k0) : 0.0;
+        y64[1][q] = ok1 ? __ldcg(st + (size_t)q * nkp + k1) : 0.0;
         yhi[q] = make_float2(float(y64[0][q]), float(y64[1][q]));
-        acc[q] = make_float2(ok0 ? float(st[(size_t)(LW_ACC + q) * nkp + k0]) : 0.f,
-                             ok1 ? float(st[(size_t)(LW_ACC + q) * nkp + k1]) : 0.f);
+        acc[q] = make_float2(ok0 ? float(__ldcg(st + (size_t)(LW_ACC + q) * nkp + k0)) : 0.f,
+                             ok1 ? float(__ldcg(st + (size_t)(LW_ACC + q) * nkp + k1)) : 0.f);
         yr[q] = add2(yhi[q], acc[q]);
     }
     const int nwarp = blockDim.x >> 5, warp = threadIdx.x >> 5;
@@ -1325,7 +1383,7 @@ __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restr
         if (e % VSTEP == VSTEP - 1 || e == nb - 1) stage.sum(red, e - e % VSTEP, e % VSTEP + 1);
       }
       __pipeline_wait_prior(0);
-      red.flush(nb, b0 - s0, ntiles, tl.tile, sd.partial);
+      red.flush(nb, b0 - sl, ntiles, tl.tile, sd.partial);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -1337,6 +1395,8 @@ __global__ void __launch_bounds__(256, 2) propagate_lw_x2(const TileDev *__restr
             st[(size_t)q * nkp + k1] = y64[1][q];
             st[(size_t)(LW_ACC + q) * nkp + k1] = double(acc[q].y);
         }
+    }
+    if (QU) tile_done(queue, sd.prog + tl.tile, s1);
     }
 }
 
@@ -1571,32 +1631,57 @@ __global__ void __launch_bounds__(256) fma_peak_x2(float *out, int iters, float 
 #define SBE_CHECK_LAUNCH() return cudaGetLastError()
 constexpr int kMaxDev = 64;
 
-// The velocity-gauge kernels' stages live in dynamic shared memory, above the
-// 48 KiB default for large CTAs: the limit is raised once per device and
-// kernel instance.
-template <class K> static cudaError_t raise_smem(K kernel, std::atomic<int> *raised, int max_bytes)
+using PropKernel = void (*)(const TileDev *, const SolveDev *, int, int, TileQueue);
+// Launch a propagate kernel: the plain instance with one CTA per tile, or the
+// queued one (q) with the CTAs the GPU holds, where the tiles outnumber them,
+// in chunks of an eighth of the launch's steps (at least 64).  A chunk costs
+// its CTA the tile's constants and state from L2, 1 to 2 us against ~0.9 us a
+// step, and the launch's tail shrinks to 1 / (8 waves).  Measured (1.4 to 3 waves;
+// us a step without / with): length gauge FP64 400^2 RK4 3.19 / 2.99, 240^2
+// Fehlberg-5 2.60 / 2.19, mixed 600^2 3.40 / 3.23; velocity gauge FP64 300^2
+// Fehlberg-5 1.13 / 1.06, RK4 600^2 2.10 / 2.10 (its last wave is FP64-pipe bound
+// too); mixed velocity gauge 600^2 1.25 / 1.26, and a burst of server requests 212 /
+// 246 ms with chunks of 32 steps: it has no queued instance.
+struct PropState {
+    std::atomic<int> raised[kMaxDev], slots[17];   // per kernel; CTAs the GPU holds by CTA size (one kind of GPU)
+};
+static cudaError_t launch_prop(const LaunchArgs &la, PropKernel plain, PropKernel queued, int bytes, int max_bytes,
+                               PropState &ps)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
-    if (raised[dev].load(std::memory_order_acquire) == 0) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_bytes);
-        if (e != cudaSuccess) return e;
-        raised[dev].store(1, std::memory_order_release);
+    if (ps.raised[dev].load(std::memory_order_acquire) == 0) {   // above the 48 KiB default for large CTAs
+        for (PropKernel k : {plain, queued})
+            if (k && (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_bytes)) != cudaSuccess) return e;
+        ps.raised[dev].store(1, std::memory_order_release);
     }
-    return cudaSuccess;
+    TileQueue q{nullptr, la.ntiles, la.S, la.ntiles};
+    std::atomic<int> &n = ps.slots[la.threads / 32];
+    if (queued && la.queue && la.S > 64 && n.load(std::memory_order_relaxed) == 0) {
+        int sms = 0, per = 0;
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, queued, la.threads, bytes)) != cudaSuccess) return e;
+        n.store(std::max(1, sms * per), std::memory_order_relaxed);
+    }
+    const int held = n.load(std::memory_order_relaxed), chunk = std::max(64, (la.S + 7) / 8);
+    const long long items = (long long)la.ntiles * ((la.S + chunk - 1) / chunk);
+    if (queued && la.queue && la.S > 64 && la.ntiles > held && items < 0x40000000ll) {
+        q = TileQueue{la.queue, la.ntiles, chunk, (int)items};
+        queued<<<held, la.threads, bytes, la.stream>>>(la.tiles, la.solves, la.tick, la.S, q);
+    } else {
+        plain<<<la.ntiles, la.threads, bytes, la.stream>>>(la.tiles, la.solves, la.tick, la.S, q);
+    }
+    SBE_CHECK_LAUNCH();
 }
 
 template <class Real, int RK, int KPT, bool G1>
 static cudaError_t launch_vg_g(const LaunchArgs &la)
 {
-    static std::atomic<int> raised[kMaxDev];
-    cudaError_t e = raise_smem(propagate_vg<Real, RK, KPT, G1>, raised, vg_stage_bytes<Real, RK>(RK == 4 ? 512 : 256));
-    if (e != cudaSuccess) return e;
-    propagate_vg<Real, RK, KPT, G1>
-        <<<la.ntiles, la.threads, vg_stage_bytes<Real, RK>(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    SBE_CHECK_LAUNCH();
+    static PropState ps;
+    return launch_prop(la, propagate_vg<Real, RK, KPT, G1, false>, propagate_vg<Real, RK, KPT, G1, true>,
+                       vg_stage_bytes<Real, RK>(la.threads), vg_stage_bytes<Real, RK>(RK == 4 ? 512 : 256), ps);
 }
 template <class Real, int RK, int KPT>
 static cudaError_t launch_vg_t(const LaunchArgs &la, bool g1)
@@ -1607,11 +1692,8 @@ static cudaError_t launch_vg_t(const LaunchArgs &la, bool g1)
 template <int RK, bool G1>
 static cudaError_t launch_vg_x2_t(const LaunchArgs &la)
 {
-    static std::atomic<int> raised[kMaxDev];
-    cudaError_t e = raise_smem(propagate_vg_x2<RK, G1>, raised, xstage_bytes(256));
-    if (e != cudaSuccess) return e;
-    propagate_vg_x2<RK, G1><<<la.ntiles, la.threads, xstage_bytes(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    SBE_CHECK_LAUNCH();
+    static PropState ps;
+    return launch_prop(la, propagate_vg_x2<RK, G1>, nullptr, xstage_bytes(la.threads), xstage_bytes(256), ps);
 }
 
 template <int RK>
@@ -1623,12 +1705,9 @@ static cudaError_t launch_vg_x2(const LaunchArgs &la, bool g1)
 template <class Real, int RK, bool G1>
 static cudaError_t launch_lw_g(const LaunchArgs &la)
 {
-    static std::atomic<int> raised[kMaxDev];
-    cudaError_t e = raise_smem(propagate_lw<Real, RK, G1>, raised, lw_stage_bytes<Real, RK>(256));
-    if (e != cudaSuccess) return e;
-    propagate_lw<Real, RK, G1>
-        <<<la.ntiles, la.threads, lw_stage_bytes<Real, RK>(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    SBE_CHECK_LAUNCH();
+    static PropState ps;
+    return launch_prop(la, propagate_lw<Real, RK, G1, false>, propagate_lw<Real, RK, G1, true>,
+                       lw_stage_bytes<Real, RK>(la.threads), lw_stage_bytes<Real, RK>(256), ps);
 }
 template <class Real, int RK>
 static cudaError_t launch_lw_t(const LaunchArgs &la, bool g1)
@@ -1639,12 +1718,9 @@ static cudaError_t launch_lw_t(const LaunchArgs &la, bool g1)
 template <int RK, bool G1>
 static cudaError_t launch_lw_x2_t(const LaunchArgs &la)
 {
-    static std::atomic<int> raised[kMaxDev];
-    cudaError_t e = raise_smem(propagate_lw_x2<RK, G1>, raised, lw_stage_bytes<float, RK>(256));
-    if (e != cudaSuccess) return e;
-    propagate_lw_x2<RK, G1>
-        <<<la.ntiles, la.threads, lw_stage_bytes<float, RK>(la.threads), la.stream>>>(la.tiles, la.solves, la.tick, la.S);
-    SBE_CHECK_LAUNCH();
+    static PropState ps;
+    return launch_prop(la, propagate_lw_x2<RK, G1, false>, propagate_lw_x2<RK, G1, true>,
+                       lw_stage_bytes<float, RK>(la.threads), lw_stage_bytes<float, RK>(256), ps);
 }
 
 int propagate_max_threads(int variant, int precision, int rk, int kpt)

@@ -15,6 +15,7 @@ struct LaunchArgs {
     int tick, S;             // launch index and steps per launch
     int variant, precision, rk, kpt;
     bool has_g1;             // T1 dephasing active
+    int *queue;              // 3 zeroed ints: the launch may queue its tiles (TileQueue), or null
     cudaStream_t stream;
 };
 

@@ -116,7 +116,7 @@ Shape autotune_shape(int device, const Problem &p, int precision)
     if (vg || precision != PREC_FP64)
         for (int t = 32; t <= propagate_max_threads(variant, precision, p.rk, 2); t += 32) addc(t, 2);
     Problem q = p;
-    const int S = 128;
+    const int S = 256;   // long enough for the tile queue of the larger grids
     q.laser.Nt = std::min(p.laser.Nt, 3 * S);
     cudaStream_t st;
     cuda_check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream create");
