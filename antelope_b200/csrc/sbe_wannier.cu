@@ -1485,7 +1485,7 @@ cudaError_t launch_wan_attempt(const WanDev &w, const WanDev *dw, int precision,
 {
     if (wan_proj(w)) {
         const int unit = wan_proj_unit(w.N);
-        return launch_wan_attempt_p(w.N, w.gr_n, dw, nullptr, nullptr, (w.ntiles + unit - 1) / unit, st);
+        return launch_wan_attempt_p(w.N, w.gr_n, w.rk == 4 ? 4 : 6, dw, nullptr, nullptr, (w.nk + unit - 1) / unit, st);
     }
     if (wan_grouped(w))
         return launch_grouped(w.N, w.nR, w.rk, dw, nullptr, nullptr, (w.ntiles + WG_WARPS - 1) / WG_WARPS,

@@ -198,16 +198,17 @@ cudaError_t launch_wan_steps(const WanStepClass &c, const WanDev *dw, const WanD
 cudaError_t launch_wan_finish(const WanDev *dw, const WanDev *const *descs, int nsolves, int S, cudaStream_t st);
 cudaError_t launch_wan_step_fields(const WanDev &w, const WanDev *dw, cudaStream_t st);
 // Projection attempts (sbe_wanproj.cu): the plain method of the length gauge on
-// explicit tables at N = 3 ... 6, on grids where no bands meet.  A block covers
-// wan_proj_unit() tiles; solves of a class (equal N) share launches, ngrp and
-// nitems (rows x stages) being the largest of them.
+// explicit tables at N = 3 ... 6, on grids where no bands meet.  A block covers a
+// unit of wan_proj_unit() k-points, and batched lists have units in `tile`;
+// solves of a class (equal N) share launches, ngrp, S (stages) and nitems (rows
+// x stages) being the largest of them.
 constexpr int WAN_PROJ_MAXGRP = 64;
 bool wan_proj_applies(const WanDev &w);   // before its tables exist
 bool wan_proj(const WanDev &w);
 int wan_proj_unit(int N);
 int wan_proj_entries(int N, int ngrp, int nq);
-cudaError_t launch_wan_attempt_p(int N, int ngrp, const WanDev *dw, const WanDev *const *descs, const WanTileRef *tiles,
-                                 int nblocks, cudaStream_t st);
+cudaError_t launch_wan_attempt_p(int N, int ngrp, int S, const WanDev *dw, const WanDev *const *descs,
+                                 const WanTileRef *tiles, int nblocks, cudaStream_t st);
 cudaError_t launch_wan_next(int N, const WanDev *dw, const WanDev *const *descs, int nsolves, int nitems, bool first,
                             cudaStream_t st);
 cudaError_t launch_wan_snapshot_batch(int N, int nR_max, const WanDev *const *descs, const WanTileRef *tiles,

@@ -23,9 +23,17 @@
 //    forms the G (and those of E.D) of every row and stage between attempts.
 //    FP64 method only: the mixed method keeps its FP32 sums over the pairs.
 //
-// Layout: G lanes per k-point (8 for N > 4), one warp per block; lane l owns
-// the upper elements u = l + G j of the state, and lane m < N forms row m of
-// the products, the other factor read by element at one address per group.
+// Layout: one warp per block; N/2 lanes per k-point for even N, two rows of its
+// matrices each, and N lanes for odd N, one row each (PD below): 10 k-points per
+// warp at N = 6.  All lanes work, only the kept half of each Hermitian product is
+// formed, and an element read from shared memory serves two rows.  That read was
+// the limit of one row per lane in groups of 8 (a 16-byte element at one address
+// per group costs 4 wavefronts, whatever the number of groups; 4 k-points per
+// warp, 6 of 8 lanes at work): Cash-Karp attempts of N = 6, 4, 3 on 200 x 300
+// points took 681, 251 and 144 us, now 408, 144 and 103; on 100 x 100 162, 82 and
+// 52, now 90, 51 and 46; on 8 x 8 68, 61 and 41, now 65, 41 and 37.
+// Bound: latencies at two warps a scheduler (255 registers), half of them in the
+// table reads of the Fourier sums; FP64 issue a quarter to a third of the time.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -71,77 +79,208 @@ __constant__ PTab c_tab[3] = {
       512. / 1771. - 1. / 4.}}};
 __device__ __forceinline__ int tab_of(int rk) { return rk == 4 ? 0 : rk == 5 ? 1 : 2; }
 
+// A k-point's G lanes share its Hermitian matrices by circulant diagonals: lane m
+// owns row m (and m + N/2 when N is even) of the elements (r, r + d mod N), d <=
+// N/2 -- of the diagonal d = N/2 of an even N the rows r < N/2 only.  Every lane
+// then has the same elements relative to its row, and equal work.
 template <int N> struct PD {
-    static constexpr int G = N <= 4 ? 4 : 8, KW = 32 / G, NN = N * N, NU = N * (N + 1) / 2;
-    static constexpr int NO = (NU + G - 1) / G;   // owned upper elements per lane
-    static constexpr int LDT = N | 1;
-    // a k-point's shared memory in complex numbers: Y, H0, H0 + E.D packed, T rows
-    // (odd stride: the groups of a warp read one element each from distinct banks)
-    static constexpr int Y = 0, H0 = NU, HT = 2 * NU, T = 3 * NU, END = (T + N * LDT) | 1;
+    static constexpr bool EVEN = N % 2 == 0;
+    static constexpr int M = N / 2, G = EVEN ? M : N, KW = 32 / G, LW = KW * G, NN = N * N;
+    static constexpr int DO = EVEN ? N - 1 : M;   // owned elements off the diagonal
+    static constexpr int NE = DO + 1;             // entries of an owned set; the last: its diagonal elements
+    static constexpr int NM = (M + 1) * N;        // slots [d][r] of a matrix (d = N/2 of an even N twice)
+    // the matrices of a k-point in complex numbers: Y, H0, H0 + E.D (later T, P);
+    // the stride puts the lanes of a warp's groups on distinct banks
+    static constexpr int Y = 0, H0 = NM, HT = 2 * NM;
+    static constexpr int END = 3 * NM + (N == 6 ? 3 : N == 4 ? 2 : N == 3 ? 1 : 0);
+    static constexpr int TN = (N - 1 - M) * N;    // slots of the product's unowned elements
+    __host__ __device__ static constexpr int slot(int d, int r) { return d * N + r; }
 };
-__host__ __device__ constexpr int up(int m, int n, int N) { return m * N - m * (m - 1) / 2 + (n - m); }
 
-template <int N> __device__ __forceinline__ double2 herm(const double2 *P, int a, int b)
+// o += a x (conj(x) if CJ), of numbers known real (ar, xr) and of the parts of
+// o that are wanted; all four known when the loops are unrolled
+__device__ __forceinline__ void mac(double2 &o, const double2 &a, bool ar, const double2 &x, bool xr, bool cj, bool re, bool im)
 {
-    return a <= b ? P[up(a, b, N)] : cconj(P[up(b, a, N)]);
-}
-// Re sum_n a_n conj(b_n): three chains
-template <int N> __device__ __forceinline__ double row_dot(const double2 (&a)[N], const double2 (&b)[N])
-{
-    double s[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-        s[(2 * n) % 3] = fma(a[n].x, b[n].x, s[(2 * n) % 3]);
-        s[(2 * n + 1) % 3] = fma(a[n].y, b[n].y, s[(2 * n + 1) % 3]);
+    if (re) {
+        o.x = fma(a.x, x.x, o.x);
+        if (!ar && !xr) o.x = fma(cj ? a.y : -a.y, x.y, o.x);
     }
-    return (s[0] + s[1]) + s[2];
+    if (im) {
+        if (!xr) o.y = fma(cj ? -a.x : a.x, x.y, o.y);
+        if (!ar) o.y = fma(a.y, x.x, o.y);
+    }
 }
-template <int G> __device__ __forceinline__ double gsum(double v)
+// Tr(XY) of a lane's owned elements: three chains
+template <int N> __device__ __forceinline__ double dot(const double2 (&a)[PD<N>::NE], const double2 (&b)[PD<N>::NE])
 {
+    constexpr int DO = PD<N>::DO;
+    double s = 0.0, t = 0.0;
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(ALL, v, o);
-    return v;
+    for (int j = 0; j < DO; ++j) {
+        s = fma(a[j].x, b[j].x, s);
+        t = fma(a[j].y, b[j].y, t);
+    }
+    double u = a[DO].x * b[DO].x;
+    if (PD<N>::EVEN) u = fma(a[DO].y, b[DO].y, u);
+    return fma(2.0, s + t, u);
 }
-
-// c = row a times the Hermitian matrix M (packed upper triangle, each element
-// read once at one address per group)
-template <int N> __device__ __forceinline__ void row_herm(double2 (&c)[N], const double2 (&a)[N], const double2 *M)
+// sum over a group's lanes, in lane order (the same bits in every lane)
+template <int G> __device__ __forceinline__ double gsum(double v, int base)
 {
+    double s = __shfl_sync(ALL, v, base);
 #pragma unroll
-    for (int n = 0; n < N; ++n) c[n] = make_double2(0.0, 0.0);
+    for (int i = 1; i < G; ++i) s += __shfl_sync(ALL, v, base + i);
+    return s;
+}
+// an owned set to its slots
+template <int N> __device__ __forceinline__ void put(double2 *P, const double2 (&x)[PD<N>::NE], int m)
+{
+    using D = PD<N>;
+#pragma unroll
+    for (int d = 1; d <= D::M; ++d) P[D::slot(d, m)] = x[d - 1];
+    P[m].x = x[D::DO].x;
+    if (D::EVEN) {
+        P[D::slot(D::M, m + D::M)] = cconj(x[D::M - 1]);
+#pragma unroll
+        for (int d = 1; d < D::M; ++d) P[D::slot(d, m + D::M)] = x[D::M + d - 1];
+        P[m + D::M].x = x[D::DO].y;
+    }
+}
+// element (l, c) relative to the lane's row: ro[i] = (m + i) mod N
+template <int N> __device__ __forceinline__ double2 elem(const double2 *P, const int (&ro)[N], int l, int c)
+{
+    using D = PD<N>;
+    const int d = (c - l + N) % N;
+    if (d == 0) return make_double2(P[ro[l]].x, 0.0);
+    if (d <= D::M) return P[D::slot(d, ro[l])];
+    return cconj(P[D::slot(N - d, ro[c])]);
+}
+// the lane's rows of a matrix, columns relative to row m
+template <int N> struct Rows {
+    double2 a[N], b[N];   // row m, row m + N/2
+    __device__ __forceinline__ void load(const double2 *P, const int (&ro)[N])
+    {
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            a[c] = elem<N>(P, ro, 0, c);
+            if (PD<N>::EVEN) b[c] = elem<N>(P, ro, PD<N>::M, c);
+        }
+    }
+};
+// w = (H P) at the owned elements (H, P commute: the product is Hermitian); each
+// element of P is read once
+template <int N>
+__device__ __forceinline__ void product(double2 (&w)[PD<N>::NE], const Rows<N> &H, const double2 *P, const int (&ro)[N])
+{
+    using D = PD<N>;
+    constexpr int M = D::M;
+    double2 oa[N], ob[N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) oa[c] = ob[c] = make_double2(0.0, 0.0);
+    // columns a lane keeps: of row m 0 .. N/2, of row m + N/2 the N/2 from its own
+    auto add = [&](int l, int c, const double2 &x, bool cj) {   // the term of column c with H's element l
+        if (c <= M) mac(oa[c], H.a[l], l == 0, x, l == c, cj, true, c != 0);
+        const int d = (c - M + N) % N;
+        if (D::EVEN && d < M) mac(ob[c], H.b[l], l == M, x, l == c, cj, true, d != 0);
+    };
 #pragma unroll
     for (int l = 0; l < N; ++l)
 #pragma unroll
-        for (int n = l; n < N; ++n) {
-            const double2 x = M[up(l, n, N)];
-            cfma(c[n], a[l], x);
-            if (n != l) cfma(c[l], a[n], cconj(x));
+        for (int c = l; c < N; ++c) {
+            const double2 x = elem<N>(P, ro, l, c);
+            add(l, c, x, false);
+            if (l != c) add(c, l, x, true);
         }
+#pragma unroll
+    for (int d = 1; d <= M; ++d) w[d - 1] = oa[d];
+    w[D::DO] = make_double2(oa[0].x, 0.0);
+    if (D::EVEN) {
+#pragma unroll
+        for (int d = 1; d < M; ++d) w[M + d - 1] = ob[(M + d) % N];
+        w[D::DO].y = ob[M].x;
+    }
+}
+// c = (H Y) - (H Y)^dag at the owned elements, its imaginary diagonal in the last
+// entry; T: room for the elements that other lanes need (may be H's own slots)
+template <int N>
+__device__ __forceinline__ void commutator(double2 (&w)[PD<N>::NE], const double2 *Hs, const double2 *Y, double2 *T,
+                                           const int (&ro)[N])
+{
+    using D = PD<N>;
+    constexpr int M = D::M;
+    Rows<N> H;
+    H.load(Hs, ro);
+    double2 oa[N], ob[N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) oa[c] = ob[c] = make_double2(0.0, 0.0);
+    auto add = [&](int l, int c, const double2 &x, bool cj) {
+        mac(oa[c], H.a[l], l == 0, x, l == c, cj, c != 0, true);
+        if (D::EVEN) mac(ob[c], H.b[l], l == M, x, l == c, cj, c != M, true);
+    };
+#pragma unroll
+    for (int l = 0; l < N; ++l)
+#pragma unroll
+        for (int c = l; c < N; ++c) {
+            const double2 x = elem<N>(Y, ro, l, c);
+            add(l, c, x, false);
+            if (l != c) add(c, l, x, true);
+        }
+    __syncwarp();
+#pragma unroll
+    for (int d = M + 1; d < N; ++d) {
+        T[(d - M - 1) * N + ro[0]] = oa[d];
+        if (D::EVEN) T[(d - M - 1) * N + ro[M]] = ob[(M + d) % N];
+    }
+    __syncwarp();
+    auto diff = [](const double2 &x, const double2 &y) { return make_double2(x.x - y.x, x.y + y.y); };
+#pragma unroll
+    for (int d = 1; d <= M; ++d)
+        w[d - 1] = diff(oa[d], D::EVEN && d == M ? ob[0] : T[(N - d - M - 1) * N + ro[d]]);
+    w[D::DO] = make_double2(2.0 * oa[0].y, 0.0);
+    if (D::EVEN) {
+#pragma unroll
+        for (int d = 1; d < M; ++d) w[M + d - 1] = diff(ob[(M + d) % N], T[(N - d - M - 1) * N + ro[(M + d) % N]]);
+        w[D::DO].y = 2.0 * ob[M].y;
+    }
+    __syncwarp();
+}
+// Re Tr(X (-i S)) of the owned elements, S anti-Hermitian with its imaginary
+// diagonal in the last entry
+template <int N>
+__device__ __forceinline__ double tr_s(const double2 (&x)[PD<N>::NE], const double2 (&s)[PD<N>::NE])
+{
+    constexpr int DO = PD<N>::DO;
+    double t = 0.0;
+#pragma unroll
+    for (int j = 0; j < DO; ++j) t += x[j].y * s[j].x - x[j].x * s[j].y;
+    double u = x[DO].x * s[DO].x;
+    if (PD<N>::EVEN) u += x[DO].y * s[DO].y;
+    return u - 2.0 * t;
 }
 
 }  // namespace
 
 // Shared memory of a block: slopes, the groups' matrices, the phases along the row
-template <int N> static int proj_bytes(int ngrp)
+template <int N> static int proj_bytes(int ngrp, int S)
 {
     using D = PD<N>;
-    return (5 * D::NO * 32 + D::KW * D::END + D::KW * ngrp) * 16;
+    return ((S - 1) * D::NE * D::LW + D::KW * D::END + D::KW * ngrp) * 16;
 }
 
 template <int N>
-__global__ void __launch_bounds__(32, N <= 4 ? 16 : 12)
+__global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
     wan_attempt_p(const WanDev *__restrict__ Pp, const WanDev *const *__restrict__ descs,
                   const WanTileRef *__restrict__ tiles)
 {
     using D = PD<N>;
-    constexpr int G = D::G, KW = D::KW, NU = D::NU, NO = D::NO, NN = D::NN;
+    constexpr int G = D::G, KW = D::KW, LW = D::LW, NE = D::NE, DO = D::DO, M = D::M, NN = D::NN;
     extern __shared__ __align__(16) double2 sm[];
     const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
     // KW k-points; consecutive units (they share the tables of a row) to the
     // blocks of one SM, which get every SPREAD-th block of the grid
     int unit;
     if (tiles) {
-        unit = tiles[blockIdx.x].tile * WAN_WARPS / KW;
+        unit = tiles[blockIdx.x].tile;
     } else {
         const int nu = (P.nk + KW - 1) / KW, i = (int)blockIdx.x % SPREAD;
         unit = (int)((long long)i * nu / SPREAD) + (int)blockIdx.x / SPREAD;
@@ -149,20 +288,21 @@ __global__ void __launch_bounds__(32, N <= 4 ? 16 : 12)
     }
     const WanCtl &ctl = *P.ctl;
     if (ctl.done) return;
-    const int lane = threadIdx.x, grp = lane / G, m = lane % G;
+    // lanes past the last group shadow its first lanes: same values, same addresses
+    const int lane = threadIdx.x, grp = min(lane / G, KW - 1), m = lane < LW ? lane % G : lane - LW;
+    const int base = grp * G, col = base + m;
     const int k = unit * KW + grp;
-    const bool live = k < P.nk, own = m < N;
-    const int kc = live ? k : P.nk - 1;   // a group past the grid shadows the last k-point
-    const int mr = own ? m : N - 1;
-    double2 *const ks = sm;                                      // [5][NO][32] slopes, a column per lane
-    double2 *const v = ks + 5 * NO * 32 + grp * D::END;
+    const bool live = k < P.nk && lane < LW;
+    const int kc = min(k, P.nk - 1);   // a group past the grid shadows the last k-point
+    const int S = c_tab[tab_of(P.rk)].S;
+    double2 *const ks = sm + col;                                // [S - 1][NE][LW] slopes, a column per lane
+    double2 *const v = sm + (S - 1) * NE * LW + grp * D::END;
     const int ng = P.gr_n, nent = 2 * ng - 1;                    // group pairs (g = 0 first), table entries
-    double2 *const ph = ks + 5 * NO * 32 + KW * D::END + grp * ng;
+    double2 *const ph = sm + (S - 1) * NE * LW + KW * D::END + grp * ng;
     const double h = ctl.hs;
     const int buf = ctl.buf;
     const bool cur = ctl.need_current;
     const PTab &tb = c_tab[tab_of(P.rk)];
-    const int S = tb.S;
     double kv[3], wk;
     kpoint(P, kc, kv, wk);
     // the row of this k-point and its phases along it
@@ -173,190 +313,178 @@ __global__ void __launch_bounds__(32, N <= 4 ? 16 : 12)
         sincos(f1 * P.gr_a[q], &sn, &cs);
         ph[q] = make_double2(cs, sn);
     }
-    // owned upper elements: (row, column) packed in bytes
-    int om[NO], on[NO];
-    double2 r64[NO];
+    int ro[N];   // rows and columns relative to the lane's row
+#pragma unroll
+    for (int i = 0; i < N; ++i) ro[i] = m + i < N ? m + i : m + i - N;
+    // the owned element j < DO: row m (m + N/2) and its column
+    auto erow = [&](int j) { return j < M ? ro[0] : ro[M % N]; };
+    auto ecol = [&](int j) { return j < M ? ro[j + 1] : ro[(j + 1) % N]; };
+    double2 r64[NE];
     const double2 *rho = P.rho[buf] + (size_t)kc * NN;
 #pragma unroll
-    for (int j = 0; j < NO; ++j) {
-        int u = min(m + G * j, NU - 1), a = 0;
-        while (u >= N - a) { u -= N - a; ++a; }
-        om[j] = a;
-        on[j] = a + u;
-        r64[j] = __ldcg(rho + om[j] * N + on[j]);
-        if (om[j] == on[j]) r64[j].y = 0.0;
+    for (int j = 0; j < DO; ++j) {
+        const int a = erow(j), b = ecol(j);
+        r64[j] = __ldcg(rho + min(a, b) * N + max(a, b));
+        if (a > b) r64[j].y = -r64[j].y;
     }
+    r64[DO].x = __ldcg(&rho[m * (N + 1)].x);
+    r64[DO].y = D::EVEN ? __ldcg(&rho[(m + M) * (N + 1)].x) : 0.0;
     const bool dip = P.has_dip;
     const int NQ = dip ? 2 : 1;
     const double g1 = P.g1, g2 = P.g2, gd = g1 - g2;
     const bool deph = g1 != 0.0 || g2 != 0.0;
-    double emax = 0.0;
-    double2 kl[NO];   // the last stage's slope
-    const size_t ent = (size_t)nent * NO * NQ * G;   // table entries of a (row, stage)
+    double2 kl[NE];   // the last stage's slope
+    const size_t ent = (size_t)nent * NE * NQ * G;   // table entries of a (row, stage)
     const double2 *tab = P.gr_tab + (size_t)row * S * ent + m;
     __syncwarp();
 
 #pragma unroll 1
     for (int s = 0; s < S; ++s, tab += ent) {
-        // stage input Y = rho + h sum_j a_sj k_j
-#pragma unroll
-        for (int j = 0; j < NO; ++j) {
-            double2 y = r64[j];
-            for (int i = 0; i < s; ++i) {
-                const double a = h * tb.a[s][i];
-                const double2 q = ks[(i * NO + j) * 32 + lane];
-                y = make_double2(fma(a, q.x, y.x), fma(a, q.y, y.y));
-            }
-            if (m + G * j < NU) v[D::Y + m + G * j] = y;
-        }
         // H0 and E.D at the owned elements; the next stage's table lines (128
         // bytes each) are fetched towards L1 meanwhile
         if (s + 1 < S)
             for (int i = lane * 8; i < (int)ent; i += 256)
                 asm volatile("prefetch.global.L1 [%0];" ::"l"(tab - m + ent + i));
-        double2 a0[NO], a1[NO];
+        {
+            double2 a0[NE], a1[NE];
 #pragma unroll
-        for (int j = 0; j < NO; ++j) {
-            a0[j] = __ldg(tab + (size_t)j * NQ * G);
-            a1[j] = dip ? __ldg(tab + (size_t)(j * NQ + 1) * G) : make_double2(0.0, 0.0);
-        }
-#pragma unroll 1
-        for (int q = 1; q < ng; ++q) {
-            const double2 e = ph[q];
-            const double2 *t0 = tab + (size_t)(2 * q - 1) * NO * NQ * G, *t1 = t0 + (size_t)NO * NQ * G;
-#pragma unroll
-            for (int j = 0; j < NO; ++j) {
-                const double2 sg = __ldg(t0 + j * NQ * G), ta = __ldg(t1 + j * NQ * G);
-                a0[j] = make_double2(fma(e.x, sg.x, fma(e.y, ta.x, a0[j].x)), fma(e.x, sg.y, fma(e.y, ta.y, a0[j].y)));
-                if (dip) {
-                    const double2 sd = __ldg(t0 + (j * NQ + 1) * G), td = __ldg(t1 + (j * NQ + 1) * G);
-                    a1[j] = make_double2(fma(e.x, sd.x, fma(e.y, td.x, a1[j].x)), fma(e.x, sd.y, fma(e.y, td.y, a1[j].y)));
-                }
+            for (int j = 0; j < NE; ++j) {
+                a0[j] = __ldg(tab + (size_t)j * NQ * G);
+                a1[j] = dip ? __ldg(tab + (size_t)(j * NQ + 1) * G) : make_double2(0.0, 0.0);
             }
-        }
-#pragma unroll
-        for (int j = 0; j < NO; ++j) {
-            if (m + G * j >= NU) continue;
-            if (om[j] == on[j]) a0[j].y = a1[j].y = 0.0;
-            v[D::H0 + m + G * j] = a0[j];
-            v[D::HT + m + G * j] = make_double2(a0[j].x + a1[j].x, a0[j].y + a1[j].y);
-        }
-        __syncwarp();
-        const bool with_cur = cur && s == 0;
-        double tot[2] = {0.0, 0.0};
-        // S_a waits in the columns of slopes that do not exist yet
-        double2 *const sv = ks + NO * 32 + lane;   // [a][j] at (a NO + j) 32
-        if (with_cur) {
-            // total current Re Tr(Y J_a), J_a = -i S_a + i [D_a, H0] (S_a = sum R_a h_R
-            // e^{iKR}): over the owned upper elements, with C = H0 Y - (H0 Y)^dag, the
-            // diagonal Y_mm Im(S_mm) - Im(C_mm) Re(D_mm), off it -2 Im(Y_mn conj(S_mn))
-            // - 2 Im(C_mn conj(D_mn))
-            const int NC = dip ? 4 : 2;   // S_x, S_y (, D_x, D_y)
-            const double2 *tc = P.gr_cur + (size_t)row * nent * NO * NC * G + m;
-            double2 dd[2][NO], sx[2][NO];
-#pragma unroll
-            for (int j = 0; j < NO; ++j)
-#pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    sx[a][j] = __ldg(tc + (size_t)(j * NC + a) * G);
-                    dd[a][j] = dip ? __ldg(tc + (size_t)(j * NC + 2 + a) * G) : make_double2(0.0, 0.0);
-                }
 #pragma unroll 1
             for (int q = 1; q < ng; ++q) {
                 const double2 e = ph[q];
-                const double2 *t0 = tc + (size_t)(2 * q - 1) * NO * NC * G, *t1 = t0 + (size_t)NO * NC * G;
+                const double2 *t0 = tab + (size_t)(2 * q - 1) * NE * NQ * G, *t1 = t0 + (size_t)NE * NQ * G;
 #pragma unroll
-                for (int j = 0; j < NO; ++j)
+                for (int j = 0; j < NE; ++j) {
+                    const double2 sg = __ldg(t0 + j * NQ * G), ta = __ldg(t1 + j * NQ * G);
+                    a0[j] = make_double2(fma(e.x, sg.x, fma(e.y, ta.x, a0[j].x)), fma(e.x, sg.y, fma(e.y, ta.y, a0[j].y)));
+                    if (dip) {
+                        const double2 sd = __ldg(t0 + (j * NQ + 1) * G), td = __ldg(t1 + (j * NQ + 1) * G);
+                        a1[j] = make_double2(fma(e.x, sd.x, fma(e.y, td.x, a1[j].x)), fma(e.x, sd.y, fma(e.y, td.y, a1[j].y)));
+                    }
+                }
+            }
+            put<N>(v + D::H0, a0, m);
 #pragma unroll
-                    for (int a = 0; a < 2; ++a) {
-                        const double2 x = __ldg(t0 + (j * NC + a) * G), y = __ldg(t1 + (j * NC + a) * G);
-                        double2 &z = sx[a][j];
-                        z = make_double2(fma(e.x, x.x, fma(e.y, y.x, z.x)), fma(e.x, x.y, fma(e.y, y.y, z.y)));
+            for (int j = 0; j < NE; ++j) a1[j] = make_double2(a0[j].x + a1[j].x, a0[j].y + a1[j].y);
+            put<N>(v + D::HT, a1, m);
+        }
+        // stage input Y = rho + h sum_j a_sj k_j
+        double2 y[NE];
+#pragma unroll
+        for (int j = 0; j < NE; ++j) y[j] = r64[j];
+#pragma unroll 1
+        for (int i = 0; i < s; ++i) {
+            const double a = h * tb.a[s][i];
+#pragma unroll
+            for (int j = 0; j < NE; ++j) {
+                const double2 q = ks[(i * NE + j) * LW];
+                y[j] = make_double2(fma(a, q.x, y[j].x), fma(a, q.y, y[j].y));
+            }
+        }
+        put<N>(v + D::Y, y, m);
+        __syncwarp();
+        const bool with_cur = cur && s == 0;
+        double tot[2] = {0.0, 0.0};
+        if (with_cur) {
+            // total current Re Tr(Y J_a), J_a = -i S_a + i [D_a, H0] (S_a = sum R_a h_R
+            // e^{iKR}): over the owned elements, with C = H0 Y - (H0 Y)^dag, the
+            // diagonal Y_mm Im(S_mm) - Im(C_mm) Re(D_mm), off it -2 Im(Y_mn conj(S_mn))
+            // - 2 Im(C_mn conj(D_mn)).  S_a and T wait in the columns of slopes that do
+            // not exist yet.
+            const int NC = dip ? 4 : 2;   // S_x, S_y (, D_x, D_y)
+            const double2 *tc = P.gr_cur + (size_t)row * nent * NE * NC * G + m;
+            double2 c[NE];
+            if (dip) commutator<N>(c, v + D::H0, v + D::Y, sm + 2 * NE * LW + grp * D::TN, ro);
+#pragma unroll 1
+            for (int a = 0; a < 2; ++a) {
+                double2 x[NE], d[NE];
+#pragma unroll
+                for (int j = 0; j < NE; ++j) {
+                    x[j] = __ldg(tc + (size_t)(j * NC + a) * G);
+                    d[j] = dip ? __ldg(tc + (size_t)(j * NC + 2 + a) * G) : make_double2(0.0, 0.0);
+                }
+#pragma unroll 1
+                for (int q = 1; q < ng; ++q) {
+                    const double2 e = ph[q];
+                    const double2 *t0 = tc + (size_t)(2 * q - 1) * NE * NC * G, *t1 = t0 + (size_t)NE * NC * G;
+#pragma unroll
+                    for (int j = 0; j < NE; ++j) {
+                        const double2 x1 = __ldg(t0 + (j * NC + a) * G), y1 = __ldg(t1 + (j * NC + a) * G);
+                        x[j] = make_double2(fma(e.x, x1.x, fma(e.y, y1.x, x[j].x)), fma(e.x, x1.y, fma(e.y, y1.y, x[j].y)));
                         if (dip) {
                             const double2 x2 = __ldg(t0 + (j * NC + 2 + a) * G), y2 = __ldg(t1 + (j * NC + 2 + a) * G);
-                            double2 &z2 = dd[a][j];
-                            z2 = make_double2(fma(e.x, x2.x, fma(e.y, y2.x, z2.x)), fma(e.x, x2.y, fma(e.y, y2.y, z2.y)));
+                            d[j] = make_double2(fma(e.x, x2.x, fma(e.y, y2.x, d[j].x)), fma(e.x, x2.y, fma(e.y, y2.y, d[j].y)));
                         }
                     }
-            }
-            if (dip) {
-                double2 hr[N], c[N];
-#pragma unroll
-                for (int l = 0; l < N; ++l) hr[l] = herm<N>(v + D::H0, mr, l);
-                row_herm<N>(c, hr, v + D::Y);
-                if (own)
-#pragma unroll
-                    for (int n = 0; n < N; ++n) v[D::T + m * D::LDT + n] = c[n];
-            }
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < NO; ++j) {
-                if (m + G * j >= NU) continue;
-                double2 c = make_double2(0.0, 0.0);
+                }
+                double t = tr_s<N>(y, x);
                 if (dip) {
-                    const double2 c1 = v[D::T + om[j] * D::LDT + on[j]], c2 = v[D::T + on[j] * D::LDT + om[j]];
-                    c = make_double2(c1.x - c2.x, c1.y + c2.y);
-                }
-                const double2 y = v[D::Y + m + G * j];
+                    double u = 0.0;
 #pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    const double2 x = sx[a][j], d = dd[a][j];
-                    sv[(a * NO + j) * 32] = x;
-                    if (om[j] == on[j]) tot[a] += y.x * x.y - c.y * d.x;
-                    else tot[a] -= 2.0 * (y.y * x.x - y.x * x.y) + 2.0 * (c.y * d.x - c.x * d.y);
+                    for (int j = 0; j < DO; ++j) u += c[j].y * d[j].x - c[j].x * d[j].y;
+                    t -= 2.0 * u + c[DO].x * d[DO].x;
+                    if (D::EVEN) t -= c[DO].y * d[DO].y;
                 }
+#pragma unroll
+                for (int j = 0; j < NE; ++j) ks[(a * NE + j) * LW] = x[j];
+                if (a == 0) tot[0] = t;
+                else tot[1] = t;
             }
-            __syncwarp();
         }
-        {   // row m of (H0 + E.D) Y
-            double2 hr[N], c[N];
+        // -i [H0 + E.D, Y] - g2 Y
+        double2 kn[NE];
+        commutator<N>(kn, v + D::HT, v + D::Y, v + D::HT, ro);
 #pragma unroll
-            for (int l = 0; l < N; ++l) hr[l] = herm<N>(v + D::HT, mr, l);
-            row_herm<N>(c, hr, v + D::Y);
-            if (own)
-#pragma unroll
-                for (int n = 0; n < N; ++n) v[D::T + m * D::LDT + n] = c[n];
+        for (int j = 0; j < NE; ++j) {
+            const double2 c = kn[j];
+            kn[j] = j < DO ? make_double2(fma(-g2, y[j].x, c.y), fma(-g2, y[j].y, -c.x))
+                           : make_double2(fma(-g2, y[j].x, c.x), fma(-g2, y[j].y, c.y));
         }
-        __syncwarp();   // HT is free for the projection below
         if (deph || with_cur) {
-            double2 p[N], q[N], y[N], d[N];   // rows of P_j, P_{j-1}, Y and D(Y)
-            double t0 = 0.0, ty = 0.0;
+            Rows<N> H;
+            H.load(v + D::H0, ro);
+            double2 *const Ps = v + D::HT;
+            double2 p[NE], q[NE], d[NE];   // P_j, P_{j-1} and D(Y)
 #pragma unroll
-            for (int n = 0; n < N; ++n) {
-                p[n] = own ? herm<N>(v + D::H0, mr, n) : make_double2(0.0, 0.0);
-                y[n] = own ? herm<N>(v + D::Y, mr, n) : make_double2(0.0, 0.0);
-                q[n] = make_double2(0.0, 0.0);
-                if (n == m) { t0 = p[n].x; ty = y[n].x; }
-            }
-            t0 = gsum<G>(t0) * (1.0 / N);
-            ty = gsum<G>(ty) * (1.0 / N);
-#pragma unroll
-            for (int n = 0; n < N; ++n) {
-                if (n == m) p[n].x -= t0;
-                d[n] = make_double2(n == m ? ty : 0.0, 0.0);
-            }
-            double p2 = gsum<G>(row_dot<N>(p, p));
-            const double py = gsum<G>(row_dot<N>(p, y));
+            for (int j = 0; j < DO; ++j) p[j] = j < M ? H.a[j + 1] : H.b[(j + 1) % N];
+            p[DO] = make_double2(H.a[0].x, D::EVEN ? H.b[M].x : 0.0);
+            const double t0 = gsum<G>(p[DO].x + p[DO].y, base) * (1.0 / N);
+            const double ty = gsum<G>(D::EVEN ? y[DO].x + y[DO].y : y[DO].x, base) * (1.0 / N);
+            p[DO].x -= t0;
+            if (D::EVEN) p[DO].y -= t0;
+            put<N>(Ps, p, m);
+            double p2 = gsum<G>(dot<N>(p, p), base);
+            const double py = gsum<G>(dot<N>(p, y), base);
             const double a2 = p2;
             double ip = p2 > 0.0 ? 1.0 / p2 : 0.0, b = 0.0;
 #pragma unroll
-            for (int n = 0; n < N; ++n) {
+            for (int j = 0; j < NE; ++j) {
                 const double x = py * ip;
-                d[n] = make_double2(fma(x, p[n].x, d[n].x), fma(x, p[n].y, d[n].y));
+                d[j] = make_double2(x * p[j].x, x * p[j].y);
+                q[j] = make_double2(0.0, 0.0);
             }
+            d[DO].x += ty;
+            if (D::EVEN) d[DO].y += ty;
+            __syncwarp();
+#pragma unroll 1
+            for (int i = 2; i < N; ++i) {
+                double2 w[NE];
+                product<N>(w, H, Ps, ro);
+                const double a = gsum<G>(dot<N>(w, p), base) * ip;
 #pragma unroll
-            for (int j = 2; j < N; ++j) {
-                double2 w[N];
-                row_herm<N>(w, p, v + D::H0);
-                const double a = gsum<G>(row_dot<N>(w, p)) * ip;
-#pragma unroll
-                for (int n = 0; n < N; ++n) {
-                    w[n].x = fma(-a, p[n].x, fma(-b, q[n].x, w[n].x));
-                    w[n].y = fma(-a, p[n].y, fma(-b, q[n].y, w[n].y));
-                    if (j == 2 && n == m) w[n].x -= p2 * (1.0 / N);   // Tr(H0 P_1) / N
-                    q[n] = p[n];
+                for (int j = 0; j < NE; ++j) {
+                    w[j].x = fma(-a, p[j].x, fma(-b, q[j].x, w[j].x));
+                    w[j].y = fma(-a, p[j].y, fma(-b, q[j].y, w[j].y));
+                    q[j] = p[j];
                 }
-                const double w2 = gsum<G>(row_dot<N>(w, w)), wy = gsum<G>(row_dot<N>(w, y));
+                if (i == 2) {   // Tr(H0 P_1) / N
+                    w[DO].x -= p2 * (1.0 / N);
+                    if (D::EVEN) w[DO].y -= p2 * (1.0 / N);
+                }
+                const double w2 = gsum<G>(dot<N>(w, w), base), wy = gsum<G>(dot<N>(w, y), base);
                 // a basis matrix that is rounding only (two bands meet) is left out
                 const bool ok = w2 > 1e-26 * a2 * p2;
                 b = w2 * ip;
@@ -364,90 +492,93 @@ __global__ void __launch_bounds__(32, N <= 4 ? 16 : 12)
                 p2 = w2;
                 const double x = wy * ip;
 #pragma unroll
-                for (int n = 0; n < N; ++n) {
-                    p[n] = w[n];
-                    d[n] = make_double2(fma(x, p[n].x, d[n].x), fma(x, p[n].y, d[n].y));
+                for (int j = 0; j < NE; ++j) {
+                    d[j] = make_double2(fma(x, w[j].x, d[j].x), fma(x, w[j].y, d[j].y));
+                    p[j] = ok ? w[j] : make_double2(0.0, 0.0);
                 }
-                if (!ok)
-#pragma unroll
-                    for (int n = 0; n < N; ++n) p[n] = make_double2(0.0, 0.0);
+                if (i + 1 < N) put<N>(Ps, p, m);
+                __syncwarp();
             }
-            if (own)
 #pragma unroll
-                for (int n = 0; n < N; ++n)
-                    if (n >= m) v[D::HT + up(m, n, N)] = d[n];
-        }
-        __syncwarp();
-        if (with_cur) {
-            // intraband current Re Tr(D(Y) J_a) = Re Tr(D(Y) (-i S_a)): D(Y) commutes with H0
-            double ii[2] = {0.0, 0.0};
-            double *out = P.cur_part + (size_t)unit * WAN_NSLOT;
-#pragma unroll
-            for (int j = 0; j < NO; ++j) {
-                if (m + G * j >= NU) continue;
-                const double2 y = v[D::HT + m + G * j];
+            for (int j = 0; j < NE; ++j) kn[j] = make_double2(fma(-gd, d[j].x, kn[j].x), fma(-gd, d[j].y, kn[j].y));
+            if (with_cur) {
+                // intraband current Re Tr(D(Y) J_a) = Re Tr(D(Y) (-i S_a)): D(Y) commutes with H0
+                double ii[2];
 #pragma unroll
                 for (int a = 0; a < 2; ++a) {
-                    const double2 x = sv[(a * NO + j) * 32];
-                    if (om[j] == on[j]) ii[a] += y.x * x.y;
-                    else ii[a] -= 2.0 * (y.y * x.x - y.x * x.y);
+                    double2 x[NE];
+#pragma unroll
+                    for (int j = 0; j < NE; ++j) x[j] = ks[(a * NE + j) * LW];
+                    ii[a] = tr_s<N>(d, x);
                 }
-            }
-            const double w = live ? wk : 0.0;
-            double z[4] = {w * (tot[0] - ii[0]), w * (tot[1] - ii[1]), w * ii[0], w * ii[1]};
-            const bool h4 = lane & 16, h3 = lane & 8;
-            double u0 = (h4 ? z[2] : z[0]) + __shfl_xor_sync(ALL, h4 ? z[0] : z[2], 16);
-            double u1 = (h4 ? z[3] : z[1]) + __shfl_xor_sync(ALL, h4 ? z[1] : z[3], 16);
-            double x = (h3 ? u1 : u0) + __shfl_xor_sync(ALL, h3 ? u0 : u1, 8);
+                double *out = P.cur_part + (size_t)unit * WAN_NSLOT;
+                const double w = live ? wk : 0.0;
+                double z[4] = {w * (tot[0] - ii[0]), w * (tot[1] - ii[1]), w * ii[0], w * ii[1]};
+                const bool h4 = lane & 16, h3 = lane & 8;
+                double u0 = (h4 ? z[2] : z[0]) + __shfl_xor_sync(ALL, h4 ? z[0] : z[2], 16);
+                double u1 = (h4 ? z[3] : z[1]) + __shfl_xor_sync(ALL, h4 ? z[1] : z[3], 16);
+                double x = (h3 ? u1 : u0) + __shfl_xor_sync(ALL, h3 ? u0 : u1, 8);
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(ALL, x, o);
-            if ((lane & 7) == 0) out[lane >> 3] = x;
-            // occupations, and the element of the coherence file (antelope.cpp:539-542)
-            const int ce = (P.nval * N + P.nval + 1) % NN;
-            double oc = own ? w * v[D::Y + up(mr, mr, N)].x : 0.0;
-            const double2 yc = herm<N>(v + D::Y, ce / N, ce % N);
-            double co = m == 0 ? w * yc.x : m == 1 ? w * yc.y : 0.0;
-#pragma unroll
-            for (int o = 16; o >= G; o >>= 1) {
-                oc += __shfl_xor_sync(ALL, oc, o);
-                co += __shfl_xor_sync(ALL, co, o);
+                for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(ALL, x, o);
+                if ((lane & 7) == 0) out[lane >> 3] = x;
+                // lane l < N: occupation l; the next two: the element of the coherence
+                // file (antelope.cpp:539-542)
+                const int ce = (P.nval * N + P.nval + 1) % NN, ca = ce / N, cb = ce % N, cd = (cb - ca + N) % N;
+                const bool up = cd <= M;
+                const double *src = reinterpret_cast<const double *>(sm + (S - 1) * NE * LW + D::Y);
+                if (lane < N) src += 2 * lane;
+                else src += 2 * (up ? D::slot(cd, ca) : D::slot(N - cd, cb)) + (lane == N + 1);
+                double oc = 0.0;
+#pragma unroll 2
+                for (int g = 0; g < KW; ++g) {
+                    const double wg = __shfl_sync(ALL, w, g * G);
+                    if (lane < N + 2) oc = fma(wg, src[2 * g * D::END], oc);
+                }
+                if (lane == N + 1) oc = cd == 0 ? 0.0 : up ? oc : -oc;
+                if (lane < N + 2) out[4 + lane] = oc;
+                __syncwarp();
             }
-            if (lane < N) out[4 + lane] = oc;
-            if (lane < 2) out[4 + N + lane] = co;
         }
-        // -i((HY) - (HY)^dag) - (g2 Y + (g1 - g2) D(Y)) at the owned elements (SBEs.h:808-861)
 #pragma unroll
-        for (int j = 0; j < NO; ++j) {
-            const int u = min(m + G * j, NU - 1);
-            const double2 c = v[D::T + om[j] * D::LDT + on[j]], c2 = v[D::T + on[j] * D::LDT + om[j]];
-            double2 kn = make_double2(c.y + c2.y, c2.x - c.x);
-            if (deph) {
-                const double2 d = v[D::HT + u], y = v[D::Y + u];
-                kn.x -= g2 * y.x + gd * d.x;
-                kn.y -= g2 * y.y + gd * d.y;
-            }
-            if (om[j] == on[j]) kn.y = 0.0;
-            if (s + 1 < S) ks[(s * NO + j) * 32 + lane] = kn;
-            else kl[j] = kn;
+        for (int j = 0; j < NE; ++j) {
+            if (s + 1 < S) ks[(s * NE + j) * LW] = kn[j];
+            else kl[j] = kn[j];
         }
-        __syncwarp();
     }
     // trial state and error estimate
+    double emax = 0.0;
     double2 *rout = P.rho[1 - buf] + (size_t)kc * NN;
+    double2 er[NE];
 #pragma unroll
-    for (int j = 0; j < NO; ++j) {
-        if (m + G * j >= NU || !live) continue;
-        double2 inc = make_double2(0.0, 0.0), er = inc;
-        for (int s = 0; s < S; ++s) {
-            const double2 q = s + 1 < S ? ks[(s * NO + j) * 32 + lane] : kl[j];
-            const double b = h * tb.b[s], e = h * tb.e[s];
-            inc = make_double2(fma(b, q.x, inc.x), fma(b, q.y, inc.y));
-            er = make_double2(fma(e, q.x, er.x), fma(e, q.y, er.y));
+    for (int j = 0; j < NE; ++j) er[j] = make_double2(0.0, 0.0);
+    double2 inc[NE];
+#pragma unroll
+    for (int j = 0; j < NE; ++j) inc[j] = make_double2(0.0, 0.0);
+#pragma unroll 1
+    for (int s = 0; s < S; ++s) {
+        const double b = h * tb.b[s], e = h * tb.e[s];
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+            const double2 q = s + 1 < S ? ks[(s * NE + j) * LW] : kl[j];
+            inc[j] = make_double2(fma(b, q.x, inc[j].x), fma(b, q.y, inc[j].y));
+            er[j] = make_double2(fma(e, q.x, er[j].x), fma(e, q.y, er[j].y));
         }
-        const double2 x = make_double2(r64[j].x + inc.x, r64[j].y + inc.y);
-        __stcg(rout + om[j] * N + on[j], x);
-        if (om[j] != on[j]) __stcg(rout + on[j] * N + om[j], cconj(x));
-        emax = fmax(emax, sqrt(er.x * er.x + er.y * er.y));
+    }
+    if (live) {
+#pragma unroll
+        for (int j = 0; j < DO; ++j) {
+            const double2 x = make_double2(r64[j].x + inc[j].x, r64[j].y + inc[j].y);
+            const int a = erow(j), b = ecol(j);
+            __stcg(rout + a * N + b, x);
+            __stcg(rout + b * N + a, cconj(x));
+            emax = fmax(emax, sqrt(er[j].x * er[j].x + er[j].y * er[j].y));
+        }
+        __stcg(rout + m * (N + 1), make_double2(r64[DO].x + inc[DO].x, 0.0));
+        emax = fmax(emax, fabs(er[DO].x));
+        if (D::EVEN) {
+            __stcg(rout + (m + M) * (N + 1), make_double2(r64[DO].y + inc[DO].y, 0.0));
+            emax = fmax(emax, fabs(er[DO].y));
+        }
     }
     if (P.rk == 45) {
 #pragma unroll
@@ -467,7 +598,7 @@ __global__ void __launch_bounds__(128) wan_next(const WanDev *__restrict__ Pp, c
                                                 bool first)
 {
     using D = PD<N>;
-    constexpr int G = D::G, NU = D::NU, NO = D::NO, NN = D::NN;
+    constexpr int G = D::G, NE = D::NE, DO = D::DO, M = D::M, NN = D::NN, NU = N * (N + 1) / 2;
     __shared__ __align__(16) unsigned char sp[sizeof(WanDev)];
     __shared__ WanCtl c;
     __shared__ double AE[6][6], red[128];
@@ -554,13 +685,15 @@ __global__ void __launch_bounds__(128) wan_next(const WanDev *__restrict__ Pp, c
             __syncthreads();
             const bool cur = s == 0 && c.need_current;
             const double ex = AE[s][3], ey = AE[s][4];
-            double2 *out = P.gr_tab + (size_t)item * nent * NO * NQ * G;
-            double2 *oc = P.gr_cur + (size_t)row * nent * NO * NC * G;
+            double2 *out = P.gr_tab + (size_t)item * nent * NE * NQ * G;
+            double2 *oc = P.gr_cur + (size_t)row * nent * NE * NC * G;
             for (int w = t; w < ng * NU; w += blockDim.x) {
-                const int q = w / NU, u = w % NU;
-                int mu = u, a = 0;
-                while (mu >= N - a) { mu -= N - a; ++a; }
-                const int e = a * N + a + mu;
+                // owned element j of lane l; the diagonal ones last, two to an entry
+                const int q = w / NU, u = w % NU, j = u / G, l = u % G;
+                const int r0 = j < DO ? (j < M ? l : l + M) : l + (j - DO) * M;
+                const int c0 = j < DO ? (r0 + 1 + (j < M ? j : j - M)) % N : r0;
+                const bool low = r0 > c0;   // from the upper triangle by symmetry
+                const int e = low ? c0 * N + r0 : r0 * N + c0;
                 double2 x[2][6];   // h, E.D, S_x, S_y, D_x, D_y of the group at +g and -g
 #pragma unroll
                 for (int z = 0; z < 2; ++z) {
@@ -584,24 +717,40 @@ __global__ void __launch_bounds__(128) wan_next(const WanDev *__restrict__ Pp, c
                     }
                     x[z][1] = make_double2(fma(ey, x[z][5].x, ex * x[z][4].x), fma(ey, x[z][5].y, ex * x[z][4].y));
                 }
-                const int j = u / G, l = u % G;
-                // sig = G_g + G_-g, tau = i (G_g - G_-g); the group g = 0 is sig alone
-                auto store = [&](double2 *o, int nq, int y, const double2 &xp, const double2 &xm) {
-                    if (q == 0) {
-                        o[(size_t)(j * nq + y) * G + l] = xp;
+                // sig = G_g + G_-g, tau = i (G_g - G_-g); the group g = 0 is sig alone.
+                // Of the diagonal the real part (h, D Hermitian), of S the imaginary one.
+                auto store = [&](double2 *o, int nq, int y, double2 sg, double2 ta, bool anti) {
+                    const size_t step = (size_t)NE * nq * G;
+                    o += (size_t)max(2 * q - 1, 0) * step + (size_t)(min(j, DO) * nq + y) * G + l;
+                    if (j < DO) {
+                        if (low) {
+                            sg = anti ? make_double2(-sg.x, sg.y) : cconj(sg);
+                            ta = anti ? make_double2(-ta.x, ta.y) : cconj(ta);
+                        }
+                        o[0] = sg;
+                        if (q > 0) o[step] = ta;
                     } else {
-                        o[((size_t)((2 * q - 1) * NO + j) * nq + y) * G + l] = make_double2(xp.x + xm.x, xp.y + xm.y);
-                        o[((size_t)(2 * q * NO + j) * nq + y) * G + l] = make_double2(xm.y - xp.y, xp.x - xm.x);
+                        double *z = reinterpret_cast<double *>(o) + (j - DO);
+                        z[0] = anti ? sg.y : sg.x;
+                        if (q > 0) z[2 * step] = anti ? ta.y : ta.x;
+                        if (!D::EVEN) {
+                            z[1] = 0.0;
+                            if (q > 0) z[2 * step + 1] = 0.0;
+                        }
                     }
                 };
-                store(out, NQ, 0, x[0][0], x[1][0]);
-                if (dip) store(out, NQ, 1, x[0][1], x[1][1]);
+                auto pair = [&](double2 *o, int nq, int y, const double2 &xp, const double2 &xm, bool anti) {
+                    store(o, nq, y, q == 0 ? xp : make_double2(xp.x + xm.x, xp.y + xm.y), make_double2(xm.y - xp.y, xp.x - xm.x),
+                          anti);
+                };
+                pair(out, NQ, 0, x[0][0], x[1][0], false);
+                if (dip) pair(out, NQ, 1, x[0][1], x[1][1], false);
                 if (cur) {
-                    store(oc, NC, 0, x[0][2], x[1][2]);
-                    store(oc, NC, 1, x[0][3], x[1][3]);
+                    pair(oc, NC, 0, x[0][2], x[1][2], true);
+                    pair(oc, NC, 1, x[0][3], x[1][3], true);
                     if (dip) {
-                        store(oc, NC, 2, x[0][4], x[1][4]);
-                        store(oc, NC, 3, x[0][5], x[1][5]);
+                        pair(oc, NC, 2, x[0][4], x[1][4], false);
+                        pair(oc, NC, 3, x[0][5], x[1][5], false);
                     }
                 }
             }
@@ -630,28 +779,28 @@ bool wan_proj(const WanDev &w) { return w.gr_tab != nullptr && wan_proj_applies(
 // Entries of the row tables per row (gr_tab has one set per stage)
 int wan_proj_entries(int N, int ngrp, int nq)
 {
-    const int G = N <= 4 ? 4 : 8;
-    return (2 * ngrp - 1) * ((N * (N + 1) / 2 + G - 1) / G) * nq * G;
+    const int even = N % 2 == 0, G = even ? N / 2 : N, NE = even ? N : (N + 1) / 2;   // PD
+    return (2 * ngrp - 1) * NE * nq * G;
 }
-int wan_proj_unit(int N) { return N <= 4 ? 2 : 1; }   // tiles per block
+int wan_proj_unit(int N) { return 32 / (N % 2 == 0 ? N / 2 : N); }
 
 template <int N>
 static cudaError_t proj_attempt(const WanDev *dw, const WanDev *const *descs, const WanTileRef *tiles, int nblocks,
-                                int ngrp, cudaStream_t st)
+                                int ngrp, int S, cudaStream_t st)
 {
     const int grid = tiles ? nblocks : (nblocks + SPREAD - 1) / SPREAD * SPREAD;
-    wan_attempt_p<N><<<grid, 32, proj_bytes<N>(ngrp), st>>>(dw, descs, tiles);
+    wan_attempt_p<N><<<grid, 32, proj_bytes<N>(ngrp, S), st>>>(dw, descs, tiles);
     return cudaGetLastError();
 }
-cudaError_t launch_wan_attempt_p(int N, int ngrp, const WanDev *dw, const WanDev *const *descs, const WanTileRef *tiles,
+cudaError_t launch_wan_attempt_p(int N, int ngrp, int S, const WanDev *dw, const WanDev *const *descs, const WanTileRef *tiles,
                                  int nblocks, cudaStream_t st)
 {
     if (nblocks <= 0) return cudaSuccess;
     switch (N) {
-    case 3: return proj_attempt<3>(dw, descs, tiles, nblocks, ngrp, st);
-    case 4: return proj_attempt<4>(dw, descs, tiles, nblocks, ngrp, st);
-    case 5: return proj_attempt<5>(dw, descs, tiles, nblocks, ngrp, st);
-    case 6: return proj_attempt<6>(dw, descs, tiles, nblocks, ngrp, st);
+    case 3: return proj_attempt<3>(dw, descs, tiles, nblocks, ngrp, S, st);
+    case 4: return proj_attempt<4>(dw, descs, tiles, nblocks, ngrp, S, st);
+    case 5: return proj_attempt<5>(dw, descs, tiles, nblocks, ngrp, S, st);
+    case 6: return proj_attempt<6>(dw, descs, tiles, nblocks, ngrp, S, st);
     default: return cudaErrorInvalidValue;
     }
 }

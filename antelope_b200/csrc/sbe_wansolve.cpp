@@ -454,12 +454,16 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         // interleave the solves' tiles round-robin (longest first), so that
         // the blocks of one launch spread every solve over the whole GPU
         // (grouped classes: one entry per block of WAN_GROUP_TILES tiles)
-        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.proj ? wan_proj_unit(c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.grouped_rk && !c.proj ? WAN_GROUP_TILES : 1;
+        auto count = [&](int m) {   // entries are tiles; of the projection attempts, units
+            const WanDev &w = solves_[m]->dev();
+            return c.proj ? (w.nk + wan_proj_unit(c.N) - 1) / wan_proj_unit(c.N) : w.ntiles;
+        };
         int maxt = 0;
-        for (int m : c.members) maxt = std::max(maxt, solves_[m]->dev().ntiles);
+        for (int m : c.members) maxt = std::max(maxt, count(m));
         for (int t = 0; t < maxt; t += unit)
             for (int j = 0; j < (int)c.members.size(); ++j)
-                if (t < solves_[c.members[j]]->dev().ntiles) tiles.push_back(WanTileRef{j, t});
+                if (t < count(c.members[j])) tiles.push_back(WanTileRef{j, t});
         c.ntiles = (int)tiles.size();
         dalloc(&c.d_descs, sizeof(WanDev *) * descs.size(), st, "alloc batch descriptors");
         dalloc(&c.d_tiles, sizeof(WanTileRef) * tiles.size(), st, "alloc batch tiles");
@@ -512,7 +516,7 @@ int WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
             }
             launched += c.shots ? 3 : 2;
             if (c.proj) {
-                cuda_check(launch_wan_attempt_p(c.N, c.ngrp, nullptr, c.d_descs, c.d_tiles, c.ntiles, st),
+                cuda_check(launch_wan_attempt_p(c.N, c.ngrp, 6, nullptr, c.d_descs, c.d_tiles, c.ntiles, st),
                            "Wannier attempt kernel (batch)");
                 cuda_check(launch_wan_next(c.N, nullptr, c.d_descs, (int)c.members.size(), c.nitems, false, st),
                            "Wannier control kernel (batch)");
@@ -696,15 +700,19 @@ void WannierPool::rebuild()
     for (Class &c : classes_) {
         std::vector<const WanDev *> descs;
         std::vector<WanTileRef> tiles;
-        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.proj ? wan_proj_unit(c.N) : c.grouped_rk ? WAN_GROUP_TILES : 1;
+        const int unit = c.steps.mode ? wan_steps_unit(c.steps.mode, c.N) : c.grouped_rk && !c.proj ? WAN_GROUP_TILES : 1;
+        auto count = [&](int id) {   // entries are tiles; of the projection attempts, units
+            const WanDev &w = solves_.at(id).s->dev();
+            return c.proj ? (w.nk + wan_proj_unit(c.N) - 1) / wan_proj_unit(c.N) : w.ntiles;
+        };
         int maxt = 0;
         for (int id : c.ids) {
             descs.push_back(solves_.at(id).s->dev_ptr());
-            maxt = std::max(maxt, solves_.at(id).s->dev().ntiles);
+            maxt = std::max(maxt, count(id));
         }
         for (int t = 0; t < maxt; t += unit)
             for (int j = 0; j < (int)c.ids.size(); ++j)
-                if (t < solves_.at(c.ids[j]).s->dev().ntiles) tiles.push_back(WanTileRef{j, t});
+                if (t < count(c.ids[j])) tiles.push_back(WanTileRef{j, t});
         c.ntiles = (int)tiles.size();
         dalloc(&c.d_descs, sizeof(WanDev *) * descs.size(), st_, "alloc pool descriptors");
         dalloc(&c.d_tiles, sizeof(WanTileRef) * tiles.size(), st_, "alloc pool tiles");
@@ -733,7 +741,7 @@ void WannierPool::step(int iters)
                 continue;
             }
             if (c.proj) {
-                cuda_check(launch_wan_attempt_p(c.N, c.ngrp, nullptr, c.d_descs, c.d_tiles, c.ntiles, st_),
+                cuda_check(launch_wan_attempt_p(c.N, c.ngrp, 6, nullptr, c.d_descs, c.d_tiles, c.ntiles, st_),
                            "Wannier attempt kernel (server)");
                 cuda_check(launch_wan_next(c.N, nullptr, c.d_descs, (int)c.ids.size(), c.nitems, false, st_),
                            "Wannier control kernel (server)");

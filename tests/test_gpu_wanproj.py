@@ -61,3 +61,25 @@ def test_slices_add_up():
     for key in ("inter", "intra", "occ"):
         x, y = getattr(out, key), getattr(whole, key)
         assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max(), key
+
+
+@pytest.mark.parametrize("nband,npoints", [(3, (1, 10)), (3, (3, 7)), (4, (1, 16)), (4, (17, 1)), (5, (1, 6)), (5, (1, 7)),
+                                           (6, (1, 10)), (6, (11, 1)), (6, (2, 5)), (6, (7, 3))])
+def test_edges_of_a_block(nband, npoints):
+    """A block's k-points (32 lanes in whole groups): full, one more, and rows that end inside it."""
+    _check(_case(nband, npoints, "cashkarp45"))
+
+
+def test_batch_of_step_rules_equals_the_solves_alone():
+    """Solves of one launch differ in their stages, grids and lengths."""
+    cases = [_case(6, (3, 7), "rk4", steps=20.5), _case(6, (5, 5), "cashkarp45"), _case(6, (1, 11), "rk5", steps=12.5),
+             _case(4, (3, 7), "cashkarp45"), _case(4, (1, 17), "rk4")]
+    problems = [ab.Problem.from_dict(c) for c in cases]
+    b = ab.Batch(problems, precision="fp64")
+    b.run()
+    outs = [b.get(i) for i in range(len(cases))]
+    b.close()
+    for p, out in zip(problems, outs):
+        one = ab.solve(p, precision="fp64")
+        for key in ("inter", "intra", "occ"):
+            np.testing.assert_array_equal(getattr(out, key), getattr(one, key))
