@@ -30,10 +30,13 @@
 // the limit of one row per lane in groups of 8 (a 16-byte element at one address
 // per group costs 4 wavefronts, whatever the number of groups; 4 k-points per
 // warp, 6 of 8 lanes at work): Cash-Karp attempts of N = 6, 4, 3 on 200 x 300
-// points took 681, 251 and 144 us, now 408, 144 and 103; on 100 x 100 162, 82 and
-// 52, now 90, 51 and 46; on 8 x 8 68, 61 and 41, now 65, 41 and 37.
-// Bound: latencies at two warps a scheduler (255 registers), half of them in the
-// table reads of the Fourier sums; FP64 issue a quarter to a third of the time.
+// points took 681, 251 and 144 us, now 361, 137 and 108; on 100 x 100 162, 82 and
+// 52, now 85, 51 and 46; on 8 x 8 68, 61 and 41, now 60, 41 and 37.  What does not
+// fit the 255 registers of N = 6 stays in shared memory (the slope while the
+// projection adds to it) or is read again (the state): 408 and 90 us with both
+// kept, their spills missing an L1 that the blocks' shared memory leaves 28 KB.
+// Bound: latencies at two warps a scheduler; FP64 issue a quarter to a third of
+// the time.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -89,10 +92,10 @@ template <int N> struct PD {
     static constexpr int DO = EVEN ? N - 1 : M;   // owned elements off the diagonal
     static constexpr int NE = DO + 1;             // entries of an owned set; the last: its diagonal elements
     static constexpr int NM = (M + 1) * N;        // slots [d][r] of a matrix (d = N/2 of an even N twice)
-    // the matrices of a k-point in complex numbers: Y, H0, H0 + E.D (later T, P);
-    // the stride puts the lanes of a warp's groups on distinct banks
-    static constexpr int Y = 0, H0 = NM, HT = 2 * NM;
-    static constexpr int END = 3 * NM + (N == 6 ? 3 : N == 4 ? 2 : N == 3 ? 1 : 0);
+    // a k-point's two matrices in complex numbers: Y, then H0; H0 + E.D (T, P); the
+    // stride puts the lanes of a warp's groups on distinct banks
+    static constexpr int Y = 0, HT = NM;
+    static constexpr int END = 2 * NM + (N == 5 ? 5 : N == 3 ? 1 : N == 6 ? 3 : 2);
     static constexpr int TN = (N - 1 - M) * N;    // slots of the product's unowned elements
     __host__ __device__ static constexpr int slot(int d, int r) { return d * N + r; }
 };
@@ -264,7 +267,7 @@ __device__ __forceinline__ double tr_s(const double2 (&x)[PD<N>::NE], const doub
 template <int N> static int proj_bytes(int ngrp, int S)
 {
     using D = PD<N>;
-    return ((S - 1) * D::NE * D::LW + D::KW * D::END + D::KW * ngrp) * 16;
+    return (S * D::NE * 32 + D::KW * D::END + D::KW * ngrp) * 16;
 }
 
 template <int N>
@@ -288,17 +291,18 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
     }
     const WanCtl &ctl = *P.ctl;
     if (ctl.done) return;
-    // lanes past the last group shadow its first lanes: same values, same addresses
+    // lanes past the last group shadow its first lanes: same values, to the same
+    // addresses where the group shares them
     const int lane = threadIdx.x, grp = min(lane / G, KW - 1), m = lane < LW ? lane % G : lane - LW;
-    const int base = grp * G, col = base + m;
+    const int base = grp * G;
     const int k = unit * KW + grp;
     const bool live = k < P.nk && lane < LW;
     const int kc = min(k, P.nk - 1);   // a group past the grid shadows the last k-point
     const int S = c_tab[tab_of(P.rk)].S;
-    double2 *const ks = sm + col;                                // [S - 1][NE][LW] slopes, a column per lane
-    double2 *const v = sm + (S - 1) * NE * LW + grp * D::END;
+    double2 *const ks = sm + lane;                               // [S][NE][32] slopes, a column per lane
+    double2 *const v = sm + S * NE * 32 + grp * D::END;
     const int ng = P.gr_n, nent = 2 * ng - 1;                    // group pairs (g = 0 first), table entries
-    double2 *const ph = sm + (S - 1) * NE * LW + KW * D::END + grp * ng;
+    double2 *const ph = sm + S * NE * 32 + KW * D::END + grp * ng;
     const double h = ctl.hs;
     const int buf = ctl.buf;
     const bool cur = ctl.need_current;
@@ -319,34 +323,36 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
     // the owned element j < DO: row m (m + N/2) and its column
     auto erow = [&](int j) { return j < M ? ro[0] : ro[M % N]; };
     auto ecol = [&](int j) { return j < M ? ro[j + 1] : ro[(j + 1) % N]; };
-    double2 r64[NE];
+    // the state's owned elements; at N = 6 read again at each stage: they do not
+    // fit the registers beside the projection's matrices
+    constexpr bool KEEP = N < 6;
     const double2 *rho = P.rho[buf] + (size_t)kc * NN;
+    auto state = [&](double2 (&r)[NE]) {
 #pragma unroll
-    for (int j = 0; j < DO; ++j) {
-        const int a = erow(j), b = ecol(j);
-        r64[j] = __ldcg(rho + min(a, b) * N + max(a, b));
-        if (a > b) r64[j].y = -r64[j].y;
-    }
-    r64[DO].x = __ldcg(&rho[m * (N + 1)].x);
-    r64[DO].y = D::EVEN ? __ldcg(&rho[(m + M) * (N + 1)].x) : 0.0;
+        for (int j = 0; j < DO; ++j) {
+            const int a = erow(j), b = ecol(j);
+            r[j] = __ldcg(rho + min(a, b) * N + max(a, b));
+            if (a > b) r[j].y = -r[j].y;
+        }
+        r[DO].x = __ldcg(&rho[m * (N + 1)].x);
+        r[DO].y = D::EVEN ? __ldcg(&rho[(m + M) * (N + 1)].x) : 0.0;
+    };
+    double2 r64[NE];
+    if (KEEP) state(r64);
     const bool dip = P.has_dip;
     const int NQ = dip ? 2 : 1;
     const double g1 = P.g1, g2 = P.g2, gd = g1 - g2;
     const bool deph = g1 != 0.0 || g2 != 0.0;
-    double2 kl[NE];   // the last stage's slope
     const size_t ent = (size_t)nent * NE * NQ * G;   // table entries of a (row, stage)
     const double2 *tab = P.gr_tab + (size_t)row * S * ent + m;
     __syncwarp();
 
 #pragma unroll 1
     for (int s = 0; s < S; ++s, tab += ent) {
-        // H0 and E.D at the owned elements; the next stage's table lines (128
-        // bytes each) are fetched towards L1 meanwhile
-        if (s + 1 < S)
-            for (int i = lane * 8; i < (int)ent; i += 256)
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(tab - m + ent + i));
+        // H0 and E.D at the owned elements
+        double2 y[NE], a0[NE], a1[NE];
+        if (!KEEP) state(y);
         {
-            double2 a0[NE], a1[NE];
 #pragma unroll
             for (int j = 0; j < NE; ++j) {
                 a0[j] = __ldg(tab + (size_t)j * NQ * G);
@@ -366,38 +372,40 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
                     }
                 }
             }
-            put<N>(v + D::H0, a0, m);
 #pragma unroll
             for (int j = 0; j < NE; ++j) a1[j] = make_double2(a0[j].x + a1[j].x, a0[j].y + a1[j].y);
-            put<N>(v + D::HT, a1, m);
         }
         // stage input Y = rho + h sum_j a_sj k_j
-        double2 y[NE];
+        if (KEEP)
 #pragma unroll
-        for (int j = 0; j < NE; ++j) y[j] = r64[j];
+            for (int j = 0; j < NE; ++j) y[j] = r64[j];
 #pragma unroll 1
         for (int i = 0; i < s; ++i) {
             const double a = h * tb.a[s][i];
 #pragma unroll
             for (int j = 0; j < NE; ++j) {
-                const double2 q = ks[(i * NE + j) * LW];
+                const double2 q = ks[(i * NE + j) * 32];
                 y[j] = make_double2(fma(a, q.x, y[j].x), fma(a, q.y, y[j].y));
             }
         }
-        put<N>(v + D::Y, y, m);
-        __syncwarp();
         const bool with_cur = cur && s == 0;
+        put<N>(v + D::Y, y, m);
+        if (!with_cur) put<N>(v + D::HT, a1, m);
+        else put<N>(v + D::HT, a0, m);
+        __syncwarp();
         double tot[2] = {0.0, 0.0};
         if (with_cur) {
             // total current Re Tr(Y J_a), J_a = -i S_a + i [D_a, H0] (S_a = sum R_a h_R
             // e^{iKR}): over the owned elements, with C = H0 Y - (H0 Y)^dag, the
             // diagonal Y_mm Im(S_mm) - Im(C_mm) Re(D_mm), off it -2 Im(Y_mn conj(S_mn))
-            // - 2 Im(C_mn conj(D_mn)).  S_a and T wait in the columns of slopes that do
-            // not exist yet.
+            // - 2 Im(C_mn conj(D_mn)).  S_a, T and H0 + E.D wait in the columns of
+            // slopes that do not exist yet.
             const int NC = dip ? 4 : 2;   // S_x, S_y (, D_x, D_y)
             const double2 *tc = P.gr_cur + (size_t)row * nent * NE * NC * G + m;
             double2 c[NE];
-            if (dip) commutator<N>(c, v + D::H0, v + D::Y, sm + 2 * NE * LW + grp * D::TN, ro);
+#pragma unroll
+            for (int j = 0; j < NE; ++j) ks[(3 * NE + j) * 32] = a1[j];
+            if (dip) commutator<N>(c, v + D::HT, v + D::Y, sm + grp * D::TN, ro);
 #pragma unroll 1
             for (int a = 0; a < 2; ++a) {
                 double2 x[NE], d[NE];
@@ -429,28 +437,53 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
                     if (D::EVEN) t -= c[DO].y * d[DO].y;
                 }
 #pragma unroll
-                for (int j = 0; j < NE; ++j) ks[(a * NE + j) * LW] = x[j];
+                for (int j = 0; j < NE; ++j) ks[((a + 1) * NE + j) * 32] = x[j];
                 if (a == 0) tot[0] = t;
                 else tot[1] = t;
             }
-        }
-        // -i [H0 + E.D, Y] - g2 Y
-        double2 kn[NE];
-        commutator<N>(kn, v + D::HT, v + D::Y, v + D::HT, ro);
+            double *out = P.cur_part + (size_t)unit * WAN_NSLOT;
+            const double w = live ? wk : 0.0;
+            // lane l < N: occupation l; the next two: the element of the coherence
+            // file (antelope.cpp:539-542)
+            const int ce = (P.nval * N + P.nval + 1) % NN, ca = ce / N, cb = ce % N, cd = (cb - ca + N) % N;
+            const bool up = cd <= M;
+            const double *src = reinterpret_cast<const double *>(sm + S * NE * 32 + D::Y);
+            if (lane < N) src += 2 * lane;
+            else src += 2 * (up ? D::slot(cd, ca) : D::slot(N - cd, cb)) + (lane == N + 1);
+            double oc = 0.0;
+#pragma unroll 2
+            for (int g = 0; g < KW; ++g) {
+                const double wg = __shfl_sync(ALL, w, g * G);
+                if (lane < N + 2) oc = fma(wg, src[2 * g * D::END], oc);
+            }
+            if (lane == N + 1) oc = cd == 0 ? 0.0 : up ? oc : -oc;
+            if (lane < N + 2) out[4 + lane] = oc;
+            __syncwarp();
 #pragma unroll
-        for (int j = 0; j < NE; ++j) {
-            const double2 c = kn[j];
-            kn[j] = j < DO ? make_double2(fma(-g2, y[j].x, c.y), fma(-g2, y[j].y, -c.x))
-                           : make_double2(fma(-g2, y[j].x, c.x), fma(-g2, y[j].y, c.y));
+            for (int j = 0; j < NE; ++j) a1[j] = ks[(3 * NE + j) * 32];
+            put<N>(v + D::HT, a1, m);
+            __syncwarp();
+        }
+        // the slope -i [H0 + E.D, Y] - g2 Y, to which the projection adds
+        double2 *const kn = ks + s * NE * 32;
+        double2 c[NE];
+        {
+            commutator<N>(c, v + D::HT, v + D::Y, v + D::HT, ro);
+#pragma unroll
+            for (int j = 0; j < NE; ++j)
+                c[j] = j < DO ? make_double2(fma(-g2, y[j].x, c[j].y), fma(-g2, y[j].y, -c[j].x))
+                              : make_double2(fma(-g2, y[j].x, c[j].x), fma(-g2, y[j].y, c[j].y));
+            if (!KEEP || !(deph || with_cur))
+#pragma unroll
+                for (int j = 0; j < NE; ++j) kn[j * 32] = c[j];
         }
         if (deph || with_cur) {
-            Rows<N> H;
-            H.load(v + D::H0, ro);
             double2 *const Ps = v + D::HT;
             double2 p[NE], q[NE], d[NE];   // P_j, P_{j-1} and D(Y)
 #pragma unroll
-            for (int j = 0; j < DO; ++j) p[j] = j < M ? H.a[j + 1] : H.b[(j + 1) % N];
-            p[DO] = make_double2(H.a[0].x, D::EVEN ? H.b[M].x : 0.0);
+            for (int j = 0; j < NE; ++j) p[j] = a0[j];
+            if (!D::EVEN) p[DO].y = 0.0;
+            put<N>(v + D::Y, a0, m);   // Y is done with
             const double t0 = gsum<G>(p[DO].x + p[DO].y, base) * (1.0 / N);
             const double ty = gsum<G>(D::EVEN ? y[DO].x + y[DO].y : y[DO].x, base) * (1.0 / N);
             p[DO].x -= t0;
@@ -469,6 +502,8 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
             d[DO].x += ty;
             if (D::EVEN) d[DO].y += ty;
             __syncwarp();
+            Rows<N> H;
+            H.load(v + D::Y, ro);
 #pragma unroll 1
             for (int i = 2; i < N; ++i) {
                 double2 w[NE];
@@ -500,7 +535,10 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
                 __syncwarp();
             }
 #pragma unroll
-            for (int j = 0; j < NE; ++j) kn[j] = make_double2(fma(-gd, d[j].x, kn[j].x), fma(-gd, d[j].y, kn[j].y));
+            for (int j = 0; j < NE; ++j) {
+                const double2 x = KEEP ? c[j] : kn[j * 32];
+                kn[j * 32] = make_double2(fma(-gd, d[j].x, x.x), fma(-gd, d[j].y, x.y));
+            }
             if (with_cur) {
                 // intraband current Re Tr(D(Y) J_a) = Re Tr(D(Y) (-i S_a)): D(Y) commutes with H0
                 double ii[2];
@@ -508,7 +546,7 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
                 for (int a = 0; a < 2; ++a) {
                     double2 x[NE];
 #pragma unroll
-                    for (int j = 0; j < NE; ++j) x[j] = ks[(a * NE + j) * LW];
+                    for (int j = 0; j < NE; ++j) x[j] = ks[((a + 1) * NE + j) * 32];
                     ii[a] = tr_s<N>(d, x);
                 }
                 double *out = P.cur_part + (size_t)unit * WAN_NSLOT;
@@ -521,28 +559,7 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
 #pragma unroll
                 for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(ALL, x, o);
                 if ((lane & 7) == 0) out[lane >> 3] = x;
-                // lane l < N: occupation l; the next two: the element of the coherence
-                // file (antelope.cpp:539-542)
-                const int ce = (P.nval * N + P.nval + 1) % NN, ca = ce / N, cb = ce % N, cd = (cb - ca + N) % N;
-                const bool up = cd <= M;
-                const double *src = reinterpret_cast<const double *>(sm + (S - 1) * NE * LW + D::Y);
-                if (lane < N) src += 2 * lane;
-                else src += 2 * (up ? D::slot(cd, ca) : D::slot(N - cd, cb)) + (lane == N + 1);
-                double oc = 0.0;
-#pragma unroll 2
-                for (int g = 0; g < KW; ++g) {
-                    const double wg = __shfl_sync(ALL, w, g * G);
-                    if (lane < N + 2) oc = fma(wg, src[2 * g * D::END], oc);
-                }
-                if (lane == N + 1) oc = cd == 0 ? 0.0 : up ? oc : -oc;
-                if (lane < N + 2) out[4 + lane] = oc;
-                __syncwarp();
             }
-        }
-#pragma unroll
-        for (int j = 0; j < NE; ++j) {
-            if (s + 1 < S) ks[(s * NE + j) * LW] = kn[j];
-            else kl[j] = kn[j];
         }
     }
     // trial state and error estimate
@@ -552,6 +569,7 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
 #pragma unroll
     for (int j = 0; j < NE; ++j) er[j] = make_double2(0.0, 0.0);
     double2 inc[NE];
+    if (!KEEP) state(r64);
 #pragma unroll
     for (int j = 0; j < NE; ++j) inc[j] = make_double2(0.0, 0.0);
 #pragma unroll 1
@@ -559,7 +577,7 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
         const double b = h * tb.b[s], e = h * tb.e[s];
 #pragma unroll
         for (int j = 0; j < NE; ++j) {
-            const double2 q = s + 1 < S ? ks[(s * NE + j) * LW] : kl[j];
+            const double2 q = ks[(s * NE + j) * 32];
             inc[j] = make_double2(fma(b, q.x, inc[j].x), fma(b, q.y, inc[j].y));
             er[j] = make_double2(fma(e, q.x, er[j].x), fma(e, q.y, er[j].y));
         }
