@@ -595,8 +595,6 @@ extern "C" sbe_status sbe_batch_run(sbe_batch *b, void *stream)
             run_engine(*b->eng, b->use_graph, &b->launches);
             for (int id : b->ids)
                 if (id >= 0) b->eng->fetch_async(id);
-            // host work of sbe_batch_get done while the GPU propagates
-            if (!b->wan) b->eng->prepare_outputs();
         }
         if (b->wan) {
             b->wan->run(st, b->use_graph);
@@ -614,6 +612,7 @@ extern "C" sbe_status sbe_batch_get(sbe_batch *b, int index, const sbe_outputs *
     return guard([&]() -> sbe_status {
         cuda_check(cudaSetDevice(b->device), "cudaSetDevice");
         const int id = b->ids[index];
+        if (id >= 0) b->eng->prepare_outputs(id);
         copy_out(id >= 0 ? b->eng->outputs(id) : b->wan->solve(-1 - id).outputs(), out);
         return SBE_OK;
     });

@@ -141,7 +141,6 @@ struct Engine::Solve {
     std::vector<double> laser;                     // output columns (prepare_outputs), or empty
     cudaEvent_t ev = nullptr;
     bool fetched = false;
-    int nqueues = 0;   // queue states copied behind h_const
     size_t bytes = 0;
 };
 
@@ -223,7 +222,7 @@ Engine::~Engine()
             cudaEventDestroy(s.ev);
         }
         pinned_.put(s.h_jout, (size_t)s.Nt * NSLOT * 8);
-        pinned_.put(s.h_const, ((size_t)s.ntiles * NSLOT + kMaxGroups) * 8);
+        pinned_.put(s.h_const, (size_t)s.ntiles * NSLOT * 8);
     }
     for (auto &kv : groups_) {
         cudaFreeAsync(kv.second->d_tiles, stream_);
@@ -234,6 +233,7 @@ Engine::~Engine()
     for (auto &e : prop_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     for (auto &e : red_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     cudaStreamSynchronize(stream_);
+    if (h_queue_) pinned_.put(h_queue_, kMaxGroups * sizeof(int));
     for (auto ev : pending_) cudaEventDestroy(ev);
     for (auto ev : spare_ev_) cudaEventDestroy(ev);
     cudaStreamDestroy(up_);
@@ -535,6 +535,7 @@ void Engine::step_frozen()
         la.kpt = g.kpt;
         la.has_g1 = g.g1;
         la.queue = g.d_queue;
+        queue_unread_ = true;
         la.stream = stream_;
         std::pair<cudaEvent_t, cudaEvent_t> ev{};
         if (profile_) {
@@ -598,19 +599,27 @@ void Engine::fetch_async(int id)
     // pinned result buffers are taken when a solve finishes, not when it is
     // admitted (a burst of admissions would otherwise wait on page locking)
     if (!s.h_jout) s.h_jout = static_cast<double *>(pinned_.get((size_t)s.Nt * NSLOT * 8));
-    if (!s.h_const) s.h_const = static_cast<double *>(pinned_.get(((size_t)s.ntiles * NSLOT + kMaxGroups) * 8));
+    if (!s.h_const) s.h_const = static_cast<double *>(pinned_.get((size_t)s.ntiles * NSLOT * 8));
     cuda_check(cudaMemcpyAsync(s.h_jout, s.jout, (size_t)s.Nt * NSLOT * 8, cudaMemcpyDeviceToHost, stream_),
                "copy outputs");
     cuda_check(cudaMemcpyAsync(s.h_const, s.constpart, (size_t)s.ntiles * NSLOT * 8, cudaMemcpyDeviceToHost, stream_),
                "copy constant parts");
-    // a queued launch that gave up waiting on a tile says so here
-    int i = 0;
-    for (auto &kv : groups_)
-        if (kv.second->d_queue && i < kMaxGroups)
-            cuda_check(cudaMemcpyAsync(s.h_const + (size_t)s.ntiles * NSLOT + i++, kv.second->d_queue + 2, sizeof(int),
-                                       cudaMemcpyDeviceToHost, stream_),
-                       "copy queue state");
-    s.nqueues = i;
+    // a queued launch that gave up waiting on a tile says so for good; one copy
+    // serves every solve fetched after the same launches (a copy per solve and
+    // class filled the stream's queue of a 256-solve batch and held up its run)
+    if (queue_unread_) {
+        if (!h_queue_) {
+            h_queue_ = static_cast<int *>(pinned_.get(kMaxGroups * sizeof(int)));
+            std::memset(h_queue_, 0, kMaxGroups * sizeof(int));
+        }
+        int i = 0;
+        for (auto &kv : groups_)
+            if (kv.second->d_queue && i < kMaxGroups)
+                cuda_check(cudaMemcpyAsync(h_queue_ + i++, kv.second->d_queue + 2, sizeof(int), cudaMemcpyDeviceToHost,
+                                           stream_),
+                           "copy queue state");
+        queue_unread_ = false;
+    }
     cuda_check(cudaEventRecord(s.ev, stream_), "event record");
     s.fetched = true;
 }
@@ -630,11 +639,8 @@ void Engine::raw_outputs(int id, std::vector<double> &jout, double cp[NSLOT])
     Solve &s = get(id);
     if (!s.fetched) fetch_async(id);
     cuda_check(cudaEventSynchronize(s.ev), "event sync");
-    for (int i = 0; i < s.nqueues; ++i) {
-        int err;
-        std::memcpy(&err, s.h_const + (size_t)s.ntiles * NSLOT + i, sizeof(int));
-        if (err) throw CudaError("a launch gave up waiting for a tile's earlier steps");
-    }
+    for (int i = 0; h_queue_ && i < kMaxGroups; ++i)
+        if (*static_cast<volatile int *>(h_queue_ + i)) throw CudaError("a launch gave up waiting for a tile's earlier steps");
     for (int q = 0; q < NSLOT; ++q) cp[q] = 0.0;
     for (int t = 0; t < s.ntiles; ++t)
         for (int q = 0; q < NSLOT; ++q) cp[q] += s.h_const[(size_t)t * NSLOT + q];
@@ -700,19 +706,30 @@ SolveOutputs Engine::outputs(int id, const std::vector<double> *laser)
     raw_outputs(id, j, cp);
     SolveOutputs o;
     const Solve &s = get(id);
-    assemble_outputs(s.prob, j, cp, o, laser ? laser : &s.laser);
+    if (!laser) {
+        std::lock_guard<std::mutex> lk(laser_mu_);   // once there, a solve's columns stay
+        if (!s.laser.empty()) laser = &s.laser;
+    }
+    assemble_outputs(s.prob, j, cp, o, laser);
     return o;
 }
 
-void Engine::prepare_outputs()
+void Engine::prepare_outputs(int id)
 {
+    const Solve &want = get(id);
+    if (!want.fetched) return;
     size_t bytes = 0;
-    for (auto &kv : live_) {
-        Solve &s = *kv.second;
+    auto prepare = [&](Solve &s) {
         bytes += (size_t)s.Nt * 56;
-        if (bytes > ((size_t)128 << 20)) return;
+        if (bytes > ((size_t)128 << 20) || cudaEventQuery(want.ev) != cudaErrorNotReady) return false;
+        cudaGetLastError();   // "not ready" stays behind as the thread's last error
+        std::lock_guard<std::mutex> lk(laser_mu_);
         if (s.laser.empty()) s.laser = laser_rows(s.prob);
-    }
+        return true;
+    };
+    if (!prepare(get(id))) return;
+    for (auto &kv : live_)
+        if (!prepare(*kv.second)) return;
 }
 
 void Engine::remove(int id)
@@ -731,7 +748,7 @@ void Engine::remove(int id)
     if (s.snap_pi) cudaFreeAsync(s.snap_pi, stream_);
     if (s.fetched) cudaEventSynchronize(s.ev);
     pinned_.put(s.h_jout, (size_t)s.Nt * NSLOT * 8);
-    pinned_.put(s.h_const, ((size_t)s.ntiles * NSLOT + kMaxGroups) * 8);
+    pinned_.put(s.h_const, (size_t)s.ntiles * NSLOT * 8);
     cudaEventDestroy(s.ev);
     bytes_in_use_ -= s.bytes;
     free_slots_.push_back(s.slot);

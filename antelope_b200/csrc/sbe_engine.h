@@ -119,9 +119,11 @@ public:
     bool ready(int id);
     // `laser` may hold the problem's laser_rows() already built by the caller
     SolveOutputs outputs(int id, const std::vector<double> *laser = nullptr);
-    // Evaluate the laser columns of the resident solves' outputs (host work
-    // that can run while the GPU propagates), up to 128 MB of them
-    void prepare_outputs();
+    // Evaluate laser columns of the resident solves' outputs -- `id`'s, then
+    // others', up to 128 MB of them -- while `id`'s results are still to come.
+    // (Done at the run's end instead, they held up callers that leave the GPU
+    // to itself.)
+    void prepare_outputs(int id);
     // The raw per-step sums [Nt][NSLOT] and the summed constant parts of a
     // fetched solve (waits for the copy); assemble_outputs() turns them into
     // the output arrays.
@@ -176,6 +178,9 @@ private:
     std::pair<cudaEvent_t, cudaEvent_t> new_pair();
     size_t bytes_in_use_ = 0;
     std::map<int, std::unique_ptr<Solve>> live_;
+    std::mutex laser_mu_;   // the solves' laser columns
+    int *h_queue_ = nullptr;       // the tile queues' error marks (pinned)
+    bool queue_unread_ = false;    // launches since they were copied
     std::vector<int> free_slots_;
     SolveDev *d_solves_ = nullptr;
     std::vector<SolveDev> h_solves_;   // host mirror of the descriptors
