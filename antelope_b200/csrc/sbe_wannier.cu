@@ -27,6 +27,15 @@
 // FP32 rounding of -i[H0, rho] or of the eigenbasis would add a field-
 // independent source that accumulates over the pulse; an FP32-synthesised H0
 // only perturbs the model itself, smoothly.
+//
+// The general kernels: one attempted step per launch, any N <= 8, any model,
+// step rule and method.  Three classes of solves run elsewhere in the plain
+// method: fixed steps of the velocity gauge (both methods) and, in the length
+// gauge, of the analytic materials (sbe_wanstep.cu), and the length gauge of
+// explicit tables at N = 3 ... 6 (sbe_wanproj.cu).  Here remain the Cash-Karp
+// steps of the velocity gauge, the mixed method of the length gauge, the
+// continuum model, and grids with a point where two bands meet (in the length
+// gauge the outcome there depends on the eigenbasis taken).
 #include <cuda_runtime.h>
 
 #include <type_traits>

@@ -148,7 +148,7 @@ cudaError_t launch_field_table(const LaserDev &L, double atmin, double dt, int N
 size_t wan_smem_bytes(int N, int nR, int precision);
 // The grouped attempt kernel (eight lanes per k-point) runs the length-gauge
 // attempts of explicit tables with the -dH/dk + i[D, H] current operator at
-// N = 4 and 6: wan_grouped_applies says whether a solve qualifies (before its
+// N = 4 and 6 that wan_proj does not take: wan_grouped_applies says whether a solve qualifies (before its
 // re-laid tables exist), wan_grouped whether it runs on it; its blocks cover
 // WAN_GROUP_TILES tiles, so batched tile lists of such a class are in blocks.
 constexpr int WAN_GROUP_TILES = 4;

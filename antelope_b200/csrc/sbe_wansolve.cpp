@@ -1,5 +1,5 @@
-// Host side of the N-band Wannier solves (length gauge): device buffers,
-// model upload, the attempt/controller launch loop, and the assembly of the
+// Host side of the N-band solves: device buffers, model upload, the launch
+// loop (attempt and controller, or many fixed steps), and the assembly of the
 // reference's output quantities for N bands (antelope.cpp:514-548).
 #include "sbe_wansolve.h"
 

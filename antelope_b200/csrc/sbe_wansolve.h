@@ -1,4 +1,4 @@
-// One N-band Wannier solve (length gauge) on the GPU; see sbe_wannier.cu.
+// One N-band solve on the GPU; see sbe_wannier.cu, sbe_wanstep.cu, sbe_wanproj.cu.
 #pragma once
 
 #include <cuda_runtime.h>
