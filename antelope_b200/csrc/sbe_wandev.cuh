@@ -164,6 +164,91 @@ __device__ void kpoint(const WanDev &P, int kl, double kv[3], double &wt)
         kv[dd] = P.origin[dd] + f[0] * P.axes[0 * 3 + dd] + f[1] * P.axes[1 * 3 + dd] + f[2] * P.axes[2 * 3 + dd];
 }
 
+// Where the Lanczos projections of wan_attempt_p and wan_lw_steps lose the
+// eigenvectors' accuracy: do bands crowd?  A basis matrix amplifies the rounding
+// of the one before by r_j^-1/2, r_j = |P_j|^2 / (|A|^2 |P_{j-1}|^2) (A: H0 without
+// its trace), so D(Y) is good to eps / sqrt(prod r_j) -- 0.1 to 2 times that in
+// random frames at N = 4, 5, 6 -- where eigenvectors are to eps / gap.  A close pair
+// makes one small factor and costs nothing beyond eps / gap; a cluster of m bands of
+// relative width d costs eps / d^(m-1).  The projection stands where the estimate is
+// below 5.5e-12, or all of it but a factor of 30 is the last r_j's (of N = 4: or the
+// other's).  The product telescopes to |P_{N-1}|^2 / |A|^(2N-2); hh = |H0|^2 in place of
+// one |A|^2 is H0's own rounding.  p2, b: |P_{N-1}|^2 and its ratio to the one
+// before.  Not for N = 3: three close bands are the whole spectrum there.
+template <int N> __device__ __forceinline__ bool bands_crowd(double p2, double b, double a2, double hh)
+{
+    double s = hh;
+#pragma unroll
+    for (int j = 3; j < N; ++j) s *= a2;
+    return N > 3 && p2 < 4e-10 * s * a2 && p2 < 1e-3 * s * b && (N != 4 || b < 1e-3 * a2);
+}
+// The same from band energies
+template <int N> __device__ bool bands_crowd(const double *e)
+{
+    double a[N], p[N], q[N], t0 = 0.0, a2 = 0.0, b = 0.0;
+    for (int n = 0; n < N; ++n) t0 += e[n] / N;
+    for (int n = 0; n < N; ++n) {
+        p[n] = a[n] = e[n] - t0;
+        q[n] = 0.0;
+        a2 += a[n] * a[n];
+    }
+    double p2 = a2;
+    for (int j = 2; j < N && p2 > 0.0; ++j) {
+        double s = 0.0, w2 = 0.0;
+        for (int n = 0; n < N; ++n) s += a[n] * p[n] * p[n];
+        for (int n = 0; n < N; ++n) {
+            const double w = (a[n] - s / p2) * p[n] - b * q[n] - (j == 2 ? p2 / N : 0.0);
+            q[n] = p[n];
+            p[n] = w;
+            w2 += w * w;
+        }
+        b = w2 / p2;
+        p2 = w2;
+    }
+    return !(p2 > 0.0) || bands_crowd<N>(p2, b, a2, a2 + N * t0 * t0);
+}
+
+// Jacobi rotation of the 2 x 2 block (a, z; conj z, b): V = (c, s; -conj s, c) makes
+// V^dag (...) V diagonal, a - dl and b + dl
+struct Turn {
+    double c;
+    double2 s;
+    __device__ __forceinline__ void find(double a, double b, double2 z, double &dl)
+    {
+        const double m2 = fma(z.x, z.x, z.y * z.y), d = b - a;
+        c = 1.0;
+        s = make_double2(0.0, 0.0);
+        dl = 0.0;
+        if (m2 > 0.0) {
+            const double rh = rsqrt(fma(d, d, 4.0 * m2));   // of twice the angle: cos |d| rh, sin 2 |z| rh
+            const double c2 = fma(0.5 * fabs(d), rh, 0.5), rc = rsqrt(c2), g = copysign(rh * rc, d);
+            c = c2 * rc;
+            s = make_double2(z.x * g, z.y * g);
+            dl = m2 * g * rc;
+        }
+    }
+    // (x, y) -> (x, y) V of a row of a matrix; V^dag (x, y) of a column takes conj(s)
+    __device__ __forceinline__ void on(double2 &x, double2 &y, double2 s) const
+    {
+        const double2 u = x;
+        x = make_double2(fma(-s.x, y.x, fma(-s.y, y.y, c * u.x)), fma(-s.x, y.y, fma(s.y, y.x, c * u.y)));
+        y = make_double2(fma(s.x, u.x, fma(-s.y, u.y, c * y.x)), fma(s.x, u.y, fma(s.y, u.x, c * y.y)));
+    }
+    // V^dag B V of the pair's own block (a, z; conj z, b)
+    __device__ __forceinline__ void own(double &a, double2 &z, double &b) const
+    {
+        double2 p = make_double2(a, 0.0), q = z, r = cconj(z), t = make_double2(b, 0.0);
+        on(p, q, s);
+        on(r, t, s);
+        on(p, r, cconj(s));
+        on(q, t, cconj(s));
+        a = p.x;
+        z = q;
+        b = t.x;
+    }
+};
+constexpr int MAX_SWEEPS = 12;
+
 // Accept or reject an attempt of error emax and set up the next one.  The
 // step-size rule is the oracle's (oracle/sbe_oracle.c, run_adaptive).
 __device__ void control_decide(const WanDev &P, WanCtl *ctl, double emax)

@@ -565,6 +565,10 @@ __global__ void __launch_bounds__(32 * WAN_WARPS) wan_init(WanDev P)
         if (lane == 0) {   // non-negative doubles order as their bits
             atomicMin(P.band_gap, (unsigned long long)__double_as_longlong(gap));
             atomicMax(P.band_gap + 1, (unsigned long long)__double_as_longlong(wid));
+            double ev[WAN_MAXN];
+            for (int n = 0; n < N; ++n) ev[n] = w.B[n * N + n].x;
+            if (N == 4 ? bands_crowd<4>(ev) : N == 5 ? bands_crowd<5>(ev) : N == 6 ? bands_crowd<6>(ev) : false)
+                atomicAdd(P.band_gap + 2, 1ull);
         }
     }
     // occupations of the eigenstates: the Nval lowest filled, or Fermi-Dirac (SBEs.h:319-340)

@@ -108,9 +108,11 @@ struct WanDev {
     const int *gmate;
     int mixed;              // the mixed method (FP32 Fourier sums)
     // length gauge: bits of the smallest gap between two bands and of the
-    // largest spread of the bands over the grid (wan_init), or null
+    // largest spread of the bands over the grid, and the number of its points
+    // where bands crowd (wan_init), or null
     unsigned long long *band_gap;
-    int degenerate;   // bands meet at a grid point: neither wan_steps nor wan_proj applies
+    int degenerate;   // neither wan_steps nor wan_proj applies: bands meet on the grid, or crowd
+                      // and it is one that wan_crowded_slow names
     // projection attempt kernel (wan_proj): the grid's rows along its fast axis
     // (axis gr_fast, gr_nf points; the solve's rows start at gr_row0), the
     // groups of vectors R with equal b.R = +-gr_a (b the fast axis; gr_n of
@@ -182,6 +184,9 @@ cudaError_t launch_wan_control_batch(const WanDev *const *descs, int nsolves, in
 // (tile = the first one).  `descs` / `tiles` null: a single solve (`dw`).
 constexpr int WAN_STEPS = 64;
 int wan_steps(const WanDev &w);   // 0: no; otherwise the kernel form (mode)
+// Is the length-gauge kernel of wan_steps or wan_proj slower than the tracked one on a
+// grid where bands crowd at `points` of its points?
+bool wan_crowded_slow(const WanDev &w, unsigned long long points);
 int wan_steps_rows(const WanDev &w);
 int wan_steps_fields(int rk);
 int wan_steps_unit(int mode, int N);

@@ -14,8 +14,9 @@
 //    a_j P_j - b_j P_{j-1} from I gives an orthogonal basis of them in N - 2
 //    products; tracking the eigenbasis took 1.9 rotation steps a stage of four
 //    products each, and half of the kernel's time.  Conditioned like the
-//    eigenvectors: over a 100 x 100 grid of N = 6 models D(Y) is within 1.5e-14
-//    of the eigensolver's, its own rounding over the smallest gap.
+//    eigenvectors -- over a 100 x 100 grid of N = 6 models D(Y) is within 1.5e-14
+//    of the eigensolver's, its own rounding over the smallest gap -- except where
+//    three or more bands crowd (bands_crowd); those k-points go by eigenvectors.
 //  - Fourier sums in two levels.  A row of the grid has k = k_row + f b, so the
 //    vectors R with equal b.R share their phase along the row: with G_g =
 //    sum of h_R e^{i(k_row + A).R} over such a group, H0(k + A) = sum_g G_g
@@ -30,10 +31,10 @@
 // the limit of one row per lane in groups of 8 (a 16-byte element at one address
 // per group costs 4 wavefronts, whatever the number of groups; 4 k-points per
 // warp, 6 of 8 lanes at work): Cash-Karp attempts of N = 6, 4, 3 on 200 x 300
-// points took 681, 251 and 144 us, now 361, 137 and 108; on 100 x 100 162, 82 and
-// 52, now 85, 51 and 46; on 8 x 8 68, 61 and 41, now 60, 41 and 37.  What does not
+// points took 681, 251 and 144 us, now 380, 141 and 111; on 100 x 100 162, 82 and
+// 52, now 88, 52 and 46; on 8 x 8 68, 61 and 41, now 65, 42 and 38.  What does not
 // fit the 255 registers of N = 6 stays in shared memory (the slope while the
-// projection adds to it) or is read again (the state): 408 and 90 us with both
+// projection adds to it) or is read again (the state): 11 and 6 % more with both
 // kept, their spills missing an L1 that the blocks' shared memory leaves 28 KB.
 // Bound: latencies at two warps a scheduler; FP64 issue a quarter to a third of
 // the time.
@@ -261,6 +262,146 @@ __device__ __forceinline__ double tr_s(const double2 (&x)[PD<N>::NE], const doub
     return u - 2.0 * t;
 }
 
+
+// D(Y) by eigenvectors, for the k-points where bands crowd, the groups of the warp at
+// once: Jacobi rotations of A until it is diagonal and of Y along with it, then Y's
+// diagonal back through them.  In a round a lane has one of the N/2 disjoint pairs
+// and keeps its rotation; the blocks between two pairs (and, of odd N, between a pair
+// and the row left over) are dealt out to the group's lanes.  Two matrices of room,
+// no eigenvectors kept.
+template <int N> struct Slots {   // elements of a Hermitian matrix in its slots, each kept once
+    using D = PD<N>;
+    double2 *P;
+    __device__ __forceinline__ double2 *at(int r, int c, bool &cj) const
+    {
+        const int d = c >= r ? c - r : c - r + N;
+        cj = d > D::M || (D::EVEN && d == D::M && r >= D::M);
+        return P + (cj ? D::slot(N - d, c) : D::slot(d, r));
+    }
+    __device__ __forceinline__ double2 get(int r, int c) const
+    {
+        bool cj;
+        const double2 x = *at(r, c, cj);
+        return cj ? cconj(x) : x;
+    }
+    __device__ __forceinline__ void set(int r, int c, const double2 &x) const
+    {
+        bool cj;
+        double2 *p = at(r, c, cj);
+        *p = cj ? cconj(x) : x;
+    }
+};
+// The row at place x of round rd (pair i: places 2 i and 2 i + 1), round robin
+template <int N> __device__ __forceinline__ int round_row(int rd, int x)
+{
+    constexpr int n = N % 2 ? N : N - 1;
+    if (N % 2 == 0 && x == 1) return N - 1;
+    const int j = (x >> 1) + N % 2, y = x == N - 1 && N % 2 ? rd : rd + (x & 1 ? n - j : j);
+    return y >= n ? y - n : y;
+}
+// A round's rotations on the blocks off the pairs of X (and of X2)
+template <int N, int NM>
+__device__ __forceinline__ void turn_blocks(const Slots<N> (&X)[NM], int rd, const Turn &own, int m, int base, bool work)
+{
+    constexpr int NP = N / 2, NB = NP * (NP - 1) / 2, NT = NB + N % 2 * NP, G = PD<N>::G;
+#pragma unroll 1
+    for (int x0 = 0; x0 < NM * NT; x0 += G) {
+        const int x = min(x0 + m, NM * NT - 1), e = x % NT;
+        const int i = e < NB ? (NP == 3 && e == 2) : e - NB, j = e < NB ? (NP == 3 ? min(e + 1, 2) : 1) : NP;
+        Turn ti, tj;
+        ti.c = __shfl_sync(ALL, own.c, base + i);
+        ti.s = make_double2(__shfl_sync(ALL, own.s.x, base + i), __shfl_sync(ALL, own.s.y, base + i));
+        tj.c = __shfl_sync(ALL, own.c, base + min(j, NP - 1));
+        tj.s = make_double2(__shfl_sync(ALL, own.s.x, base + min(j, NP - 1)), __shfl_sync(ALL, own.s.y, base + min(j, NP - 1)));
+        if (!work || x0 + m >= NM * NT) continue;
+        const Slots<N> Z = NM == 1 || x < NT ? X[0] : X[NM - 1];
+        const int p = round_row<N>(rd, 2 * i), q = round_row<N>(rd, 2 * i + 1), r = round_row<N>(rd, 2 * j);
+        double2 pr = Z.get(p, r), qr = Z.get(q, r);
+        if (j < NP) {
+            const int u = round_row<N>(rd, 2 * j + 1);
+            double2 pu = Z.get(p, u), qu = Z.get(q, u);
+            tj.on(pr, pu, tj.s);
+            tj.on(qr, qu, tj.s);
+            ti.on(pu, qu, cconj(ti.s));
+            Z.set(p, u, pu);
+            Z.set(q, u, qu);
+        }
+        ti.on(pr, qr, cconj(ti.s));
+        Z.set(p, r, pr);
+        Z.set(q, r, qr);
+    }
+}
+// at: the group's matrices in shared memory, A in the second slots and Y in the
+// first; D(Y) is left in the second.  Groups without `work` only pass through.
+template <int N> __device__ __noinline__ void eigen_diagonal(int at, int m, int base, bool work)
+{
+    using D = PD<N>;
+    constexpr int NP = N / 2, NR = N % 2 ? N : N - 1, G = D::G;
+    extern __shared__ __align__(16) double2 sm[];
+    double2 *const v = sm + at;
+    const Slots<N> AY[2] = {{v + D::HT}, {v + D::Y}}, A[1] = {{v + D::HT}};
+    Turn rot[MAX_SWEEPS * NR];
+    const bool mine = work && m < NP;
+    const int place = 2 * min(m, NP - 1);
+    int n = 0;
+#pragma unroll 1
+    for (int sweep = 0; sweep < MAX_SWEEPS; ++sweep) {
+        double off = 0.0, all = 0.0;
+#pragma unroll 1
+        for (int e = m; e < N * N; e += G) {
+            const double2 z = A[0].get(e / N, e % N);
+            const bool diag = e / N == e % N;
+            const double q = diag ? z.x * z.x : fma(z.x, z.x, z.y * z.y);
+            all += q;
+            off += diag ? 0.0 : q;
+        }
+        off = gsum<G>(off, base);
+        all = gsum<G>(all, base);
+        if (!__any_sync(ALL, work && off > 1e-36 * all)) break;
+#pragma unroll 1
+        for (int rd = 0; rd < NR; ++rd, ++n) {
+            const int p = round_row<N>(rd, place), q = round_row<N>(rd, place + 1);
+            Turn t;
+            t.c = 1.0;
+            t.s = make_double2(0.0, 0.0);
+            if (mine) {
+                double dl, a = v[D::Y + p].x, b = v[D::Y + q].x;
+                double2 z = AY[1].get(p, q);
+                t.find(v[D::HT + p].x, v[D::HT + q].x, A[0].get(p, q), dl);
+                v[D::HT + p].x -= dl;
+                v[D::HT + q].x += dl;
+                A[0].set(p, q, make_double2(0.0, 0.0));
+                t.own(a, z, b);
+                v[D::Y + p].x = a;
+                v[D::Y + q].x = b;
+                AY[1].set(p, q, z);
+            }
+            rot[n] = t;
+            turn_blocks<N, 2>(AY, rd, t, m, base, work);
+            __syncwarp();
+        }
+    }
+    if (work)
+        for (int e = m; e < D::NM; e += G) v[D::HT + e] = make_double2(e < N ? v[D::Y + e].x : 0.0, 0.0);
+    __syncwarp();
+#pragma unroll 1
+    while (n > 0) {   // D = V D' V^dag, the last rotation first
+        const int rd = --n % NR, p = round_row<N>(rd, place), q = round_row<N>(rd, place + 1);
+        Turn t = rot[n];
+        t.s = make_double2(-t.s.x, -t.s.y);
+        if (mine) {
+            double a = v[D::HT + p].x, b = v[D::HT + q].x;
+            double2 z = A[0].get(p, q);
+            t.own(a, z, b);
+            v[D::HT + p].x = a;
+            v[D::HT + q].x = b;
+            A[0].set(p, q, z);
+        }
+        turn_blocks<N, 1>(A, rd, t, m, base, work);
+        __syncwarp();
+    }
+}
+
 }  // namespace
 
 // Shared memory of a block: slopes, the groups' matrices, the phases along the row
@@ -270,27 +411,17 @@ template <int N> static int proj_bytes(int ngrp, int S)
     return (S * D::NE * 32 + D::KW * D::END + D::KW * ngrp) * 16;
 }
 
-template <int N>
-__global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
-    wan_attempt_p(const WanDev *__restrict__ Pp, const WanDev *const *__restrict__ descs,
-                  const WanTileRef *__restrict__ tiles)
+// One attempted step of a unit of KW k-points; false: bands crowd at a stage of one
+// of them, and nothing but current sums was written.  EIG: those k-points by
+// eigenvectors, in a pass of its own (with the call in the first pass N = 6 took 390
+// us an attempt of 200 x 300 points, with the check alone 380, without 367).
+template <int N, bool EIG>
+__device__ __forceinline__ bool attempt(const WanDev &P, int unit)
 {
+    extern __shared__ __align__(16) double2 sm[];
     using D = PD<N>;
     constexpr int G = D::G, KW = D::KW, LW = D::LW, NE = D::NE, DO = D::DO, M = D::M, NN = D::NN;
-    extern __shared__ __align__(16) double2 sm[];
-    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
-    // KW k-points; consecutive units (they share the tables of a row) to the
-    // blocks of one SM, which get every SPREAD-th block of the grid
-    int unit;
-    if (tiles) {
-        unit = tiles[blockIdx.x].tile;
-    } else {
-        const int nu = (P.nk + KW - 1) / KW, i = (int)blockIdx.x % SPREAD;
-        unit = (int)((long long)i * nu / SPREAD) + (int)blockIdx.x / SPREAD;
-        if (unit >= (int)((long long)(i + 1) * nu / SPREAD)) return;
-    }
     const WanCtl &ctl = *P.ctl;
-    if (ctl.done) return;
     // lanes past the last group shadow its first lanes: same values, to the same
     // addresses where the group shares them
     const int lane = threadIdx.x, grp = min(lane / G, KW - 1), m = lane < LW ? lane % G : lane - LW;
@@ -301,6 +432,8 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
     const int S = c_tab[tab_of(P.rk)].S;
     double2 *const ks = sm + lane;                               // [S][NE][32] slopes, a column per lane
     double2 *const v = sm + S * NE * 32 + grp * D::END;
+    constexpr int CR = 2 * D::NM;                                // past the matrices: |H0|^2; have bands crowded?
+    if (N > 3 && m == 0) v[CR].y = 0.0;
     const int ng = P.gr_n, nent = 2 * ng - 1;                    // group pairs (g = 0 first), table entries
     double2 *const ph = sm + S * NE * 32 + KW * D::END + grp * ng;
     const double h = ctl.hs;
@@ -483,16 +616,16 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
 #pragma unroll
             for (int j = 0; j < NE; ++j) p[j] = a0[j];
             if (!D::EVEN) p[DO].y = 0.0;
-            put<N>(v + D::Y, a0, m);   // Y is done with
             const double t0 = gsum<G>(p[DO].x + p[DO].y, base) * (1.0 / N);
             const double ty = gsum<G>(D::EVEN ? y[DO].x + y[DO].y : y[DO].x, base) * (1.0 / N);
             p[DO].x -= t0;
             if (D::EVEN) p[DO].y -= t0;
-            put<N>(Ps, p, m);
+            put<N>(v + D::Y, p, m);   // A: H0 without its trace (Y is done with)
             double p2 = gsum<G>(dot<N>(p, p), base);
             const double py = gsum<G>(dot<N>(p, y), base);
             const double a2 = p2;
             double ip = p2 > 0.0 ? 1.0 / p2 : 0.0, b = 0.0;
+            if (N > 3 && m == 0) v[CR].x = fma(N * t0, t0, a2);   // |H0|^2
 #pragma unroll
             for (int j = 0; j < NE; ++j) {
                 const double x = py * ip;
@@ -507,7 +640,7 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
 #pragma unroll 1
             for (int i = 2; i < N; ++i) {
                 double2 w[NE];
-                product<N>(w, H, Ps, ro);
+                product<N>(w, H, i == 2 ? v + D::Y : Ps, ro);
                 const double a = gsum<G>(dot<N>(w, p), base) * ip;
 #pragma unroll
                 for (int j = 0; j < NE; ++j) {
@@ -515,7 +648,7 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
                     w[j].y = fma(-a, p[j].y, fma(-b, q[j].y, w[j].y));
                     q[j] = p[j];
                 }
-                if (i == 2) {   // Tr(H0 P_1) / N
+                if (i == 2) {   // Tr(A P_1) / N
                     w[DO].x -= p2 * (1.0 / N);
                     if (D::EVEN) w[DO].y -= p2 * (1.0 / N);
                 }
@@ -533,6 +666,25 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
                 }
                 if (i + 1 < N) put<N>(Ps, p, m);
                 __syncwarp();
+            }
+            if (N > 3 && !EIG && m == 0 && bands_crowd<N>(p2, b, a2, v[CR].x)) v[CR].y = 1.0;
+            if constexpr (EIG) {
+                const bool bad = bands_crowd<N>(p2, b, a2, v[CR].x);
+                if (__any_sync(ALL, live && bad)) {
+                    for (int e = m; e < D::NM; e += G)
+                        if (lane < LW) Ps[e] = v[D::Y + e];
+                    __syncwarp();
+                    put<N>(v + D::Y, y, m);
+                    __syncwarp();
+                    eigen_diagonal<N>((int)(v - sm), m, base, live && bad);
+                    if (bad) {
+                        const Slots<N> Dy{Ps};
+#pragma unroll
+                        for (int j = 0; j < DO; ++j) d[j] = Dy.get(erow(j), ecol(j));
+                        d[DO] = make_double2(Ps[m].x, D::EVEN ? Ps[m + M].x : 0.0);
+                    }
+                    __syncwarp();
+                }
             }
 #pragma unroll
             for (int j = 0; j < NE; ++j) {
@@ -561,6 +713,10 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
                 if ((lane & 7) == 0) out[lane >> 3] = x;
             }
         }
+    }
+    if (N > 3 && !EIG) {
+        __syncwarp();
+        if (__any_sync(ALL, live && v[CR].y != 0.0)) return false;
     }
     // trial state and error estimate
     double emax = 0.0;
@@ -603,6 +759,35 @@ __global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
         for (int o = 16; o > 0; o >>= 1) emax = fmax(emax, __shfl_xor_sync(ALL, emax, o));
         // non-negative doubles order as their bits; a NaN's are above all
         if (lane == 0) atomicMax(P.gr_err, (unsigned long long)__double_as_longlong(fabs(emax)));
+    }
+    return true;
+}
+// A block's unit of KW k-points (-1: none): consecutive units (they share the tables of a
+// row) go to the blocks of one SM, which get every SPREAD-th block of the grid
+template <int N> __device__ __forceinline__ int block_unit(const WanDev &P, const WanTileRef *tiles)
+{
+    if (tiles) return tiles[blockIdx.x].tile;
+    const int nu = (P.nk + PD<N>::KW - 1) / PD<N>::KW, i = (int)blockIdx.x % SPREAD;
+    const int unit = (int)((long long)i * nu / SPREAD) + (int)blockIdx.x / SPREAD;
+    return unit < (int)((long long)(i + 1) * nu / SPREAD) ? unit : -1;
+}
+template <int N>
+__device__ __noinline__ void attempt_eig(const WanDev *Pp, const WanDev *const *descs, const WanTileRef *tiles)
+{
+    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
+    attempt<N, true>(P, block_unit<N>(P, tiles));
+}
+
+template <int N>
+__global__ void __launch_bounds__(32, N == 6 || N == 4 ? 8 : N == 5 ? 12 : 16)
+    wan_attempt_p(const WanDev *__restrict__ Pp, const WanDev *const *__restrict__ descs,
+                  const WanTileRef *__restrict__ tiles)
+{
+    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
+    const int unit = block_unit<N>(P, tiles);
+    if (unit < 0 || P.ctl->done) return;
+    if (!attempt<N, false>(P, unit)) {
+        if constexpr (N > 3) attempt_eig<N>(Pp, descs, tiles);
     }
 }
 

@@ -117,16 +117,18 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     // the projections of the length gauge need bands that do not meet on the grid
     const bool lw_new = !w_.vg && (wan_steps(w_) != 0 || wan_proj_applies(w_));
     if (lw_new) {
-        dalloc(&w_.band_gap, 16, st, "alloc band gap");
+        dalloc(&w_.band_gap, 24, st, "alloc band gap");
         cuda_check(cudaMemsetAsync(w_.band_gap, 0x7f, 8, st), "clear band gap");   // a large double
-        cuda_check(cudaMemsetAsync(w_.band_gap + 1, 0, 8, st), "clear band gap");
+        cuda_check(cudaMemsetAsync(w_.band_gap + 1, 0, 16, st), "clear band gap");
     }
     cuda_check(launch_wan_init(w_, precision_, st), "Wannier init kernel");
     if (lw_new) {
+        unsigned long long bits[3];
         double gw[2];
-        cuda_check(cudaMemcpyAsync(gw, w_.band_gap, 16, cudaMemcpyDeviceToHost, st), "copy band gap");
+        cuda_check(cudaMemcpyAsync(bits, w_.band_gap, 24, cudaMemcpyDeviceToHost, st), "copy band gap");
         cuda_check(cudaStreamSynchronize(st), "sync");
-        w_.degenerate = !(gw[0] > 1e-7 * gw[1]);
+        std::memcpy(gw, bits, 16);
+        w_.degenerate = !(gw[0] > 1e-7 * gw[1]) || wan_crowded_slow(w_, bits[2]);
     }
     if (wan_steps(w_)) {
         w_.step_rows = wan_steps_rows(w_);

@@ -590,6 +590,66 @@ template <int N> __device__ __forceinline__ void mul_traceless(Herm<N> &W, const
     traceless<N>(W);
 }
 
+// V^dag X V, rows p < q
+template <int N> __device__ __forceinline__ void turn(Herm<N> &X, int p, int q, const Turn &t)
+{
+    t.own(X.d[p], X.o[oidx(p, q, N)], X.d[q]);
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        if (r == p || r == q) continue;
+        double2 x = el<N>(X, r, p), y = el<N>(X, r, q);
+        t.on(x, y, t.s);
+        if (r < p) X.o[oidx(r, p, N)] = x;
+        else X.o[oidx(p, r, N)] = cconj(x);
+        if (r < q) X.o[oidx(r, q, N)] = y;
+        else X.o[oidx(q, r, N)] = cconj(y);
+    }
+}
+// D(Y) by eigenvectors, for k-points where bands crowd: Jacobi rotations of A until it is
+// diagonal and of Y along with it, then Y's diagonal back through them.  Out of line.
+template <int N> __device__ __noinline__ void eigen_diagonal(Herm<N> *D, const Herm<N> *A0, const Herm<N> *Y0)
+{
+    Turn rot[MAX_SWEEPS * Herm<N>::NO];
+    Herm<N> A = *A0, Y = *Y0;
+    int n = 0;
+#pragma unroll 1
+    for (int sweep = 0; sweep < MAX_SWEEPS; ++sweep) {
+        double off = 0.0;
+#pragma unroll
+        for (int i = 0; i < Herm<N>::NO; ++i) off += A.o[i].x * A.o[i].x + A.o[i].y * A.o[i].y;
+        if (!(off > 1e-36 * tr2<N>(A, A))) break;
+#pragma unroll
+        for (int p = 0; p < N - 1; ++p)
+#pragma unroll
+            for (int q = p + 1; q < N; ++q) {
+                Turn t;
+                double dl;
+                t.find(A.d[p], A.d[q], A.o[oidx(p, q, N)], dl);
+                turn<N>(Y, p, q, t);
+                const double a = A.d[p] - dl, b = A.d[q] + dl;
+                turn<N>(A, p, q, t);
+                A.d[p] = a;
+                A.d[q] = b;
+                A.o[oidx(p, q, N)] = make_double2(0.0, 0.0);
+                rot[n++] = t;
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < Herm<N>::NO; ++i) Y.o[i] = make_double2(0.0, 0.0);
+#pragma unroll 1
+    while (n > 0) {   // the last rotation first
+#pragma unroll
+        for (int p = N - 2; p >= 0; --p)
+#pragma unroll
+            for (int q = N - 1; q > p; --q) {
+                Turn t = rot[--n];
+                t.s = make_double2(-t.s.x, -t.s.y);
+                turn<N>(Y, p, q, t);
+            }
+    }
+    *D = Y;
+}
+
 // D = the band-diagonal part of Y in the eigenbasis of A, U diag(U^dag Y U)
 // U^dag, without the eigenbasis: for distinct eigenvalues it is the orthogonal
 // projection (inner product Tr(XY)) of Y on the span of I, A, ..., A^{N-1},
@@ -597,13 +657,18 @@ template <int N> __device__ __forceinline__ void mul_traceless(Herm<N> &W, const
 // multiplication by A is self-adjoint) gives an orthogonal basis of Hermitian
 // matrices in N - 2 products, where a tracked eigenbasis takes B = U^dag A U,
 // rotations until it is diagonal, and U diag U^dag.  Conditioned like the
-// eigenvectors (rounding over the smallest gap).  N = 2 is the closed form
-// (s.n) n of the Bloch vector.  A is made traceless.
-template <int N> __device__ __forceinline__ void band_diagonal(Herm<N> &D, Herm<N> &A, const Herm<N> &Y)
+// eigenvectors (rounding over the smallest gap) but for three close bands of
+// N = 4 (bands_crowd), which go by eigenvectors.  N = 2 is the closed form (s.n) n
+// of the Bloch vector.  A is made traceless.  Returns whether bands crowd; D is by
+// eigenvectors then if EIG.
+template <int N, bool EIG> __device__ __forceinline__ bool band_diagonal(Herm<N> &D, Herm<N> &A, const Herm<N> &Y)
 {
-    double ty = 0.0;
+    double ty = 0.0, th = 0.0;
 #pragma unroll
-    for (int m = 0; m < N; ++m) ty += Y.d[m];
+    for (int m = 0; m < N; ++m) {
+        ty += Y.d[m];
+        th += A.d[m];
+    }
     traceless<N>(A);
     const double a2 = tr2<N>(A, A), ia = a2 > 0.0 ? 1.0 / a2 : 0.0;
     clear<N>(D);
@@ -625,8 +690,17 @@ template <int N> __device__ __forceinline__ void band_diagonal(Herm<N> &D, Herm<
             axpy<N>(V, -vw, W);
             const double v2 = tr2<N>(V, V), iv = v2 > 1e-26 * a2 * w2 ? 1.0 / v2 : 0.0;
             axpy<N>(D, tr2<N>(V, Y) * iv, V);
+            if (bands_crowd<N>(v2, v2 * iw, a2, fma(th * th, 1.0 / N, a2))) {
+                if constexpr (EIG) {
+                    Herm<N> d, a = A, y = Y;
+                    eigen_diagonal<N>(&d, &a, &y);
+                    D = d;
+                }
+                return true;
+            }
         }
     }
+    return false;
 }
 
 // H += a pair's term: table entry s [2][NU], phase e
@@ -678,18 +752,16 @@ static int lw_bytes(int N, int rk, int npair)
 // of 367 steps with their set-up, us a step, 168 to 14 640 k-points alike): N =
 // 2, 3, 4 RK4 2.5, 5.7, 9.4, RK5 4.1, 9.2, 15; one attempt and one control
 // launch a step take 78 (N = 3, RK5, 2 400 k-points).
-template <int N, int RK>
-__global__ void __launch_bounds__(WL_T) wan_lw_steps(const WanDev *__restrict__ Pp,
-                                                     const WanDev *const *__restrict__ descs,
-                                                     const WanTileRef *__restrict__ tiles, int S)
+//
+// lw_advance: false if bands crowded at a stage of a k-point; nothing but partial
+// rows was written then.  EIG: those by eigenvectors (in a pass of their own: with
+// the call in the first pass a step took 9.9 us, with the check alone 9.5, without 9.3).
+template <int N, int RK, bool EIG>
+__device__ __forceinline__ bool lw_advance(const WanDev &P, int k0, int S, unsigned char *smem)
 {
     using TB = StepTab<RK>;
     using HN = Herm<N>;
     constexpr int NN = N * N, NU = N * (N + 1) / 2, NO = HN::NO, NK = RK == 4 ? 1 : 5;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
-    const int k0 = tiles ? tiles[blockIdx.x].tile * WAN_WARPS : (int)blockIdx.x * WL_T;
-    if (P.ctl->done) return;
     const int n0 = P.ctl->n, steps = launch_steps(P, n0, S), np = P.npair, ncA = TB::NT * np;
     const int t = threadIdx.x, lane = t & 31;
     const int k = k0 + t;
@@ -745,6 +817,7 @@ __global__ void __launch_bounds__(WL_T) wan_lw_steps(const WanDev *__restrict__ 
     // the step's phase factors go to shared memory; the next step's first 64
     // are on their way in registers meanwhile
     const double2 *cg = P.step_cA;
+    bool crowded = false;
     double2 pre[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) pre[x] = t + x * WL_T < ncA ? cg[t + x * WL_T] : make_double2(0.0, 0.0);
@@ -792,7 +865,7 @@ __global__ void __launch_bounds__(WL_T) wan_lw_steps(const WanDev *__restrict__ 
             }
             {
                 HN A = H;
-                band_diagonal<N>(K, A, Y);   // K = D(Y)
+                crowded |= band_diagonal<N, EIG>(K, A, Y);   // K = D(Y)
             }
             if (s == 0) {   // currents at k + A(t_n) (SBEs.h:694-760): intraband Re Tr(D J), the rest interband
 #pragma unroll
@@ -861,7 +934,8 @@ __global__ void __launch_bounds__(WL_T) wan_lw_steps(const WanDev *__restrict__ 
             }
         }
     }
-    if (!live) return;
+    if (N > 3 && !EIG && __any_sync(0xffffffffu, live && crowded)) return false;
+    if (!live) return true;
     HN Y;
     get(0, Y);
 #pragma unroll
@@ -872,6 +946,25 @@ __global__ void __launch_bounds__(WL_T) wan_lw_steps(const WanDev *__restrict__ 
             rho[m * N + n] = Y.o[oidx(m, n, N)];
             rho[n * N + m] = cconj(Y.o[oidx(m, n, N)]);
         }
+    }
+    return true;
+}
+template <int N, int RK> __device__ __noinline__ void lw_advance_eig(const WanDev &P, int k0, int S, unsigned char *smem)
+{
+    lw_advance<N, RK, true>(P, k0, S, smem);
+}
+
+template <int N, int RK>
+__global__ void __launch_bounds__(WL_T) wan_lw_steps(const WanDev *__restrict__ Pp,
+                                                     const WanDev *const *__restrict__ descs,
+                                                     const WanTileRef *__restrict__ tiles, int S)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const WanDev &P = tiles ? *descs[tiles[blockIdx.x].solve] : *Pp;
+    const int k0 = tiles ? tiles[blockIdx.x].tile * WAN_WARPS : (int)blockIdx.x * WL_T;
+    if (P.ctl->done) return;
+    if (!lw_advance<N, RK, false>(P, k0, S, smem)) {
+        if constexpr (N > 3) lw_advance_eig<N, RK>(P, k0, S, smem);
     }
 }
 
@@ -940,7 +1033,7 @@ __global__ void __launch_bounds__(256) wan_finish(const WanDev *__restrict__ Pp,
 // tables stay with it and with wan_attempt_g, and so do solves with bands that
 // meet at a grid point (to 1e-7 of their spread): what the dephasing does
 // inside such a pair depends on its basis, which only a tracked eigenbasis
-// carries along.
+// carries along; and small grids where three bands crowd (wan_crowded_slow).
 enum StepMode : int { VG_THREAD = 1, VG_ROWS = 2, LW_THREAD = 3 };
 static int row_lanes(int N) { return N <= 4 ? 4 : 8; }
 // dynamic shared memory of a block
@@ -956,6 +1049,19 @@ int wan_steps(const WanDev &w)
     if (w.vg) return w.N <= 3 ? VG_THREAD : VG_ROWS;
     if (w.mixed || !w.has_jtab || w.has_dip || w.cont || w.N > 4 || w.degenerate) return 0;
     return steps_bytes(LW_THREAD, w.N, 2, w.rk, w.nR) <= STEPS_MAX_BYTES ? LW_THREAD : 0;
+}
+// A k-point where bands crowd makes its block take its pass again, with eigenvectors.
+// Measured with such points, us a step or attempt, against the tracked kernels:
+// wan_lw_steps (N = 4, RK4) 50 / 40 on 168 points, 52 / 77 on 3 720, 55 / 199 on
+// 14 640; wan_attempt_p (Cash-Karp) at 64, 10 000 and 60 000 points, all of them or
+// one in 30 crowded, N = 4: 208, 243, 812 all and 206, 292 some / 97, 207, 818; N = 5:
+// 450, 582, 3015 and 507, 768 / 164, 769, 4261; N = 6: 500, 595, 3268 and 595, 1221 /
+// 146, 390, 1433.
+bool wan_crowded_slow(const WanDev &w, unsigned long long points)
+{
+    if (points == 0) return false;
+    if (wan_steps(w)) return w.nk < 2048;
+    return w.N < 6 ? w.nk < 10000 : w.nk < 60000 || points * 32 > (unsigned long long)w.nk;
 }
 static int block_threads(int mode) { return mode == VG_ROWS ? WR_T : mode == LW_THREAD ? WL_T : WS_T; }
 int wan_steps_rows(const WanDev &w)
