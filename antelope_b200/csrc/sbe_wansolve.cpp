@@ -261,10 +261,12 @@ void WannierSolve::setup_rows(const Problem &p, cudaStream_t st)
     std::vector<double> b(nR);
     double bmax = 0.0;
     for (int r = 0; r < nR; ++r) {
-        b[r] = p.bzaxes[3 * fast] * p.w_vec[2 * r] + p.bzaxes[3 * fast + 1] * p.w_vec[2 * r + 1];
-        bmax = std::max(bmax, std::fabs(b[r]));
+        const double bx = p.bzaxes[3 * fast] * p.w_vec[2 * r], by = p.bzaxes[3 * fast + 1] * p.w_vec[2 * r + 1];
+        b[r] = bx + by;
+        bmax = std::max(bmax, std::fabs(bx) + std::fabs(by));
     }
-    const double tol = 1e-10 * bmax;   // the rounding of b.R
+    // the rounding of b.R (axes given to ten digits leave larger differences, which count)
+    const double tol = 1e-14 * bmax;
     std::vector<double> ga{0.0};
     std::vector<std::vector<int>> lists(2);
     for (int r = 0; r < nR; ++r) {
