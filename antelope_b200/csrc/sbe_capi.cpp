@@ -898,7 +898,7 @@ void sbe_server::loop()
                 try {
                     if (wpool->failed(r.wsolve)) {
                         r.state = Request::FAILED;
-                        r.err = "Cash-Karp step size underflow: tolerance unreachable";
+                        r.err = wpool->error(r.wsolve);
                         ++n_failed;
                     } else {
                         r.jout = wpool->sums(r.wsolve);

@@ -21,7 +21,8 @@ template <class T> void dalloc(T **p, size_t bytes, cudaStream_t st, const char 
 }
 }  // namespace
 
-WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin, int k_end)
+WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin, int k_end,
+                           bool defer)
     : prob_(p), precision_(precision), device_(device), stream_(st)
 {
     if (p.model != MODEL_SYNTHETIC_WANNIER && p.model != MODEL_TB && p.model != MODEL_MULTIWSM)
@@ -101,16 +102,8 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     w_.d = d;
     w_.jt = j;
     w_.mixed = precision_ != 0;
-    UploadRing &ring = UploadRing::shared();
-    if (!p.w_vec.empty()) ring.upload(V, p.w_vec.data(), sizeof(double) * p.w_vec.size(), st);
-    auto up_real = [&](void *dst, const std::vector<double> &src) {
-        if (precision_ == 0) {
-            ring.upload(dst, src.data(), src.size() * 8, st);
-        } else {
-            std::vector<float> f(src.begin(), src.end());
-            ring.upload(dst, f.data(), f.size() * 4, st);
-        }
-    };
+    if (!p.w_vec.empty()) UploadRing::shared().upload(V, p.w_vec.data(), sizeof(double) * p.w_vec.size(), st);
+    auto up_real = [&](void *dst, const std::vector<double> &src) { upload_real(dst, src, st); };
     if (!p.w_h.empty()) up_real(h, p.w_h);
     if (w_.has_dip) up_real(d, p.w_d);
     if (w_.has_jtab && !w_.cont) up_real(j, p.w_j);
@@ -123,12 +116,40 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     }
     cuda_check(launch_wan_init(w_, precision_, st), "Wannier init kernel");
     if (lw_new) {
-        unsigned long long bits[3];
+        h_gap_ = static_cast<unsigned long long *>(PinnedPool::shared().get(24));
+        cuda_check(cudaEventCreateWithFlags(&gap_ev_, cudaEventDisableTiming), "event create");
+        cuda_check(cudaMemcpyAsync(h_gap_, w_.band_gap, 24, cudaMemcpyDeviceToHost, st), "copy band gap");
+        cuda_check(cudaEventRecord(gap_ev_, st), "event record");
+    }
+    if (!defer) finish_setup();
+}
+
+bool WannierSolve::setup_ready()
+{
+    if (!gap_ev_) return true;
+    const cudaError_t q = cudaEventQuery(gap_ev_);
+    if (q == cudaErrorNotReady) {
+        cudaGetLastError();   // "not ready" stays behind as the thread's last error
+        return false;
+    }
+    cuda_check(q, "band gap event");
+    return true;
+}
+
+// The second half of the set-up, once the bands over the grid are known: which
+// kernels run the solve, and their tables.
+void WannierSolve::finish_setup()
+{
+    cudaStream_t st = stream_;
+    const Problem &p = prob_;
+    const int N = w_.N;
+    const size_t cplx = precision_ == 0 ? 16 : 8;
+    if (gap_ev_) {
+        cuda_check(cudaEventSynchronize(gap_ev_), "band gap");
         double gw[2];
-        cuda_check(cudaMemcpyAsync(bits, w_.band_gap, 24, cudaMemcpyDeviceToHost, st), "copy band gap");
-        cuda_check(cudaStreamSynchronize(st), "sync");
-        std::memcpy(gw, bits, 16);
-        w_.degenerate = !(gw[0] > 1e-7 * gw[1]) || wan_crowded_slow(w_, bits[2]);
+        std::memcpy(gw, h_gap_, 16);
+        w_.degenerate = !(gw[0] > 1e-7 * gw[1]) || wan_crowded_slow(w_, h_gap_[2]);
+        drop_gap();
     }
     if (wan_steps(w_)) {
         w_.step_rows = wan_steps_rows(w_);
@@ -225,7 +246,8 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
             w_.stage_gt = sg;
         }
     }
-    if (w_.gtab) up_real(const_cast<void *>(w_.gtab), gt);
+    UploadRing &ring = UploadRing::shared();
+    if (w_.gtab) upload_real(const_cast<void *>(w_.gtab), gt, st);
     if (w_.gpair) ring.upload(const_cast<int *>(w_.gpair), gpair.data(), sizeof(int) * gpair.size(), st);
     if (w_.gmate) ring.upload(const_cast<int *>(w_.gmate), gmate.data(), sizeof(int) * gmate.size(), st);
     cuda_check(cudaMemsetAsync(w_.jout, 0, sizeof(double) * (size_t)w_.Nt * WAN_NSLOT, st), "clear outputs");
@@ -249,6 +271,26 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     if (wan_steps(w_)) cuda_check(launch_wan_step_fields(w_, d_w_, st), "Wannier step fields");
     else cuda_check(launch_wan_prepare(w_, d_w_, precision_, st), "Wannier stage preparation");
     h_ctl_ = static_cast<WanCtl *>(PinnedPool::shared().get(sizeof(WanCtl)));
+}
+
+void WannierSolve::drop_gap()
+{
+    if (gap_ev_) cudaEventDestroy(gap_ev_);
+    gap_ev_ = nullptr;
+    PinnedPool::shared().put(h_gap_, 24);
+    h_gap_ = nullptr;
+}
+
+// To the solve's table precision
+void WannierSolve::upload_real(void *dst, const std::vector<double> &src, cudaStream_t st)
+{
+    UploadRing &ring = UploadRing::shared();
+    if (precision_ == 0) {
+        ring.upload(dst, src.data(), src.size() * 8, st);
+    } else {
+        std::vector<float> f(src.begin(), src.end());
+        ring.upload(dst, f.data(), f.size() * 4, st);
+    }
 }
 
 // The groups of lattice vectors that share their phase along the grid's rows,
@@ -353,6 +395,7 @@ WannierSolve::~WannierSolve()
     if (w_.snap_pi) cudaFreeAsync(w_.snap_pi, stream_);
     cudaStreamSynchronize(stream_);
     PinnedPool::shared().put(h_ctl_, sizeof(WanCtl));
+    drop_gap();
 }
 
 void WannierSolve::run(cudaStream_t st)
@@ -412,8 +455,9 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     for (const Problem *p : probs) {
         const int prec = precision >= 0 ? precision : p->precision;
-        solves_.push_back(std::make_unique<WannierSolve>(*p, prec, device_, st));
+        solves_.push_back(std::make_unique<WannierSolve>(*p, prec, device_, st, 0, 0, true));
     }
+    for (auto &s : solves_) s->finish_setup();   // one wait for all of them
     // launch classes; within a class the solves with the most k-point steps
     // lead the tile list, so their blocks are scheduled first
     for (int i = 0; i < (int)solves_.size(); ++i) {
@@ -619,7 +663,11 @@ size_t WannierPool::bytes_needed(const Problem &p, int precision)
 int WannierPool::add(const Problem &p, int precision)
 {
     Entry e;
-    e.s = std::make_unique<WannierSolve>(p, precision, device_, st_);
+    e.s = std::make_unique<WannierSolve>(p, precision, device_, st_, 0, 0, true);
+    // a solve that waits for its bands waits on the GPU's side: the host would stand
+    // until every tick queued before is done (step() takes it up)
+    e.ready = e.s->setup_ready();
+    if (e.ready) e.s->finish_setup();
     e.bytes = bytes_needed(p, precision);
     bytes_ += e.bytes;
     const int id = next_id_++;
@@ -658,6 +706,12 @@ bool WannierPool::failed(int id) const
     return it != solves_.end() && it->second.failed;
 }
 
+std::string WannierPool::error(int id) const
+{
+    auto it = solves_.find(id);
+    return it == solves_.end() || it->second.err.empty() ? "Cash-Karp step size underflow: tolerance unreachable" : it->second.err;
+}
+
 std::vector<double> WannierPool::sums(int id)
 {
     auto it = solves_.find(id);
@@ -673,7 +727,7 @@ void WannierPool::rebuild()
     }
     classes_.clear();
     for (auto &kv : solves_) {
-        if (kv.second.done) continue;
+        if (kv.second.done || !kv.second.ready) continue;
         const WannierSolve &s = *kv.second.s;
         const WanDev &w = s.dev();
         const int grk = wan_grouped(w) ? w.rk : 0;
@@ -730,6 +784,17 @@ void WannierPool::step(int iters)
 {
     last_launches_ = 0;
     if (pending_) poll();
+    for (auto &kv : solves_) {
+        Entry &e = kv.second;
+        if (e.ready || !e.s->setup_ready()) continue;
+        e.ready = dirty_ = true;
+        try {
+            e.s->finish_setup();
+        } catch (const std::exception &x) {
+            e.done = e.failed = true;
+            e.err = x.what();
+        }
+    }
     if (dirty_) rebuild();
     if (classes_.empty()) return;
     for (int it = 0; it < iters; ++it)

@@ -5,6 +5,7 @@
 
 #include <map>
 #include <memory>
+#include <string>
 #include <vector>
 
 #include "sbe_engine.h"
@@ -14,8 +15,11 @@ namespace sbe {
 
 class WannierSolve {
 public:
-    // k_begin/k_end: a k-slice [k_begin, k_end) of the grid (0, 0: all of it)
-    WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin = 0, int k_end = 0);
+    // k_begin/k_end: a k-slice [k_begin, k_end) of the grid (0, 0: all of it);
+    // defer: finish_setup() is left to the caller (it waits for the bands over the
+    // grid where the choice of kernels depends on them; setup_ready(): it will not wait)
+    WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin = 0, int k_end = 0,
+                 bool defer = false);
     ~WannierSolve();
     WannierSolve(const WannierSolve &) = delete;
     WannierSolve &operator=(const WannierSolve &) = delete;
@@ -38,8 +42,14 @@ public:
     void set_stream(cudaStream_t st) { stream_ = st; }
     // the controller state after a batched run (copied in by the batch)
     void finish_batched(const WanCtl &c, int launches);
+    bool setup_ready();
+    void finish_setup();
 
 private:
+    void drop_gap();
+    void upload_real(void *dst, const std::vector<double> &src, cudaStream_t st);
+    unsigned long long *h_gap_ = nullptr;   // WanDev::band_gap (pinned) until finish_setup()
+    cudaEvent_t gap_ev_ = nullptr;
     void setup_rows(const Problem &p, cudaStream_t st);
     Problem prob_;
     int precision_, device_, nshots_ = 0;
@@ -114,8 +124,10 @@ public:
     void step(int iters);
     void poll();
     bool finished(int id) const;
-    // a finished solve whose step-size controller gave up (tolerance unreachable)
+    // a finished solve whose step-size controller gave up (tolerance unreachable) or
+    // whose set-up failed; and why
     bool failed(int id) const;
+    std::string error(int id) const;
     std::vector<double> sums(int id);
     int last_launches() const { return last_launches_; }
 
@@ -123,7 +135,9 @@ private:
     struct Entry {
         std::unique_ptr<WannierSolve> s;
         size_t bytes = 0;
+        bool ready = true;   // its set-up is finished
         bool done = false, failed = false;
+        std::string err;
     };
     void rebuild();
     std::map<int, Entry> solves_;

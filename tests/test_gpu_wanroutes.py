@@ -4,7 +4,7 @@ import pytest
 
 import antelope_b200 as ab
 from antelope_b200 import wannier
-from cases import variant
+from cases import material, variant
 from oracle import pyoracle
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +37,39 @@ def test_axes_of_ten_digits(tilt):
     scale = max(np.abs(ref["inter"]).max(), np.abs(ref["intra"]).max())
     for key in ("inter", "intra"):
         assert np.abs(getattr(out, key) - ref[key]).max() <= 1e-10 * scale, key
+
+
+def _equal(out, one):
+    for key in ("inter", "intra", "occ"):
+        np.testing.assert_array_equal(getattr(out, key), getattr(one, key))
+
+
+def test_requests_that_join_and_leave():
+    """Plain length-gauge, velocity-gauge and two-band requests come in while
+    others run; some are cancelled at once.  Each result is the solve's alone."""
+    cases = [_table(6, (7, 5)), _table(6, (5, 9), rk="cashkarp45", steps=25.5), _table(3, (4, 4), rk="rk5"),
+             material("KaneMele", "Wannier"), material("TMDCs", "Wannier", calc__RKorder=5),
+             _table(5, (9, 3), gauge="Velocity"), variant(calc__Npoints=[40, 41]), _table(4, (1, 17), steps=90.5)]
+    probs = [ab.Problem.from_dict(c) for c in cases]
+    alone = [ab.solve(p, precision="fp64") for p in probs]
+    srv = ab.api.Server(precision="fp64")
+    ids, dropped = [], []
+    for rep in range(3):
+        for i, p in enumerate(probs):
+            ids.append((i, srv.submit(p)))
+            if (i + rep) % 3 == 0:
+                dropped.append(srv.submit(p))
+                srv.cancel(dropped[-1])
+        if rep == 1:
+            out, _ = srv.wait(ids[0][1], timeout=120.0)
+            _equal(out, alone[0])
+            ids.pop(0)
+    for i, rid in ids:
+        out, _ = srv.wait(rid, timeout=120.0)
+        if cases[i]["target"] == "Haldane":   # the server's CTA sizes: other sums over k
+            for key in ("inter", "intra"):
+                x, y = getattr(out, key), getattr(alone[i], key)
+                assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max()
+        else:
+            _equal(out, alone[i])
+    srv.close()
