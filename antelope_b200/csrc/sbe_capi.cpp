@@ -712,6 +712,7 @@ struct Request {
     int solve = -1;               // engine solve id while the engine holds it
     bool nband = false;           // a table or continuum model: held by the N-band pool
     int wsolve = -1;              // its pool id
+    bool lean = false;            // without the tables that the budget has no room for
     bool fetching = false;
     bool cancel_asked = false;    // cancelled while ADMITTING
     bool delivered = false;       // a wait returned its final state: the worker may erase it
@@ -784,6 +785,10 @@ void sbe_server::loop()
                     continue;
                 }
                 const int resident = eng->nresident() + wpool->nresident() + (int)batch.size();
+                if (resident == 0 && r.nband && (double)need > budget) {
+                    r.lean = true;
+                    need = WannierPool::bytes_needed(r.prob, nband_precision(r.prob), true);
+                }
                 const bool slots_ok = opts.max_resident <= 0 || resident < opts.max_resident;
                 if (!slots_ok || (double)(eng->bytes_in_use() + wpool->bytes_in_use() + planned + need) > budget) {
                     if (resident == 0) {  // can never fit
@@ -811,7 +816,7 @@ void sbe_server::loop()
         // and waiting threads are not held up by it
         for (Request *r : batch) {
             try {
-                if (r->nband) r->wsolve = wpool->add(r->prob, nband_precision(r->prob));
+                if (r->nband) r->wsolve = wpool->add(r->prob, nband_precision(r->prob), r->lean);
                 else r->solve = eng->add(r->prob, eo);
             } catch (const std::exception &e) {
                 r->solve = r->wsolve = -1;

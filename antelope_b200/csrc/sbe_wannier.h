@@ -96,11 +96,12 @@ struct WanDev {
     double *snap_pi;
     // many steps per launch (wan_steps): A at the distinct stage times of
     // every step [Nt][wan_steps_fields][3], the output partials of a launch
-    // [WAN_STEPS][step_rows][WAN_NSLOT] and the finishing blocks' counter
+    // [step_max][step_rows][WAN_NSLOT] and the finishing blocks' counter
     double *step_fld;
     double *step_part;
     unsigned *step_ticket;
-    int step_rows;
+    int step_rows, step_max;   // step_max: steps of a launch at most
+    int lean;                  // neither wan_steps nor wan_proj applies: no memory for their tables
     // ... in the length gauge the launch's phase factors e^{iA(t)R}
     // [WAN_STEPS][wan_steps_fields][npair] at the pairs' vectors gpair (gmate:
     // the index of a pair's other vector, or -1)

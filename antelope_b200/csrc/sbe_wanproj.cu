@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(128) wan_next(const WanDev *__restrict__ Pp, c
 // ============================================================= launchers
 bool wan_proj_applies(const WanDev &w)
 {
-    return !w.mixed && !w.vg && !w.cont && !w.has_jtab && !w.degenerate && w.N >= 3 && w.N <= 6 && w.nR >= 1 &&
+    return !w.lean && !w.mixed && !w.vg && !w.cont && !w.has_jtab && !w.degenerate && w.N >= 3 && w.N <= 6 && w.nR >= 1 &&
            w.Ngrid[2] == 1;
 }
 bool wan_proj(const WanDev &w) { return w.gr_tab != nullptr && wan_proj_applies(w); }

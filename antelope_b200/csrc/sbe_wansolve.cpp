@@ -21,8 +21,49 @@ template <class T> void dalloc(T **p, size_t bytes, cudaStream_t st, const char 
 }
 }  // namespace
 
+// The numbers of a solve's descriptor, and none of its buffers
+static WanDev describe(const Problem &p, int precision, int k_begin, int k_end)
+{
+    WanDev w;
+    std::memset(&w, 0, sizeof(w));
+    w.N = p.nband;
+    w.nval = p.nval;
+    w.nR = p.w_nR;
+    const int kb = k_end > 0 ? k_begin : 0, ke = k_end > 0 ? k_end : p.ntotal();
+    if (kb < 0 || ke > p.ntotal() || kb >= ke) throw CfgError("k-slice outside the grid");
+    w.nk = ke - kb;
+    w.k_offset = kb;
+    w.Nt = p.laser.Nt;
+    w.ntiles = (w.nk + WAN_WARPS - 1) / WAN_WARPS;
+    w.rk = p.rk;
+    w.inter_intra = p.inter_intra ? 1 : 0;
+    w.use_fermi = p.use_fermi ? 1 : 0;
+    w.has_dip = p.w_d.empty() ? 0 : 1;
+    w.has_jtab = p.w_j.empty() ? 0 : 1;
+    w.vg = p.gauge == GAUGE_VELOCITY ? 1 : 0;
+    if (p.model == MODEL_MULTIWSM) {   // formulas in place of tables; its own current operator
+        w.cont = 1;
+        w.has_jtab = 1;
+        w.mw_n = p.mw_n;
+        w.mw_v = p.mw_v;
+        w.mw_alphan = p.mw_alphan;
+    }
+    w.Ef = p.Ef;
+    w.dt = p.dt;
+    w.atmin = p.laser.atmin;
+    w.tol = p.rk_tol;
+    w.g1 = p.T1 > 1.0e-16 ? 1.0 / p.T1 : 0.0;  // SBEs.h:484-493
+    w.g2 = p.T2 > 1.0e-16 ? 1.0 / p.T2 : 0.0;
+    for (int i = 0; i < 3; ++i) w.Ngrid[i] = p.Nk[i];
+    for (int i = 0; i < 9; ++i) w.axes[i] = p.bzaxes[i];
+    for (int i = 0; i < 3; ++i) w.origin[i] = p.bzorigin[i];
+    w.laser = laser_dev(p.laser);
+    w.mixed = precision != 0;
+    return w;
+}
+
 WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin, int k_end,
-                           bool defer)
+                           bool defer, bool lean)
     : prob_(p), precision_(precision), device_(device), stream_(st)
 {
     if (p.model != MODEL_SYNTHETIC_WANNIER && p.model != MODEL_TB && p.model != MODEL_MULTIWSM)
@@ -32,39 +73,8 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     if (p.w_nR > WAN_MAXR) throw CfgError("tight-binding model: at most 64 hopping vectors");
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     const int N = p.nband, NN = N * N;
-    std::memset(&w_, 0, sizeof(w_));
-    w_.N = N;
-    w_.nval = p.nval;
-    w_.nR = p.w_nR;
-    const int kb = k_end > 0 ? k_begin : 0, ke = k_end > 0 ? k_end : p.ntotal();
-    if (kb < 0 || ke > p.ntotal() || kb >= ke) throw CfgError("k-slice outside the grid");
-    w_.nk = ke - kb;
-    w_.k_offset = kb;
-    w_.Nt = p.laser.Nt;
-    w_.ntiles = (w_.nk + WAN_WARPS - 1) / WAN_WARPS;
-    w_.rk = p.rk;
-    w_.inter_intra = p.inter_intra ? 1 : 0;
-    w_.use_fermi = p.use_fermi ? 1 : 0;
-    w_.has_dip = p.w_d.empty() ? 0 : 1;
-    w_.has_jtab = p.w_j.empty() ? 0 : 1;
-    w_.vg = p.gauge == GAUGE_VELOCITY ? 1 : 0;
-    if (p.model == MODEL_MULTIWSM) {   // formulas in place of tables; its own current operator
-        w_.cont = 1;
-        w_.has_jtab = 1;
-        w_.mw_n = p.mw_n;
-        w_.mw_v = p.mw_v;
-        w_.mw_alphan = p.mw_alphan;
-    }
-    w_.Ef = p.Ef;
-    w_.dt = p.dt;
-    w_.atmin = p.laser.atmin;
-    w_.tol = p.rk_tol;
-    w_.g1 = p.T1 > 1.0e-16 ? 1.0 / p.T1 : 0.0;  // SBEs.h:484-493
-    w_.g2 = p.T2 > 1.0e-16 ? 1.0 / p.T2 : 0.0;
-    for (int i = 0; i < 3; ++i) w_.Ngrid[i] = p.Nk[i];
-    for (int i = 0; i < 9; ++i) w_.axes[i] = p.bzaxes[i];
-    for (int i = 0; i < 3; ++i) w_.origin[i] = p.bzorigin[i];
-    w_.laser = laser_dev(p.laser);
+    w_ = describe(p, precision_, k_begin, k_end);
+    w_.lean = lean;
 
     const size_t real = precision_ == 0 ? 8 : 4, cplx = 2 * real;
     const size_t nk = (size_t)w_.nk;
@@ -76,7 +86,7 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     if (w_.has_jtab && !w_.cont) dalloc(&j, cplx * p.w_j.size() / 2, st, "alloc current tables");
     for (int b = 0; b < 2; ++b) {
         dalloc(&w_.rho[b], sizeof(double2) * nk * NN, st, "alloc rho");
-        dalloc(&w_.U[b], sizeof(double2) * nk * NN, st, "alloc U");
+        if (!w_.vg) dalloc(&w_.U[b], sizeof(double2) * nk * NN, st, "alloc U");
     }
     dalloc(&w_.weight, sizeof(double) * nk, st, "alloc weights");
     if (w_.vg) {
@@ -101,7 +111,6 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     w_.h = h;
     w_.d = d;
     w_.jt = j;
-    w_.mixed = precision_ != 0;
     if (!p.w_vec.empty()) UploadRing::shared().upload(V, p.w_vec.data(), sizeof(double) * p.w_vec.size(), st);
     auto up_real = [&](void *dst, const std::vector<double> &src) { upload_real(dst, src, st); };
     if (!p.w_h.empty()) up_real(h, p.w_h);
@@ -151,19 +160,26 @@ void WannierSolve::finish_setup()
         w_.degenerate = !(gw[0] > 1e-7 * gw[1]) || wan_crowded_slow(w_, h_gap_[2]);
         drop_gap();
     }
-    if (wan_steps(w_)) {
-        w_.step_rows = wan_steps_rows(w_);
-        dalloc(&w_.step_fld, sizeof(double) * (size_t)w_.Nt * wan_steps_fields(w_.rk) * 3, st, "alloc step fields");
-        dalloc(&w_.step_part, sizeof(double) * (size_t)std::min(WAN_STEPS, w_.Nt) * w_.step_rows * WAN_NSLOT, st,
-               "alloc step partials");
-        // slots that a model has no values for stay zero
-        cuda_check(cudaMemsetAsync(w_.step_part, 0,
-                                   sizeof(double) * (size_t)std::min(WAN_STEPS, w_.Nt) * w_.step_rows * WAN_NSLOT, st),
-                   "clear step partials");
-        dalloc(&w_.step_ticket, sizeof(unsigned), st, "alloc step counter");
-        cuda_check(cudaMemsetAsync(w_.step_ticket, 0, sizeof(unsigned), st), "clear step counter");
+    try {
+        if (wan_steps(w_)) setup_steps(st);
+        if (wan_proj_applies(w_)) setup_rows(p, st);
+    } catch (const OomError &) {   // these tables are for speed
+        for (void **q : {(void **)&w_.step_fld, (void **)&w_.step_part, (void **)&w_.gr_tab, (void **)&w_.gr_cur}) {
+            if (*q) cudaFreeAsync(*q, st);
+            *q = nullptr;
+        }
+        w_.lean = 1;
     }
-    if (wan_proj_applies(w_)) setup_rows(p, st);
+    if (wan_steps(w_) || wan_proj(w_)) {   // what only the attempt kernels use
+        for (void **q : {(void **)&w_.U[0], (void **)&w_.U[1], (void **)&w_.tile_err}) {
+            if (*q) cudaFreeAsync(*q, st);
+            *q = nullptr;
+        }
+        if (wan_steps(w_)) {
+            cudaFreeAsync(w_.cur_part, st);
+            w_.cur_part = nullptr;
+        }
+    }
     // the tables re-laid for the grouped attempt kernel.  The lattice vectors
     // are taken in pairs (R, -R) (a vector without its negative, R = 0
     // included, stands alone): h_R e^{iKR} + h_-R e^{-iKR} = c sig + s tau
@@ -293,33 +309,79 @@ void WannierSolve::upload_real(void *dst, const std::vector<double> &src, cudaSt
     }
 }
 
-// The groups of lattice vectors that share their phase along the grid's rows,
-// and the row tables of the projection attempt kernel.  Left undone (the
-// other attempt kernels run the solve) where the tables would pass 1 GiB: grids
-// of very many short rows.
+// Fields and output partials of the many-step kernels
+static size_t step_bytes(const WanDev &w)
+{
+    return sizeof(double) * ((size_t)w.Nt * wan_steps_fields(w.rk) * 3 +
+                             (size_t)std::min(WAN_STEPS, w.Nt) * wan_steps_rows(w) * WAN_NSLOT) +
+           (w.vg ? 0 : sizeof(double2) * WAN_STEPS * (size_t)wan_steps_fields(w.rk) * w.nR);
+}
+void WannierSolve::setup_steps(cudaStream_t st)
+{
+    w_.step_rows = wan_steps_rows(w_);
+    dalloc(&w_.step_fld, sizeof(double) * (size_t)w_.Nt * wan_steps_fields(w_.rk) * 3, st, "alloc step fields");
+    // fewer steps per launch where memory is short (64 of 10^6 k-points at N = 8 take 2 GB)
+    size_t part = 0;
+    for (w_.step_max = std::min(WAN_STEPS, w_.Nt); !w_.step_part; w_.step_max = std::max(1, w_.step_max / 4)) {
+        part = sizeof(double) * (size_t)w_.step_max * w_.step_rows * WAN_NSLOT;
+        try {
+            dalloc(&w_.step_part, part, st, "alloc step partials");
+            break;
+        } catch (const OomError &) {
+            if (w_.step_max == 1) throw;
+        }
+    }
+    // slots that a model has no values for stay zero
+    cuda_check(cudaMemsetAsync(w_.step_part, 0, part, st), "clear step partials");
+    dalloc(&w_.step_ticket, sizeof(unsigned), st, "alloc step counter");
+    cuda_check(cudaMemsetAsync(w_.step_ticket, 0, sizeof(unsigned), st), "clear step counter");
+}
+
+// The groups of lattice vectors that share their phase along the grid's rows: b.R at
+// + and - ga[g] (0 first), lists[2 g] and [2 g + 1]
+struct RowGroups {
+    int fast;
+    std::vector<double> ga{0.0};
+    std::vector<std::vector<int>> lists = std::vector<std::vector<int>>(2);
+    explicit RowGroups(const Problem &p) : fast(p.Nk[1] > 1 ? 1 : 0)
+    {
+        const int nR = p.w_nR;
+        std::vector<double> b(nR);
+        double bmax = 0.0;
+        for (int r = 0; r < nR; ++r) {
+            const double bx = p.bzaxes[3 * fast] * p.w_vec[2 * r], by = p.bzaxes[3 * fast + 1] * p.w_vec[2 * r + 1];
+            b[r] = bx + by;
+            bmax = std::max(bmax, std::fabs(bx) + std::fabs(by));
+        }
+        // the rounding of b.R (axes given to ten digits leave larger differences, which count)
+        const double tol = 1e-14 * bmax;
+        for (int r = 0; r < nR; ++r) {
+            int g = 0;
+            while (g < (int)ga.size() && std::fabs(ga[g] - std::fabs(b[r])) > tol) ++g;
+            if (g == (int)ga.size()) {
+                ga.push_back(std::fabs(b[r]));
+                lists.resize(2 * ga.size());
+            }
+            lists[2 * g + (g > 0 && b[r] < 0.0 ? 1 : 0)].push_back(r);
+        }
+    }
+};
+// Bytes of a solve's row tables; 0: none (grids of very many short rows, or too many
+// groups: the other attempt kernels run the solve)
+static size_t row_bytes(const WanDev &w, const RowGroups &rg)
+{
+    const int nf = w.Ngrid[rg.fast], ng = (int)rg.ga.size(), nq = w.has_dip ? 2 : 1;
+    const size_t rows = (size_t)((w.k_offset + w.nk - 1) / nf - w.k_offset / nf + 1);
+    const size_t n = rows * ((w.rk == 4 ? 4 : 6) * (size_t)wan_proj_entries(w.N, ng, nq) + wan_proj_entries(w.N, ng, 2 * nq));
+    return ng > WAN_PROJ_MAXGRP || n * 16 > ((size_t)1 << 30) ? 0 : n * 16;
+}
+// The groups and the row tables of the projection attempt kernel
 void WannierSolve::setup_rows(const Problem &p, cudaStream_t st)
 {
-    const int nR = w_.nR, N = w_.N, fast = w_.Ngrid[1] > 1 ? 1 : 0;
-    std::vector<double> b(nR);
-    double bmax = 0.0;
-    for (int r = 0; r < nR; ++r) {
-        const double bx = p.bzaxes[3 * fast] * p.w_vec[2 * r], by = p.bzaxes[3 * fast + 1] * p.w_vec[2 * r + 1];
-        b[r] = bx + by;
-        bmax = std::max(bmax, std::fabs(bx) + std::fabs(by));
-    }
-    // the rounding of b.R (axes given to ten digits leave larger differences, which count)
-    const double tol = 1e-14 * bmax;
-    std::vector<double> ga{0.0};
-    std::vector<std::vector<int>> lists(2);
-    for (int r = 0; r < nR; ++r) {
-        int g = 0;
-        while (g < (int)ga.size() && std::fabs(ga[g] - std::fabs(b[r])) > tol) ++g;
-        if (g == (int)ga.size()) {
-            ga.push_back(std::fabs(b[r]));
-            lists.resize(2 * ga.size());
-        }
-        lists[2 * g + (g > 0 && b[r] < 0.0 ? 1 : 0)].push_back(r);
-    }
+    const RowGroups rg(p);
+    const std::vector<double> &ga = rg.ga;
+    if (row_bytes(w_, rg) == 0) return;
+    const int N = w_.N, fast = rg.fast;
     const int ng = (int)ga.size(), nq = w_.has_dip ? 2 : 1;
     w_.gr_fast = fast;
     w_.gr_nf = w_.Ngrid[fast];
@@ -328,9 +390,8 @@ void WannierSolve::setup_rows(const Problem &p, cudaStream_t st)
     w_.gr_n = ng;
     const int S = w_.rk == 4 ? 4 : 6;
     const size_t nt = (size_t)w_.gr_rows * S * wan_proj_entries(N, ng, nq), nc = (size_t)w_.gr_rows * wan_proj_entries(N, ng, 2 * nq);
-    if (ng > WAN_PROJ_MAXGRP || (nt + nc) * 16 > ((size_t)1 << 30)) return;
     std::vector<int> off{0}, idx;
-    for (const auto &l : lists) {
+    for (const auto &l : rg.lists) {
         idx.insert(idx.end(), l.begin(), l.end());
         off.push_back((int)idx.size());
     }
@@ -366,14 +427,14 @@ WannierSolve::~WannierSolve()
     if (w_.stage_gt) cudaFreeAsync(w_.stage_gt, stream_);
     for (int b = 0; b < 2; ++b) {
         cudaFreeAsync(w_.rho[b], stream_);
-        cudaFreeAsync(w_.U[b], stream_);
+        if (w_.U[b]) cudaFreeAsync(w_.U[b], stream_);
     }
     cudaFreeAsync(w_.weight, stream_);
     if (w_.vg_eps) cudaFreeAsync(w_.vg_eps, stream_);
     if (w_.vg_f) cudaFreeAsync(w_.vg_f, stream_);
     if (w_.vg_P) cudaFreeAsync(w_.vg_P, stream_);
-    cudaFreeAsync(w_.tile_err, stream_);
-    cudaFreeAsync(w_.cur_part, stream_);
+    if (w_.tile_err) cudaFreeAsync(w_.tile_err, stream_);
+    if (w_.cur_part) cudaFreeAsync(w_.cur_part, stream_);
     cudaFreeAsync(w_.jout, stream_);
     cudaFreeAsync(w_.ctl, stream_);
     cudaFreeAsync(w_.stage_AE, stream_);
@@ -407,11 +468,11 @@ void WannierSolve::run(cudaStream_t st)
         launches_ = 0;
         for (int n = 0; n < w_.Nt;) {
             // the steps the kernels take from n (a launch ends at a snapshot)
-            int m = std::min(WAN_STEPS, w_.Nt - n);
+            int m = std::min(w_.step_max, w_.Nt - n);
             if (F > 0) m = std::min(m, (n + F - 1) / F * F + 1 - n);
-            cuda_check(launch_wan_steps(sc, d_w_, nullptr, nullptr, (w_.ntiles + unit - 1) / unit, WAN_STEPS, st),
+            cuda_check(launch_wan_steps(sc, d_w_, nullptr, nullptr, (w_.ntiles + unit - 1) / unit, w_.step_max, st),
                        "Wannier step kernel");
-            cuda_check(launch_wan_finish(d_w_, nullptr, 1, WAN_STEPS, st), "Wannier finish kernel");
+            cuda_check(launch_wan_finish(d_w_, nullptr, 1, w_.step_max, st), "Wannier finish kernel");
             cuda_check(launch_wan_snapshot(w_, d_w_, precision_, st), "Wannier snapshot kernel");
             launches_ += F > 0 ? 3 : 2;
             n += m;
@@ -483,6 +544,7 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         c->members.push_back(i);
         c->nR = std::max(c->nR, w.nR);
         c->steps.npair = std::max(c->steps.npair, sc.npair);
+        if (c->steps.mode) c->step_max = std::min(c->step_max, w.step_max);
         c->ngrp = std::max(c->ngrp, w.gr_n);
         c->nitems = std::max(c->nitems, w.gr_rows * (w.rk == 4 ? 4 : 6));
         c->shots = c->shots || w.shot_every > 0;
@@ -547,12 +609,12 @@ int WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
     int launched = 0;
     for (int it = 0; it < iters; ++it)
         for (const Class &c : classes_) {
-            if (c.steps.mode) {   // WAN_STEPS iterations in one launch
-                if (it % WAN_STEPS) continue;
-                cuda_check(launch_wan_steps(c.steps, nullptr, c.d_descs, c.d_tiles, c.ntiles,
-                                            std::min(WAN_STEPS, iters - it), st),
+            if (c.steps.mode) {   // step_max iterations in one launch
+                if (it % c.step_max) continue;
+                const int S = std::min(c.step_max, iters - it);
+                cuda_check(launch_wan_steps(c.steps, nullptr, c.d_descs, c.d_tiles, c.ntiles, S, st),
                            "Wannier step kernel (batch)");
-                cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.members.size(), std::min(WAN_STEPS, iters - it), st),
+                cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.members.size(), S, st),
                            "Wannier finish kernel (batch)");
                 launched += 2;
                 if (c.shots) {
@@ -643,7 +705,7 @@ WannierPool::~WannierPool()
     if (copied_) cudaEventDestroy(copied_);
 }
 
-size_t WannierPool::bytes_needed(const Problem &p, int precision)
+size_t WannierPool::bytes_needed(const Problem &p, int precision, bool lean)
 {
     const size_t N = (size_t)p.nband, NN = N * N, nk = (size_t)p.ntotal(), nR = (size_t)std::max(p.w_nR, 1);
     const size_t real = precision == 0 ? 8 : 4, cplx = 2 * real;
@@ -652,23 +714,23 @@ size_t WannierPool::bytes_needed(const Problem &p, int precision)
     b += nR * NN * cplx * 5 + nR * 16 + nR * 216 * cplx;               // h, d, current, re-laid and stage tables, vectors
     b += ntiles * 8 * (1 + WAN_NSLOT) + (size_t)p.laser.Nt * WAN_NSLOT * 8;   // tile results, per-step sums
     if (p.gauge == GAUGE_VELOCITY) b += nk * N * 16 + nk * 3 * NN * 16;  // bands, momentum matrices
-    // row tables of the projection attempts (at most a group per vector pair)
-    if (p.gauge != GAUGE_VELOCITY && precision == 0)
-        b += (size_t)p.Nk[0] * 10 * wan_proj_entries((int)std::max<size_t>(N, 2), (int)nR / 2 + 1, 2) * 16;
-    if (p.rk != 45)   // step fields, phases and partials
-        b += (size_t)WAN_STEPS * 6 * nR * cplx + (size_t)p.laser.Nt * 6 * 24 + (size_t)WAN_STEPS * (nk / 4 + 1) * WAN_NSLOT * 8;
+    if (!lean) {   // tables of the many-step and projection kernels
+        const WanDev w = describe(p, precision, 0, 0);
+        if (wan_steps(w)) b += step_bytes(w);
+        if (wan_proj_applies(w)) b += row_bytes(w, RowGroups(p));
+    }
     return b + 4096;
 }
 
-int WannierPool::add(const Problem &p, int precision)
+int WannierPool::add(const Problem &p, int precision, bool lean)
 {
     Entry e;
-    e.s = std::make_unique<WannierSolve>(p, precision, device_, st_, 0, 0, true);
+    e.s = std::make_unique<WannierSolve>(p, precision, device_, st_, 0, 0, true, lean);
     // a solve that waits for its bands waits on the GPU's side: the host would stand
     // until every tick queued before is done (step() takes it up)
     e.ready = e.s->setup_ready();
     if (e.ready) e.s->finish_setup();
-    e.bytes = bytes_needed(p, precision);
+    e.bytes = bytes_needed(p, precision, lean);
     bytes_ += e.bytes;
     const int id = next_id_++;
     solves_.emplace(id, std::move(e));
@@ -751,6 +813,7 @@ void WannierPool::rebuild()
         c->ids.push_back(kv.first);
         c->nR = std::max(c->nR, w.nR);
         c->steps.npair = std::max(c->steps.npair, sc.npair);
+        if (c->steps.mode) c->step_max = std::min(c->step_max, w.step_max);
         c->ngrp = std::max(c->ngrp, w.gr_n);
         c->nitems = std::max(c->nitems, w.gr_rows * (w.rk == 4 ? 4 : 6));
     }
@@ -799,9 +862,9 @@ void WannierPool::step(int iters)
     if (classes_.empty()) return;
     for (int it = 0; it < iters; ++it)
         for (const Class &c : classes_) {
-            if (c.steps.mode) {   // up to WAN_STEPS iterations in one launch
-                if (it % WAN_STEPS) continue;
-                const int S = std::min(WAN_STEPS, iters - it);
+            if (c.steps.mode) {   // up to step_max iterations in one launch
+                if (it % c.step_max) continue;
+                const int S = std::min(c.step_max, iters - it);
                 cuda_check(launch_wan_steps(c.steps, nullptr, c.d_descs, c.d_tiles, c.ntiles, S, st_),
                            "Wannier step kernel (server)");
                 cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.ids.size(), S, st_),

@@ -17,9 +17,11 @@ class WannierSolve {
 public:
     // k_begin/k_end: a k-slice [k_begin, k_end) of the grid (0, 0: all of it);
     // defer: finish_setup() is left to the caller (it waits for the bands over the
-    // grid where the choice of kernels depends on them; setup_ready(): it will not wait)
+    // grid where the choice of kernels depends on them; setup_ready(): it will not wait);
+    // lean: the attempt kernels, which hold least memory (so does a solve for whose
+    // other tables there is none)
     WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin = 0, int k_end = 0,
-                 bool defer = false);
+                 bool defer = false, bool lean = false);
     ~WannierSolve();
     WannierSolve(const WannierSolve &) = delete;
     WannierSolve &operator=(const WannierSolve &) = delete;
@@ -50,6 +52,7 @@ private:
     void upload_real(void *dst, const std::vector<double> &src, cudaStream_t st);
     unsigned long long *h_gap_ = nullptr;   // WanDev::band_gap (pinned) until finish_setup()
     cudaEvent_t gap_ev_ = nullptr;
+    void setup_steps(cudaStream_t st);
     void setup_rows(const Problem &p, cudaStream_t st);
     Problem prob_;
     int precision_, device_, nshots_ = 0;
@@ -84,6 +87,7 @@ private:
         int N = 0, nR = 0, precision = 0;
         int grouped_rk = 0;   // the grouped attempt kernel (and its RK order), or 0
         WanStepClass steps;   // the many-step kernels (mode 0: not)
+        int step_max = WAN_STEPS;
         bool proj = false;    // the projection attempts
         int ngrp = 0, nitems = 0;
         bool vg = false, shots = false;
@@ -115,8 +119,8 @@ public:
     WannierPool(const WannierPool &) = delete;
     WannierPool &operator=(const WannierPool &) = delete;
     // device memory a solve of this problem holds
-    static size_t bytes_needed(const Problem &p, int precision);
-    int add(const Problem &p, int precision);   // returns its id
+    static size_t bytes_needed(const Problem &p, int precision, bool lean = false);
+    int add(const Problem &p, int precision, bool lean = false);   // returns its id
     void remove(int id);
     size_t bytes_in_use() const { return bytes_; }
     int nresident() const { return (int)solves_.size(); }
@@ -148,6 +152,7 @@ private:
     struct Class {
         int N = 0, nR = 0, precision = 0, grouped_rk = 0;
         WanStepClass steps;
+        int step_max = WAN_STEPS;
         bool proj = false;
         int ngrp = 0, nitems = 0;
         bool vg = false;

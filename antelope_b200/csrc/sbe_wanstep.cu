@@ -74,7 +74,7 @@ template <> struct StepTab<5> {
 // past a step whose density snapshot is due (it is taken between launches).
 __device__ __forceinline__ int launch_steps(const WanDev &P, int n, int S)
 {
-    int m = min(S, P.Nt - n);
+    int m = min(min(S, P.step_max), P.Nt - n);
     if (P.shot_every > 0) m = min(m, ((n + P.shot_every - 1) / P.shot_every) * P.shot_every + 1 - n);
     return m;
 }
@@ -1001,7 +1001,7 @@ __global__ void __launch_bounds__(256) wan_finish(const WanDev *__restrict__ Pp,
             P.jout[(size_t)(n0 + j) * WAN_NSLOT + t] = s;
         }
     }
-    launch_phases(P, n0 + steps, j);   // of the next launch
+    for (int x = j; x < WAN_STEPS; x += gridDim.x) launch_phases(P, n0 + steps, x);   // of the next launch, whatever its S
     __syncthreads();
     if (t == 0) {
         __threadfence();
@@ -1045,7 +1045,7 @@ static int steps_bytes(int mode, int N, int na, int rk, int npair)
 constexpr int STEPS_MAX_BYTES = 96 * 1024;   // at least two blocks per SM
 int wan_steps(const WanDev &w)
 {
-    if ((w.rk != 4 && w.rk != 5) || w.N < 2 || w.N > WAN_MAXN) return 0;
+    if (w.lean || (w.rk != 4 && w.rk != 5) || w.N < 2 || w.N > WAN_MAXN) return 0;
     if (w.vg) return w.N <= 3 ? VG_THREAD : VG_ROWS;
     if (w.mixed || !w.has_jtab || w.has_dip || w.cont || w.N > 4 || w.degenerate) return 0;
     return steps_bytes(LW_THREAD, w.N, 2, w.rk, w.nR) <= STEPS_MAX_BYTES ? LW_THREAD : 0;

@@ -1,4 +1,5 @@
-"""Which N-band solves the many-step and projection kernels take, and how."""
+"""Which N-band solves the many-step and projection kernels take, and what the
+server's admission counts for them."""
 import numpy as np
 import pytest
 
@@ -42,6 +43,46 @@ def test_axes_of_ten_digits(tilt):
 def _equal(out, one):
     for key in ("inter", "intra", "occ"):
         np.testing.assert_array_equal(getattr(out, key), getattr(one, key))
+
+
+def _base_bytes(p, nR):
+    """Device memory of a solve on the attempt kernels alone."""
+    N, nk, Nt = p.dims.nband, p.dims.ntotal, p.dims.Nt
+    return 4 * nk * N * N * 16 + nk * 8 + nR * N * N * 80 + nR * 16 + nR * 3456 + nk // 4 * 136 + Nt * 128 + (1 << 20)
+
+
+def _served(p, budget):
+    srv = ab.api.Server(precision="fp64", mem_budget_bytes=float(budget))
+    try:
+        return srv.wait(srv.submit(p), timeout=120.0)[0]
+    finally:
+        srv.close()
+
+
+def _close(out, one, tol=1e-12):
+    scale = max(np.abs(one.inter).max(), np.abs(one.intra).max())
+    for key in ("inter", "intra"):
+        assert np.abs(getattr(out, key) - getattr(one, key)).max() <= tol * scale, key
+
+
+def test_admission_of_long_and_thin_grids():
+    """No row tables for a material, and none above their limit."""
+    km = material("KaneMele", "Wannier", pulse__ncycles=0.05)
+    km["calc"]["Npoints"] = [4000, 1]
+    for c, nR in ((_table(6, (1200, 1), rk="cashkarp45", steps=3.5), 37), (km, 19)):
+        p = ab.Problem.from_dict(c)
+        out = _served(p, _base_bytes(p, nR))
+        assert np.abs(out.intra).max() > 0.0
+
+
+@pytest.mark.parametrize("gauge", ["Velocity", "Wannier"])
+def test_a_budget_without_room_for_tables(gauge):
+    """The solve runs on the kernels that need none: no less is admitted than they hold."""
+    c = _table(6, (64, 60), steps=10.5, gauge=gauge)
+    p = ab.Problem.from_dict(c)
+    nk = p.dims.ntotal
+    budget = _base_bytes(p, 37) + (nk * 6 * 16 + nk * 3 * 36 * 16 if gauge == "Velocity" else 0)
+    _close(_served(p, budget), ab.solve(p, precision="fp64"), 1e-11)
 
 
 def test_requests_that_join_and_leave():
