@@ -886,7 +886,10 @@ void WannierPool::step(int iters)
             }
             last_launches_ += 2;
         }
-    // controllers of the running solves, read by a later poll()
+    // controllers of the running solves, read by a later poll(); not again before it
+    // has read them (the event would always be the newest launches', and a poll that
+    // comes while those run would never see a solve done)
+    if (pending_) return;
     polled_.clear();
     for (const Class &c : classes_)
         for (int id : c.ids) polled_.push_back(id);

@@ -85,6 +85,18 @@ def test_a_budget_without_room_for_tables(gauge):
     _close(_served(p, budget), ab.solve(p, precision="fp64"), 1e-11)
 
 
+def test_a_finished_request_is_noticed():
+    """A request alone on the server: its 10 steps are one tick (32 attempts, 64
+    launches), and the server sees it done a few ticks later."""
+    p = ab.Problem.from_dict(_table(6, (64, 60), steps=10.5))
+    for _ in range(3):
+        srv = ab.api.Server(precision="fp64")
+        srv.wait(srv.submit(p), timeout=120.0)
+        launches = srv.stats()["launches"]
+        srv.close()
+        assert launches <= 20 * 64, launches
+
+
 def test_requests_that_join_and_leave():
     """Plain length-gauge, velocity-gauge and two-band requests come in while
     others run; some are cancelled at once.  Each result is the solve's alone."""
