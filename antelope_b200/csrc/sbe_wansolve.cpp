@@ -63,7 +63,7 @@ static WanDev describe(const Problem &p, int precision, int k_begin, int k_end)
 }
 
 WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin, int k_end,
-                           bool defer, bool lean)
+                           bool defer, bool lean, bool snapshots)
     : prob_(p), precision_(precision), device_(device), stream_(st)
 {
     if (p.model != MODEL_SYNTHETIC_WANNIER && p.model != MODEL_TB && p.model != MODEL_MULTIWSM)
@@ -100,7 +100,7 @@ WannierSolve::WannierSolve(const Problem &p, int precision, int device, cudaStre
     dalloc(&w_.ctl, sizeof(WanCtl), st, "alloc control");
     dalloc(&w_.stage_AE, sizeof(double) * 36, st, "alloc stage fields");
     dalloc(&w_.stage_cA, cplx * 6 * (size_t)w_.nR, st, "alloc stage phases");
-    nshots_ = p.nshots();
+    nshots_ = snapshots ? p.nshots() : 0;
     if (nshots_ > 0) {   // density snapshots (antelope.cpp:267-422)
         w_.shot_every = p.shot_every();
         dalloc(&w_.snap_nc, sizeof(double) * nshots_ * nk, st, "alloc snapshots");
@@ -548,6 +548,7 @@ WannierBatch::WannierBatch(const std::vector<const Problem *> &probs, int precis
         c->ngrp = std::max(c->ngrp, w.gr_n);
         c->nitems = std::max(c->nitems, w.gr_rows * (w.rk == 4 ? 4 : 6));
         c->shots = c->shots || w.shot_every > 0;
+        if (w.shot_every > 0) c->stride = std::min(c->stride, w.shot_every);   // its launches end at snapshots
     }
     UploadRing &ring = UploadRing::shared();
     for (Class &c : classes_) {
@@ -610,8 +611,8 @@ int WannierBatch::enqueue_chunk(cudaStream_t st, int iters)
     for (int it = 0; it < iters; ++it)
         for (const Class &c : classes_) {
             if (c.steps.mode) {   // step_max iterations in one launch
-                if (it % c.step_max) continue;
-                const int S = std::min(c.step_max, iters - it);
+                if (it % std::min(c.step_max, c.stride)) continue;
+                const int S = std::min(c.step_max, iters);
                 cuda_check(launch_wan_steps(c.steps, nullptr, c.d_descs, c.d_tiles, c.ntiles, S, st),
                            "Wannier step kernel (batch)");
                 cuda_check(launch_wan_finish(nullptr, c.d_descs, (int)c.members.size(), S, st),
@@ -725,7 +726,7 @@ size_t WannierPool::bytes_needed(const Problem &p, int precision, bool lean)
 int WannierPool::add(const Problem &p, int precision, bool lean)
 {
     Entry e;
-    e.s = std::make_unique<WannierSolve>(p, precision, device_, st_, 0, 0, true, lean);
+    e.s = std::make_unique<WannierSolve>(p, precision, device_, st_, 0, 0, true, lean, false);
     // a solve that waits for its bands waits on the GPU's side: the host would stand
     // until every tick queued before is done (step() takes it up)
     e.ready = e.s->setup_ready();

@@ -21,7 +21,7 @@ public:
     // lean: the attempt kernels, which hold least memory (so does a solve for whose
     // other tables there is none)
     WannierSolve(const Problem &p, int precision, int device, cudaStream_t st, int k_begin = 0, int k_end = 0,
-                 bool defer = false, bool lean = false);
+                 bool defer = false, bool lean = false, bool snapshots = true);
     ~WannierSolve();
     WannierSolve(const WannierSolve &) = delete;
     WannierSolve &operator=(const WannierSolve &) = delete;
@@ -87,7 +87,7 @@ private:
         int N = 0, nR = 0, precision = 0;
         int grouped_rk = 0;   // the grouped attempt kernel (and its RK order), or 0
         WanStepClass steps;   // the many-step kernels (mode 0: not)
-        int step_max = WAN_STEPS;
+        int step_max = WAN_STEPS, stride = WAN_STEPS;   // steps of a launch; iterations between two
         bool proj = false;    // the projection attempts
         int ngrp = 0, nitems = 0;
         bool vg = false, shots = false;

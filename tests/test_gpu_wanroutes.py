@@ -52,7 +52,7 @@ def _base_bytes(p, nR):
 
 
 def _served(p, budget):
-    srv = ab.api.Server(precision="fp64", mem_budget_bytes=float(budget))
+    srv = ab.Server(precision="fp64", mem_budget_bytes=float(budget))
     try:
         return srv.wait(srv.submit(p), timeout=120.0)[0]
     finally:
@@ -90,11 +90,51 @@ def test_a_finished_request_is_noticed():
     launches), and the server sees it done a few ticks later."""
     p = ab.Problem.from_dict(_table(6, (64, 60), steps=10.5))
     for _ in range(3):
-        srv = ab.api.Server(precision="fp64")
+        srv = ab.Server(precision="fp64")
         srv.wait(srv.submit(p), timeout=120.0)
         launches = srv.stats()["launches"]
         srv.close()
         assert launches <= 20 * 64, launches
+
+
+@pytest.mark.parametrize("shots", [1, 400])
+def test_snapshots_do_not_slow_the_server(shots):
+    """A request returns the output files' arrays: beside a long two-band solve
+    (one turn of the server per tick of it) the turns it takes do not depend on
+    its snapshot count."""
+    long = variant(calc__Npoints=[200, 200], pulse__ncycles=60000.5 * 0.1 * 0.0855 / (2 * np.pi))
+    launches, outs = [], []
+    for n in (0, shots):
+        c = _table(4, (6, 5), steps=300.5, gauge="Velocity", shotNumber=n)
+        srv = ab.Server(precision="fp64", steps_per_launch=64)
+        other = srv.submit(ab.Problem.from_dict(long))
+        while srv.stats()["launches"] < 4:
+            pass
+        before = srv.stats()["launches"]
+        out, _ = srv.wait(srv.submit(ab.Problem.from_dict(c)), timeout=120.0)
+        launches.append(srv.stats()["launches"] - before)
+        srv.cancel(other)
+        srv.close()
+        outs.append(out)
+    _equal(outs[1], outs[0])
+    assert launches[1] <= 3 * launches[0], launches
+
+
+@pytest.mark.parametrize("shots", [200, 700])
+def test_snapshots_do_not_idle_a_batch(shots):
+    """Launches end at snapshots: a batch queues as many between two looks at its
+    controllers as 64 steps take.  A short solve with snapshots beside a long
+    adaptive one, whose attempts every look costs 64 of."""
+    c = _table(4, (6, 5), steps=600.5, gauge="Velocity", shotNumber=shots)
+    other = _table(3, (4, 4), rk="cashkarp45", steps=10.5)
+    n = []
+    for cases in ([other], [c, other]):
+        b = ab.Batch([ab.Problem.from_dict(x) for x in cases], precision="fp64")
+        b.run()
+        n.append(b.launches)
+        b.close()
+    # 600 steps are 10 looks: 128 launches of the other class each, and at most 3 per step
+    assert n[1] <= 12 * 128 + 3 * 700, n
 
 
 def test_requests_that_join_and_leave():
@@ -105,7 +145,7 @@ def test_requests_that_join_and_leave():
              _table(5, (9, 3), gauge="Velocity"), variant(calc__Npoints=[40, 41]), _table(4, (1, 17), steps=90.5)]
     probs = [ab.Problem.from_dict(c) for c in cases]
     alone = [ab.solve(p, precision="fp64") for p in probs]
-    srv = ab.api.Server(precision="fp64")
+    srv = ab.Server(precision="fp64")
     ids, dropped = [], []
     for rep in range(3):
         for i, p in enumerate(probs):
