@@ -105,10 +105,10 @@ struct TileDev {
 // from the counter until none are left, so that only the last chunk of the last
 // tiles leaves SMs idle.  An item waits until its tile's chunk before is done:
 // that one was taken earlier, by a CTA that is running.  ctr: [0] next item,
-// [1] CTAs that are done (the last one clears both), [2] error; null: one tile
-// per CTA, all of its steps.
+// [1] CTAs that are done (the last one clears both); null: one tile per CTA, all
+// of its steps.  err: set when a wait ran out, for good.
 struct TileQueue {
-    int *ctr;
+    int *ctr, *err;
     int ntiles, chunk, nitems;
 };
 

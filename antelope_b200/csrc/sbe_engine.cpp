@@ -144,8 +144,6 @@ struct Engine::Solve {
     size_t bytes = 0;
 };
 
-constexpr int kMaxGroups = 32;   // launch classes: gauge x precision x RK x KPT x CTA size x T1 in use
-
 struct Engine::Group {
     int variant, precision, rk, kpt, threads;
     bool g1;
@@ -195,6 +193,8 @@ Engine::Engine(int device, cudaStream_t stream, int steps_per_launch, int capaci
     h_solves_.resize(capacity_);
     cuda_check(cudaMallocFromPoolAsync((void **)&d_ids_, sizeof(int) * capacity_, pool_, stream_), "alloc ids");
     h_ids_.assign(capacity_, 0);
+    cuda_check(cudaMallocFromPoolAsync((void **)&d_queue_err_, sizeof(int), pool_, stream_), "alloc queue state");
+    cuda_check(cudaMemsetAsync(d_queue_err_, 0, sizeof(int), stream_), "clear queue state");
     for (int i = capacity_ - 1; i >= 0; --i) free_slots_.push_back(i);
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device_) == cudaSuccess) {
@@ -230,10 +230,11 @@ Engine::~Engine()
     }
     cudaFreeAsync(d_solves_, stream_);
     cudaFreeAsync(d_ids_, stream_);
+    cudaFreeAsync(d_queue_err_, stream_);
     for (auto &e : prop_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     for (auto &e : red_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     cudaStreamSynchronize(stream_);
-    if (h_queue_) pinned_.put(h_queue_, kMaxGroups * sizeof(int));
+    pinned_.put(h_queue_err_, sizeof(int));
     for (auto ev : pending_) cudaEventDestroy(ev);
     for (auto ev : spare_ev_) cudaEventDestroy(ev);
     cudaStreamDestroy(up_);
@@ -480,8 +481,8 @@ void Engine::rebuild_lists()
             g->kpt = s.shape.kpt;
             g->threads = s.shape.threads;
             g->g1 = s.g1;
-            cuda_check(cudaMallocFromPoolAsync((void **)&g->d_queue, 3 * sizeof(int), pool_, stream_), "alloc queue");
-            cuda_check(cudaMemsetAsync(g->d_queue, 0, 3 * sizeof(int), stream_), "clear queue");
+            cuda_check(cudaMallocFromPoolAsync((void **)&g->d_queue, 2 * sizeof(int), pool_, stream_), "alloc queue");
+            cuda_check(cudaMemsetAsync(g->d_queue, 0, 2 * sizeof(int), stream_), "clear queue");
         }
         for (int t = 0; t < s.ntiles; ++t) {
             TileDev td;
@@ -535,6 +536,7 @@ void Engine::step_frozen()
         la.kpt = g.kpt;
         la.has_g1 = g.g1;
         la.queue = g.d_queue;
+        la.queue_err = d_queue_err_;
         queue_unread_ = true;
         la.stream = stream_;
         std::pair<cudaEvent_t, cudaEvent_t> ev{};
@@ -604,24 +606,28 @@ void Engine::fetch_async(int id)
                "copy outputs");
     cuda_check(cudaMemcpyAsync(s.h_const, s.constpart, (size_t)s.ntiles * NSLOT * 8, cudaMemcpyDeviceToHost, stream_),
                "copy constant parts");
-    // a queued launch that gave up waiting on a tile says so for good; one copy
-    // serves every solve fetched after the same launches (a copy per solve and
-    // class filled the stream's queue of a 256-solve batch and held up its run)
-    if (queue_unread_) {
-        if (!h_queue_) {
-            h_queue_ = static_cast<int *>(pinned_.get(kMaxGroups * sizeof(int)));
-            std::memset(h_queue_, 0, kMaxGroups * sizeof(int));
-        }
-        int i = 0;
-        for (auto &kv : groups_)
-            if (kv.second->d_queue && i < kMaxGroups)
-                cuda_check(cudaMemcpyAsync(h_queue_ + i++, kv.second->d_queue + 2, sizeof(int), cudaMemcpyDeviceToHost,
-                                           stream_),
-                           "copy queue state");
-        queue_unread_ = false;
-    }
+    read_queue_error();
     cuda_check(cudaEventRecord(s.ev, stream_), "event record");
     s.fetched = true;
+}
+
+// A queued launch that gave up waiting for a tile says so for good: what the engine
+// holds is then not what it should be.  One copy serves every result read after the
+// same launches (a copy per solve of a 256-solve batch filled the stream's queue and
+// held up its run).
+void Engine::read_queue_error()
+{
+    if (!h_queue_err_) {
+        h_queue_err_ = static_cast<int *>(pinned_.get(sizeof(int)));
+        *h_queue_err_ = 0;
+    }
+    if (!queue_unread_) return;
+    cuda_check(cudaMemcpyAsync(h_queue_err_, d_queue_err_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "copy queue state");
+    queue_unread_ = false;
+}
+void Engine::check_queue_error() const
+{
+    if (*static_cast<volatile int *>(h_queue_err_)) throw CudaError("a launch gave up waiting for a tile's earlier steps");
 }
 
 bool Engine::ready(int id)
@@ -639,8 +645,7 @@ void Engine::raw_outputs(int id, std::vector<double> &jout, double cp[NSLOT])
     Solve &s = get(id);
     if (!s.fetched) fetch_async(id);
     cuda_check(cudaEventSynchronize(s.ev), "event sync");
-    for (int i = 0; h_queue_ && i < kMaxGroups; ++i)
-        if (*static_cast<volatile int *>(h_queue_ + i)) throw CudaError("a launch gave up waiting for a tile's earlier steps");
+    check_queue_error();
     for (int q = 0; q < NSLOT; ++q) cp[q] = 0.0;
     for (int t = 0; t < s.ntiles; ++t)
         for (int q = 0; q < NSLOT; ++q) cp[q] += s.h_const[(size_t)t * NSLOT + q];
@@ -665,7 +670,9 @@ int Engine::snapshots(int id, double *occ1d, double *nc, double *pi)
     }
     if (nc) cuda_check(cudaMemcpyAsync(nc, s.snap_nc, n * 8, cudaMemcpyDeviceToHost, stream_), "copy snapshots");
     if (pi) cuda_check(cudaMemcpyAsync(pi, s.snap_pi, n * 16, cudaMemcpyDeviceToHost, stream_), "copy snapshots");
+    read_queue_error();
     cuda_check(cudaStreamSynchronize(stream_), "snapshot sync");
+    check_queue_error();
     return s.nshots;
 }
 
@@ -695,8 +702,10 @@ void Engine::harmonics(int id, double w0, int hmax, double *band_power)
         in.A = A;
         in.nvw = p.nval * p.total_weight;
     }
-    harmonics_on_device(in, w0, hmax, band_power, stream_);
+    read_queue_error();
+    harmonics_on_device(in, w0, hmax, band_power, stream_);   // waits for its result
     if (A) cudaFreeAsync(A, stream_);
+    check_queue_error();
 }
 
 SolveOutputs Engine::outputs(int id, const std::vector<double> *laser)

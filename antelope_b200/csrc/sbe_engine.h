@@ -143,6 +143,12 @@ public:
     cudaStream_t stream() const { return stream_; }
     size_t bytes_in_use() const { return bytes_in_use_; }
     // Number of propagate launches issued by the last step() (telemetry).
+    // the device word that a launch sets when its wait for a tile runs out
+    int *queue_error()
+    {
+        queue_unread_ = true;
+        return d_queue_err_;
+    }
     int last_launches() const { return last_launches_; }
     // CUDA-event timing of every propagate / reduce launch (telemetry for the
     // roofline; off by default, not usable under graph capture).
@@ -179,8 +185,10 @@ private:
     size_t bytes_in_use_ = 0;
     std::map<int, std::unique_ptr<Solve>> live_;
     std::mutex laser_mu_;   // the solves' laser columns
-    int *h_queue_ = nullptr;       // the tile queues' error marks (pinned)
-    bool queue_unread_ = false;    // launches since they were copied
+    void read_queue_error();
+    void check_queue_error() const;
+    int *d_queue_err_ = nullptr, *h_queue_err_ = nullptr;   // set by a queued launch whose wait ran out; its pinned copy
+    bool queue_unread_ = false;                             // launches since it was copied
     std::vector<int> free_slots_;
     SolveDev *d_solves_ = nullptr;
     std::vector<SolveDev> h_solves_;   // host mirror of the descriptors

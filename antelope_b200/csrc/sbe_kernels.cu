@@ -36,6 +36,7 @@
 
 #include "sbe_dev.h"
 #include "sbe_kernels.h"
+#include "sbe_queue.cuh"
 
 namespace sbe {
 
@@ -179,50 +180,6 @@ struct TileReducer {
         half ^= 1;
     }
 };
-
-// -------------------------------------------------------------- tile queue
-// The CTA's next item, or -1 (see TileQueue).  The propagate kernels have an
-// instance with the queue (QU) and one without: the loop around the tile costs
-// registers (14 % of a small length-gauge solve, which needs no queue).
-__device__ __forceinline__ int next_item(const TileQueue &q)
-{
-    __shared__ int item;
-    __syncthreads();   // the item before is finished with shared memory
-    if (threadIdx.x == 0) {
-        item = atomicAdd(q.ctr, 1);
-        if (item >= q.nitems && atomicAdd(q.ctr + 1, 1) == (int)gridDim.x - 1) {
-            q.ctr[1] = 0;   // every CTA has taken its last item
-            __threadfence();
-            q.ctr[0] = 0;
-        }
-    }
-    __syncthreads();
-    return item < q.nitems ? item : -1;
-}
-// Wait until the tile's state at step s0 is in memory (bounded; false: gave up)
-__device__ __forceinline__ bool tile_ready(const TileQueue &q, const int *prog, int s0, bool first)
-{
-    __shared__ int ok;
-    if (first) return true;
-    if (threadIdx.x == 0) {
-        int v = 0, n = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(prog) : "memory");
-        } while (v < s0 && ++n < (1 << 25) && *(volatile int *)(q.ctr + 2) == 0);
-        if (v < s0) q.ctr[2] = 1;
-        ok = v >= s0;
-    }
-    __syncthreads();
-    return ok;
-}
-__device__ __forceinline__ void tile_done(const TileQueue &q, int *prog, int s1)
-{
-    __syncthreads();   // the CTA's state stores
-    if (threadIdx.x == 0) {
-        __threadfence();
-        asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(prog), "r"(s1) : "memory");
-    }
-}
 
 // ------------------------------------------------------ velocity gauge
 // The state is rho - rho0 in the band basis: (da, db, z) = (drho_00,
@@ -1657,7 +1614,7 @@ static cudaError_t launch_prop(const LaunchArgs &la, PropKernel plain, PropKerne
             if (k && (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_bytes)) != cudaSuccess) return e;
         ps.raised[dev].store(1, std::memory_order_release);
     }
-    TileQueue q{nullptr, la.ntiles, la.S, la.ntiles};
+    TileQueue q{nullptr, nullptr, la.ntiles, la.S, la.ntiles};
     std::atomic<int> &n = ps.slots[la.threads / 32];
     if (queued && la.queue && la.S > 64 && n.load(std::memory_order_relaxed) == 0) {
         int sms = 0, per = 0;
@@ -1668,7 +1625,7 @@ static cudaError_t launch_prop(const LaunchArgs &la, PropKernel plain, PropKerne
     const int held = n.load(std::memory_order_relaxed), chunk = std::max(64, (la.S + 7) / 8);
     const long long items = (long long)la.ntiles * ((la.S + chunk - 1) / chunk);
     if (queued && la.queue && la.S > 64 && la.ntiles > held && items < 0x40000000ll) {
-        q = TileQueue{la.queue, la.ntiles, chunk, (int)items};
+        q = TileQueue{la.queue, la.queue_err, la.ntiles, chunk, (int)items};
         queued<<<held, la.threads, bytes, la.stream>>>(la.tiles, la.solves, la.tick, la.S, q);
     } else {
         plain<<<la.ntiles, la.threads, bytes, la.stream>>>(la.tiles, la.solves, la.tick, la.S, q);

@@ -15,7 +15,8 @@ struct LaunchArgs {
     int tick, S;             // launch index and steps per launch
     int variant, precision, rk, kpt;
     bool has_g1;             // T1 dephasing active
-    int *queue;              // 3 zeroed ints: the launch may queue its tiles (TileQueue), or null
+    int *queue, *queue_err;  // 2 zeroed ints of the launch class and the engine's error word: the launch
+                             // may queue its tiles (TileQueue); or null
     cudaStream_t stream;
 };
 
