@@ -138,7 +138,9 @@ struct Engine::Solve {
     double *snap_nc = nullptr, *snap_pi = nullptr;  // density snapshots (or null)
     int nshots = 0, k_begin = 0;
     double *h_jout = nullptr, *h_const = nullptr;  // pinned
-    std::vector<double> laser;                     // output columns (prepare_outputs), or empty
+    // output columns evaluated ahead (prepare_outputs); given away with the first outputs
+    enum { NONE, BUSY, THERE, GONE } columns = NONE;
+    std::vector<double> laser;
     cudaEvent_t ev = nullptr;
     bool fetched = false;
     size_t bytes = 0;
@@ -714,10 +716,16 @@ SolveOutputs Engine::outputs(int id, const std::vector<double> *laser)
     double cp[NSLOT];
     raw_outputs(id, j, cp);
     SolveOutputs o;
-    const Solve &s = get(id);
+    Solve &s = get(id);
+    std::vector<double> own;
     if (!laser) {
-        std::lock_guard<std::mutex> lk(laser_mu_);   // once there, a solve's columns stay
-        if (!s.laser.empty()) laser = &s.laser;
+        std::lock_guard<std::mutex> lk(laser_mu_);
+        if (s.columns == Solve::THERE) {
+            own = std::move(s.laser);
+            laser_bytes_ -= own.size() * 8;
+            laser = &own;
+        }
+        s.columns = Solve::GONE;
     }
     assemble_outputs(s.prob, j, cp, o, laser);
     return o;
@@ -727,13 +735,24 @@ void Engine::prepare_outputs(int id)
 {
     const Solve &want = get(id);
     if (!want.fetched) return;
-    size_t bytes = 0;
     auto prepare = [&](Solve &s) {
-        bytes += (size_t)s.Nt * 56;
-        if (bytes > ((size_t)128 << 20) || cudaEventQuery(want.ev) != cudaErrorNotReady) return false;
+        if (cudaEventQuery(want.ev) != cudaErrorNotReady) return false;
         cudaGetLastError();   // "not ready" stays behind as the thread's last error
+        const size_t bytes = (size_t)s.Nt * 56;
+        {
+            std::lock_guard<std::mutex> lk(laser_mu_);
+            if (s.columns != Solve::NONE || laser_bytes_ + bytes > kLaserBytes) return true;
+            s.columns = Solve::BUSY;
+            laser_bytes_ += bytes;
+        }
+        std::vector<double> rows = laser_rows(s.prob);   // other threads evaluate other solves' meanwhile
         std::lock_guard<std::mutex> lk(laser_mu_);
-        if (s.laser.empty()) s.laser = laser_rows(s.prob);
+        if (s.columns == Solve::BUSY) {
+            s.laser = std::move(rows);
+            s.columns = Solve::THERE;
+        } else {
+            laser_bytes_ -= bytes;   // its outputs did not wait
+        }
         return true;
     };
     if (!prepare(get(id))) return;

@@ -122,7 +122,7 @@ public:
     // Evaluate laser columns of the resident solves' outputs -- `id`'s, then
     // others', up to 128 MB of them -- while `id`'s results are still to come.
     // (Done at the run's end instead, they held up callers that leave the GPU
-    // to itself.)
+    // to itself.)  Threads share the work; outputs() takes a solve's columns away.
     void prepare_outputs(int id);
     // The raw per-step sums [Nt][NSLOT] and the summed constant parts of a
     // fetched solve (waits for the copy); assemble_outputs() turns them into
@@ -184,7 +184,9 @@ private:
     std::pair<cudaEvent_t, cudaEvent_t> new_pair();
     size_t bytes_in_use_ = 0;
     std::map<int, std::unique_ptr<Solve>> live_;
-    std::mutex laser_mu_;   // the solves' laser columns
+    std::mutex laser_mu_;   // the solves' laser columns, and how many bytes of them there are
+    static constexpr size_t kLaserBytes = (size_t)128 << 20;
+    size_t laser_bytes_ = 0;
     void read_queue_error();
     void check_queue_error() const;
     int *d_queue_err_ = nullptr, *h_queue_err_ = nullptr;   // set by a queued launch whose wait ran out; its pinned copy
