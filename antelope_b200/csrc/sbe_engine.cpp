@@ -195,8 +195,6 @@ Engine::Engine(int device, cudaStream_t stream, int steps_per_launch, int capaci
     h_solves_.resize(capacity_);
     cuda_check(cudaMallocFromPoolAsync((void **)&d_ids_, sizeof(int) * capacity_, pool_, stream_), "alloc ids");
     h_ids_.assign(capacity_, 0);
-    cuda_check(cudaMallocFromPoolAsync((void **)&d_queue_err_, sizeof(int), pool_, stream_), "alloc queue state");
-    cuda_check(cudaMemsetAsync(d_queue_err_, 0, sizeof(int), stream_), "clear queue state");
     for (int i = capacity_ - 1; i >= 0; --i) free_slots_.push_back(i);
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device_) == cudaSuccess) {
@@ -228,11 +226,11 @@ Engine::~Engine()
     }
     for (auto &kv : groups_) {
         cudaFreeAsync(kv.second->d_tiles, stream_);
-        cudaFreeAsync(kv.second->d_queue, stream_);
+        if (kv.second->d_queue != d_queue_err_ + 1) cudaFreeAsync(kv.second->d_queue, stream_);
     }
+    if (d_queue_err_) cudaFreeAsync(d_queue_err_, stream_);
     cudaFreeAsync(d_solves_, stream_);
     cudaFreeAsync(d_ids_, stream_);
-    cudaFreeAsync(d_queue_err_, stream_);
     for (auto &e : prop_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     for (auto &e : red_ev_) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     cudaStreamSynchronize(stream_);
@@ -483,8 +481,13 @@ void Engine::rebuild_lists()
             g->kpt = s.shape.kpt;
             g->threads = s.shape.threads;
             g->g1 = s.g1;
-            cuda_check(cudaMallocFromPoolAsync((void **)&g->d_queue, 2 * sizeof(int), pool_, stream_), "alloc queue");
-            cuda_check(cudaMemsetAsync(g->d_queue, 0, 2 * sizeof(int), stream_), "clear queue");
+            // the first class's counters follow the engine's error word
+            const int err = d_queue_err_ ? 0 : 1;
+            int *q = nullptr;
+            cuda_check(cudaMallocFromPoolAsync((void **)&q, (2 + err) * sizeof(int), pool_, stream_), "alloc queue");
+            cuda_check(cudaMemsetAsync(q, 0, (2 + err) * sizeof(int), stream_), "clear queue");
+            if (err) d_queue_err_ = q;
+            g->d_queue = q + err;
         }
         for (int t = 0; t < s.ntiles; ++t) {
             TileDev td;

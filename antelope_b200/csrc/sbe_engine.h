@@ -143,7 +143,7 @@ public:
     cudaStream_t stream() const { return stream_; }
     size_t bytes_in_use() const { return bytes_in_use_; }
     // Number of propagate launches issued by the last step() (telemetry).
-    // the device word that a launch sets when its wait for a tile runs out
+    // the device word that a launch sets when its wait for a tile runs out (after the first step)
     int *queue_error()
     {
         queue_unread_ = true;

@@ -757,8 +757,8 @@ __device__ __forceinline__ bool attempt(const WanDev &P, int unit)
     if (P.rk == 45) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) emax = fmax(emax, __shfl_xor_sync(ALL, emax, o));
-        // non-negative doubles order as their bits; a NaN's are above all
-        if (lane == 0) atomicMax(P.gr_err, (unsigned long long)__double_as_longlong(fabs(emax)));
+        // non-negative doubles order as their bits (fmax has dropped a NaN, as in wan_attempt)
+        if (lane == 0) atomicMax(P.gr_err, (unsigned long long)__double_as_longlong(emax));
     }
     return true;
 }
