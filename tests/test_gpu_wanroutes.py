@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import antelope_b200 as ab
-from antelope_b200 import wannier
+from antelope_b200 import api, wannier
 from cases import material, variant
 from oracle import pyoracle
 
@@ -95,6 +95,20 @@ def test_a_finished_request_is_noticed():
         launches = srv.stats()["launches"]
         srv.close()
         assert launches <= 20 * 64, launches
+
+
+def test_row_tables_above_their_limit():
+    """A grid of very many short rows runs on the tracked kernel; its slices, whose
+    tables fit, on the projections.  Bar: 1e-10 of max_t |J| (FP64 parity)."""
+    n = (50000, 2)   # 24 kB of tables a row: 1.2 GB
+    p = ab.Problem.from_dict(_table(6, n, steps=6.5))
+    total = 0.0
+    for a in range(0, 100000, 25000):
+        s = api.Solver(p, k_slice=(a, a + 25000), precision="fp64")
+        s.run()
+        total = total + s.sums()
+        s.close()
+    _close(api.assemble(p, total), ab.solve(p, precision="fp64"), 1e-10)
 
 
 @pytest.mark.parametrize("shots", [1, 400])
