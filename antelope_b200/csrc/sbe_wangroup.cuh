@@ -30,8 +30,9 @@
 // of H0 (eps_n D_nn - D_nn eps_n), which the reference evaluates to rounding.
 // Used for the tables of the SyntheticWannier group (current operator
 // -dH/dk + i[D, H], BaseMaterial.h:62-68) at N = 4 and 6, in the mixed method
-// and, in the plain one, on grids where bands meet and for row tables above 1 GB
-// (otherwise wan_attempt_p: 85 us against 402 us for an attempt of 100 x 100
+// and, in the plain one, on grids where bands meet or crowd and where there is no
+// room for row tables (1 GB at most)
+// (otherwise wan_attempt_p: 88 us against 402 us for an attempt of 100 x 100
 // points at N = 6); other models and band counts run on wan_attempt.
 
 // Tuning: resident blocks per SM the registers are sized for.  (Tables

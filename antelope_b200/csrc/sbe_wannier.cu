@@ -33,9 +33,10 @@
 // method: fixed steps of the velocity gauge (both methods) and, in the length
 // gauge, of the analytic materials (sbe_wanstep.cu), and the length gauge of
 // explicit tables at N = 3 ... 6 (sbe_wanproj.cu).  Here remain the Cash-Karp
-// steps of the velocity gauge, the mixed method of the length gauge, the
-// continuum model, and grids with a point where two bands meet (in the length
-// gauge the outcome there depends on the eigenbasis taken).
+// steps of the velocity gauge, and in the length gauge the mixed method, the
+// continuum model, grids with a point where two bands meet (the outcome there
+// depends on the eigenbasis taken), small grids where three or more crowd
+// (wan_crowded_slow), and solves for whose other tables there is no memory.
 #include <cuda_runtime.h>
 
 #include <type_traits>

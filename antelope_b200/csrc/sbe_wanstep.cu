@@ -750,7 +750,7 @@ static int lw_bytes(int N, int rk, int npair)
 // SM.  Latency-bound (a step is a serial chain of stages) until the grid gives
 // every scheduler a few warps, FP64-pipe bound beyond.  Measured (whole solves
 // of 367 steps with their set-up, us a step, 168 to 14 640 k-points alike): N =
-// 2, 3, 4 RK4 2.5, 5.7, 9.4, RK5 4.1, 9.2, 15; one attempt and one control
+// 2, 3, 4 RK4 2.5, 5.7, 9.5, RK5 4.1, 9.2, 15; one attempt and one control
 // launch a step take 78 (N = 3, RK5, 2 400 k-points).
 //
 // lw_advance: false if bands crowded at a stage of a k-point; nothing but partial
