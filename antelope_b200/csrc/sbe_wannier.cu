@@ -570,6 +570,7 @@ __global__ void __launch_bounds__(32 * WAN_WARPS) wan_init(WanDev P)
             for (int n = 0; n < N; ++n) ev[n] = w.B[n * N + n].x;
             if (N == 4 ? bands_crowd<4>(ev) : N == 5 ? bands_crowd<5>(ev) : N == 6 ? bands_crowd<6>(ev) : false)
                 atomicAdd(P.band_gap + 2, 1ull);
+            if (N > 2) atomicAdd(P.band_gap + 3, (unsigned long long)fmin(wid / gap, 1e9));
         }
     }
     // occupations of the eigenstates: the Nval lowest filled, or Fermi-Dirac (SBEs.h:319-340)

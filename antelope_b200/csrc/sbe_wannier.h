@@ -109,11 +109,11 @@ struct WanDev {
     const int *gmate;
     int mixed;              // the mixed method (FP32 Fourier sums)
     // length gauge: bits of the smallest gap between two bands and of the
-    // largest spread of the bands over the grid, and the number of its points
-    // where bands crowd (wan_init), or null
+    // largest spread of the bands over the grid, the number of its points where
+    // bands crowd, and the sum over them of the spread over the gap (wan_init), or null
     unsigned long long *band_gap;
-    int degenerate;   // neither wan_steps nor wan_proj applies: bands meet on the grid, or crowd
-                      // and it is one that wan_crowded_slow names
+    int degenerate;   // neither wan_steps nor wan_proj applies: bands meet on the grid or are close
+                      // over much of it, or crowd and it is one that wan_crowded_slow names
     // projection attempt kernel (wan_proj): the grid's rows along its fast axis
     // (axis gr_fast, gr_nf points; the solve's rows start at gr_row0), the
     // groups of vectors R with equal b.R = +-gr_a (b the fast axis; gr_n of

@@ -39,7 +39,7 @@ def _frame(nband, nval):
 
 def _levels(nband, m):
     """Energies of the bands outside a cluster of m at 0: below, then above."""
-    return np.array({1: [0.3], 2: [-0.3, 0.3], 3: [-0.3, 0.25, 0.5]}[nband - m])
+    return np.array({1: [0.3], 2: [-0.3, 0.3], 3: [-0.3, 0.25, 0.5], 4: [-0.3, 0.2, 0.4, 0.6]}[nband - m])
 
 
 def _cluster(nband, m, width):
@@ -91,6 +91,13 @@ def _check(case):
 @pytest.mark.parametrize("width", [1e-1, 1e-2, 1e-3, 1e-4])
 def test_clusters_over_the_zone(nband, m, width):
     _check(_case(_cluster(nband, m, width), (4, 4), "rk4"))
+
+
+@pytest.mark.parametrize("nband", [3, 4, 5, 6])
+@pytest.mark.parametrize("width", [1e-2, 1e-4, 1e-6, 2e-7])
+def test_close_pairs_over_the_zone(nband, width):
+    """Two bands with gaps down to 2e-7 of the spectrum's width."""
+    _check(_case(_cluster(nband, 2, width), (4, 4), "rk4"))
 
 
 def _turn(c):
